@@ -265,6 +265,7 @@ extern "C" int gnr_destroy(GnrModel* m) {
   free_dev(m->alpha_bits);
   free_dev(m->alpha_coarse);
   free_dev(m->alpha_full);
+  free_dev(m->alpha_any8);
   free_dev(m->hull_near_term);
   free_dev(m->hull_u);
   free_dev(m->mlp.basis_blocked);
@@ -433,6 +434,24 @@ __global__ void full_bits_kernel(const uint32_t* __restrict__ bits, int D, int H
   if ((threadIdx.x & 31) == 0 && c < (((long long)cD * cH * cW + 31) / 32) * 32) full[c >> 5] = word;
 }
 
+// Per cell: is any of the eight cells a trilinear test with this lower corner reads set (cells outside the volume are not)?
+__global__ void any8_bits_kernel(const uint32_t* __restrict__ bits, int D, int H, int W, uint32_t* __restrict__ any8) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = (long long)D * H * W;
+  bool any = false;
+  if (c < n) {
+    const int x = (int)(c % W), y = (int)((c / W) % H), z = (int)(c / ((long long)W * H));
+    for (int e = 0; e < 8 && !any; ++e) {
+      const int xx = x + (e & 1), yy = y + ((e >> 1) & 1), zz = z + (e >> 2);
+      if (xx < W && yy < H && zz < D) {
+        const long long bit = ((long long)zz * H + yy) * W + xx;
+        any = (bits[bit >> 5] >> (bit & 31)) & 1u;
+      }
+    }
+  }
+  const uint32_t word = __ballot_sync(0xffffffffu, any);  // 32 consecutive cells = one word
+  if ((threadIdx.x & 31) == 0 && c < ((n + 31) / 32) * 32) any8[c >> 5] = word;
+}
+
 extern "C" int gnr_upload_alpha_mask(GnrModel* m, const uint8_t* vol, int D, int H, int W, const float* aabb_h,
                                      const float* inv_size_h, void* stream) {
   if (!m) {
@@ -443,7 +462,8 @@ extern "C" int gnr_upload_alpha_mask(GnrModel* m, const uint8_t* vol, int D, int
   free_dev(m->alpha_bits);
   free_dev(m->alpha_coarse);
   free_dev(m->alpha_full);
-  m->alpha_bits = m->alpha_coarse = m->alpha_full = nullptr;
+  free_dev(m->alpha_any8);
+  m->alpha_bits = m->alpha_coarse = m->alpha_full = m->alpha_any8 = nullptr;
   m->aD = m->aH = m->aW = 0;
   if (!vol) return 0;
   if (D < 1 || H < 1 || W < 1 || !aabb_h || !inv_size_h || (long long)D * H * W > 0xffffffffLL) {
@@ -464,6 +484,9 @@ extern "C" int gnr_upload_alpha_mask(GnrModel* m, const uint8_t* vol, int D, int
     GNR_CUDA_OK(cudaMalloc(&m->alpha_full, (size_t)n_cwords * sizeof(uint32_t)));
     full_bits_kernel<<<(unsigned)((n_cwords * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->alpha_bits, D, H, W, cD, cH, cW,
                                                                                           m->alpha_full);
+    GNR_CUDA_OK(cudaGetLastError());
+    GNR_CUDA_OK(cudaMalloc(&m->alpha_any8, (size_t)n_words * sizeof(uint32_t)));
+    any8_bits_kernel<<<(unsigned)((n_words * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->alpha_bits, D, H, W, m->alpha_any8);
     GNR_CUDA_OK(cudaGetLastError());
   }
   m->aD = D;
@@ -690,10 +713,14 @@ GnrSampleParams gnr_sample_params(const GnrModel* m, int S) {
   p.aD = m->aD;
   p.aH = m->aH;
   p.aW = m->aW;
-  p.has_mask = m->alpha_bits != nullptr;
+  p.has_mask = m->alpha_any8 != nullptr;  // (the last of the four bit volumes to be made)
   p.a_bits = m->alpha_bits;
   p.a_coarse = m->alpha_coarse;
   p.a_full = m->alpha_full;
+  p.a_any8 = m->alpha_any8;
+  p.a_half[0] = 0.5f * (float)(m->aW - 1);
+  p.a_half[1] = 0.5f * (float)(m->aH - 1);
+  p.a_half[2] = 0.5f * (float)(m->aD - 1);
   p.cD = (m->aD + 3) / 4;
   p.cH = (m->aH + 3) / 4;
   p.cW = (m->aW + 3) / 4;

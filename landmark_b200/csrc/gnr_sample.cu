@@ -59,25 +59,20 @@ __global__ void raygen_dev_kernel(const float* __restrict__ pose_dev, const floa
 }
 
 // ---------------------------------------------------------------------------------------------
-// sampling: one thread per ray, samples in order, 32 validity bits per register word
+// sampling: a warp per group of rays, 32 samples at a time
 // ---------------------------------------------------------------------------------------------
+// Continuous mask index of a coordinate: ((p - aabb0) * invgridSize - 1 + 1) / 2 * (size - 1), each operation rounded
+// as torch rounds it.  The halving is exact, so it is folded into the last factor (`half` = (size - 1) / 2, exact too).
+__device__ __forceinline__ float mask_index(float px, float lo, float inv, float half) {
+  return __fmul_rn(__fadd_rn(gnr_normalize(px, lo, inv), 1.0f), half);
+}
+
 // AlphaGridMask.sample_alpha (app/models/alpha_mask.py:35-59): trilinear interpolation of the 0/1
 // volume with zero padding, then `> threshold`.  The sum runs over the corners in grid_sample's
-// order with individually rounded operations.  Two exact shortcuts come first: a clear bit of the
-// coarse grid proves that all eight corners are empty (threshold >= 0 then fails), and with a
-// threshold of exactly zero the sum of non-negative weights is positive as soon as one occupied
-// corner has a positive weight, so the loop can stop there.
-// `skip` (optional): when the coarse grids decide the sample (empty block: invalid; full block and
-// threshold 0: valid), the number of FOLLOWING samples that provably lie in the same block and so
-// get the same answer, given the index-space step `di` per sample
-// (dense sampler: positions advance by d * stepSize).  The bound keeps 1/100 of a mask cell away
-// from the block's faces, far more than the rounding of the index arithmetic (a few 1e-4).
-__device__ __forceinline__ bool occupancy_test(const GnrSampleParams& p, float px, float py, float pz,
-                                               const float* di = nullptr, int* skip = nullptr) {
-  // q = (p - aabb0) * invgridSize - 1 ; index = ((q + 1) / 2) * (size - 1)
-  const float ix = __fmul_rn(__fmul_rn(__fadd_rn(gnr_normalize(px, p.a_lo[0], p.a_inv[0]), 1.0f), 0.5f), (float)(p.aW - 1));
-  const float iy = __fmul_rn(__fmul_rn(__fadd_rn(gnr_normalize(py, p.a_lo[1], p.a_inv[1]), 1.0f), 0.5f), (float)(p.aH - 1));
-  const float iz = __fmul_rn(__fmul_rn(__fadd_rn(gnr_normalize(pz, p.a_lo[2], p.a_inv[2]), 1.0f), 0.5f), (float)(p.aD - 1));
+// order with individually rounded operations.  With a threshold of exactly zero the sum of
+// non-negative weights is positive as soon as one occupied corner has a positive weight, so the
+// loop can stop there.
+__device__ __forceinline__ bool occupancy_corners(const GnrSampleParams& p, float ix, float iy, float iz) {
   // corners outside the volume contribute zero (padding_mode="zeros"); indices that do not
   // fit an int (only possible for samples far outside the mask box) are outside too.
   const bool okx = (ix >= -1.0f) && (ix < (float)p.aW), oky = (iy >= -1.0f) && (iy < (float)p.aH),
@@ -85,29 +80,6 @@ __device__ __forceinline__ bool occupancy_test(const GnrSampleParams& p, float p
   if (!(okx && oky && okz)) return 0.0f > p.a_thres;
   const float fx0 = floorf(ix), fy0 = floorf(iy), fz0 = floorf(iz);
   const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
-  if (p.a_coarse != nullptr && p.a_thres >= 0.0f && x0 >= 0 && y0 >= 0 && z0 >= 0) {
-    const uint32_t cb = (uint32_t)(((z0 >> 2) * p.cH + (y0 >> 2)) * p.cW + (x0 >> 2));
-    const uint32_t cw = cb >> 5, cs = cb & 31;
-    const bool empty = !((__ldg(p.a_coarse + cw) >> cs) & 1u);
-    // a full block decides the test when the threshold is exactly zero: the lower corner is occupied
-    // and its weight (x0 + 1 - ix)(y0 + 1 - iy)(z0 + 1 - iz) is a product of three positive floats
-    const bool full = !empty && p.a_thres == 0.0f && ((__ldg(p.a_full + cw) >> cs) & 1u);
-    if (empty || full) {
-      if (skip) {
-        const float idx[3] = {ix, iy, iz};
-        const int lo[3] = {x0 & ~3, y0 & ~3, z0 & ~3};
-        float n = 64.0f;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const float room = di[a] > 0.0f ? ((float)(lo[a] + 4) - idx[a] - 0.01f) : (idx[a] - (float)lo[a] - 0.01f);
-          const float speed = fabsf(di[a]);
-          if (speed > 0.0f) n = fminf(n, room / speed);
-        }
-        *skip = n > 0.0f ? (int)n : 0;
-      }
-      return full;
-    }
-  }
   const float fx1 = __fadd_rn(fx0, 1.0f), fy1 = __fadd_rn(fy0, 1.0f), fz1 = __fadd_rn(fz0, 1.0f);
   const float wx[2] = {__fsub_rn(fx1, ix), __fsub_rn(ix, fx0)};
   const float wy[2] = {__fsub_rn(fy1, iy), __fsub_rn(iy, fy0)};
@@ -138,123 +110,222 @@ __device__ __forceinline__ bool occupancy_test(const GnrSampleParams& p, float p
   return out > p.a_thres;
 }
 
-constexpr int kSampleBlock = 128;
+// floor of 0 <= x < 2^22 as a float and an int with two full-rate additions: rounding towards minus infinity at
+// 2^23 leaves the integer part in the low mantissa bits.
+__device__ __forceinline__ float floor_small(float x, int& i) {
+  const float m = __fadd_rd(x, 8388608.0f);
+  i = __float_as_int(m) & 0x7fffff;
+  return __fsub_rn(m, 8388608.0f);
+}
 
-__global__ void __launch_bounds__(kSampleBlock)
-sample_mask_kernel(GnrSampleParams p, const float* __restrict__ rays, int64_t n_rays, float* __restrict__ t_min_out,
-                   uint32_t* __restrict__ words_out, int32_t* __restrict__ counts_out) {
-  const int64_t ray_raw = (int64_t)blockIdx.x * kSampleBlock + threadIdx.x;
-  const bool live = ray_raw < n_rays;  // lanes past the end keep their warp company (warp votes below) and write nothing
-  const int64_t ray = live ? ray_raw : n_rays - 1;
-  const float* r = rays + ray * 6;
-  const float o[3] = {__ldg(r), __ldg(r + 1), __ldg(r + 2)};
-  const float d[3] = {__ldg(r + 3), __ldg(r + 4), __ldg(r + 5)};
-  // slab entry: max over axes of min(rate_a, rate_b), clamped to [near, far]
-  float t_min = -INFINITY;
+__device__ __forceinline__ bool occupancy_test(const GnrSampleParams& p, float px, float py, float pz) {
+  const float ix = mask_index(px, p.a_lo[0], p.a_inv[0], p.a_half[0]);
+  const float iy = mask_index(py, p.a_lo[1], p.a_inv[1], p.a_half[1]);
+  const float iz = mask_index(pz, p.a_lo[2], p.a_inv[2], p.a_half[2]);
+  if (p.a_thres == 0.0f && fminf(fminf(ix, iy), iz) > 0.0f && ix < (float)(p.aW - 1) && iy < (float)(p.aH - 1) && iz < (float)(p.aD - 1)) {
+    int x0, y0, z0;
+    const float fx = floor_small(ix, x0), fy = floor_small(iy, y0), fz = floor_small(iz, z0);
+    // strictly inside a cell all eight corner weights are positive (differences of floats that are not equal; their
+    // product is far above the smallest float), so the sum is positive exactly if one of the corners is occupied
+    if (fx != ix && fy != iy && fz != iz) {
+      const uint32_t bit = ((uint32_t)z0 * (uint32_t)p.aH + (uint32_t)y0) * (uint32_t)p.aW + (uint32_t)x0;
+      return (__ldg(p.a_any8 + (bit >> 5)) >> (bit & 31)) & 1u;
+    }
+  }
+  return occupancy_corners(p, ix, iy, iz);
+}
+
+struct RaySetup {  // what the sample tests need of a ray, in shared memory
+  float o[3], t_min, d[3], pad;
+};
+
+// What the two end samples of a run prove about all samples k0 .. k1 between them (dense sampler): 0 = none is valid,
+// 1 = all are, 2 = still open.  fl(t_min + fl(step k)), the point, and the mask index are each monotone in their
+// argument (every operation is a correctly rounded monotone function), so along each axis every sample between the two
+// lies between them, without any tolerance: if both are inside the box all are, if both are outside on the same side
+// none is, and the mask cells of all samples lie in the range spanned by the cells of the two.
+// BLOCKS: the occupancy of that range is looked up in blocks of 4x4x4 cells, else cell by cell.
+template <bool BLOCKS>
+__device__ __forceinline__ int run_by_ends(const GnrSampleParams& p, const RaySetup& r, int k0, int k1) {
+  const float t0 = gnr_sample_t(p, r.t_min, k0), t1 = gnr_sample_t(p, r.t_min, k1);
+  float q0[3], q1[3];
+  bool in = true;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const float vec = (d[a] == 0.0f) ? 1e-6f : d[a];
-    const float ra = __fdiv_rn(__fsub_rn(p.hi[a], o[a]), vec);
-    const float rb = __fdiv_rn(__fsub_rn(p.lo[a], o[a]), vec);
-    t_min = fmaxf(t_min, fminf(ra, rb));
+    q0[a] = gnr_point(r.o[a], r.d[a], t0);
+    q1[a] = gnr_point(r.o[a], r.d[a], t1);
+    const float lo = fminf(q0[a], q1[a]), hi = fmaxf(q0[a], q1[a]);
+    if (hi < p.lo[a] || lo > p.hi[a]) return 0;
+    in = in && !(p.lo[a] > lo) && !(hi > p.hi[a]);
   }
-  t_min = fminf(fmaxf(t_min, p.near_t), p.far_t);
-  if (p.mode == 1) {
-    // hull sampler: the per-ray parameter is `far`, the hit with the ground plane z = aabb_min_z
-    // (far = -(o_z - z0) / d_z, replaced by near_far[1] for rays that do not point down)
-    const float far = -__fdiv_rn(__fsub_rn(o[2], p.lo[2]), d[2]);
-    t_min = (d[2] >= 0.0f) ? p.far_t : far;
+  if (!in) return 2;
+  if (!p.has_mask) return 1;
+  if (!(p.a_thres >= 0.0f)) return 2;
+  int b0[3], b1[3];
+  const int size[3] = {p.aW, p.aH, p.aD};
+  bool inside_cell = true;  // all samples strictly inside one cell
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float i0 = mask_index(q0[a], p.a_lo[a], p.a_inv[a], p.a_half[a]), i1 = mask_index(q1[a], p.a_lo[a], p.a_inv[a], p.a_half[a]);
+    const float lo = fminf(i0, i1), hi = fmaxf(i0, i1);
+    if (!(lo >= 0.0f && hi < (float)size[a])) return 2;
+    b0[a] = (int)lo;
+    b1[a] = (int)hi;
+    if (BLOCKS) {
+      b0[a] >>= 2;
+      b1[a] >>= 2;
+    } else {
+      inside_cell = inside_cell && b0[a] == b1[a] && (float)b0[a] != lo;
+    }
+    if (b1[a] - b0[a] > 1) return 2;
   }
-  if (live) t_min_out[ray] = t_min;
+  const uint32_t nx = (uint32_t)(BLOCKS ? p.cW : p.aW), ny = (uint32_t)(BLOCKS ? p.cH : p.aH);
+  const uint32_t* any_bits = BLOCKS ? p.a_coarse : p.a_any8;
+  const uint32_t* all_bits = BLOCKS ? p.a_full : p.a_bits;
+  bool any = false, all = p.a_thres == 0.0f;
+  for (int z = b0[2]; z <= b1[2]; ++z)
+    for (int y = b0[1]; y <= b1[1]; ++y)
+      for (int x = b0[0]; x <= b1[0]; ++x) {
+        const uint32_t at = ((uint32_t)z * ny + (uint32_t)y) * nx + (uint32_t)x;
+        any = any || ((__ldg(any_bits + (at >> 5)) >> (at & 31)) & 1u);
+        all = all && ((__ldg(all_bits + (at >> 5)) >> (at & 31)) & 1u);
+      }
+  // no occupied corner in reach: the sum is zero.  Threshold zero: with its lower corner occupied a sample has a positive
+  // weight, (x0 + 1 - ix)(y0 + 1 - iy)(z0 + 1 - iz), wherever in the cell it lies; strictly inside a cell any corner will do
+  if (!any) return 0;
+  if (!BLOCKS && inside_cell && p.a_thres == 0.0f) return 1;
+  return all ? 1 : 2;
+}
 
-  int count = 0;
-  uint32_t* wrow = words_out + ray * p.words;
-  // fl(o + fl(d * fl(t_min + fl(step * k)))) is monotone in k, so once a sample has left the
-  // box through the far side of an axis every later sample is outside as well.
-  // (The hull sampler's distances are a sum of a falling and a rising term and need not be
-  // monotone to the last bit, so only the dense sampler stops at the first exit and skips.)
-  // The 32 rays of a warp walk the sample index k together.  When every ray of the warp stands in
-  // an empty coarse block (or has left the box) the warp jumps over the samples that all of them
-  // can rule out; jumping together keeps neighbouring rays, which see the same occupancy, in step.
-  const float di[3] = {d[0] * p.step * p.a_inv[0] * 0.5f * (float)(p.aW - 1), d[1] * p.step * p.a_inv[1] * 0.5f * (float)(p.aH - 1),
-                       d[2] * p.step * p.a_inv[2] * 0.5f * (float)(p.aD - 1)};
-  const bool can_skip = p.mode == 0 && p.has_mask;
-  constexpr int kMaxSkip = 64;
-  // Samples that are skipped as VALID (full blocks) must also lie inside the box: they do while their
-  // index stays two samples short of the slab exit (the positions are monotone along the ray and the
-  // sample that started the run was tested inside).
-  int k_inside = -1;
-  if (can_skip) {
-    float t_far = INFINITY;
+__device__ __forceinline__ bool sample_valid(const GnrSampleParams& p, const RaySetup& r, int k) {
+  const float t = gnr_sample_t(p, r.t_min, k);
+  const float px = gnr_point(r.o[0], r.d[0], t), py = gnr_point(r.o[1], r.d[1], t), pz = gnr_point(r.o[2], r.d[2], t);
+  const bool lo_out = (p.lo[0] > px) | (p.lo[1] > py) | (p.lo[2] > pz);
+  const bool hi_out = (px > p.hi[0]) | (py > p.hi[1]) | (pz > p.hi[2]);
+  return !(lo_out | hi_out) && (!p.has_mask || occupancy_test(p, px, py, pz));
+}
+
+constexpr int kSampleWarps = 4;
+
+// A warp takes `per_warp` consecutive rays.  It sets them up one ray per lane, then walks their validity words, 32 words
+// (of one or several rays) at a time, in three steps: every lane tries to decide its own word from the word's two end
+// samples; the words that stay open are cut into runs of eight samples, 32 runs at a time, and decided the same way cell
+// by cell; the runs that stay open are tested sample by sample, four runs at a time.  Each step queues what it leaves
+// open in shared memory, so that the lanes of the next one are full.
+// Bound by instruction issue (77 % of the slots).  A ray's latency is a few passes instead of one dependent step per
+// sample, and most samples are never looked at: of a city frame's words 40 % stay open after the first step and 0.5 runs
+// of each after the second.  98,304 rays x 256 samples: 65 us, 51 warp instructions per word (104 us and 87 when every
+// open word was tested sample by sample); 333 rays x 128 samples: 14 us, 121 us with a thread walking each ray.
+__global__ void __launch_bounds__(kSampleWarps * 32, 8)
+sample_words_kernel(const __grid_constant__ GnrSampleParams p, const float* __restrict__ rays, int64_t n_rays, int per_warp,
+                    float* __restrict__ t_min_out, uint32_t* __restrict__ words_out, int32_t* __restrict__ counts_out) {
+  __shared__ RaySetup s_ray[kSampleWarps][32];
+  __shared__ int s_count[kSampleWarps][32];
+  __shared__ uint32_t s_bits[kSampleWarps][32];   // the 32 words of a pass
+  __shared__ uint32_t s_item[kSampleWarps][32];   // ray << 16 | word of each of them
+  __shared__ uint8_t s_open[kSampleWarps][32];    // open words: number in the pass
+  __shared__ uint8_t s_run[kSampleWarps][128];    // open runs: number in the pass << 2 | run
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t below = (1u << lane) - 1u;
+  const int64_t first = ((int64_t)blockIdx.x * kSampleWarps + warp) * per_warp;
+  if (first >= n_rays) return;
+  const int mine = (int)min((int64_t)per_warp, n_rays - first);
+  if (lane < mine) {
+    const float* r = rays + (first + lane) * 6;
+    RaySetup s;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      if (d[a] != 0.0f) t_far = fminf(t_far, fmaxf((p.hi[a] - o[a]) / d[a], (p.lo[a] - o[a]) / d[a]));
+      s.o[a] = __ldg(r + a);
+      s.d[a] = __ldg(r + 3 + a);
     }
-    const float ksafe = floorf((t_far - t_min) / p.step) - 2.0f;
-    k_inside = ksafe > 0.0f ? (int)fminf(ksafe, (float)p.S) : -1;
+    // slab entry: max over axes of min(rate_a, rate_b), clamped to [near, far]
+    float t_min = -INFINITY;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float vec = (s.d[a] == 0.0f) ? 1e-6f : s.d[a];
+      const float ra = __fdiv_rn(__fsub_rn(p.hi[a], s.o[a]), vec);
+      const float rb = __fdiv_rn(__fsub_rn(p.lo[a], s.o[a]), vec);
+      t_min = fmaxf(t_min, fminf(ra, rb));
+    }
+    t_min = fminf(fmaxf(t_min, p.near_t), p.far_t);
+    if (p.mode == 1) {
+      // hull sampler: the per-ray parameter is `far`, the hit with the ground plane z = aabb_min_z
+      // (far = -(o_z - z0) / d_z, replaced by near_far[1] for rays that do not point down)
+      const float far = -__fdiv_rn(__fsub_rn(s.o[2], p.lo[2]), s.d[2]);
+      t_min = (s.d[2] >= 0.0f) ? p.far_t : far;
+    }
+    s.t_min = t_min;
+    s.pad = 0.0f;
+    s_ray[warp][lane] = s;
+    s_count[warp][lane] = 0;
+    t_min_out[first + lane] = t_min;
   }
-  bool done = !live;
-  uint32_t bits = 0;
-  int word = 0, k = 0;
-  int ones_beg = 0, ones_end = 0;  // samples [ones_beg, ones_end) of this ray are valid without a test
-  auto with_ones = [&](uint32_t b, int wd) {
-    const int lo = max(ones_beg, wd * 32), hi = min(ones_end, wd * 32 + 32);
-    if (lo < hi) b |= (hi - lo == 32 ? 0xffffffffu : ((1u << (hi - lo)) - 1u)) << (lo - wd * 32);
-    return b;
-  };
-  while (k < p.S) {
-    const int w = k >> 5;
-    while (word < w) {  // words completed since the last sample (all of them when samples were skipped)
-      bits = with_ones(bits, word);
-      if (live) wrow[word] = bits;
-      ++word;
-      count += __popc(bits);
-      bits = 0;
-    }
-    int skip = kMaxSkip;  // a finished ray never holds the warp back
-    bool run_valid = false;
-    if (!done) {
-      skip = 0;
-      const float t = gnr_sample_t(p, t_min, k);
-      const float px = gnr_point(o[0], d[0], t), py = gnr_point(o[1], d[1], t), pz = gnr_point(o[2], d[2], t);
-      const bool lo_out = (p.lo[0] > px) | (p.lo[1] > py) | (p.lo[2] > pz);
-      const bool hi_out = (px > p.hi[0]) | (py > p.hi[1]) | (pz > p.hi[2]);
-      if (!(lo_out | hi_out)) {
-        if (!p.has_mask || occupancy_test(p, px, py, pz, di, can_skip ? &skip : nullptr)) {
-          bits |= 1u << (k & 31);
-          run_valid = true;
-          skip = max(0, min(skip, k_inside - k));  // a run of valid samples ends before the box does
-        }
-      } else if (p.mode == 0) {
-        const bool exited = ((d[0] > 0.0f) & (px > p.hi[0])) | ((d[0] < 0.0f) & (p.lo[0] > px)) |
-                            ((d[1] > 0.0f) & (py > p.hi[1])) | ((d[1] < 0.0f) & (p.lo[1] > py)) |
-                            ((d[2] > 0.0f) & (pz > p.hi[2])) | ((d[2] < 0.0f) & (p.lo[2] > pz)) |
-                            ((d[0] == 0.0f) & ((p.lo[0] > px) | (px > p.hi[0]))) |
-                            ((d[1] == 0.0f) & ((p.lo[1] > py) | (py > p.hi[1]))) |
-                            ((d[2] == 0.0f) & ((p.lo[2] > pz) | (pz > p.hi[2])));
-        if (exited) {
-          done = true;
-          skip = kMaxSkip;
+  __syncwarp();
+  const int W = p.words, items = mine * W;
+  int ray = lane / W, word = lane - ray * W;  // this lane's item: word `word` of ray `ray` of the warp
+  const int ray_step = 32 / W, word_step = 32 - ray_step * W;
+  // (the hull sampler's distances are a sum of a falling and a rising term and need not be monotone to the last bit:
+  // its samples are all tested one by one)
+  const bool dense = p.mode == 0;
+  for (int i0 = 0; i0 < items; i0 += 32) {
+    const bool has = i0 + lane < items;
+    int verdict = 0;
+    if (has) verdict = dense ? run_by_ends<true>(p, s_ray[warp][ray], 32 * word, min(32 * word + 31, p.S - 1)) : 2;
+    const uint32_t open = __ballot_sync(0xffffffffu, verdict == 2);
+    s_bits[warp][lane] = verdict != 1 ? 0u : (p.S - 32 * word >= 32 ? 0xffffffffu : (1u << (p.S - 32 * word)) - 1u);
+    s_item[warp][lane] = ((uint32_t)ray << 16) | (uint32_t)word;
+    if (verdict == 2) s_open[warp][__popc(open & below)] = (uint8_t)lane;
+    __syncwarp();
+    const int n_open = __popc(open);
+    int n_run = 0;
+    for (int j0 = 0; j0 < 4 * n_open; j0 += 32) {  // lane = run of eight samples
+      const int j = j0 + lane;
+      int v = 0, at = 0, run = j & 3;
+      if (j < 4 * n_open) {
+        at = s_open[warp][j >> 2];
+        const uint32_t it = s_item[warp][at];
+        const int k = 32 * (int)(it & 0xffffu) + 8 * run;
+        if (k < p.S) {
+          v = dense ? run_by_ends<false>(p, s_ray[warp][it >> 16], k, min(k + 7, p.S - 1)) : 2;
+          if (v == 1) atomicOr(&s_bits[warp][at], (k + 8 <= p.S ? 0xffu : (1u << (p.S - k)) - 1u) << (8 * run));
         }
       }
+      const uint32_t still = __ballot_sync(0xffffffffu, v == 2);
+      if (v == 2) s_run[warp][n_run + __popc(still & below)] = (uint8_t)(at << 2 | run);
+      n_run += __popc(still);
     }
-    if (__all_sync(0xffffffffu, done)) break;
-    const int jump = __reduce_min_sync(0xffffffffu, min(skip, kMaxSkip));
-    if (run_valid && jump > 0) {  // (jump > 0 implies this lane's own run is at least that long)
-      bits = with_ones(bits, w);  // what an earlier run left in the current word, before the range moves on
-      ones_beg = k + 1;
-      ones_end = min(k + 1 + jump, p.S);
+    __syncwarp();
+    for (int j0 = 0; j0 < n_run; j0 += 4) {  // lane = sample
+      const int j = j0 + (lane >> 3);
+      bool valid = false;
+      int at = 0, run = 0;
+      if (j < n_run) {
+        const int e = s_run[warp][j];
+        at = e >> 2;
+        run = e & 3;
+        const uint32_t it = s_item[warp][at];
+        const int k = 32 * (int)(it & 0xffffu) + 8 * run + (lane & 7);
+        valid = k < p.S && sample_valid(p, s_ray[warp][it >> 16], k);
+      }
+      const uint32_t vote = __ballot_sync(0xffffffffu, valid);
+      const uint32_t byte = (vote >> (lane & 24)) & 0xffu;
+      if ((lane & 7) == 0 && byte) atomicOr(&s_bits[warp][at], byte << (8 * run));
     }
-    k += 1 + jump;
+    __syncwarp();
+    if (has) {
+      const uint32_t bits = s_bits[warp][lane];
+      words_out[first * W + i0 + lane] = bits;
+      if (bits) atomicAdd(&s_count[warp][ray], __popc(bits));
+    }
+    ray += ray_step;
+    word += word_step;
+    if (word >= W) {
+      word -= W;
+      ++ray;
+    }
+    __syncwarp();
   }
-  while (word < p.words) {
-    bits = with_ones(bits, word);
-    if (live) wrow[word] = bits;
-    ++word;
-    count += __popc(bits);
-    bits = 0;
-  }
-  if (live) counts_out[ray] = count;
+  if (lane < mine) counts_out[first + lane] = s_count[warp][lane];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -363,13 +434,21 @@ int launch_exclusive_scan(const int32_t* counts, int32_t* offsets, int32_t* bloc
   return (int)cudaGetLastError();
 }
 
+// Rays per warp: 32 when there are enough rays to fill the GPU (the slab set-up then uses every lane), fewer below that,
+// down to one, so that a small chunk still spreads over all SMs.
+static int launch_sample_words(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, float* t_min,
+                               uint32_t* words, int32_t* counts, cudaStream_t st) {
+  const int64_t warps = (int64_t)m->sm_count * 32;
+  const int per_warp = (int)min((int64_t)32, max((int64_t)1, n / warps));
+  const int64_t per_block = (int64_t)per_warp * kSampleWarps;
+  sample_words_kernel<<<(unsigned)((n + per_block - 1) / per_block), kSampleWarps * 32, 0, st>>>(p, rays, n, per_warp, t_min, words,
+                                                                                               counts);
+  return (int)cudaGetLastError();
+}
+
 int launch_sample_mask(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws,
                        const GnrWs& L, cudaStream_t st) {
-  (void)m;
-  unsigned blocks = (unsigned)((n + kSampleBlock - 1) / kSampleBlock);
-  sample_mask_kernel<<<blocks, kSampleBlock, 0, st>>>(p, rays, n, (float*)(ws + L.t_min), (uint32_t*)(ws + L.words),
-                                                            (int32_t*)(ws + L.counts));
-  return (int)cudaGetLastError();
+  return launch_sample_words(m, p, rays, n, (float*)(ws + L.t_min), (uint32_t*)(ws + L.words), (int32_t*)(ws + L.counts), st);
 }
 
 int launch_sample_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, char* ws, const GnrWs& L,
@@ -512,8 +591,9 @@ extern "C" int gnr_sample_static(GnrModel* m, const float* rays, int64_t n_rays,
     if (e == cudaSuccess) {
       // every word of mask_words and block_sums that is read below is written first by these
       // launches, so what an earlier call left in the array is never seen
-      sample_mask_kernel<<<(unsigned)((n_rays + kSampleBlock - 1) / kSampleBlock), kSampleBlock, 0, st>>>(p, rays, n_rays, t_min,
-                                                                                                  mask_words, counts);
+      e = (cudaError_t)launch_sample_words(m, p, rays, n_rays, t_min, mask_words, counts, st);
+    }
+    if (e == cudaSuccess) {
       e = (cudaError_t)launch_exclusive_scan(counts, offsets, block_sums, n_rays, status, GNR_ST_NUM_VALID,
                                              GNR_ST_OVERFLOW_VALID, max_valid, st);
     }
