@@ -881,12 +881,9 @@ static int copy_out(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   return 0;
 }
 
-static int run_app_gather(GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws, const GnrWs& L,
-                          int64_t max_valid, int64_t max_app, cudaStream_t st) {
-  (void)n;
-  (void)max_valid;
-  (void)max_app;
-  const GnrCoords c = gnr_coords_app(rays, ws, L);
+static int run_app_gather(GnrModel* m, const GnrSampleParams& p, const float* rays, char* ws, const GnrWs& L, int lanes,
+                          cudaStream_t st) {
+  const GnrCoords c = gnr_coords_app(rays, ws, L, lanes);
   if (gnr_tc_basis_fused(m)) {
     unsigned char* hi = (unsigned char*)(ws + L.app_prod);
     return launch_app_products(m, p, c, hi, hi + L.app_prod_image, L.app_prod_tile, m->cfg.mlp_mode == 1 ? 2 : 1, st);
@@ -894,9 +891,9 @@ static int run_app_gather(GnrModel* m, const GnrSampleParams& p, const float* ra
   return launch_app_gather(m, p, c, L.feat_stride, (float*)(ws + L.app_feat), st);
 }
 
-static int run_mlp(GnrModel* m, const GnrSampleParams& p, const float* rays, char* ws, const GnrWs& L, int write_features,
-                   cudaStream_t st) {
-  const GnrCoords c = gnr_coords_app(rays, ws, L);
+static int run_mlp(GnrModel* m, const GnrSampleParams& p, const float* rays, char* ws, const GnrWs& L, int lanes,
+                   int write_features, cudaStream_t st) {
+  const GnrCoords c = gnr_coords_app(rays, ws, L, lanes);
   float* feat = (float*)(ws + L.app_feat);
   float* rgb = (float*)(ws + L.app_rgb);
   if (m->cfg.mlp_mode == 0) return launch_mlp_simt(m, p, c, L.feat_stride, feat, rgb, st);
@@ -905,10 +902,9 @@ static int run_mlp(GnrModel* m, const GnrSampleParams& p, const float* rays, cha
                        L.app_prod_tile, rgb, (int32_t*)(ws + L.status), 0, st);
 }
 
-static int run_appearance(GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws, const GnrWs& L,
-                          int64_t max_valid, int64_t max_app, cudaStream_t st) {
-  GNR_LAUNCH_OK(run_app_gather(m, p, rays, n, ws, L, max_valid, max_app, st));
-  GNR_LAUNCH_OK(run_mlp(m, p, rays, ws, L, /*write_features=*/1, st));
+static int run_appearance(GnrModel* m, const GnrSampleParams& p, const float* rays, char* ws, const GnrWs& L, cudaStream_t st) {
+  GNR_LAUNCH_OK(run_app_gather(m, p, rays, ws, L, /*lanes=*/0, st));
+  GNR_LAUNCH_OK(run_mlp(m, p, rays, ws, L, /*lanes=*/0, /*write_features=*/1, st));
   return 0;
 }
 
@@ -1009,7 +1005,7 @@ extern "C" int gnr_appearance(GnrModel* m, const float* rays, int64_t n, int S, 
   char* ws = (char*)workspace;
   GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app);
   GnrSampleParams p = gnr_sample_params(m, S);
-  rc = run_appearance(m, p, rays, n, ws, L, max_valid, max_app, st);
+  rc = run_appearance(m, p, rays, ws, L, st);
   if (rc) return rc;
   if (app_features) {
     GNR_CUDA_OK(cudaMemcpy2DAsync(app_features, (size_t)m->cfg.app_dim * 4, ws + L.app_feat, (size_t)L.feat_stride * 4,
@@ -1034,54 +1030,60 @@ static int render_chunk_impl(GnrModel* m, const float* rays, int64_t n, int S, i
                              int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, cudaStream_t st) {
   GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app);
   GnrSampleParams p = gnr_sample_params(m, S);
-  GNR_CUDA_OK(cudaMemsetAsync(ws + L.status, 0, GNR_ST_WORDS * sizeof(int32_t), st));
+  const int lanes = gnr_march_lanes(m, n, S, max_valid);
   {
     StageScope sc(m, GNR_STAGE_SAMPLE, 1, st);
-    GNR_LAUNCH_OK(launch_sample_mask(m, p, rays, n, ws, L, st));
+    GNR_LAUNCH_OK(launch_sample_mask(m, p, rays, n, ws, L, st, (int32_t*)(ws + L.status)));
   }
-  {
-    const int fused = m->cfg.ert_transmittance >= 0.0f;
-    StageScope sc(m, GNR_STAGE_COMPACT, fused ? 3 : 4, st);
-    GNR_LAUNCH_OK(launch_sample_compact(m, p, n, ws, L, max_valid, fused ? 0 : 1, st));
-  }
-  if (m->cfg.ert_transmittance >= 0.0f) {
-    // fused density + weights pass (with early ray termination when the threshold is > 0)
+  if (lanes != 0) {
+    // density + weights (with early ray termination when the threshold is > 0) + the appearance list
     StageScope sc(m, GNR_STAGE_DENSITY, 1, st);
-    GNR_LAUNCH_OK(launch_march(m, p, rays, n, ws, L, st, /*list_only=*/1));
+    GNR_LAUNCH_OK(launch_march(m, p, rays, n, ws, L, st, /*list_only=*/1, lanes));
   } else {
+    const int fused = m->cfg.ert_transmittance >= 0.0f;
     {
+      StageScope sc(m, GNR_STAGE_COMPACT, fused ? 3 : 4, st);
+      GNR_LAUNCH_OK(launch_sample_compact(m, p, n, ws, L, max_valid, fused ? 0 : 1, st));
+    }
+    if (fused) {
       StageScope sc(m, GNR_STAGE_DENSITY, 1, st);
-      GNR_LAUNCH_OK(launch_density(m, p, gnr_coords_valid(rays, ws, L), (float*)(ws + L.sigma_feat), (float*)(ws + L.sigma), st));
+      GNR_LAUNCH_OK(launch_march(m, p, rays, n, ws, L, st, /*list_only=*/1));
+    } else {
+      {
+        StageScope sc(m, GNR_STAGE_DENSITY, 1, st);
+        GNR_LAUNCH_OK(launch_density(m, p, gnr_coords_valid(rays, ws, L), (float*)(ws + L.sigma_feat), (float*)(ws + L.sigma), st));
+      }
+      {
+        StageScope sc(m, GNR_STAGE_WEIGHTS, 1, st);
+        GNR_LAUNCH_OK(launch_weights_only(m, p, n, ws, L, max_valid, st));
+      }
     }
     {
-      StageScope sc(m, GNR_STAGE_WEIGHTS, 1, st);
-      GNR_LAUNCH_OK(launch_weights_only(m, p, n, ws, L, max_valid, st));
+      StageScope sc(m, GNR_STAGE_COMPACT_APP, 4, st);
+      GNR_LAUNCH_OK(launch_app_compact(m, p, n, ws, L, max_valid, max_app, st, /*packed=*/fused ? 1 : 0));
     }
-  }
-  {
-    StageScope sc(m, GNR_STAGE_COMPACT_APP, 4, st);
-    GNR_LAUNCH_OK(launch_app_compact(m, p, n, ws, L, max_valid, max_app, st, /*packed=*/m->cfg.ert_transmittance >= 0.0f ? 1 : 0));
   }
   if (gnr_app_fusable(m)) {
     // gather + basis projection + MLP as one kernel: no operand of a sample leaves the SM
     StageScope sc(m, GNR_STAGE_MLP, 1, st);
+    const GnrCoords c = gnr_coords_app(rays, ws, L, lanes);
     if (m->cfg.unfused_appearance == 2 && !m->debug_prof)
-      GNR_LAUNCH_OK(launch_app_mlp_stream(m, p, gnr_coords_app(rays, ws, L), (float*)(ws + L.app_rgb), (int32_t*)(ws + L.status), st));
+      GNR_LAUNCH_OK(launch_app_mlp_stream(m, p, c, (float*)(ws + L.app_rgb), (int32_t*)(ws + L.status), st));
     else
-      GNR_LAUNCH_OK(launch_app_mlp_fused(m, p, gnr_coords_app(rays, ws, L), (float*)(ws + L.app_rgb), (int32_t*)(ws + L.status), st));
+      GNR_LAUNCH_OK(launch_app_mlp_fused(m, p, c, (float*)(ws + L.app_rgb), (int32_t*)(ws + L.status), st));
   } else {
     {
       StageScope sc(m, GNR_STAGE_APP_GATHER, 1, st);
-      GNR_LAUNCH_OK(run_app_gather(m, p, rays, n, ws, L, max_valid, max_app, st));
+      GNR_LAUNCH_OK(run_app_gather(m, p, rays, ws, L, lanes, st));
     }
     {
       StageScope sc(m, GNR_STAGE_MLP, 1, st);
-      GNR_LAUNCH_OK(run_mlp(m, p, rays, ws, L, /*write_features=*/0, st));
+      GNR_LAUNCH_OK(run_mlp(m, p, rays, ws, L, lanes, /*write_features=*/0, st));
     }
   }
   {
     StageScope sc(m, GNR_STAGE_COMPOSITE, 1, st);
-    GNR_LAUNCH_OK(launch_composite(m, n, white_bg, ws, L, rgb_map, depth_map, st));
+    GNR_LAUNCH_OK(launch_composite(m, n, white_bg, ws, L, rgb_map, depth_map, st, lanes));
   }
   return 0;
 }

@@ -43,13 +43,13 @@ weights_kernel(GnrSampleParams p, float distance_scale, float thres, const float
       const float dist = (k == p.S - 1) ? 0.0f : __fsub_rn(gnr_sample_t(p, t_min, k + 1), t);
       const float sg = __ldg(sigma + (rows ? (long long)__ldg(rows + i) : i));
       const float alpha = __fsub_rn(1.0f, expf(__fmul_rn(-sg, __fmul_rn(dist, distance_scale))));
-      const float w = alpha * T;
+      const float w = __fmul_rn(alpha, T);
       if (packed) {
         if (w > thres) packed[beg + n_app] = make_float2(w, __int_as_float(k));
       } else {
         weight[i] = w;
       }
-      acc += w;
+      acc = __fadd_rn(acc, w);
       dep = fmaf(w, t, dep);
       n_app += (w > thres) ? 1 : 0;
       T *= __fadd_rn(__fsub_rn(1.0f, alpha), 1e-10f);
@@ -156,7 +156,20 @@ expand_app_packed_kernel(const float2* __restrict__ packed, int kbits,
 }
 
 // rgb_map = sum_j w_j rgb_j (+ 1 - acc), clamp to [0,1]; depth_map = sum w t
-// (app/models/gridnerf_sequential.py:493-501).  One thread per ray, ranks in order.
+// (app/models/gridnerf_sequential.py:493-501).
+__device__ __forceinline__ void write_pixel(float r, float g, float b, const float* __restrict__ acc, const float* __restrict__ depth,
+                                            int64_t ray, int white_bg, float* __restrict__ rgb_map, float* __restrict__ depth_map) {
+  if (rgb_map) {
+    const float bg = white_bg ? (1.0f - acc[ray]) : 0.0f;
+    rgb_map[ray * 3 + 0] = fminf(fmaxf(r + bg, 0.0f), 1.0f);
+    rgb_map[ray * 3 + 1] = fminf(fmaxf(g + bg, 0.0f), 1.0f);
+    rgb_map[ray * 3 + 2] = fminf(fmaxf(b + bg, 0.0f), 1.0f);
+  }
+  if (depth_map) depth_map[ray] = depth[ray];
+}
+
+// One thread per ray, ranks in order, the loads of eight ranks in flight (one rank at a time, each step waited for its
+// four loads: 17 us against 10 for 8192 rays with 12 samples each).
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 composite_kernel(const float* __restrict__ app_weight, const int32_t* __restrict__ app_counts,
                  const int32_t* __restrict__ app_offsets, const float* __restrict__ app_rgb, const float* __restrict__ acc, const float* __restrict__ depth,
@@ -167,31 +180,65 @@ composite_kernel(const float* __restrict__ app_weight, const int32_t* __restrict
   if (group * 32 >= n_rays) return;
   const int64_t ray = group * 32 + lane;
   const bool has_ray = ray < n_rays;
-  int left = has_ray ? app_counts[ray] : 0;
+  const int count = has_ray ? app_counts[ray] : 0;
+  const int ranks = __reduce_max_sync(0xffffffffu, count);
   float r = 0.0f, g = 0.0f, b = 0.0f;
   AppGroupWalk walk;
   walk.pos = app_offsets[group * 32];
-  long long at;
-  while (walk.step(lane, left > 0, at)) {
-    if (left > 0) {
-      if (at < app_capacity) {
-        const float w = __ldg(app_weight + at);
-        r = fmaf(w, __ldg(app_rgb + at * 3 + 0), r);
-        g = fmaf(w, __ldg(app_rgb + at * 3 + 1), g);
-        b = fmaf(w, __ldg(app_rgb + at * 3 + 2), b);
+  for (int j0 = 0; j0 < ranks; j0 += 8) {
+    float w[8], cr[8], cg[8], cb[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      long long at = 0;
+      walk.step(lane, count > j0 + i, at);
+      w[i] = cr[i] = cg[i] = cb[i] = 0.0f;
+      if (count > j0 + i && at < app_capacity) {
+        w[i] = __ldg(app_weight + at);
+        cr[i] = __ldg(app_rgb + at * 3 + 0);
+        cg[i] = __ldg(app_rgb + at * 3 + 1);
+        cb[i] = __ldg(app_rgb + at * 3 + 2);
       }
-      --left;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {  // (a rank the ray does not have adds +0, which changes no bit of a sum that starts at +0)
+      r = fmaf(w[i], cr[i], r);
+      g = fmaf(w[i], cg[i], g);
+      b = fmaf(w[i], cb[i], b);
     }
   }
-  if (has_ray) {
-    if (rgb_map) {
-      const float bg = white_bg ? (1.0f - acc[ray]) : 0.0f;
-      rgb_map[ray * 3 + 0] = fminf(fmaxf(r + bg, 0.0f), 1.0f);
-      rgb_map[ray * 3 + 1] = fminf(fmaxf(g + bg, 0.0f), 1.0f);
-      rgb_map[ray * 3 + 2] = fminf(fmaxf(b + bg, 0.0f), 1.0f);
+  if (has_ray) write_pixel(r, g, b, acc, depth, ray, white_bg, rgb_map, depth_map);
+}
+
+// Ray-by-ray lists (small chunks): one warp per ray, 32 entries loaded at a time, summed in order with shuffles.
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+composite_rays_kernel(const float* __restrict__ app_weight, const int32_t* __restrict__ app_counts,
+                      const int32_t* __restrict__ app_base, const float* __restrict__ app_rgb, const float* __restrict__ acc,
+                      const float* __restrict__ depth, int64_t n_rays, long long app_capacity, int white_bg,
+                      float* __restrict__ rgb_map, float* __restrict__ depth_map) {
+  const int lane = threadIdx.x & 31;
+  const int64_t ray = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (ray >= n_rays) return;
+  const int count = app_counts[ray];
+  const long long base = app_base[ray];
+  float r = 0.0f, g = 0.0f, b = 0.0f;
+  for (int j0 = 0; j0 < count; j0 += 32) {
+    const long long at = base + j0 + lane;
+    float w = 0.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
+    if (j0 + lane < count && at < app_capacity) {
+      w = __ldg(app_weight + at);
+      cr = __ldg(app_rgb + at * 3 + 0);
+      cg = __ldg(app_rgb + at * 3 + 1);
+      cb = __ldg(app_rgb + at * 3 + 2);
     }
-    if (depth_map) depth_map[ray] = depth[ray];
+    const int m = min(32, count - j0);
+    for (int i = 0; i < m; ++i) {
+      const float wi = __shfl_sync(0xffffffffu, w, i);
+      r = fmaf(wi, __shfl_sync(0xffffffffu, cr, i), r);
+      g = fmaf(wi, __shfl_sync(0xffffffffu, cg, i), g);
+      b = fmaf(wi, __shfl_sync(0xffffffffu, cb, i), b);
+    }
   }
+  if (lane == 0) write_pixel(r, g, b, acc, depth, ray, white_bg, rgb_map, depth_map);
 }
 
 }  // namespace
@@ -234,8 +281,15 @@ int launch_app_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, c
 }
 
 int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const GnrWs& L, float* rgb_map,
-                     float* depth_map, cudaStream_t st) {
+                     float* depth_map, cudaStream_t st, int march_lanes) {
   (void)m;
+  if (march_lanes == 32) {  // ray-by-ray lists
+    composite_rays_kernel<<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
+        (const float*)(ws + L.app_weight), (const int32_t*)(ws + L.app_counts), (const int32_t*)(ws + L.app_offsets),
+        (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc), (const float*)(ws + L.depth), n, L.max_app, white_bg, rgb_map,
+        depth_map);
+    return (int)cudaGetLastError();
+  }
   const int64_t groups = (n + 31) / 32;
   unsigned blocks = (unsigned)((groups + kWarpsPerBlock - 1) / kWarpsPerBlock);
   long long app_capacity = L.max_app;

@@ -403,89 +403,229 @@ density_lattice_kernel(GnrSampleParams p, PlaneSet planes, LatticeRef lat, GnrCo
   }
 }
 
-// Fused density + weights pass ("march"): one thread walks one ray's valid samples (the set bits of
-// its validity words; sample j of the ray owns entry offsets[ray] + j of the per-sample arrays): density feature (density_thread), activation, raw2alpha's alpha, the
-// running transmittance product in sample order (as torch.cumprod computes it on the CPU), weight,
-// and the ray's accumulated opacity and depth.  The 32 rays of a warp are consecutive rays of the
-// chunk; when those are neighbouring pixels (tile order) their samples of equal rank lie within a
-// few voxels of each other, so the lanes of one load instruction read a handful of texels and the
-// L1 serves them as broadcasts.  When the transmittance falls below t_stop the ray stops: the
-// remaining samples get weight 0 and never touch the planes.  What they would have added to acc
-// (and, with a white background, taken from rgb) is bounded by the transmittance at the stop,
-// i.e. by t_stop.  With t_stop == 0 the weights are bit-identical to density_kernel followed by
-// weights_kernel.
-constexpr int kMarchBlock = 32;  // one warp per CTA: a finished warp frees its slot at once
+// Fused density + weights pass ("march"): G lanes walk one ray's valid samples (the set bits of its validity words)
+// together, G consecutive sample numbers at a time starting at the next valid one: each lane evaluates its own sample
+// (density_thread or the lattice, activation, raw2alpha's alpha), then the group takes the running transmittance product,
+// the accumulated opacity and the depth over its G samples in sample order (as torch.cumprod computes it on the CPU),
+// with shuffles.  A sample that is not valid has alpha 0 and a factor of exactly 1.  When the transmittance falls below
+// t_stop the ray stops: the remaining samples get weight 0 and never touch the planes.  What they would have added to
+// acc (and, with a white background, taken from rgb) is bounded by the transmittance at the stop, i.e. by t_stop.  With
+// t_stop == 0 the weights are bit-identical to density_kernel followed by weights_kernel.
+// Neighbouring groups of a warp are consecutive rays of the chunk; when those are neighbouring pixels (tile order) their
+// samples lie within a few voxels of each other and the L1 serves the lanes of a load from a few sectors.
+//
+// LIST: the kernel also builds the appearance list.  A ray's samples above the appearance threshold go, as (weight,
+// sample number) pairs of 8 bytes, to the front of the ray's own S entries of the pair array; at the end the rays that
+// share a list group know their counts, take a range of the list with one atomic, and write it in the group's order
+// (G < 32: the 32 rays of the block, by rank first and ray second, see AppGroupWalk in gnr_composite.cu; G == 32: the
+// warp's one ray).  The order of the GROUPS in the list is whatever the atomics give; nothing depends on it, since every
+// entry is evaluated by itself and a group's base is kept for the compositing.
+// What bounds it: with few rays the chain of a ray's dependent steps (eight lattice loads at L2 latency, exp, log), which
+// more lanes per ray shorten; with many rays load latency and issue slots, where more lanes only add shuffles and samples
+// evaluated behind a ray's stop.  gnr_march_lanes holds the rule and its figures.
+// Without LIST the valid samples are indexed through `offsets` (exclusive scan of the counts), and either the weight of
+// every valid sample is written (`weight`) or the pairs are packed at the front of the ray's range.
+template <int G>
+constexpr int kMarchBlock = G == 32 ? 128 : 32 * G;  // 32 rays = one list group per block; four rays with G == 32
 
-template <int J, int NP, bool HALF = false, bool LAT = false>
-__global__ void __launch_bounds__(kMarchBlock, LAT ? 32 : 16)
-march_kernel(GnrSampleParams p, PlaneSet planes, LatticeRef lat, const float* __restrict__ rays, const float* __restrict__ t_min_arr,
-             const uint32_t* __restrict__ words, const int32_t* __restrict__ offsets, long long n_rays, long long capacity,
-             float shift, int act, float distance_scale, float thres, float t_stop, float* __restrict__ weight,
-             float* __restrict__ acc_out, float* __restrict__ depth_out, int32_t* __restrict__ app_counts,
-             int32_t* __restrict__ evaluated_total, int list_only, float2* __restrict__ packed) {
-  __shared__ int s_evaluated;
-  if (threadIdx.x == 0) s_evaluated = 0;
-  __syncthreads();
-  const long long ray = (long long)blockIdx.x * kMarchBlock + threadIdx.x;
-  int evaluated = 0;
-  if (ray < n_rays) {
-    const long long beg = offsets[ray], end = min((long long)offsets[ray + 1], capacity);
-    float acc = 0.0f, dep = 0.0f;
-    int n_app = 0;
-    if (beg < end) {
-      const float* r = rays + (size_t)ray * 6;
-      const float ox = __ldg(r + 0), oy = __ldg(r + 1), oz = __ldg(r + 2);
-      const float dx = __ldg(r + 3), dy = __ldg(r + 4), dz = __ldg(r + 5);
-      const float t_min = t_min_arr[ray];
-      float T = 1.0f;
-      long long i = beg;
-      // the ray's valid samples are the set bits of its validity words, in order
-      const uint32_t* wrow = words + (size_t)ray * p.words;
-      int word = 0;
-      uint32_t bits = __ldg(wrow);
-      while (i < end) {
-        while (bits == 0u && word + 1 < p.words) bits = __ldg(wrow + ++word);
-        if (bits == 0u) break;  // (cannot happen: offsets count exactly the set bits)
-        const int k = word * 32 + (__ffs(bits) - 1);
-        bits &= bits - 1u;
-        const float t = gnr_sample_t(p, t_min, k);
-        const float x = gnr_normalize(gnr_point(ox, dx, t), p.lo[0], p.inv[0]);
-        const float y = gnr_normalize(gnr_point(oy, dy, t), p.lo[1], p.inv[1]);
-        const float z = gnr_normalize(gnr_point(oz, dz, t), p.lo[2], p.inv[2]);
-        float feat;
-        if constexpr (LAT) feat = lattice_density_feature(lat, planes, x, y, z);
-        else feat = density_thread<J, NP, HALF>(planes, x, y, z);
-        const float sg = density_activation(feat, shift, act);
-        const float dist = (k == p.S - 1) ? 0.0f : __fsub_rn(gnr_sample_t(p, t_min, k + 1), t);
-        const float alpha = __fsub_rn(1.0f, expf(__fmul_rn(-sg, __fmul_rn(dist, distance_scale))));
-        const float w = alpha * T;
-        if (list_only) {
-          // the frame loop reads nothing but the samples that pass the appearance threshold: they go, as (weight,
-          // sample number) pairs of 8 bytes, to the front of the ray's own range of the pair array, in order
-          if (w > thres) packed[beg + n_app] = make_float2(w, __int_as_float(k));
-        } else {
-          weight[i] = w;
-        }
-        acc += w;
-        dep = fmaf(w, t, dep);
-        n_app += (w > thres) ? 1 : 0;
-        T *= __fadd_rn(__fsub_rn(1.0f, alpha), 1e-10f);
-        ++i;
-        if (T < t_stop) break;
-      }
-      evaluated = (int)(i - beg);
-      // Weights behind the stop are zero (written for callers that look at the weight array itself).
-      if (!list_only)
-        for (; i < end; ++i) weight[i] = 0.0f;
+struct MarchArgs {
+  const float* rays;
+  const float* t_min;
+  const uint32_t* words;
+  const int32_t* counts;   // LIST: valid samples per ray
+  const int32_t* offsets;  // !LIST
+  long long n_rays, capacity, app_capacity;
+  float shift, distance_scale, thres, t_stop;
+  int act;
+  float* weight;           // !LIST: null = packed
+  float* acc;
+  float* depth;
+  int32_t* app_counts;
+  int32_t* status;
+  float2* packed;
+  int32_t* app_base;       // LIST: first list entry of the group of ray 32 g (G < 32) or of the ray (G == 32)
+  uint32_t* app_ids;
+  float* app_weight;
+};
+
+template <int J, int NP, bool HALF, bool LAT, int G, bool LIST>
+__global__ void __launch_bounds__(kMarchBlock<G>, (LAT ? 40 : 16) / (kMarchBlock<G> / 32))
+march_kernel(const __grid_constant__ GnrSampleParams p, const __grid_constant__ PlaneSet planes, LatticeRef lat,
+             const __grid_constant__ MarchArgs a) {
+  constexpr uint32_t kGroup = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+  const int lane = threadIdx.x & 31, g = lane & (G - 1);
+  const long long ray = (long long)blockIdx.x * (kMarchBlock<G> / G) + threadIdx.x / G;
+  const bool has_ray = ray < a.n_rays;
+  long long beg = 0;
+  int limit = 0;  // valid samples of the ray that have an entry
+  if (has_ray) {
+    if (LIST) {
+      beg = ray * p.S;
+      limit = p.S;
+    } else {
+      beg = a.offsets[ray];
+      limit = (int)max(0LL, min((long long)a.offsets[ray + 1], a.capacity) - beg);
     }
-    acc_out[ray] = acc;
-    depth_out[ray] = dep;
-    app_counts[ray] = n_app;
+  }
+  float acc = 0.0f, dep = 0.0f, T = 1.0f;
+  int n_app = 0, seen = 0, evaluated = 0;
+  float o[3] = {0.0f, 0.0f, 0.0f}, d[3] = {0.0f, 0.0f, 0.0f}, t_min = 0.0f;
+  const uint32_t* wrow = a.words + (size_t)(has_ray ? ray : 0) * p.words;
+  int word = p.words - 1;
+  uint32_t bits = 0u;
+  if (limit > 0) {
+    const float* r = a.rays + (size_t)ray * 6;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      o[e] = __ldg(r + e);
+      d[e] = __ldg(r + 3 + e);
+    }
+    t_min = a.t_min[ray];
+    word = 0;
+    bits = __ldg(wrow);
+  }
+  while (true) {
+    while (bits == 0u && word + 1 < p.words) bits = __ldg(wrow + ++word);
+    if (!__any_sync(0xffffffffu, bits != 0u)) break;
+    const int pos = bits ? __ffs(bits) - 1 : 0;
+    const uint32_t window = (bits >> pos) & kGroup;  // this step's samples: bit i = sample word * 32 + pos + i
+    bool valid = (window >> g) & 1u;
+    const int rank = LIST ? 0 : seen + __popc(window & ((1u << g) - 1u));
+    if (!LIST) valid = valid && rank < limit;
+    const int k = word * 32 + pos + g;
+    float t = 0.0f, alpha = 0.0f;
+    if (valid) {
+      t = gnr_sample_t(p, t_min, k);
+      const float x = gnr_normalize(gnr_point(o[0], d[0], t), p.lo[0], p.inv[0]);
+      const float y = gnr_normalize(gnr_point(o[1], d[1], t), p.lo[1], p.inv[1]);
+      const float z = gnr_normalize(gnr_point(o[2], d[2], t), p.lo[2], p.inv[2]);
+      float feat;
+      if constexpr (LAT) feat = lattice_density_feature(lat, planes, x, y, z);
+      else feat = density_thread<J, NP, HALF>(planes, x, y, z);
+      const float sg = density_activation(feat, a.shift, a.act);
+      const float dist = (k == p.S - 1) ? 0.0f : __fsub_rn(gnr_sample_t(p, t_min, k + 1), t);
+      alpha = __fsub_rn(1.0f, expf(__fmul_rn(-sg, __fmul_rn(dist, a.distance_scale))));
+    }
+    // transmittance in front of this lane's sample, in sample order; nothing counts behind the sample that stops the ray
+    const float factor = __fadd_rn(__fsub_rn(1.0f, alpha), 1e-10f);
+    float before = T;
+    bool stopped = false, live = true;
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const float f = __shfl_sync(0xffffffffu, factor, i, G);
+      if (g == i) {
+        before = T;
+        live = !stopped;
+      }
+      T = __fmul_rn(T, f);
+      stopped = stopped || T < a.t_stop;
+    }
+    const bool counted = valid && live;
+    const float w = counted ? __fmul_rn(alpha, before) : 0.0f;
+    const bool pass = counted && w > a.thres;
+    evaluated += counted ? 1 : 0;
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const float wi = __shfl_sync(0xffffffffu, w, i, G), ti = __shfl_sync(0xffffffffu, t, i, G);
+      acc = __fadd_rn(acc, wi);
+      dep = fmaf(wi, ti, dep);
+    }
+    const uint32_t passed = (__ballot_sync(0xffffffffu, pass) >> (lane & ~(G - 1) & 31)) & kGroup;
+    if (LIST || a.weight == nullptr) {
+      if (pass) a.packed[beg + n_app + __popc(passed & ((1u << g) - 1u))] = make_float2(w, __int_as_float(k));
+    } else if (valid) {
+      a.weight[beg + rank] = w;
+    }
+    n_app += __popc(passed);
+    seen += __popc(window);
+    bits = G == 32 ? 0u : bits & ~(kGroup << pos);
+    if (stopped || (!LIST && seen >= limit)) {
+      bits = 0u;
+      word = p.words - 1;
+    }
+  }
+  if (!LIST && a.weight != nullptr)  // weights behind the stop are zero
+    for (int i = seen + g; i < limit; i += G) a.weight[beg + i] = 0.0f;
+  if (has_ray && g == 0) {
+    a.acc[ray] = acc;
+    a.depth[ray] = dep;
+    a.app_counts[ray] = n_app;
   }
   evaluated = __reduce_add_sync(0xffffffffu, evaluated);
-  if ((threadIdx.x & 31) == 0 && evaluated) atomicAdd(&s_evaluated, evaluated);
-  __syncthreads();
-  if (threadIdx.x == 0 && s_evaluated) atomicAdd(evaluated_total, s_evaluated);
+  if (!LIST) {
+    if (lane == 0 && evaluated) atomicAdd(a.status + GNR_ST_NUM_DENSITY, evaluated);
+    return;
+  }
+
+  if constexpr (LIST && G == 32) {
+    int base = 0;
+    if (lane == 0 && has_ray) {
+      const int valid_samples = a.counts[ray];
+      if (valid_samples) atomicAdd(a.status + GNR_ST_NUM_VALID, valid_samples);
+      if (evaluated) atomicAdd(a.status + GNR_ST_NUM_DENSITY, evaluated);
+      if (n_app) base = atomicAdd(a.status + GNR_ST_NUM_APP, n_app);
+      if ((long long)base + n_app > a.app_capacity) a.status[GNR_ST_OVERFLOW_APP] = 1;
+      a.app_base[ray] = base;
+    }
+    base = __shfl_sync(0xffffffffu, base, 0);
+    __syncwarp();  // the warp's pairs above are visible to all its lanes below
+    for (int i = lane; i < n_app; i += 32) {
+      const long long at = (long long)base + i;
+      if (at < a.app_capacity) {
+        const float2 wk = a.packed[beg + i];
+        a.app_ids[at] = ((uint32_t)ray << p.kbits) | (uint32_t)__float_as_int(wk.y);
+        a.app_weight[at] = wk.x;
+      }
+    }
+  } else if constexpr (LIST) {
+    static_assert(kMarchBlock<G> / G == 32, "a block holds the 32 rays of one list group");
+    __shared__ int s_count[32], s_evaluated[kMarchBlock<G> / 32], s_base;
+    const int warp = threadIdx.x >> 5;
+    if (g == 0) s_count[threadIdx.x / G] = n_app;  // (0 for a ray past the end)
+    if (lane == 0) s_evaluated[warp] = evaluated;
+    __syncthreads();
+    const long long ray0 = (long long)blockIdx.x * 32;
+    const int mine = s_count[lane];  // lane = ray of the group from here on
+    if (warp == 0) {
+      const int valid_samples = __reduce_add_sync(0xffffffffu, ray0 + lane < a.n_rays ? a.counts[ray0 + lane] : 0);
+      const int total = __reduce_add_sync(0xffffffffu, mine);
+      if (lane == 0) {
+        int ev = 0;
+#pragma unroll
+        for (int i = 0; i < kMarchBlock<G> / 32; ++i) ev += s_evaluated[i];
+        if (valid_samples) atomicAdd(a.status + GNR_ST_NUM_VALID, valid_samples);
+        if (ev) atomicAdd(a.status + GNR_ST_NUM_DENSITY, ev);
+        const int base = total ? atomicAdd(a.status + GNR_ST_NUM_APP, total) : 0;
+        if ((long long)base + total > a.app_capacity) a.status[GNR_ST_OVERFLOW_APP] = 1;
+        a.app_base[ray0] = base;
+        s_base = base;
+      }
+    }
+    __syncthreads();
+    // ranks in runs of four (one sector of a ray's pairs), the runs dealt to the warps
+    long long at0 = s_base;
+    const int ranks = __reduce_max_sync(0xffffffffu, mine);
+    const float2* pairs = a.packed + (ray0 + lane) * p.S;
+    for (int j0 = 0; j0 < ranks; j0 += 4) {
+      const bool my_run = ((j0 >> 2) & (kMarchBlock<G> / 32 - 1)) == warp;
+      float2 wk[4];
+      long long at[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t m = __ballot_sync(0xffffffffu, mine > j0 + i);
+        at[i] = at0 + __popc(m & ((1u << lane) - 1u));
+        at0 += __popc(m);
+        if (my_run && mine > j0 + i) wk[i] = pairs[j0 + i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (my_run && mine > j0 + i && at[i] < a.app_capacity) {
+          a.app_ids[at[i]] = ((uint32_t)(ray0 + lane) << p.kbits) | (uint32_t)__float_as_int(wk[i].y);
+          a.app_weight[at[i]] = wk[i].x;
+        }
+      }
+    }
+  }
 }
 
 // Appearance gather + basis projection.  The basis weights sit in shared memory, blocked per
@@ -767,10 +907,10 @@ GnrCoords gnr_coords_valid(const float* rays, char* ws, const GnrWs& L) {
   return c;
 }
 
-GnrCoords gnr_coords_app(const float* rays, char* ws, const GnrWs& L) {
+GnrCoords gnr_coords_app(const float* rays, char* ws, const GnrWs& L, int lanes) {
   GnrCoords c = gnr_coords_valid(rays, ws, L);
-  c.ids = (const uint32_t*)(ws + L.app_ids);  // written by expand_app_kernel in list order
-  c.total_ptr = (const int32_t*)(ws + L.app_offsets) + L.n_rays;
+  c.ids = (const uint32_t*)(ws + L.app_ids);  // written in list order by the march or by expand_app_kernel
+  c.total_ptr = lanes == 0 ? (const int32_t*)(ws + L.app_offsets) + L.n_rays : (const int32_t*)(ws + L.status) + GNR_ST_NUM_APP;
   c.capacity = L.max_app;
   return c;
 }
@@ -1014,33 +1154,77 @@ int launch_positions(const GnrModel* m, const GnrSampleParams& p, const GnrCoord
   return (int)cudaGetLastError();
 }
 
+// Lanes per ray of the march, or 0 for the scanned offsets of the stage-wise entries.  The march writes the appearance
+// list itself when every ray can have its own S entries of the pair array (the worst-case capacity, the default).
+// Measured, us per launch, city at 512 samples (lattice) / city at 256 samples (planes and lines):
+//   rays     1 lane  2 lanes  4 lanes  8 lanes  32 lanes
+//   262144    398      341      376      469         -      (one thread per ray and separate scans and expansion: 530)
+//    65536    183      183      235      274         -      planes
+//    32768    114       82       67       76         -
+//    16384    111       86       93      105       119      planes
+//     8192    101       70       46       35        44
+//     8192    107       72       60       62        69      planes
+//     2048     97       70       43       30        23
+//     1024    100       64       41       37        19      planes
+// From planes and lines a step is 36 loads of 32 bytes and the L1 port is busy sooner: half as many lanes.
+int gnr_march_lanes(const GnrModel* m, int64_t n, int S, int64_t max_valid) {
+  if (m->cfg.ert_transmittance < 0.0f || max_valid < n * S) return 0;
+  if (m->den_lattice) return n >= 98304 ? 2 : (n >= 12288 ? 4 : (n >= 3072 ? 8 : 32));
+  return n >= 12288 ? 2 : (n >= 6144 ? 4 : (n >= 3072 ? 8 : 32));
+}
+
 int launch_march(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws, const GnrWs& L,
-                 cudaStream_t st, int list_only) {
-  PlaneSet set = make_set(m->den, m->cfg.n_pairs);
+                 cudaStream_t st, int list_only, int lanes) {
+  const PlaneSet set = make_set(m->den, m->cfg.n_pairs);
   const int J = m->den[0].C / 16;
-  const unsigned grid = (unsigned)((n + kMarchBlock - 1) / kMarchBlock);
-  const float t_stop = m->cfg.ert_transmittance > 0.0f ? m->cfg.ert_transmittance : 0.0f;
   const LatticeRef lat = lattice_of(m);
-#define GNR_MARCH(JJ, NPP) GNR_MARCH_H(JJ, NPP, false, false)
-#define GNR_MARCH_H(JJ, NPP, HH, LL)                                                                              \
-  march_kernel<JJ, NPP, HH, LL><<<grid, kMarchBlock, 0, st>>>(                                                    \
-      p, set, lat, rays, (const float*)(ws + L.t_min), (const uint32_t*)(ws + L.words), (const int32_t*)(ws + L.offsets), \
-      (long long)n, L.max_valid, m->cfg.density_shift, m->cfg.density_act, m->cfg.distance_scale,                 \
-      m->cfg.ray_weight_thres, t_stop, (float*)(ws + L.weight), (float*)(ws + L.acc), (float*)(ws + L.depth),     \
-      (int32_t*)(ws + L.app_counts), (int32_t*)(ws + L.status) + GNR_ST_NUM_DENSITY, list_only, (float2*)(ws + L.sigma))
-  if (m->den_lattice) GNR_MARCH_H(1, 3, false, true);
-  else if (m->cfg.den_storage == 1 && standard_vm3(set)) GNR_MARCH_H(1, 3, true, false);
-  else if (m->cfg.den_storage == 1) GNR_MARCH_H(1, 0, true, false);
-  else if (J == 1 && standard_vm3(set)) GNR_MARCH(1, 3);
-  else if (J == 1) GNR_MARCH(1, 0);
-  else if (J == 2) GNR_MARCH(2, 0);
-  else if (J == 3) GNR_MARCH(3, 0);
-  else if (J == 4) GNR_MARCH(4, 0);
+  MarchArgs a;
+  a.rays = rays;
+  a.t_min = (const float*)(ws + L.t_min);
+  a.words = (const uint32_t*)(ws + L.words);
+  a.counts = (const int32_t*)(ws + L.counts);
+  a.offsets = (const int32_t*)(ws + L.offsets);
+  a.n_rays = n;
+  a.capacity = L.max_valid;
+  a.app_capacity = L.max_app;
+  a.shift = m->cfg.density_shift;
+  a.distance_scale = m->cfg.distance_scale;
+  a.thres = m->cfg.ray_weight_thres;
+  a.t_stop = m->cfg.ert_transmittance > 0.0f ? m->cfg.ert_transmittance : 0.0f;
+  a.act = m->cfg.density_act;
+  a.weight = list_only ? nullptr : (float*)(ws + L.weight);
+  a.acc = (float*)(ws + L.acc);
+  a.depth = (float*)(ws + L.depth);
+  a.app_counts = (int32_t*)(ws + L.app_counts);
+  a.status = (int32_t*)(ws + L.status);
+  a.packed = (float2*)(ws + L.sigma);
+  a.app_base = (int32_t*)(ws + L.app_offsets);
+  a.app_ids = (uint32_t*)(ws + L.app_ids);
+  a.app_weight = (float*)(ws + L.app_weight);
+  const unsigned rays_per_block = lanes == 32 ? 4 : 32;
+  const unsigned grid = (unsigned)((n + rays_per_block - 1) / rays_per_block);
+#define GNR_MARCH_G(JJ, NPP, HH, LL, GG, LIST) march_kernel<JJ, NPP, HH, LL, GG, LIST><<<grid, kMarchBlock<GG>, 0, st>>>(p, set, lat, a)
+#define GNR_MARCH(JJ, NPP, HH, LL)                                   \
+  do {                                                               \
+    if (lanes == 0) GNR_MARCH_G(JJ, NPP, HH, LL, 4, false);          \
+    else if (lanes == 2) GNR_MARCH_G(JJ, NPP, HH, LL, 2, true);      \
+    else if (lanes == 4) GNR_MARCH_G(JJ, NPP, HH, LL, 4, true);      \
+    else if (lanes == 8) GNR_MARCH_G(JJ, NPP, HH, LL, 8, true);      \
+    else GNR_MARCH_G(JJ, NPP, HH, LL, 32, true);                     \
+  } while (0)
+  if (m->den_lattice) GNR_MARCH(1, 3, false, true);
+  else if (m->cfg.den_storage == 1 && standard_vm3(set)) GNR_MARCH(1, 3, true, false);
+  else if (m->cfg.den_storage == 1) GNR_MARCH(1, 0, true, false);
+  else if (J == 1 && standard_vm3(set)) GNR_MARCH(1, 3, false, false);
+  else if (J == 1) GNR_MARCH(1, 0, false, false);
+  else if (J == 2) GNR_MARCH(2, 0, false, false);
+  else if (J == 3) GNR_MARCH(3, 0, false, false);
+  else if (J == 4) GNR_MARCH(4, 0, false, false);
   else {
     gnr_set_error("density channels (padded) %d not supported (16..64)", m->den[0].C);
     return -1;
   }
 #undef GNR_MARCH
-#undef GNR_MARCH_H
+#undef GNR_MARCH_G
   return (int)cudaGetLastError();
 }

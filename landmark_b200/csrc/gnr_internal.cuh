@@ -155,8 +155,9 @@ int gnr_check_chunk(const GnrModel* m, int64_t n_rays, int S, int64_t max_valid,
                     const void* ws, size_t ws_bytes);
 
 // launchers (each enqueues on `st`, returns cudaGetLastError as int)
+// (`status`: also zero this status block)
 int launch_sample_mask(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws,
-                       const GnrWs& L, cudaStream_t st);
+                       const GnrWs& L, cudaStream_t st, int32_t* status = nullptr);
 // with_ids == 0: offsets only (the compacted id list is needed by the list-based density kernel and the stage API)
 int launch_sample_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, char* ws, const GnrWs& L,
                           int64_t max_valid, int with_ids, cudaStream_t st);
@@ -165,7 +166,10 @@ int launch_build_app_lattice(const GnrModel* m, void* V, cudaStream_t st);
 int gnr_app_lattice_dims(const GnrModel* m, int* dims);
 int gnr_lattice_dims(const GnrModel* m, int* dims);  // grid of the density field if it has the standard VM3 layout, else -1
 GnrCoords gnr_coords_valid(const float* rays, char* ws, const GnrWs& L);
-GnrCoords gnr_coords_app(const float* rays, char* ws, const GnrWs& L);
+// How a chunk's appearance list comes about: written by the march itself with that many lanes per ray (32: ray by ray,
+// fewer: in groups of 32 rays), or (0) through the scanned offsets of the stage-wise entries.
+int gnr_march_lanes(const GnrModel* m, int64_t n_rays, int S, int64_t max_valid);
+GnrCoords gnr_coords_app(const float* rays, char* ws, const GnrWs& L, int lanes = 0);
 int launch_density(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, float* sigma_feat, float* sigma,
                    cudaStream_t st);
 // (`sigma_rows` + `rows`: sigma of list entry i is sigma_rows[rows[i]], read in place; the output is then the packed
@@ -175,13 +179,13 @@ int launch_weights_only(const GnrModel* m, const GnrSampleParams& p, int64_t n, 
 // (`packed`: the march ran with list_only)
 int launch_app_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, char* ws, const GnrWs& L,
                        int64_t max_valid, int64_t max_app, cudaStream_t st, int packed = 0);
-// Fused density gather + transmittance scan + early termination, one warp per ray.
+// Fused density gather + transmittance scan + early termination.
 // (`list_only`: instead of one weight per valid sample, write only the samples above the appearance threshold, packed
 // at the front of every ray's range as 8-byte (weight, sample number) pairs in the sigma + weight arrays, which lie
-// back to back in the workspace; what
-// launch_app_compact(..., packed = 1) reads)
+// back to back in the workspace; what launch_app_compact(..., packed = 1) reads.  With `lanes` from gnr_march_lanes above
+// 0 the kernel builds the appearance list itself: no scan, no expansion.)
 int launch_march(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws, const GnrWs& L,
-                 cudaStream_t st, int list_only = 0);
+                 cudaStream_t st, int list_only = 0, int lanes = 0);
 int launch_app_gather(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, float* feat,
                       cudaStream_t st);
 int launch_app_products(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, unsigned char* prod_hi,
@@ -216,7 +220,7 @@ int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& 
                   float* feat_out, const unsigned char* prod_hi, const unsigned char* prod_lo, int tile_bytes, float* rgb,
                   int32_t* status, int force_unfused, cudaStream_t st, int basis_only = 0);
 int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const GnrWs& L, float* rgb_map,
-                     float* depth_map, cudaStream_t st);
+                     float* depth_map, cudaStream_t st, int march_lanes = 0);
 int launch_exclusive_scan(const int32_t* counts, int32_t* offsets, int32_t* block_sums, int64_t n,
                           int32_t* status, int total_slot, int overflow_slot, int64_t capacity,
                           cudaStream_t st);

@@ -218,7 +218,9 @@ constexpr int kSampleWarps = 4;
 // open word was tested sample by sample); 333 rays x 128 samples: 14 us, 121 us with a thread walking each ray.
 __global__ void __launch_bounds__(kSampleWarps * 32, 8)
 sample_words_kernel(const __grid_constant__ GnrSampleParams p, const float* __restrict__ rays, int64_t n_rays, int per_warp,
-                    float* __restrict__ t_min_out, uint32_t* __restrict__ words_out, int32_t* __restrict__ counts_out) {
+                    float* __restrict__ t_min_out, uint32_t* __restrict__ words_out, int32_t* __restrict__ counts_out,
+                    int32_t* __restrict__ status) {
+  if (status != nullptr && blockIdx.x == 0 && threadIdx.x < GNR_ST_WORDS) status[threadIdx.x] = 0;
   __shared__ RaySetup s_ray[kSampleWarps][32];
   __shared__ int s_count[kSampleWarps][32];
   __shared__ uint32_t s_bits[kSampleWarps][32];   // the 32 words of a pass
@@ -437,18 +439,19 @@ int launch_exclusive_scan(const int32_t* counts, int32_t* offsets, int32_t* bloc
 // Rays per warp: 32 when there are enough rays to fill the GPU (the slab set-up then uses every lane), fewer below that,
 // down to one, so that a small chunk still spreads over all SMs.
 static int launch_sample_words(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, float* t_min,
-                               uint32_t* words, int32_t* counts, cudaStream_t st) {
+                               uint32_t* words, int32_t* counts, cudaStream_t st, int32_t* status = nullptr) {
   const int64_t warps = (int64_t)m->sm_count * 32;
   const int per_warp = (int)min((int64_t)32, max((int64_t)1, n / warps));
   const int64_t per_block = (int64_t)per_warp * kSampleWarps;
   sample_words_kernel<<<(unsigned)((n + per_block - 1) / per_block), kSampleWarps * 32, 0, st>>>(p, rays, n, per_warp, t_min, words,
-                                                                                               counts);
+                                                                                               counts, status);
   return (int)cudaGetLastError();
 }
 
 int launch_sample_mask(const GnrModel* m, const GnrSampleParams& p, const float* rays, int64_t n, char* ws,
-                       const GnrWs& L, cudaStream_t st) {
-  return launch_sample_words(m, p, rays, n, (float*)(ws + L.t_min), (uint32_t*)(ws + L.words), (int32_t*)(ws + L.counts), st);
+                       const GnrWs& L, cudaStream_t st, int32_t* status) {
+  return launch_sample_words(m, p, rays, n, (float*)(ws + L.t_min), (uint32_t*)(ws + L.words), (int32_t*)(ws + L.counts), st,
+                             status);
 }
 
 int launch_sample_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, char* ws, const GnrWs& L,
