@@ -276,6 +276,7 @@ extern "C" int gnr_destroy(GnrModel* m) {
   free_dev(m->mlp.b2);
   free_dev(m->mlp.b3);
   free_dev(m->mlp.tc_image);
+  free_dev(m->mlp.split_image);
   free_dev(m->host_ws);
   free_dev(m->host_rays);
   free_dev(m->host_rgb);
@@ -561,6 +562,7 @@ extern "C" int gnr_upload_mlp(GnrModel* m, const float* basis_w, const float* w1
   copy_or_zero_kernel<<<1, 32, 0, st>>>(b3, q.b3, 3, 4);
   GNR_CUDA_OK(cudaGetLastError());
   if (m->cfg.mlp_mode != 0) return gnr_mlp_tc_prepare(m, basis_w, w1, w2, w3, st);
+  if (gnr_mlp_split_usable(m)) return gnr_mlp_split_prepare(m, w1, w2, st);
   return 0;
 }
 
@@ -896,6 +898,7 @@ static int run_mlp(GnrModel* m, const GnrSampleParams& p, const float* rays, cha
   const GnrCoords c = gnr_coords_app(rays, ws, L, lanes);
   float* feat = (float*)(ws + L.app_feat);
   float* rgb = (float*)(ws + L.app_rgb);
+  if (gnr_mlp_split_usable(m)) return launch_mlp_split(m, p, c, L.feat_stride, feat, rgb, (int32_t*)(ws + L.status), st);
   if (m->cfg.mlp_mode == 0) return launch_mlp_simt(m, p, c, L.feat_stride, feat, rgb, st);
   const unsigned char* hi = (const unsigned char*)(ws + L.app_prod);
   return launch_mlp_tc(m, p, c, L.feat_stride, feat, write_features ? feat : nullptr, hi, hi + L.app_prod_image,
@@ -1229,7 +1232,9 @@ extern "C" int gnr_density_points(GnrModel* m, const float* xyz, int64_t n, floa
 static int mlp_points(GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, char* sc, const PointScratch& S, int fused,
                       float* feat_copy, float* rgb, cudaStream_t st) {
   float* feat = (float*)(sc + S.feat);
-  if (m->cfg.mlp_mode == 0) {
+  if (gnr_mlp_split_usable(m)) {
+    GNR_LAUNCH_OK(launch_mlp_split(m, p, c, 28, feat, rgb, (int32_t*)(sc + S.status), st));
+  } else if (m->cfg.mlp_mode == 0) {
     GNR_LAUNCH_OK(launch_mlp_simt(m, p, c, 28, feat, rgb, st));
   } else {
     const unsigned char* hi = (const unsigned char*)(sc + S.prod);

@@ -33,6 +33,7 @@ struct GnrMlp {
   // tensor-core images (pre-tiled, see gnr_mlp_tc.cu)
   void* tc_image;
   size_t tc_image_bytes;
+  void* split_image;  // weights as sums of bf16 terms (gnr_mlp_split.cu), mlp_mode 0
   int in_dim;   // 150
   int k1_pad;   // in_dim rounded up to 8
   int n_prod;   // sum of padded appearance channels (144)
@@ -214,6 +215,11 @@ int launch_positions(const GnrModel* m, const GnrSampleParams& p, const GnrCoord
                      cudaStream_t st);
 int launch_mlp_simt(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat,
                     float* rgb, cudaStream_t st);
+// the fp32 network on the tensor cores (gnr_mlp_split.cu): 1 if this model's layer sizes are the ones it is built for
+int gnr_mlp_split_usable(const GnrModel* m);
+int gnr_mlp_split_prepare(GnrModel* m, const float* w1, const float* w2, cudaStream_t st);
+int launch_mlp_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat,
+                     float* rgb, int32_t* status, cudaStream_t st);
 // feat_in: features for the non-fused variant; feat_out: optional copy of the projected features
 // (fused variant); prod_*: product tiles (fused variant); status: 8-word block for the wait flag.
 int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat_in,

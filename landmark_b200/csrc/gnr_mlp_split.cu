@@ -1,0 +1,440 @@
+// Appearance MLP (150 -> 128 -> 128 -> 3) on the tensor cores with every operand carried as a sum of 16-bit terms.
+//
+// MLPRender_Fea.forward (app/models/mlp_render_fea.py:44-68) with positional_encoding
+// (app/tools/utils.py:42-48): input = [feat, view, sin(feat 2^f), cos(feat 2^f), sin(view 2^f), cos(view 2^f)].
+//
+// fp32 network (mlp_mode 0): an fp32 number is EXACTLY the sum of three bf16 numbers (8 + 8 + 8 significand bits;
+// bf16 has the exponent range of fp32), x = h + m + l with |m| <= 2^-8 |x|, |l| <= 2^-16 |x| up to rounding.  A product
+// of two such sums needs six of the nine partial products, hh, hm, mh, mm, hl, lh: what is left out is below 2^-24 of
+// the product, i.e. below the rounding of one fp32 multiplication.  Partial products of 16-bit terms are exact, sums are
+// fp32 in tensor memory.  Biases, ReLU, the encodings (sincosf) and layer 3 are fp32 on the CUDA cores.
+//
+// Work split: one persistent CTA per SM, tiles of 128 samples (row = lane of tensor memory).  Two groups of 256 threads
+// (two per row) take alternate tiles and do the CUDA-core work; one warp issues every MMA.  Layer inputs travel in
+// CHUNKS of 32 columns (two K steps; in tensor memory 16 columns per term) through a ring of slots in tensor memory:
+// five chunks of layer 1, then four of layer 2, per tile.  A chunk's MMAs run as soon as its 8 warps have stored it, and
+// its slot is free when they have completed (tcgen05.commit), so the encoding of the next tile and the conversion of
+// layer 1's result into layer 2's input run beside the MMAs of earlier chunks.  The K order of layer 1 is
+// permuted so that each K step holds three values u with their sin u, sin 2u, cos u, cos 2u (and one zero): a thread
+// encodes three values, splits 16 numbers, and stores 8 columns per term.
+// Tensor memory: D1 (layer 1 result) [0, 128), D2 [128, 256), the ring [256, 512).  Shared memory: the weight images
+// (216 KB with three terms), biases, layer-3 weights.
+//
+// Every wait is bounded; when one runs out the CTA raises status[GNR_ST_WAIT_EXPIRED] and all its roles stop.
+#include <cuda_bf16.h>
+
+#include "gnr_tc.cuh"
+
+namespace {
+
+constexpr int GROUP = 256;                 // threads of a group (two per row)
+constexpr int THREADS = 2 * GROUP + 32;    // + the warp that issues MMAs
+constexpr int L1_CHUNKS = 5, L2_CHUNKS = 4, CHUNKS = L1_CHUNKS + L2_CHUNKS;
+constexpr int CHUNK_COLS = 16;             // tensor-memory columns of one term of a chunk (32 values)
+constexpr int RING_COL = 256;
+constexpr int W1S_BYTES = 160 * HID * 2, W2S_BYTES = HID * HID * 2;  // one term of a weight image
+
+struct SplitArgs {
+  GnrCoords crd;
+  const float* feat;             // [n][FEAT_STRIDE]
+  const unsigned char* w_image;  // [term][W1 image, permuted K][...], then [term][W2 image]
+  const float* w3;
+  const float* b1;
+  const float* b2;
+  const float* b3;
+  float* rgb_out;
+  int32_t* status;
+  int kbits;
+  uint32_t wait_limit;
+  int debug_skip_commit;         // test hook: CTA 0 leaves out the commit of its first layer-1 result
+};
+
+// TA x TW terms of activations and weights; partial products in the order they are issued.
+template <bool EXACT>
+struct Terms;
+template <>
+struct Terms<true> {
+  static constexpr int TA = 3, TW = 3, PRODUCTS = 6, SLOTS = 5;
+  static constexpr uint32_t kFormat = (1u << 7) | (1u << 10);  // A and B bf16
+  __device__ static constexpr int a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
+  __device__ static constexpr int w(int i) { return i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : i == 3 ? 0 : i == 4 ? 1 : 0; }
+};
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32"
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
+// Two fp32 numbers as three packed bf16 pairs that sum to them exactly (`a` in the low halves).
+__device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
+  return d;
+}
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pack_bf2(a, b);
+  a -= __uint_as_float(h << 16);
+  b -= __uint_as_float(h & 0xffff0000u);
+  m = pack_bf2(a, b);
+  a -= __uint_as_float(m << 16);
+  b -= __uint_as_float(m & 0xffff0000u);
+  l = pack_bf2(a, b);
+}
+
+// All lanes of a warp wait together (bounded); false if the wait ran out or another role gave up.
+__device__ __forceinline__ bool warp_wait(uint32_t mbar, uint32_t parity, volatile int* abort_flag, int32_t* status, uint32_t limit) {
+  bool ok = false;
+  for (uint32_t it = 0; it < limit; ++it) {
+    ok = mbar_try_wait(mbar, parity);
+    if (ok || *abort_flag) break;
+    if (it > 64) __nanosleep(64);
+  }
+  if (__all_sync(0xffffffffu, ok)) return true;
+  if ((threadIdx.x & 31) == 0) {
+    *abort_flag = 1;
+    atomicExch(status + GNR_ST_WAIT_EXPIRED, 1);
+  }
+  return false;
+}
+
+template <bool EXACT>
+__global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_constant__ SplitArgs a) {
+  using T = Terms<EXACT>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned char* s_w1 = smem;                                  // [TW][W1S_BYTES]
+  unsigned char* s_w2 = s_w1 + T::TW * W1S_BYTES;              // [TW][W2S_BYTES]
+  float* s_w3 = reinterpret_cast<float*>(s_w2 + T::TW * W2S_BYTES);  // [3][HID]
+  float* s_b1 = s_w3 + 3 * HID;
+  float* s_b2 = s_b1 + HID;
+  float* s_b3 = s_b2 + HID;                                    // [4]
+  float* s_part = s_b3 + 4;                                    // [2 groups][128][3] layer-3 sums of the second half of a row
+  uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_part + 2 * ROWS * 3);
+  enum { FULL = 0, EMPTY = T::SLOTS, D1_READY = 2 * T::SLOTS, D2_READY, D2_FREE, WEIGHTS, DRAIN, PART, N_BARS = PART + 2 };
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + N_BARS);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int lane = tid & 31;
+  const long long total = min(a.crd.total_ptr ? (long long)*a.crd.total_ptr : a.crd.total_direct, a.crd.capacity);
+  const long long n_tiles = (total + ROWS - 1) / ROWS;
+  if ((long long)blockIdx.x >= n_tiles) return;  // (the whole CTA)
+  const int my_tiles = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  const uint32_t bars = smem_u32(s_bar);
+  auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+
+  // ---- set-up: barriers, tensor memory; the weight images come in by bulk copies while the first tile is encoded ----
+  constexpr uint32_t kImage = T::TW * (W1S_BYTES + W2S_BYTES);
+  if (warp == 2 * GROUP / 32) {
+    if (lane == 0) {
+      for (int s = 0; s < T::SLOTS; ++s) {
+        mbar_init(bar(FULL + s), GROUP / 32);
+        mbar_init(bar(EMPTY + s), 1);
+      }
+      mbar_init(bar(D1_READY), 1);
+      mbar_init(bar(D2_READY), 1);
+      mbar_init(bar(D2_FREE), GROUP / 32);
+      mbar_init(bar(WEIGHTS), 1);
+      mbar_init(bar(DRAIN), 1);
+      for (int g = 0; g < 2; ++g) mbar_init(bar(PART + g), GROUP / 64);
+      *s_abort = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    if (lane == 0) {
+      mbar_expect_tx(bar(WEIGHTS), kImage);
+      for (uint32_t at = 0; at < kImage; at += 16384u)
+        bulk_load(smem_u32(smem) + at, a.w_image + at, min(16384u, kImage - at), bar(WEIGHTS));
+    }
+  } else {
+    for (int i = tid; i < 3 * HID; i += 2 * GROUP) s_w3[i] = a.w3[i];
+    if (tid < HID) {
+      s_b1[tid] = a.b1[tid];
+      s_b2[tid] = a.b2[tid];
+    }
+    if (tid < 4) s_b3[tid] = a.b3[tid];
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
+  const uint32_t d1 = tmem, d2 = tmem + HID, ring = tmem + RING_COL;
+
+  if (warp == 2 * GROUP / 32) {
+    // ---- the warp that issues MMAs: chunks strictly in order ---------------------------------------------------------
+    constexpr uint32_t kIdesc = kIdescHid | T::kFormat;
+    bool ok = warp_wait(bar(WEIGHTS), 0, s_abort, a.status, a.wait_limit);
+    const uint32_t w1 = smem_u32(s_w1), w2 = smem_u32(s_w2);
+    int q = 0;  // chunks taken so far
+    for (int n = 0; n < my_tiles && ok; ++n) {
+#pragma unroll 1
+      for (int layer = 0; layer < 2 && ok; ++layer) {
+        const int chunks = layer == 0 ? L1_CHUNKS : L2_CHUNKS;
+        const uint32_t d = layer == 0 ? d1 : d2, wb = layer == 0 ? w1 : w2, w_term = layer == 0 ? W1S_BYTES : W2S_BYTES;
+        auto products = [&](int i, int c, uint32_t leader) {
+          const uint32_t at = ring + (uint32_t)(((q + c) % T::SLOTS) * T::TA * CHUNK_COLS);
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+            mma_f16_ts(d, at + T::a(i) * CHUNK_COLS + ks * 8,
+                       make_desc(wb + T::w(i) * w_term + (uint32_t)(4 * c + 2 * ks) * KG_BYTES, KG_BYTES), kIdesc,
+                       (c > 0 || i > 0 || ks > 0) ? 1u : 0u, leader);
+        };
+#pragma unroll 1
+        for (int c = 0; c < chunks && ok; ++c) {  // everything but the leading products, chunk by chunk as they arrive
+          ok = warp_wait(bar(FULL + (q + c) % T::SLOTS), (uint32_t)((q + c) / T::SLOTS) & 1u, s_abort, a.status, a.wait_limit);
+          if (ok && c == 0 && layer == 1 && n > 0)  // layer 2 of the tile before must have been read out
+            ok = warp_wait(bar(D2_FREE), (uint32_t)(n - 1) & 1u, s_abort, a.status, a.wait_limit);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t leader = elect_one();
+#pragma unroll
+          for (int i = 0; i + 1 < T::PRODUCTS; ++i) products(i, c, leader);
+        }
+        if (!ok) break;
+        const uint32_t leader = elect_one();
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c) {  // the leading products
+          products(T::PRODUCTS - 1, c, leader);
+          mma_commit(bar(EMPTY + (q + c) % T::SLOTS), leader);
+        }
+        const bool skip = a.debug_skip_commit != 0 && blockIdx.x == 0 && n == 0 && layer == 0;
+        mma_commit(bar(layer == 0 ? D1_READY : D2_READY), skip ? 0u : leader);
+        __syncwarp();
+        q += chunks;
+      }
+    }
+    if (!ok) {
+      // stop: wait (bounded) until nothing of this CTA runs in the tensor pipe
+      mma_commit(bar(DRAIN), elect_one());
+      __syncwarp();
+      for (uint32_t it = 0; it < kWaitLimit && !mbar_try_wait(bar(DRAIN), 0); ++it) __nanosleep(64);
+    }
+  } else {
+    // ---- a group: tiles g, g + 2, ... of this CTA ----------------------------------------------------------------------
+    const int g = warp / (GROUP / 32), wg = warp % (GROUP / 32);
+    const int half = wg >> 2, row = ((wg & 3) << 5) | lane;
+    const uint32_t lane_off = (uint32_t)((wg & 3) * 32) << 16;
+    const uint32_t ring_half = ring + lane_off + (uint32_t)(half * 8);  // this thread's 8 of a chunk's 16 columns
+    float* part = s_part + (size_t)(g * ROWS + row) * 3;
+    bool ok = true;
+    // one chunk (16 numbers of this thread) -> its slot of the ring; q = number of the chunk in this CTA
+    auto put_chunk = [&](int q, const float (&x)[16]) -> bool {
+      const int slot = q % T::SLOTS, use = q / T::SLOTS;
+      uint32_t t[3][8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) split_pair(x[2 * e], x[2 * e + 1], t[0][e], t[1][e], t[2][e]);
+      if (use > 0 && !warp_wait(bar(EMPTY + slot), (uint32_t)(use - 1) & 1u, s_abort, a.status, a.wait_limit)) return false;
+      tc_fence_after();
+      const uint32_t at = ring_half + (uint32_t)(slot * T::TA * CHUNK_COLS);
+#pragma unroll
+      for (int i = 0; i < T::TA; ++i) tmem_st8(at + i * CHUNK_COLS, t[i]);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(FULL + slot));
+      return true;
+    };
+    for (int n = g; n < my_tiles && ok; n += 2) {
+      const long long j = ((long long)blockIdx.x + (long long)n * gridDim.x) * ROWS + row;
+      const bool live = j < total;
+      const long long js = live ? j : total - 1;
+      // this thread's 15 values: 6 c + 3 half + i for chunk c; the last three of half 1 are the view direction
+      float u[15];
+      const float* fr = a.feat + (size_t)js * FEAT_STRIDE + 3 * half;
+#pragma unroll
+      for (int c = 0; c < 5; ++c) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+          if (c < 4 || half == 0) u[3 * c + i] = __ldg(fr + 6 * c + i);
+      }
+      if (half == 1) {
+        const float* vsrc;
+        if (a.crd.view_direct) {
+          vsrc = a.crd.view_direct + (size_t)js * a.crd.point_stride;
+        } else {
+          const uint32_t ray = __ldg(a.crd.ids + (a.crd.index ? (long long)__ldg(a.crd.index + js) : js)) >> a.kbits;
+          vsrc = a.crd.rays + (size_t)ray * 6 + 3;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) u[12 + i] = __ldg(vsrc + i);
+      }
+      // ---- layer 1 input ------------------------------------------------------------------------------------------------
+#pragma unroll
+      for (int c = 0; c < L1_CHUNKS; ++c) {
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const float v = u[3 * c + i];
+          x[5 * i] = v;
+          sincosf(v, &x[5 * i + 1], &x[5 * i + 3]);
+          sincosf(2.0f * v, &x[5 * i + 2], &x[5 * i + 4]);
+        }
+        x[15] = 0.0f;
+        if (ok) ok = put_chunk(CHUNKS * n + c, x);
+      }
+      // ---- layer 2 input: relu(D1 + b1) ------------------------------------------------------------------------------------
+      if (ok) ok = warp_wait(bar(D1_READY), (uint32_t)n & 1u, s_abort, a.status, a.wait_limit);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < L2_CHUNKS; ++c) {
+        uint32_t v[16];
+        const int col = 32 * c + 16 * half;
+        tmem_ld16(d1 + lane_off + col, v);
+        tmem_ld_wait();
+        float x[16];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 b = *reinterpret_cast<const float4*>(s_b1 + col + 4 * q);
+          x[4 * q + 0] = fmaxf(__uint_as_float(v[4 * q + 0]) + b.x, 0.0f);
+          x[4 * q + 1] = fmaxf(__uint_as_float(v[4 * q + 1]) + b.y, 0.0f);
+          x[4 * q + 2] = fmaxf(__uint_as_float(v[4 * q + 2]) + b.z, 0.0f);
+          x[4 * q + 3] = fmaxf(__uint_as_float(v[4 * q + 3]) + b.w, 0.0f);
+        }
+        if (ok) ok = put_chunk(CHUNKS * n + L1_CHUNKS + c, x);
+      }
+      // ---- layer 3: rgb = sigmoid(W3 relu(D2 + b2) + b3), fp32; half h sums columns 64 h .. ------------------------------------
+      if (ok) ok = warp_wait(bar(D2_READY), (uint32_t)n & 1u, s_abort, a.status, a.wait_limit);
+      if (!ok) break;
+      tc_fence_after();
+      float2 p0 = make_float2(0.0f, 0.0f), p1 = p0, p2 = p0;
+#pragma unroll
+      for (int cb = 0; cb < 2; ++cb) {
+        uint32_t v[32];
+        const int col = 64 * half + 32 * cb;
+        tmem_ld32(d2 + lane_off + col, v);
+        tmem_ld_wait();
+        if (cb == 1) {  // the accumulator can be overwritten
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(D2_FREE));
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float4 b = *reinterpret_cast<const float4*>(s_b2 + col + 4 * q);
+          const float2 xa = make_float2(fmaxf(__uint_as_float(v[4 * q + 0]) + b.x, 0.0f), fmaxf(__uint_as_float(v[4 * q + 1]) + b.y, 0.0f));
+          const float2 xb = make_float2(fmaxf(__uint_as_float(v[4 * q + 2]) + b.z, 0.0f), fmaxf(__uint_as_float(v[4 * q + 3]) + b.w, 0.0f));
+          const float4 wr = *reinterpret_cast<const float4*>(s_w3 + col + 4 * q);
+          const float4 wg4 = *reinterpret_cast<const float4*>(s_w3 + HID + col + 4 * q);
+          const float4 wb4 = *reinterpret_cast<const float4*>(s_w3 + 2 * HID + col + 4 * q);
+          p0 = __ffma2_rn(xb, make_float2(wr.z, wr.w), __ffma2_rn(xa, make_float2(wr.x, wr.y), p0));
+          p1 = __ffma2_rn(xb, make_float2(wg4.z, wg4.w), __ffma2_rn(xa, make_float2(wg4.x, wg4.y), p1));
+          p2 = __ffma2_rn(xb, make_float2(wb4.z, wb4.w), __ffma2_rn(xa, make_float2(wb4.x, wb4.y), p2));
+        }
+      }
+      // (half 1 cannot overtake: its next sums follow MMAs that need half 0's next chunks, stored after the reads here)
+      if (half == 1) {
+        part[0] = p0.x + p0.y;
+        part[1] = p1.x + p1.y;
+        part[2] = p2.x + p2.y;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(PART + g));
+        continue;
+      }
+      ok = warp_wait(bar(PART + g), (uint32_t)(n >> 1) & 1u, s_abort, a.status, a.wait_limit);
+      if (ok && live) {
+        float* out = a.rgb_out + (size_t)j * 3;
+        out[0] = 1.0f / (1.0f + expf(-((p0.x + p0.y) + part[0] + s_b3[0])));
+        out[1] = 1.0f / (1.0f + expf(-((p1.x + p1.y) + part[1] + s_b3[1])));
+        out[2] = 1.0f / (1.0f + expf(-((p2.x + p2.y) + part[2] + s_b3[2])));
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2 * GROUP / 32) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+}
+
+// W [n_out][k_real] fp32 -> [term][k group][n_out][8] bf16 terms; position k of the operand takes column map[k] of W
+// (null: k itself), -1 = zero.
+__global__ void pack_split_image_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ img, int k_real, int k_groups,
+                                        int terms, bool permuted) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per (k group, n)
+  if (i >= k_groups * HID) return;
+  const int kg = i / HID, n = i - kg * HID;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int k = kg * 8 + e;
+    int col = k;
+    if (permuted) {
+      // K step s = k / 16 holds the values 3 s .. 3 s + 2 (features, then view), each as u, sin u, sin 2u, cos u, cos 2u
+      const int r = k & 15, v = 3 * (k >> 4) + r / 5, what = r % 5;
+      const bool view = v >= APP;
+      const int base_s = APP + 3, base_vs = base_s + 4 * APP;
+      const int sin0 = view ? base_vs + 2 * (v - APP) : base_s + 2 * v;
+      const int cos0 = sin0 + (view ? 6 : 2 * APP);
+      col = r == 15 ? -1 : what == 0 ? v : what <= 2 ? sin0 + what - 1 : cos0 + what - 3;
+    }
+    float x = (col >= 0 && col < k_real) ? w[(size_t)n * k_real + col] : 0.0f;
+    for (int t = 0; t < terms; ++t) {
+      const __nv_bfloat16 b = __float2bfloat16_rn(x);
+      img[(size_t)t * k_groups * HID * 8 + (size_t)i * 8 + e] = b;
+      x -= __bfloat162float(b);
+    }
+  }
+}
+
+template <bool EXACT>
+constexpr size_t split_smem() {
+  using T = Terms<EXACT>;
+  return (size_t)T::TW * (W1S_BYTES + W2S_BYTES) + (3 * HID + 2 * HID + 4 + 2 * ROWS * 3) * sizeof(float) + (2 * T::SLOTS + 7) * 8 + 16;
+}
+
+}  // namespace
+
+int gnr_mlp_split_usable(const GnrModel* m) {
+  const GnrConfig& c = m->cfg;
+  return c.mlp_mode == 0 && c.app_dim == APP && c.fea_pe == FPE && c.view_pe == VPE && c.hidden == HID;
+}
+
+int gnr_mlp_split_prepare(GnrModel* m, const float* w1, const float* w2, cudaStream_t st) {
+  using T = Terms<true>;
+  if (m->mlp.split_image == nullptr) GNR_CUDA_OK(cudaMalloc(&m->mlp.split_image, (size_t)T::TW * (W1S_BYTES + W2S_BYTES)));
+  __nv_bfloat16* img = reinterpret_cast<__nv_bfloat16*>(m->mlp.split_image);
+  pack_split_image_kernel<<<(20 * HID + 255) / 256, 256, 0, st>>>(w1, img, IN_DIM, 20, T::TW, true);
+  pack_split_image_kernel<<<(16 * HID + 255) / 256, 256, 0, st>>>(w2, img + (size_t)T::TW * W1S_BYTES / 2, HID, 16, T::TW, false);
+  GNR_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+int launch_mlp_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat,
+                     float* rgb, int32_t* status, cudaStream_t st) {
+  if (!m->mlp.split_image || feat_stride != FEAT_STRIDE) {
+    gnr_set_error("split MLP: weights were not prepared, or feature stride %d is not %d", feat_stride, FEAT_STRIDE);
+    return -1;
+  }
+  SplitArgs a;
+  a.crd = c;
+  a.feat = feat;
+  a.w_image = (const unsigned char*)m->mlp.split_image;
+  a.w3 = m->mlp.w3;
+  a.b1 = m->mlp.b1;
+  a.b2 = m->mlp.b2;
+  a.b3 = m->mlp.b3;
+  a.rgb_out = rgb;
+  a.status = status;
+  a.kbits = p.kbits;
+  a.wait_limit = m->debug_wait_limit > 0 ? (uint32_t)m->debug_wait_limit : kWaitLimit;
+  a.debug_skip_commit = m->debug_expire_wait;
+  constexpr size_t smem = split_smem<true>();
+  static_assert(smem <= 227 * 1024, "weights of the split MLP must fit shared memory");
+  cudaError_t e = cudaFuncSetAttribute(mlp_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  mlp_split_kernel<true><<<m->sm_count, THREADS, smem, st>>>(a);
+  return (int)cudaGetLastError();
+}

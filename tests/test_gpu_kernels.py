@@ -70,3 +70,55 @@ def test_appearance_list_overflow_is_reported():
     for n in (200, 4000, 10000):
         with pytest.raises(RuntimeError, match="appearance-sample list overflow"):
             model(rays[5000 - n // 2:5000 + n // 2].contiguous(), N_samples=spec.n_samples)
+
+
+def _network_fp64(sd, feats, view):
+    """MLPRender_Fea in fp64, and a bound on the error of an fp32 evaluation: every layer's sums may be off by
+    16 x 2^-24 of the sum of magnitudes (rounding of operands, encodings and bias, and ten accumulation steps at full
+    size), propagated through the layers; sigmoid has slope 1/4 at most and one rounding of its own."""
+    def pe(x):
+        p = (x[..., None] * torch.tensor([1.0, 2.0], dtype=torch.float64, device=x.device)).reshape(x.shape[0], -1)
+        return torch.cat([p.sin(), p.cos()], -1)
+
+    gamma = 16 * 2.0 ** -24
+    x = torch.cat([feats, view, pe(feats), pe(view)], -1)
+    err = torch.zeros_like(x)
+    for i in (0, 2, 4):
+        w, b = sd[f"renderModule.mlp.{i}.weight"], sd[f"renderModule.mlp.{i}.bias"]
+        err = err @ w.abs().T + gamma * (x.abs() @ w.abs().T + b.abs())
+        x = x @ w.T + b
+        if i < 4:
+            x = torch.relu(x)
+    return torch.sigmoid(x), 0.25 * err + 2.0 ** -24
+
+
+@pytest.mark.parametrize("n,scale", [(1, 0.02), (127, 0.02), (128, 1.0), (129, 0.02), (148 * 128 + 1, 5.0), (3 * 148 * 128 + 77, 0.3)])
+def test_fp32_network_on_tensor_cores(n, scale):
+    """The fp32 network as sums of bf16 terms, from given features: inside the error bound of an fp32 evaluation against
+    fp64 for partial tiles, one to four tiles per CTA, features from 0.02 to 5 (times a normal variable)."""
+    from landmark_b200.model_parallel import mlp_features
+
+    spec = scenes.tiny_spec(grid=32).lit()
+    ckpt = scenes.make_checkpoint(spec)
+    g = torch.Generator().manual_seed(n)
+    ckpt["state_dict"]["renderModule.mlp.4.bias"] = torch.randn(3, generator=g)
+    model = cuda_model(spec, ckpt)
+    feats = (torch.randn((n, 27), generator=g) * scale).cuda()
+    view = torch.randn((n, 3), generator=g).cuda()
+    rgb = mlp_features(model, feats, view)
+    ref, bound = _network_fp64({k: v.cuda().double() for k, v in ckpt["state_dict"].items()}, feats.double(), view.double())
+    worst = ((rgb.double() - ref).abs() / bound).max().item()
+    assert worst <= 1.0, f"error is {worst:.2f} of the bound"
+
+
+def test_fp32_network_wait_expires_and_the_context_survives():
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    rays = tiny_rays(spec).cuda()[4000:6000].contiguous()
+    good, _ = model(rays, N_samples=spec.n_samples)
+    model.debug_wait(expire=True, wait_limit=2000)
+    with pytest.raises(RuntimeError, match="bounded device-side wait expired"):
+        model(rays, N_samples=spec.n_samples)
+    model.debug_wait()
+    again, _ = model(rays, N_samples=spec.n_samples)
+    assert torch.equal(good["rgb_map"], again["rgb_map"])
