@@ -561,8 +561,13 @@ extern "C" int gnr_upload_mlp(GnrModel* m, const float* basis_w, const float* w1
   copy_or_zero_kernel<<<(Hd + 255) / 256, 256, 0, st>>>(b2, q.b2, Hd, Hd);
   copy_or_zero_kernel<<<1, 32, 0, st>>>(b3, q.b3, 3, 4);
   GNR_CUDA_OK(cudaGetLastError());
-  if (m->cfg.mlp_mode != 0) return gnr_mlp_tc_prepare(m, basis_w, w1, w2, w3, st);
-  if (gnr_mlp_split_usable(m)) return gnr_mlp_split_prepare(m, w1, w2, st);
+  if (m->cfg.mlp_mode == 2) return gnr_mlp_tc_prepare(m, basis_w, w1, w2, w3, st);
+  if (gnr_mlp_split_usable(m)) return gnr_mlp_split_prepare(m, basis_w, w1, w2, st);
+  if (m->cfg.mlp_mode != 0) {
+    gnr_set_error("tensor-core MLP supports app_dim 27, fea_pe 2, view_pe 2, featureC 128 (got %d, %d, %d, %d); use mlp_mode 0",
+                  m->cfg.app_dim, m->cfg.fea_pe, m->cfg.view_pe, m->cfg.hidden);
+    return -1;
+  }
   return 0;
 }
 
@@ -688,11 +693,9 @@ GnrWs gnr_ws_layout(const GnrModel* m, int64_t n, int S, int64_t max_valid, int6
   L.app_feat = take((size_t)max_app * L.feat_stride * 4);
   L.app_rgb = take((size_t)max_app * 3 * 4);
   if (gnr_tc_basis_fused(m)) {
-    const int terms = m->cfg.mlp_mode == 1 ? 2 : 1;
     const size_t tiles = (size_t)(max_app + 127) / 128;
     L.app_prod_tile = gnr_tc_tile_bytes(m);
-    L.app_prod_image = align_up(tiles * (size_t)L.app_prod_tile, 256);
-    L.app_prod = take(L.app_prod_image * terms);
+    L.app_prod = take(tiles * (size_t)L.app_prod_tile);
   }
   L.total = off;
   return L;
@@ -883,14 +886,18 @@ static int copy_out(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   return 0;
 }
 
+// projected features in fp32: gather + projection on the tensor cores where the model allows it, else on the CUDA cores
+static int launch_features(GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, float* feat, int32_t* status,
+                           cudaStream_t st) {
+  if (gnr_project_split_usable(m)) return launch_project_split(m, p, c, feat_stride, feat, status, st);
+  return launch_app_gather(m, p, c, feat_stride, feat, st);
+}
+
 static int run_app_gather(GnrModel* m, const GnrSampleParams& p, const float* rays, char* ws, const GnrWs& L, int lanes,
                           cudaStream_t st) {
   const GnrCoords c = gnr_coords_app(rays, ws, L, lanes);
-  if (gnr_tc_basis_fused(m)) {
-    unsigned char* hi = (unsigned char*)(ws + L.app_prod);
-    return launch_app_products(m, p, c, hi, hi + L.app_prod_image, L.app_prod_tile, m->cfg.mlp_mode == 1 ? 2 : 1, st);
-  }
-  return launch_app_gather(m, p, c, L.feat_stride, (float*)(ws + L.app_feat), st);
+  if (gnr_tc_basis_fused(m)) return launch_app_products(m, p, c, (unsigned char*)(ws + L.app_prod), L.app_prod_tile, st);
+  return launch_features(m, p, c, L.feat_stride, (float*)(ws + L.app_feat), (int32_t*)(ws + L.status), st);
 }
 
 static int run_mlp(GnrModel* m, const GnrSampleParams& p, const float* rays, char* ws, const GnrWs& L, int lanes,
@@ -900,8 +907,7 @@ static int run_mlp(GnrModel* m, const GnrSampleParams& p, const float* rays, cha
   float* rgb = (float*)(ws + L.app_rgb);
   if (gnr_mlp_split_usable(m)) return launch_mlp_split(m, p, c, L.feat_stride, feat, rgb, (int32_t*)(ws + L.status), st);
   if (m->cfg.mlp_mode == 0) return launch_mlp_simt(m, p, c, L.feat_stride, feat, rgb, st);
-  const unsigned char* hi = (const unsigned char*)(ws + L.app_prod);
-  return launch_mlp_tc(m, p, c, L.feat_stride, feat, write_features ? feat : nullptr, hi, hi + L.app_prod_image,
+  return launch_mlp_tc(m, p, c, L.feat_stride, feat, write_features ? feat : nullptr, (const unsigned char*)(ws + L.app_prod),
                        L.app_prod_tile, rgb, (int32_t*)(ws + L.status), 0, st);
 }
 
@@ -1159,8 +1165,8 @@ static GnrCoords coords_points(const float* xyz, const float* view, int64_t n, i
 }
 
 struct PointScratch {
-  size_t status, feat, prod, total, prod_image;
-  int tile_bytes, terms;
+  size_t status, feat, prod, total;
+  int tile_bytes;
 };
 
 static PointScratch point_scratch(const GnrModel* m, int64_t n) {
@@ -1171,12 +1177,10 @@ static PointScratch point_scratch(const GnrModel* m, int64_t n) {
   off = align_up(off + GNR_ST_WORDS * 4, 256);
   s.feat = off;
   off = align_up(off + (size_t)n * 28 * 4, 256);
-  if (m->cfg.mlp_mode != 0 && gnr_tc_basis_fused(m)) {
-    s.terms = m->cfg.mlp_mode == 1 ? 2 : 1;
+  if (gnr_tc_basis_fused(m)) {
     s.tile_bytes = gnr_tc_tile_bytes(m);
-    s.prod_image = align_up((size_t)((n + 127) / 128) * s.tile_bytes, 256);
     s.prod = off;
-    off += s.prod_image * s.terms;
+    off += align_up((size_t)((n + 127) / 128) * s.tile_bytes, 256);
   }
   s.total = off;
   return s;
@@ -1237,9 +1241,8 @@ static int mlp_points(GnrModel* m, const GnrSampleParams& p, const GnrCoords& c,
   } else if (m->cfg.mlp_mode == 0) {
     GNR_LAUNCH_OK(launch_mlp_simt(m, p, c, 28, feat, rgb, st));
   } else {
-    const unsigned char* hi = (const unsigned char*)(sc + S.prod);
-    GNR_LAUNCH_OK(launch_mlp_tc(m, p, c, 28, feat, (fused && feat_copy) ? feat : nullptr, hi, hi + S.prod_image, S.tile_bytes, rgb,
-                                (int32_t*)(sc + S.status), fused ? 0 : 1, st));
+    GNR_LAUNCH_OK(launch_mlp_tc(m, p, c, 28, feat, (fused && feat_copy) ? feat : nullptr, (const unsigned char*)(sc + S.prod),
+                                S.tile_bytes, rgb, (int32_t*)(sc + S.status), fused ? 0 : 1, st));
   }
   if (feat_copy) {
     GNR_CUDA_OK(cudaMemcpy2DAsync(feat_copy, (size_t)m->cfg.app_dim * 4, feat, 28 * 4, (size_t)m->cfg.app_dim * 4,
@@ -1288,12 +1291,11 @@ static int appearance_points_impl(GnrModel* m, const GnrCoords& c, int64_t n, vo
     GNR_LAUNCH_OK(launch_app_mlp_fused(m, p, c, rgb, (int32_t*)(sc + S.status), st));
     return 0;
   }
-  const int fused = m->cfg.mlp_mode != 0 && gnr_tc_basis_fused(m);
+  const int fused = gnr_tc_basis_fused(m);
   if (fused) {
-    unsigned char* hi = (unsigned char*)(sc + S.prod);
-    GNR_LAUNCH_OK(launch_app_products(m, p, c, hi, hi + S.prod_image, S.tile_bytes, S.terms, st));
+    GNR_LAUNCH_OK(launch_app_products(m, p, c, (unsigned char*)(sc + S.prod), S.tile_bytes, st));
   } else {
-    GNR_LAUNCH_OK(launch_app_gather(m, p, c, 28, (float*)(sc + S.feat), st));
+    GNR_LAUNCH_OK(launch_features(m, p, c, 28, (float*)(sc + S.feat), (int32_t*)(sc + S.status), st));
   }
   return mlp_points(m, p, c, sc, S, fused, features, rgb, st);
 }
@@ -1314,15 +1316,14 @@ extern "C" int gnr_app_features_points(GnrModel* m, const float* xyz, int64_t n,
   GnrSampleParams p = gnr_sample_params(m, 1);
   const GnrCoords c = coords_points(xyz, nullptr, n);
   float* feat = (float*)(sc + S.feat);
-  if (m->cfg.mlp_mode != 0 && gnr_tc_basis_fused(m)) {
+  GNR_CUDA_OK(cudaMemsetAsync(sc + S.status, 0, GNR_ST_WORDS * 4, st));
+  if (gnr_tc_basis_fused(m)) {
     // product tiles, then the projection alone on the tensor cores (fp32 accumulate)
-    GNR_CUDA_OK(cudaMemsetAsync(sc + S.status, 0, GNR_ST_WORDS * 4, st));
-    unsigned char* hi = (unsigned char*)(sc + S.prod);
-    GNR_LAUNCH_OK(launch_app_products(m, p, c, hi, hi + S.prod_image, S.tile_bytes, S.terms, st));
-    GNR_LAUNCH_OK(launch_mlp_tc(m, p, c, 28, nullptr, feat, hi, hi + S.prod_image, S.tile_bytes, nullptr, (int32_t*)(sc + S.status), 0, st,
-                                /*basis_only=*/1));
+    unsigned char* prod = (unsigned char*)(sc + S.prod);
+    GNR_LAUNCH_OK(launch_app_products(m, p, c, prod, S.tile_bytes, st));
+    GNR_LAUNCH_OK(launch_mlp_tc(m, p, c, 28, nullptr, feat, prod, S.tile_bytes, nullptr, (int32_t*)(sc + S.status), 0, st, /*basis_only=*/1));
   } else {
-    GNR_LAUNCH_OK(launch_app_gather(m, p, c, 28, feat, st));
+    GNR_LAUNCH_OK(launch_features(m, p, c, 28, feat, (int32_t*)(sc + S.status), st));
   }
   GNR_CUDA_OK(cudaMemcpy2DAsync(features, (size_t)m->cfg.app_dim * 4, feat, 28 * 4, (size_t)m->cfg.app_dim * 4, (size_t)n,
                                 cudaMemcpyDeviceToDevice, st));
@@ -1604,12 +1605,12 @@ extern "C" int gnr_app_features(GnrModel* m, const float* rays, int64_t n, int S
   const GnrCoords c = gnr_coords_app(rays, ws, L);
   if (gnr_tc_basis_fused(m)) {
     // tensor-core path: fp16 product tiles, then the projection alone (tcgen05, fp32 accumulate)
-    unsigned char* hi = (unsigned char*)(ws + L.app_prod);
-    GNR_LAUNCH_OK(launch_app_products(m, p, c, hi, hi + L.app_prod_image, L.app_prod_tile, m->cfg.mlp_mode == 1 ? 2 : 1, st));
-    GNR_LAUNCH_OK(launch_mlp_tc(m, p, c, L.feat_stride, nullptr, (float*)(ws + L.app_feat), hi, hi + L.app_prod_image,
-                                L.app_prod_tile, (float*)(ws + L.app_rgb), (int32_t*)(ws + L.status), 0, st, /*basis_only=*/1));
+    unsigned char* prod = (unsigned char*)(ws + L.app_prod);
+    GNR_LAUNCH_OK(launch_app_products(m, p, c, prod, L.app_prod_tile, st));
+    GNR_LAUNCH_OK(launch_mlp_tc(m, p, c, L.feat_stride, nullptr, (float*)(ws + L.app_feat), prod, L.app_prod_tile,
+                                (float*)(ws + L.app_rgb), (int32_t*)(ws + L.status), 0, st, /*basis_only=*/1));
   } else {
-    GNR_LAUNCH_OK(launch_app_gather(m, p, c, L.feat_stride, (float*)(ws + L.app_feat), st));
+    GNR_LAUNCH_OK(launch_features(m, p, c, L.feat_stride, (float*)(ws + L.app_feat), (int32_t*)(ws + L.status), st));
   }
   GNR_CUDA_OK(cudaMemcpy2DAsync(features, (size_t)m->cfg.app_dim * 4, ws + L.app_feat, (size_t)L.feat_stride * 4,
                                 (size_t)m->cfg.app_dim * 4, (size_t)rows, cudaMemcpyDeviceToDevice, st));

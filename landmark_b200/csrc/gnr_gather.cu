@@ -696,15 +696,14 @@ app_gather_kernel(GnrSampleParams p, PlaneSet planes, GnrCoords crd, const float
 // K dimension of the basis projection, so they are written as fp16 straight into the MMA
 // operand layout of their 128-sample tile: element (row r, k) of tile t at byte
 //   t * tile_bytes + (k / 8) * 2048 + r * 16 + (k % 8) * 2,     k = pair * C + channel.
-// With TA == 2 the fp16 rounding residual goes to a second image of the same shape.
 // One more 16-byte group per row, after the products (k group `view_group`), carries the
 // sample's view direction for the MLP kernel as fp16 pairs {hi x, hi y, hi z, lo x, lo y, lo z}:
 // hi + lo restores the fp32 value to about 2^-22, and the MLP kernel needs no list lookups.
 // (fp32 planes only; fp16 storage goes through app_products_thread_kernel.)
-template <int J, int NP, int TA>
+template <int J, int NP>
 __global__ void __launch_bounds__(kBlock)
-app_products_kernel(GnrSampleParams p, PlaneSet planes, GnrCoords crd, unsigned char* __restrict__ prod_hi,
-                    unsigned char* __restrict__ prod_lo, int tile_bytes, int view_group) {
+app_products_kernel(GnrSampleParams p, PlaneSet planes, GnrCoords crd, unsigned char* __restrict__ prod_hi, int tile_bytes,
+                    int view_group) {
   const int c4 = threadIdx.x & 3;
   const long long total = coords_total(crd);
   long long range_beg, range_end;
@@ -738,79 +737,16 @@ app_products_kernel(GnrSampleParams p, PlaneSet planes, GnrCoords crd, unsigned 
         hv.x = *reinterpret_cast<const uint32_t*>(&h0);
         hv.y = *reinterpret_cast<const uint32_t*>(&h1);
         *reinterpret_cast<uint2*>(prod_hi + at) = hv;
-        if (TA == 2) {
-          const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-          const __half2 l0 = __floats2half2_rn(prod[j].x - f0.x, prod[j].y - f0.y);
-          const __half2 l1 = __floats2half2_rn(prod[j].z - f1.x, prod[j].w - f1.y);
-          uint2 lv;
-          lv.x = *reinterpret_cast<const uint32_t*>(&l0);
-          lv.y = *reinterpret_cast<const uint32_t*>(&l1);
-          *reinterpret_cast<uint2*>(prod_lo + at) = lv;
-        }
       }
     });
   }
 }
 
-// The same for 48 channels with one thread per sample.  Consecutive list entries are samples of
+// The same for 48 channels from fp16 storage, one thread per sample.  Consecutive list entries are samples of
 // neighbouring rays at the same rank (see the order of the appearance list), so the 32 lanes of a
 // load read a few texels between them, and their rows in the tile are consecutive: every store
-// instruction writes 512 contiguous bytes.  With fp32 storage a thread takes the 48 channels of a
-// pair in six rounds of 8: six 256-bit loads, the fp32 interpolation and product of
-// pair_products_tap, and one 16-byte store, which is exactly one k group of its row (fp16 storage:
-// pair_products_thread48_h2 below).
+// instruction writes 512 contiguous bytes.
 constexpr int kThreadBlock = 128;
-
-template <bool HALF>
-__device__ __forceinline__ void load8(const void* base, uint32_t texel, int h, float4& lo, float4& hi) {
-  if constexpr (HALF) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(base) + (size_t)texel * 96u) + h);
-    const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&a.x)), a1 = __half22float2(*reinterpret_cast<const __half2*>(&a.y));
-    const float2 a2 = __half22float2(*reinterpret_cast<const __half2*>(&a.z)), a3 = __half22float2(*reinterpret_cast<const __half2*>(&a.w));
-    lo = make_float4(a0.x, a0.y, a1.x, a1.y);
-    hi = make_float4(a2.x, a2.y, a3.x, a3.y);
-  } else {
-    const F8 v = ldg8(reinterpret_cast<const float*>(base) + (size_t)texel * 48u + 8 * h);
-    lo = v.lo;
-    hi = v.hi;
-  }
-}
-
-template <bool HALF>
-__device__ __forceinline__ void pair_products_thread48(const GnrPlane& pl, Tap tx, Tap ty, Tap tl, unsigned char* out) {
-  const float ax1 = tx.f1, ay1 = ty.f1, al1 = tl.f1;
-  const float ax0 = 1.0f - ax1, ay0 = 1.0f - ay1, al0 = 1.0f - al1;
-  const float w_nw = ax0 * ay0, w_ne = ax1 * ay0, w_sw = ax0 * ay1, w_se = ax1 * ay1;
-  const uint32_t nw = (uint32_t)ty.i0 * (uint32_t)pl.W + (uint32_t)tx.i0, sw = nw + (uint32_t)pl.W;
-  const uint32_t seg = (uint32_t)tl.i0;
-#pragma unroll
-  for (int h = 0; h < 6; ++h) {
-    float4 nwl, nwh, nel, neh, swl, swh, sel, seh, l0l, l0h, l1l, l1h;
-    load8<HALF>(pl.plane, nw, h, nwl, nwh);
-    load8<HALF>(pl.plane, nw + 1u, h, nel, neh);
-    load8<HALF>(pl.plane, sw, h, swl, swh);
-    load8<HALF>(pl.plane, sw + 1u, h, sel, seh);
-    load8<HALF>(pl.line, seg, h, l0l, l0h);
-    load8<HALF>(pl.line, seg + 1u, h, l1l, l1h);
-    float4 pa = f4_scale(nwl, w_nw), pb = f4_scale(nwh, w_nw);
-    pa = f4_fma(nel, w_ne, pa);
-    pb = f4_fma(neh, w_ne, pb);
-    pa = f4_fma(swl, w_sw, pa);
-    pb = f4_fma(swh, w_sw, pb);
-    pa = f4_fma(sel, w_se, pa);
-    pb = f4_fma(seh, w_se, pb);
-    const float4 la = f4_fma(l1l, al1, f4_scale(l0l, al0)), lb = f4_fma(l1h, al1, f4_scale(l0h, al0));
-    const float4 qa = f4_mul(pa, la), qb = f4_mul(pb, lb);
-    const __half2 h0 = __floats2half2_rn(qa.x, qa.y), h1 = __floats2half2_rn(qa.z, qa.w);
-    const __half2 h2 = __floats2half2_rn(qb.x, qb.y), h3 = __floats2half2_rn(qb.z, qb.w);
-    uint4 v;
-    v.x = *reinterpret_cast<const uint32_t*>(&h0);
-    v.y = *reinterpret_cast<const uint32_t*>(&h1);
-    v.z = *reinterpret_cast<const uint32_t*>(&h2);
-    v.w = *reinterpret_cast<const uint32_t*>(&h3);
-    *reinterpret_cast<uint4*>(out + (size_t)h * 2048) = v;
-  }
-}
 
 __device__ __forceinline__ void pair_products_thread48_h2(const GnrPlane& pl, Tap tx, Tap ty, Tap tl, unsigned char* out) {
   const PairTapsH2 t = make_pair_taps_h2(pl, tx, ty, tl);
@@ -823,7 +759,7 @@ __device__ __forceinline__ void pair_products_thread48_h2(const GnrPlane& pl, Ta
   }
 }
 
-template <int NP, bool HALF>
+template <int NP>
 __global__ void __launch_bounds__(kThreadBlock, 4)
 app_products_thread_kernel(GnrSampleParams p, PlaneSet planes, GnrCoords crd, unsigned char* __restrict__ prod_hi,
                            int tile_bytes, int view_group) {
@@ -853,22 +789,15 @@ app_products_thread_kernel(GnrSampleParams p, PlaneSet planes, GnrCoords crd, un
       const Tap tx = make_tap(x, planes.p[0].fw, planes.p[0].W);
       const Tap ty = make_tap(y, planes.p[0].fh, planes.p[0].H);
       const Tap tz = make_tap(z, planes.p[0].fl, planes.p[0].L);
-      if constexpr (HALF) {
-        pair_products_thread48_h2(planes.p[0], tx, ty, tz, row);
-        pair_products_thread48_h2(planes.p[1], tx, tz, ty, row + 6 * 2048);
-        pair_products_thread48_h2(planes.p[2], ty, tz, tx, row + 12 * 2048);
-      } else {
-        pair_products_thread48<HALF>(planes.p[0], tx, ty, tz, row);
-        pair_products_thread48<HALF>(planes.p[1], tx, tz, ty, row + 6 * 2048);
-        pair_products_thread48<HALF>(planes.p[2], ty, tz, tx, row + 12 * 2048);
-      }
+      pair_products_thread48_h2(planes.p[0], tx, ty, tz, row);
+      pair_products_thread48_h2(planes.p[1], tx, tz, ty, row + 6 * 2048);
+      pair_products_thread48_h2(planes.p[2], ty, tz, tx, row + 12 * 2048);
     } else {
       for (int pi = 0; pi < planes.n; ++pi) {
         const GnrPlane& pl = planes.p[pi];
         const float u = pick(x, y, z, pl.mat0), v = pick(x, y, z, pl.mat1), l = pick(x, y, z, pl.vec);
         const Tap tu = make_tap(u, pl.fw, pl.W), tv = make_tap(v, pl.fh, pl.H), tl = make_tap(l, pl.fl, pl.L);
-        if constexpr (HALF) pair_products_thread48_h2(pl, tu, tv, tl, row + (size_t)pi * 6 * 2048);
-        else pair_products_thread48<HALF>(pl, tu, tv, tl, row + (size_t)pi * 6 * 2048);
+        pair_products_thread48_h2(pl, tu, tv, tl, row + (size_t)pi * 6 * 2048);
       }
     }
   }
@@ -1110,36 +1039,31 @@ int launch_app_gather(const GnrModel* m, const GnrSampleParams& p, const GnrCoor
   return (int)cudaGetLastError();
 }
 
-int launch_app_products(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, unsigned char* hi,
-                        unsigned char* lo, int tile_bytes, int terms, cudaStream_t st) {
+int launch_app_products(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, unsigned char* prod, int tile_bytes,
+                        cudaStream_t st) {
   PlaneSet set = make_set(m->app, m->cfg.n_pairs);
   const int J = m->app[0].C / 16;
   const int grid = m->sm_count * 4;
-#define GNR_PRD(JJ, NPP, TT) app_products_kernel<JJ, NPP, TT><<<grid, kBlock, 0, st>>>(p, set, c, hi, lo, tile_bytes, m->mlp.n_prod / 8)
-  if (m->cfg.app_storage == 1 && (J != 3 || terms != 1)) {
-    gnr_set_error("fp16 appearance planes need 48 (padded) channels and mlp_mode 2");
-    return -1;
-  }
-  if (J == 3 && terms == 1 && m->cfg.app_storage == 1) {
+  const bool vm3 = standard_vm3(set);
+#define GNR_PRD(JJ, NPP) app_products_kernel<JJ, NPP><<<grid, kBlock, 0, st>>>(p, set, c, prod, tile_bytes, m->mlp.n_prod / 8)
+  if (m->cfg.app_storage == 1) {
     // fp16 storage: one thread per sample; fp32 storage below: four lanes per sample, which the L1
     // serves better when every load instruction moves 16 bytes per lane
+    if (J != 3) {
+      gnr_set_error("fp16 appearance planes need 48 (padded) channels and mlp_mode 2");
+      return -1;
+    }
     const int tgrid = m->sm_count * 8;
-    const bool vm3 = standard_vm3(set), half = m->cfg.app_storage == 1;
-#define GNR_PRT(NPP, HH) \
-  app_products_thread_kernel<NPP, HH><<<tgrid, kThreadBlock, 0, st>>>(p, set, c, hi, tile_bytes, m->mlp.n_prod / 8)
-    if (vm3 && half) GNR_PRT(3, true);
-    else if (vm3) GNR_PRT(3, false);
-    else if (half) GNR_PRT(0, true);
-    else GNR_PRT(0, false);
-#undef GNR_PRT
-  } else if (J == 3 && standard_vm3(set)) {
-    if (terms == 2) GNR_PRD(3, 3, 2); else GNR_PRD(3, 3, 1);
+    if (vm3) app_products_thread_kernel<3><<<tgrid, kThreadBlock, 0, st>>>(p, set, c, prod, tile_bytes, m->mlp.n_prod / 8);
+    else app_products_thread_kernel<0><<<tgrid, kThreadBlock, 0, st>>>(p, set, c, prod, tile_bytes, m->mlp.n_prod / 8);
+  } else if (J == 3 && vm3) {
+    GNR_PRD(3, 3);
   } else if (J == 1) {
-    if (terms == 2) GNR_PRD(1, 0, 2); else GNR_PRD(1, 0, 1);
+    GNR_PRD(1, 0);
   } else if (J == 2) {
-    if (terms == 2) GNR_PRD(2, 0, 2); else GNR_PRD(2, 0, 1);
+    GNR_PRD(2, 0);
   } else if (J == 3) {
-    if (terms == 2) GNR_PRD(3, 0, 2); else GNR_PRD(3, 0, 1);
+    GNR_PRD(3, 0);
   } else {
     gnr_set_error("appearance channels (padded) %d not supported by the tensor-core path", m->app[0].C);
     return -1;

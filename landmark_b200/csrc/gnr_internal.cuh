@@ -33,7 +33,8 @@ struct GnrMlp {
   // tensor-core images (pre-tiled, see gnr_mlp_tc.cu)
   void* tc_image;
   size_t tc_image_bytes;
-  void* split_image;  // weights as sums of bf16 terms (gnr_mlp_split.cu), mlp_mode 0
+  void* split_image;  // weights as sums of 16-bit terms (gnr_mlp_split.cu), mlp_mode 0 and 1
+  void* split_basis;  // the basis projection's part of it
   int in_dim;   // 150
   int k1_pad;   // in_dim rounded up to 8
   int n_prod;   // sum of padded appearance channels (144)
@@ -118,8 +119,7 @@ struct GnrSampleParams {
 struct GnrWs {
   size_t status, t_min, words, counts, offsets, block_sums, ids, sigma_feat, sigma, weight, acc, depth,
       app_counts, app_offsets, app_index, app_ids, app_weight, app_feat, app_rgb, app_prod, total;
-  size_t app_prod_image;  // bytes of one fp16 product image (hi), 0 if the tensor-core path is off
-  int app_prod_tile;      // bytes of one 128-sample tile of that image
+  int app_prod_tile;      // bytes of one 128-sample tile of fp16 products (mlp_mode 2), 0 if there are none
   int feat_stride;  // floats per appearance feature row (app_dim rounded up to 4)
   long long max_valid, max_app;  // capacities of the two compacted lists
   long long n_rays;
@@ -189,8 +189,8 @@ int launch_march(const GnrModel* m, const GnrSampleParams& p, const float* rays,
                  cudaStream_t st, int list_only = 0, int lanes = 0);
 int launch_app_gather(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, float* feat,
                       cudaStream_t st);
-int launch_app_products(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, unsigned char* prod_hi,
-                        unsigned char* prod_lo, int tile_bytes, int terms, cudaStream_t st);
+int launch_app_products(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, unsigned char* prod, int tile_bytes,
+                        cudaStream_t st);
 // gather + basis + MLP in one kernel (gnr_app_fused.cu): 1 if this model can run it
 int gnr_app_fusable(const GnrModel* m);
 // the same work with dedicated gather warps feeding the MLP warps through tensor memory (gnr_app_stream.cu)
@@ -206,7 +206,7 @@ int launch_app_slice_project(const GnrModel* m, const float* xyz, int stride, in
 int launch_sum_partials(const void* parts_h, int n_parts, int64_t rows, int64_t part_stride_rows, int n_out, int out_stride,
                         float* out, cudaStream_t st);
 void gnr_fused_k1_order(int* map);  // K order of the fused kernel's layer-1 operand (160 entries)
-int gnr_tc_basis_fused(const GnrModel* m);  // 1 if the tensor-core path also runs the basis projection
+int gnr_tc_basis_fused(const GnrModel* m);  // 1 if mlp_mode 2's network kernel also runs the basis projection
 int gnr_tc_tile_bytes(const GnrModel* m);   // bytes of one 128-sample product tile (products + the view group)
 // (`mode` 0: rows of block-local points; 1: points + view directions; 2: 32-bit ids, (ray_base + ray) << kbits | sample)
 int launch_route_blocks(GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int px, int py, int mode, float* send,
@@ -215,15 +215,19 @@ int launch_positions(const GnrModel* m, const GnrSampleParams& p, const GnrCoord
                      cudaStream_t st);
 int launch_mlp_simt(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat,
                     float* rgb, cudaStream_t st);
-// the fp32 network on the tensor cores (gnr_mlp_split.cu): 1 if this model's layer sizes are the ones it is built for
+// mlp_mode 0 and 1 on the tensor cores with operands as sums of 16-bit terms: the network (gnr_mlp_split.cu; 1 if this
+// model's layer sizes are the ones it is built for) and gather + projection from fp32 planes (gnr_project_split.cu)
 int gnr_mlp_split_usable(const GnrModel* m);
-int gnr_mlp_split_prepare(GnrModel* m, const float* w1, const float* w2, cudaStream_t st);
+int gnr_mlp_split_prepare(GnrModel* m, const float* basis_w, const float* w1, const float* w2, cudaStream_t st);
+int gnr_project_split_usable(const GnrModel* m);
+int launch_project_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, float* feat,
+                         int32_t* status, cudaStream_t st);
 int launch_mlp_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat,
                      float* rgb, int32_t* status, cudaStream_t st);
 // feat_in: features for the non-fused variant; feat_out: optional copy of the projected features
 // (fused variant); prod_*: product tiles (fused variant); status: 8-word block for the wait flag.
 int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat_in,
-                  float* feat_out, const unsigned char* prod_hi, const unsigned char* prod_lo, int tile_bytes, float* rgb,
+                  float* feat_out, const unsigned char* prod, int tile_bytes, float* rgb,
                   int32_t* status, int force_unfused, cudaStream_t st, int basis_only = 0);
 int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const GnrWs& L, float* rgb_map,
                      float* depth_map, cudaStream_t st, int march_lanes = 0);

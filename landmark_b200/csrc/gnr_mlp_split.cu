@@ -3,11 +3,8 @@
 // MLPRender_Fea.forward (app/models/mlp_render_fea.py:44-68) with positional_encoding
 // (app/tools/utils.py:42-48): input = [feat, view, sin(feat 2^f), cos(feat 2^f), sin(view 2^f), cos(view 2^f)].
 //
-// fp32 network (mlp_mode 0): an fp32 number is EXACTLY the sum of three bf16 numbers (8 + 8 + 8 significand bits;
-// bf16 has the exponent range of fp32), x = h + m + l with |m| <= 2^-8 |x|, |l| <= 2^-16 |x| up to rounding.  A product
-// of two such sums needs six of the nine partial products, hh, hm, mh, mm, hl, lh: what is left out is below 2^-24 of
-// the product, i.e. below the rounding of one fp32 multiplication.  Partial products of 16-bit terms are exact, sums are
-// fp32 in tensor memory.  Biases, ReLU, the encodings (sincosf) and layer 3 are fp32 on the CUDA cores.
+// mlp_mode 0: the fp32 network, operands as exact sums of three bf16 terms; mlp_mode 1: activations as fp16 hi + lo (see
+// gnr_split.cuh).  Biases, ReLU, the encodings and layer 3 are fp32 on the CUDA cores.
 //
 // Work split: one persistent CTA per SM, tiles of 128 samples (row = lane of tensor memory).  Two groups of 256 threads
 // (two per row) take alternate tiles and do the CUDA-core work; one warp issues every MMA.  Layer inputs travel in
@@ -21,9 +18,7 @@
 // (216 KB with three terms), biases, layer-3 weights.
 //
 // Every wait is bounded; when one runs out the CTA raises status[GNR_ST_WAIT_EXPIRED] and all its roles stop.
-#include <cuda_bf16.h>
-
-#include "gnr_tc.cuh"
+#include "gnr_split.cuh"
 
 namespace {
 
@@ -32,6 +27,7 @@ constexpr int THREADS = 2 * GROUP + 32;    // + the warp that issues MMAs
 constexpr int L1_CHUNKS = 5, L2_CHUNKS = 4, CHUNKS = L1_CHUNKS + L2_CHUNKS;
 constexpr int CHUNK_COLS = 16;             // tensor-memory columns of one term of a chunk (32 values)
 constexpr int RING_COL = 256;
+constexpr int SLOTS = 5;
 constexpr int W1S_BYTES = 160 * HID * 2, W2S_BYTES = HID * HID * 2;  // one term of a weight image
 
 struct SplitArgs {
@@ -49,67 +45,9 @@ struct SplitArgs {
   int debug_skip_commit;         // test hook: CTA 0 leaves out the commit of its first layer-1 result
 };
 
-// TA x TW terms of activations and weights; partial products in the order they are issued.
-template <bool EXACT>
-struct Terms;
-template <>
-struct Terms<true> {
-  static constexpr int TA = 3, TW = 3, PRODUCTS = 6, SLOTS = 5;
-  static constexpr uint32_t kFormat = (1u << 7) | (1u << 10);  // A and B bf16
-  __device__ static constexpr int a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
-  __device__ static constexpr int w(int i) { return i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : i == 3 ? 0 : i == 4 ? 1 : 0; }
-};
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32"
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-
-// Two fp32 numbers as three packed bf16 pairs that sum to them exactly (`a` in the low halves).
-__device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
-  uint32_t d;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
-  return d;
-}
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-  h = pack_bf2(a, b);
-  a -= __uint_as_float(h << 16);
-  b -= __uint_as_float(h & 0xffff0000u);
-  m = pack_bf2(a, b);
-  a -= __uint_as_float(m << 16);
-  b -= __uint_as_float(m & 0xffff0000u);
-  l = pack_bf2(a, b);
-}
-
-// All lanes of a warp wait together (bounded); false if the wait ran out or another role gave up.
-__device__ __forceinline__ bool warp_wait(uint32_t mbar, uint32_t parity, volatile int* abort_flag, int32_t* status, uint32_t limit) {
-  bool ok = false;
-  for (uint32_t it = 0; it < limit; ++it) {
-    ok = mbar_try_wait(mbar, parity);
-    if (ok || *abort_flag) break;
-    if (it > 64) __nanosleep(64);
-  }
-  if (__all_sync(0xffffffffu, ok)) return true;
-  if ((threadIdx.x & 31) == 0) {
-    *abort_flag = 1;
-    atomicExch(status + GNR_ST_WAIT_EXPIRED, 1);
-  }
-  return false;
-}
-
-template <bool EXACT>
+template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_constant__ SplitArgs a) {
-  using T = Terms<EXACT>;
+  using T = Split<MODE>;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* s_w1 = smem;                                  // [TW][W1S_BYTES]
   unsigned char* s_w2 = s_w1 + T::TW * W1S_BYTES;              // [TW][W2S_BYTES]
@@ -119,7 +57,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   float* s_b3 = s_b2 + HID;                                    // [4]
   float* s_part = s_b3 + 4;                                    // [2 groups][128][3] layer-3 sums of the second half of a row
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_part + 2 * ROWS * 3);
-  enum { FULL = 0, EMPTY = T::SLOTS, D1_READY = 2 * T::SLOTS, D2_READY, D2_FREE, WEIGHTS, DRAIN, PART, N_BARS = PART + 2 };
+  enum { FULL = 0, EMPTY = SLOTS, D1_READY = 2 * SLOTS, D2_READY, D2_FREE, WEIGHTS, DRAIN, PART, N_BARS = PART + 2 };
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + N_BARS);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
 
@@ -137,7 +75,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   constexpr uint32_t kImage = T::TW * (W1S_BYTES + W2S_BYTES);
   if (warp == 2 * GROUP / 32) {
     if (lane == 0) {
-      for (int s = 0; s < T::SLOTS; ++s) {
+      for (int s = 0; s < SLOTS; ++s) {
         mbar_init(bar(FULL + s), GROUP / 32);
         mbar_init(bar(EMPTY + s), 1);
       }
@@ -184,7 +122,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
         const int chunks = layer == 0 ? L1_CHUNKS : L2_CHUNKS;
         const uint32_t d = layer == 0 ? d1 : d2, wb = layer == 0 ? w1 : w2, w_term = layer == 0 ? W1S_BYTES : W2S_BYTES;
         auto products = [&](int i, int c, uint32_t leader) {
-          const uint32_t at = ring + (uint32_t)(((q + c) % T::SLOTS) * T::TA * CHUNK_COLS);
+          const uint32_t at = ring + (uint32_t)(((q + c) % SLOTS) * T::TA * CHUNK_COLS);
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks)
             mma_f16_ts(d, at + T::a(i) * CHUNK_COLS + ks * 8,
@@ -193,7 +131,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
         };
 #pragma unroll 1
         for (int c = 0; c < chunks && ok; ++c) {  // everything but the leading products, chunk by chunk as they arrive
-          ok = warp_wait(bar(FULL + (q + c) % T::SLOTS), (uint32_t)((q + c) / T::SLOTS) & 1u, s_abort, a.status, a.wait_limit);
+          ok = warp_wait(bar(FULL + (q + c) % SLOTS), (uint32_t)((q + c) / SLOTS) & 1u, s_abort, a.status, a.wait_limit);
           if (ok && c == 0 && layer == 1 && n > 0)  // layer 2 of the tile before must have been read out
             ok = warp_wait(bar(D2_FREE), (uint32_t)(n - 1) & 1u, s_abort, a.status, a.wait_limit);
           if (!ok) break;
@@ -207,7 +145,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
 #pragma unroll 1
         for (int c = 0; c < chunks; ++c) {  // the leading products
           products(T::PRODUCTS - 1, c, leader);
-          mma_commit(bar(EMPTY + (q + c) % T::SLOTS), leader);
+          mma_commit(bar(EMPTY + (q + c) % SLOTS), leader);
         }
         const bool skip = a.debug_skip_commit != 0 && blockIdx.x == 0 && n == 0 && layer == 0;
         mma_commit(bar(layer == 0 ? D1_READY : D2_READY), skip ? 0u : leader);
@@ -231,10 +169,15 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
     bool ok = true;
     // one chunk (16 numbers of this thread) -> its slot of the ring; q = number of the chunk in this CTA
     auto put_chunk = [&](int q, const float (&x)[16]) -> bool {
-      const int slot = q % T::SLOTS, use = q / T::SLOTS;
-      uint32_t t[3][8];
+      const int slot = q % SLOTS, use = q / SLOTS;
+      uint32_t t[T::TA][8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) split_pair(x[2 * e], x[2 * e + 1], t[0][e], t[1][e], t[2][e]);
+      for (int e = 0; e < 8; ++e) {
+        uint32_t terms[T::TA];
+        T::split(x[2 * e], x[2 * e + 1], terms);
+#pragma unroll
+        for (int i = 0; i < T::TA; ++i) t[i][e] = terms[i];
+      }
       if (use > 0 && !warp_wait(bar(EMPTY + slot), (uint32_t)(use - 1) & 1u, s_abort, a.status, a.wait_limit)) return false;
       tc_fence_after();
       const uint32_t at = ring_half + (uint32_t)(slot * T::TA * CHUNK_COLS);
@@ -278,8 +221,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
         for (int i = 0; i < 3; ++i) {
           const float v = u[3 * c + i];
           x[5 * i] = v;
-          sincosf(v, &x[5 * i + 1], &x[5 * i + 3]);
-          sincosf(2.0f * v, &x[5 * i + 2], &x[5 * i + 4]);
+          T::encode(v, x[5 * i + 1], x[5 * i + 2], x[5 * i + 3], x[5 * i + 4]);
         }
         x[15] = 0.0f;
         if (ok) ok = put_chunk(CHUNKS * n + c, x);
@@ -360,18 +302,19 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   }
 }
 
-// W [n_out][k_real] fp32 -> [term][k group][n_out][8] bf16 terms; position k of the operand takes column map[k] of W
-// (null: k itself), -1 = zero.
-__global__ void pack_split_image_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ img, int k_real, int k_groups,
-                                        int terms, bool permuted) {
+// W [n_out][k_real] fp32 -> [term][k group][n_rows][8] 16-bit terms; rows past n_out are zero.  KIND: where position k of
+// the operand comes from: 0 = column k, 1 = the K order of layer 1, 2 = products of pairs padded from c to cp channels.
+template <int MODE, int KIND>
+__global__ void pack_split_image_kernel(const float* __restrict__ w, uint16_t* __restrict__ img, int n_out, int n_rows, int k_real,
+                                        int k_groups, int c, int cp) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;  // one thread per (k group, n)
-  if (i >= k_groups * HID) return;
-  const int kg = i / HID, n = i - kg * HID;
+  if (i >= k_groups * n_rows) return;
+  const int kg = i / n_rows, n = i - kg * n_rows;
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     const int k = kg * 8 + e;
     int col = k;
-    if (permuted) {
+    if (KIND == 1) {
       // K step s = k / 16 holds the values 3 s .. 3 s + 2 (features, then view), each as u, sin u, sin 2u, cos u, cos 2u
       const int r = k & 15, v = 3 * (k >> 4) + r / 5, what = r % 5;
       const bool view = v >= APP;
@@ -379,43 +322,60 @@ __global__ void pack_split_image_kernel(const float* __restrict__ w, __nv_bfloat
       const int sin0 = view ? base_vs + 2 * (v - APP) : base_s + 2 * v;
       const int cos0 = sin0 + (view ? 6 : 2 * APP);
       col = r == 15 ? -1 : what == 0 ? v : what <= 2 ? sin0 + what - 1 : cos0 + what - 3;
+    } else if (KIND == 2) {
+      const int pair = k / cp, ch = k - pair * cp;
+      col = ch < c ? pair * c + ch : -1;
     }
-    float x = (col >= 0 && col < k_real) ? w[(size_t)n * k_real + col] : 0.0f;
-    for (int t = 0; t < terms; ++t) {
-      const __nv_bfloat16 b = __float2bfloat16_rn(x);
-      img[(size_t)t * k_groups * HID * 8 + (size_t)i * 8 + e] = b;
-      x -= __bfloat162float(b);
-    }
+    float x = (n < n_out && col >= 0 && col < k_real) ? w[(size_t)n * k_real + col] : 0.0f;
+#pragma unroll
+    for (int t = 0; t < Split<MODE>::TW; ++t) img[((size_t)t * k_groups * n_rows + i) * 8 + e] = Split<MODE>::term(x);
   }
 }
 
-template <bool EXACT>
-constexpr size_t split_smem() {
-  using T = Terms<EXACT>;
-  return (size_t)T::TW * (W1S_BYTES + W2S_BYTES) + (3 * HID + 2 * HID + 4 + 2 * ROWS * 3) * sizeof(float) + (2 * T::SLOTS + 7) * 8 + 16;
+// [layer 1: TW terms][layer 2: TW terms][basis: TW terms], the basis only where the products fit one operand
+template <int MODE>
+int prepare_images(GnrModel* m, const float* basis_w, const float* w1, const float* w2, cudaStream_t st) {
+  constexpr int TW = Split<MODE>::TW;
+  const size_t net = (size_t)TW * (W1S_BYTES + W2S_BYTES);
+  const int cp = (m->cfg.n_app + 15) / 16 * 16, kgb = m->cfg.n_pairs * cp / 8;
+  if (m->mlp.split_image == nullptr) GNR_CUDA_OK(cudaMalloc(&m->mlp.split_image, net + (size_t)TW * kgb * KGB_BYTES));
+  unsigned char* img = (unsigned char*)m->mlp.split_image;
+  pack_split_image_kernel<MODE, 1><<<(20 * HID + 255) / 256, 256, 0, st>>>(w1, (uint16_t*)img, HID, HID, IN_DIM, 20, 0, 0);
+  pack_split_image_kernel<MODE, 0><<<(16 * HID + 255) / 256, 256, 0, st>>>(w2, (uint16_t*)(img + (size_t)TW * W1S_BYTES), HID, HID, HID,
+                                                                          16, 0, 0);
+  m->mlp.split_basis = img + net;
+  pack_split_image_kernel<MODE, 2><<<(kgb * NB + 255) / 256, 256, 0, st>>>(basis_w, (uint16_t*)m->mlp.split_basis, m->cfg.app_dim, NB,
+                                                                          m->cfg.n_pairs * m->cfg.n_app, kgb, m->cfg.n_app, cp);
+  GNR_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+template <int MODE>
+int launch_mode(const GnrModel* m, const SplitArgs& a, cudaStream_t st) {
+  constexpr size_t smem = (size_t)Split<MODE>::TW * (W1S_BYTES + W2S_BYTES) + (3 * HID + 2 * HID + 4 + 2 * ROWS * 3) * sizeof(float) +
+                          (2 * SLOTS + 7) * 8 + 16;
+  static_assert(smem <= 227 * 1024, "the weights of the split network must fit shared memory");
+  cudaError_t e = cudaFuncSetAttribute(mlp_split_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  mlp_split_kernel<MODE><<<m->sm_count, THREADS, smem, st>>>(a);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace
 
 int gnr_mlp_split_usable(const GnrModel* m) {
   const GnrConfig& c = m->cfg;
-  return c.mlp_mode == 0 && c.app_dim == APP && c.fea_pe == FPE && c.view_pe == VPE && c.hidden == HID;
+  return c.mlp_mode <= 1 && c.app_dim == APP && c.fea_pe == FPE && c.view_pe == VPE && c.hidden == HID;
 }
 
-int gnr_mlp_split_prepare(GnrModel* m, const float* w1, const float* w2, cudaStream_t st) {
-  using T = Terms<true>;
-  if (m->mlp.split_image == nullptr) GNR_CUDA_OK(cudaMalloc(&m->mlp.split_image, (size_t)T::TW * (W1S_BYTES + W2S_BYTES)));
-  __nv_bfloat16* img = reinterpret_cast<__nv_bfloat16*>(m->mlp.split_image);
-  pack_split_image_kernel<<<(20 * HID + 255) / 256, 256, 0, st>>>(w1, img, IN_DIM, 20, T::TW, true);
-  pack_split_image_kernel<<<(16 * HID + 255) / 256, 256, 0, st>>>(w2, img + (size_t)T::TW * W1S_BYTES / 2, HID, 16, T::TW, false);
-  GNR_CUDA_OK(cudaGetLastError());
-  return 0;
+int gnr_mlp_split_prepare(GnrModel* m, const float* basis_w, const float* w1, const float* w2, cudaStream_t st) {
+  return m->cfg.mlp_mode == 0 ? prepare_images<0>(m, basis_w, w1, w2, st) : prepare_images<1>(m, basis_w, w1, w2, st);
 }
 
 int launch_mlp_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat,
                      float* rgb, int32_t* status, cudaStream_t st) {
   if (!m->mlp.split_image || feat_stride != FEAT_STRIDE) {
-    gnr_set_error("split MLP: weights were not prepared, or feature stride %d is not %d", feat_stride, FEAT_STRIDE);
+    gnr_set_error("split network: weights were not prepared, or feature stride %d is not %d", feat_stride, FEAT_STRIDE);
     return -1;
   }
   SplitArgs a;
@@ -431,10 +391,5 @@ int launch_mlp_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoord
   a.kbits = p.kbits;
   a.wait_limit = m->debug_wait_limit > 0 ? (uint32_t)m->debug_wait_limit : kWaitLimit;
   a.debug_skip_commit = m->debug_expire_wait;
-  constexpr size_t smem = split_smem<true>();
-  static_assert(smem <= 227 * 1024, "weights of the split MLP must fit shared memory");
-  cudaError_t e = cudaFuncSetAttribute(mlp_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  mlp_split_kernel<true><<<m->sm_count, THREADS, smem, st>>>(a);
-  return (int)cudaGetLastError();
+  return m->cfg.mlp_mode == 0 ? launch_mode<0>(m, a, st) : launch_mode<1>(m, a, st);
 }

@@ -26,9 +26,7 @@
 // Operand layout (A and B alike): element (row r, k) at byte (k / 8) * LBO + r * 16 + (k % 8) * 2:
 // 8 rows x 16 B form one contiguous 128 B core matrix, row groups are 128 B apart (stride byte
 // offset), the two K halves of one MMA are LBO = rows * 16 bytes apart (leading byte offset).
-// TA = 2 carries the fp16 rounding residual of every activation (and product) as a second
-// operand and a second MMA per K-step (activations then hold ~22 mantissa bits; weights stay
-// single fp16).
+// (mlp_mode 2; modes 0 and 1 carry their operands as sums of terms, gnr_mlp_split.cu.)
 //
 // Every wait on an mbarrier is bounded; when one expires the group raises
 // status[GNR_ST_WAIT_EXPIRED], stops taking tiles, and the CTA frees its TMEM and returns.
@@ -40,14 +38,10 @@ struct TcArgs {
   GnrCoords crd;
   const float* feat_in;           // BASIS == false: features from the CUDA-core gather
   float* feat_out;                // BASIS == true: optional copy of the projected features
-  const unsigned char* prod_hi;   // BASIS == true: fp16 product tiles in operand layout
-  const unsigned char* prod_lo;
+  const unsigned char* prod;      // BASIS == true: fp16 product tiles in operand layout
   int tile_bytes;                 // bytes of one product tile (k0 / 8 * 2048)
   int k0;                         // products per sample
   const unsigned char* w_image;   // [basis fp16 operand image (WB_BYTES)][W1 image][W2 image][W3 image]
-  const float* w3;
-  const float* b1;
-  const float* b2;
   const float* b3;
   float* rgb_out;
   int32_t* status;
@@ -57,18 +51,15 @@ struct TcArgs {
   int debug_skip_copy;            // test hook: group 0 of CTA 0 never starts the copy of its first tile
 };
 
-template <int TA, int NSLOT, bool BASIS>
+template <int NSLOT, bool BASIS>
 __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* s_wb = smem;
   unsigned char* s_w1 = s_wb + WB_BYTES;
   unsigned char* s_w2 = s_w1 + W1_BYTES;
-  unsigned char* s_w3h = s_w2 + W2_BYTES;  // layer 3 as an fp16 operand (used when L3TC)
-  unsigned char* s_a = s_w3h + W3_BYTES;   // [NSLOT][TA][A_BYTES]
-  float* s_w3 = reinterpret_cast<float*>(s_a + NSLOT * TA * A_BYTES);
-  float* s_b1 = s_w3 + 3 * HID;
-  float* s_b2 = s_b1 + HID;
-  float* s_b3 = s_b2 + HID;
+  unsigned char* s_w3h = s_w2 + W2_BYTES;  // layer 3 as an fp16 operand
+  unsigned char* s_a = s_w3h + W3_BYTES;   // [NSLOT][A_BYTES]
+  float* s_b3 = reinterpret_cast<float*>(s_a + NSLOT * A_BYTES);
   uint64_t* s_mbar = reinterpret_cast<uint64_t*>(s_b3 + 4);  // [NSLOT][2]: MMA completion, bulk-copy completion
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_mbar + 2 * NSLOT);
   volatile uint32_t* s_flag = s_tmem + 1;  // [NSLOT] per-group outcome of the last wait (indexed below)
@@ -84,11 +75,6 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
     const uint4* src = reinterpret_cast<const uint4*>(a.w_image);
     uint4* dst = reinterpret_cast<uint4*>(s_wb);
     for (int i = tid; i < (WB_BYTES + W1_BYTES + W2_BYTES + W3_BYTES) / 16; i += NSLOT * 128) dst[i] = src[i];
-    for (int i = tid; i < 3 * HID; i += NSLOT * 128) s_w3[i] = a.w3[i];
-    for (int i = tid; i < HID; i += NSLOT * 128) {
-      s_b1[i] = a.b1[i];
-      s_b2[i] = a.b2[i];
-    }
     if (tid < 4) s_b3[tid] = a.b3[tid];
     if (tid == 0) {
       for (int s = 0; s < 2 * NSLOT; ++s)
@@ -109,11 +95,9 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
   const uint32_t d_tmem = tmem_base + (uint32_t)(slot * COLS_PER_SLOT);     // this group's D accumulator
   const uint32_t f_tmem = d_tmem + HID;                                     // this group's feature accumulator
   const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;              // this warp's TMEM lane quarter
-  unsigned char* a_hi = s_a + (slot * TA) * A_BYTES;
-  unsigned char* a_lo = a_hi + (TA == 2 ? A_BYTES : 0);
-  const uint32_t a_hi_addr = smem_u32(a_hi), a_lo_addr = smem_u32(a_lo);
+  unsigned char* a_buf = s_a + slot * A_BYTES;
+  const uint32_t a_addr = smem_u32(a_buf);
   const uint32_t wb_addr = smem_u32(s_wb), w1_addr = smem_u32(s_w1), w2_addr = smem_u32(s_w2), w3_addr = smem_u32(s_w3h);
-  constexpr bool L3TC = (TA == 1);  // layer 3 on the tensor cores too (fp16 operands); TA == 2 keeps it in fp32
   const uint32_t mbar = smem_u32(&s_mbar[2 * slot]), tbar = smem_u32(&s_mbar[2 * slot + 1]);
   const int bar_id = 1 + slot;  // named barrier of this group (0 is __syncthreads)
   s_flag += slot;
@@ -126,10 +110,9 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
   const uint32_t copy_bytes = (uint32_t)a.tile_bytes;
 
   auto start_copy = [&](long long t) {
-    // one thread: announce the bytes, then start the copies of the tile's operand image(s)
-    mbar_expect_tx(tbar, copy_bytes * TA);
-    bulk_load(a_hi_addr, a.prod_hi + (size_t)t * copy_bytes, copy_bytes, tbar);
-    if (TA == 2) bulk_load(a_lo_addr, a.prod_lo + (size_t)t * copy_bytes, copy_bytes, tbar);
+    // one thread: announce the bytes, then start the copy of the tile's operand image
+    mbar_expect_tx(tbar, copy_bytes);
+    bulk_load(a_addr, a.prod + (size_t)t * copy_bytes, copy_bytes, tbar);
   };
 
   long long tile = (long long)blockIdx.x * NSLOT + slot;
@@ -160,8 +143,7 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
         for (int ks = 0; ks < MAX_K0 / 16; ++ks) {
           if (ks < ksteps) {
             const uint64_t bd = make_desc(wb_addr + ks * 2 * KGB_BYTES, KGB_BYTES);
-            mma_f16(f_tmem, make_desc(a_hi_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescBasis, ks > 0 ? 1u : 0u, leader);
-            if (TA == 2) mma_f16(f_tmem, make_desc(a_lo_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescBasis, 1u, leader);
+            mma_f16(f_tmem, make_desc(a_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescBasis, ks > 0 ? 1u : 0u, leader);
           }
         }
         mma_commit(mbar, leader);
@@ -214,7 +196,7 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
       float view[3] = {0.0f, 0.0f, 0.0f};
       if (BASIS) {
         // the gather kernel left the view direction in the k group after the products (hi + lo fp16)
-        const uint4 vv = *reinterpret_cast<const uint4*>(a_hi + (a.k0 >> 3) * KG_BYTES + row * 16);
+        const uint4 vv = *reinterpret_cast<const uint4*>(a_buf + (a.k0 >> 3) * KG_BYTES + row * 16);
         const float2 p0 = __half22float2(*reinterpret_cast<const __half2*>(&vv.x));
         const float2 p1 = __half22float2(*reinterpret_cast<const __half2*>(&vv.y));
         const float2 p2 = __half22float2(*reinterpret_cast<const __half2*>(&vv.z));
@@ -267,7 +249,7 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
         float g[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) g[e] = x[kg * 8 + e];
-        store_group<TA>(a_hi, a_lo, kg, row, g);
+        store_group(a_buf, kg, row, g);
       }
     }
     tc_fence_before();
@@ -281,8 +263,7 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
 #pragma unroll
       for (int ks = 0; ks < K1 / 16; ++ks) {
         const uint64_t bd = make_desc(w1_addr + ks * 2 * KG_BYTES, KG_BYTES);
-        mma_f16(d_tmem, make_desc(a_hi_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescHid, ks > 0 ? 1u : 0u, leader);
-        if (TA == 2) mma_f16(d_tmem, make_desc(a_lo_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescHid, 1u, leader);
+        mma_f16(d_tmem, make_desc(a_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescHid, ks > 0 ? 1u : 0u, leader);
       }
       mma_commit(mbar, leader);
       __syncwarp();
@@ -302,27 +283,20 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
       tmem_ld_wait();
 #pragma unroll
       for (int g8 = 0; g8 < 8; ++g8) {
-        if (TA == 1) {
-          uint4 hi;
-          hi.x = pack_h2_relu(__uint_as_float(v[g8 * 8 + 0]), __uint_as_float(v[g8 * 8 + 1]));
-          hi.y = pack_h2_relu(__uint_as_float(v[g8 * 8 + 2]), __uint_as_float(v[g8 * 8 + 3]));
-          hi.z = pack_h2_relu(__uint_as_float(v[g8 * 8 + 4]), __uint_as_float(v[g8 * 8 + 5]));
-          hi.w = pack_h2_relu(__uint_as_float(v[g8 * 8 + 6]), __uint_as_float(v[g8 * 8 + 7]));
-          *reinterpret_cast<uint4*>(a_hi + (cb * 8 + g8) * KG_BYTES + row * 16) = hi;
-        } else {
-          float g[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) g[e] = fmaxf(__uint_as_float(v[g8 * 8 + e]), 0.0f);
-          store_group<TA>(a_hi, a_lo, cb * 8 + g8, row, g);
-        }
+        uint4 hi;
+        hi.x = pack_h2_relu(__uint_as_float(v[g8 * 8 + 0]), __uint_as_float(v[g8 * 8 + 1]));
+        hi.y = pack_h2_relu(__uint_as_float(v[g8 * 8 + 2]), __uint_as_float(v[g8 * 8 + 3]));
+        hi.z = pack_h2_relu(__uint_as_float(v[g8 * 8 + 4]), __uint_as_float(v[g8 * 8 + 5]));
+        hi.w = pack_h2_relu(__uint_as_float(v[g8 * 8 + 6]), __uint_as_float(v[g8 * 8 + 7]));
+        *reinterpret_cast<uint4*>(a_buf + (cb * 8 + g8) * KG_BYTES + row * 16) = hi;
       }
     }
     {
       // the constant-1 column (input 128) and the padding of the last K-step
       const float one[8] = {1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
       const float zero[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-      store_group<TA>(a_hi, a_lo, HID / 8, row, one);
-      store_group<TA>(a_hi, a_lo, HID / 8 + 1, row, zero);
+      store_group(a_buf, HID / 8, row, one);
+      store_group(a_buf, HID / 8 + 1, row, zero);
     }
     tc_fence_before();
     proxy_fence();
@@ -335,8 +309,7 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
 #pragma unroll
       for (int ks = 0; ks < K2 / 16; ++ks) {
         const uint64_t bd = make_desc(w2_addr + ks * 2 * KG_BYTES, KG_BYTES);
-        mma_f16(d_tmem, make_desc(a_hi_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescHid, ks > 0 ? 1u : 0u, leader);
-        if (TA == 2) mma_f16(d_tmem, make_desc(a_lo_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescHid, 1u, leader);
+        mma_f16(d_tmem, make_desc(a_addr + ks * 2 * KG_BYTES, KG_BYTES), bd, kIdescHid, ks > 0 ? 1u : 0u, leader);
       }
       mma_commit(mbar, leader);
       __syncwarp();
@@ -353,7 +326,7 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
     }
 
     float o0, o1, o2;
-    if (L3TC) {
+    {
       // ---- phase 3 (tensor cores): relu(D) goes back into tensor memory as packed fp16 pairs, over the
       // columns of D this thread has already read (64 columns hold k = 0..127), and is the A operand
       // of 8 more MMAs (N = 16, 3 real outputs) whose accumulator reuses the feature columns.
@@ -391,31 +364,6 @@ __global__ void __launch_bounds__(NSLOT * 128, 1) mlp_tc_kernel(TcArgs a) {
       o0 = s_b3[0] + __uint_as_float(r[0]);
       o1 = s_b3[1] + __uint_as_float(r[1]);
       o2 = s_b3[2] + __uint_as_float(r[2]);
-    } else {
-      // ---- phase 3 (CUDA cores): rgb = sigmoid(W3 relu(D) + b3) in fp32, packed fp32x2 FMAs ----------
-      float2 p0 = make_float2(0.0f, 0.0f), p1 = p0, p2 = p0;
-#pragma unroll
-      for (int cb = 0; cb < HID / 64; ++cb) {
-        uint32_t v[64];
-        tmem_ld32(d_tmem + lane_off + cb * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-        tmem_ld32(d_tmem + lane_off + cb * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
-        tmem_ld_wait();
-#pragma unroll
-        for (int e4 = 0; e4 < 16; ++e4) {
-          const int c = cb * 64 + e4 * 4;
-          const float4 wr = *reinterpret_cast<const float4*>(s_w3 + c);
-          const float4 wg = *reinterpret_cast<const float4*>(s_w3 + HID + c);
-          const float4 wb = *reinterpret_cast<const float4*>(s_w3 + 2 * HID + c);
-          const float2 ha = make_float2(fmaxf(__uint_as_float(v[e4 * 4 + 0]), 0.0f), fmaxf(__uint_as_float(v[e4 * 4 + 1]), 0.0f));
-          const float2 hb = make_float2(fmaxf(__uint_as_float(v[e4 * 4 + 2]), 0.0f), fmaxf(__uint_as_float(v[e4 * 4 + 3]), 0.0f));
-          p0 = __ffma2_rn(hb, make_float2(wr.z, wr.w), __ffma2_rn(ha, make_float2(wr.x, wr.y), p0));
-          p1 = __ffma2_rn(hb, make_float2(wg.z, wg.w), __ffma2_rn(ha, make_float2(wg.x, wg.y), p1));
-          p2 = __ffma2_rn(hb, make_float2(wb.z, wb.w), __ffma2_rn(ha, make_float2(wb.x, wb.y), p2));
-        }
-      }
-      o0 = s_b3[0] + (p0.x + p0.y);
-      o1 = s_b3[1] + (p1.x + p1.y);
-      o2 = s_b3[2] + (p2.x + p2.y);
     }
     if (live) {
       float* out = a.rgb_out + (size_t)j * 3;
@@ -491,13 +439,13 @@ __global__ void pack_weight_image_mapped_kernel(const float* __restrict__ w, __h
   }
 }
 
-template <int TA, int NSLOT, bool BASIS>
+template <int NSLOT, bool BASIS>
 int launch_variant(const GnrModel* m, const TcArgs& args, cudaStream_t st) {
-  const size_t smem = (size_t)WB_BYTES + W1_BYTES + W2_BYTES + W3_BYTES + (size_t)NSLOT * TA * A_BYTES +
-                      (3 * HID + 2 * HID + 4) * sizeof(float) + 2 * NSLOT * sizeof(uint64_t) + 32;
-  cudaError_t e = cudaFuncSetAttribute(mlp_tc_kernel<TA, NSLOT, BASIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = (size_t)WB_BYTES + W1_BYTES + W2_BYTES + W3_BYTES + (size_t)NSLOT * A_BYTES +
+                      4 * sizeof(float) + 2 * NSLOT * sizeof(uint64_t) + 32;
+  cudaError_t e = cudaFuncSetAttribute(mlp_tc_kernel<NSLOT, BASIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  mlp_tc_kernel<TA, NSLOT, BASIS><<<m->sm_count, NSLOT * 128, smem, st>>>(args);
+  mlp_tc_kernel<NSLOT, BASIS><<<m->sm_count, NSLOT * 128, smem, st>>>(args);
   return (int)cudaGetLastError();
 }
 
@@ -505,7 +453,7 @@ int launch_variant(const GnrModel* m, const TcArgs& args, cudaStream_t st) {
 
 int gnr_tc_basis_fused(const GnrModel* m) {
   // the operand buffer holds the products and one more k group (the view direction)
-  return m->cfg.mlp_mode != 0 && m->mlp.n_prod % 16 == 0 && m->mlp.n_prod + 8 <= MAX_K0 && m->cfg.app_dim <= NB;
+  return m->cfg.mlp_mode == 2 && m->mlp.n_prod % 16 == 0 && m->mlp.n_prod + 8 <= MAX_K0 && m->cfg.app_dim <= NB;
 }
 
 int gnr_tc_tile_bytes(const GnrModel* m) { return (m->mlp.n_prod / 8 + 1) * KG_BYTES; }
@@ -552,7 +500,7 @@ int gnr_mlp_tc_prepare(GnrModel* m, const float* basis_w, const float* w1, const
 }
 
 int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, const float* feat_in,
-                  float* feat_out, const unsigned char* prod_hi, const unsigned char* prod_lo, int tile_bytes, float* rgb,
+                  float* feat_out, const unsigned char* prod, int tile_bytes, float* rgb,
                   int32_t* status, int force_unfused, cudaStream_t st, int basis_only) {
   if (!m->mlp.tc_image) {
     gnr_set_error("tensor-core MLP weights were not prepared");
@@ -567,14 +515,10 @@ int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& 
   a.crd = c;
   a.feat_in = feat_in;
   a.feat_out = fused ? feat_out : nullptr;
-  a.prod_hi = fused ? prod_hi : nullptr;
-  a.prod_lo = fused ? prod_lo : nullptr;
+  a.prod = fused ? prod : nullptr;
   a.tile_bytes = tile_bytes;
   a.k0 = m->mlp.n_prod;
   a.w_image = (const unsigned char*)m->mlp.tc_image;
-  a.w3 = m->mlp.w3;
-  a.b1 = m->mlp.b1;
-  a.b2 = m->mlp.b2;
   a.b3 = m->mlp.b3;
   a.rgb_out = rgb;
   a.status = status;
@@ -586,8 +530,7 @@ int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& 
     gnr_set_error("the projection-only launch needs the fused tensor-core path");
     return -1;
   }
-  if (m->cfg.mlp_mode == 1) return fused ? launch_variant<2, 1, true>(m, a, st) : launch_variant<2, 1, false>(m, a, st);
-  if (m->cfg.mlp_mode == 2) return fused ? launch_variant<1, 3, true>(m, a, st) : launch_variant<1, 3, false>(m, a, st);
+  if (m->cfg.mlp_mode == 2) return fused ? launch_variant<3, true>(m, a, st) : launch_variant<3, false>(m, a, st);
   gnr_set_error("unknown mlp_mode %d", m->cfg.mlp_mode);
   return -1;
 }

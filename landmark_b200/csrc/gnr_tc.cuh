@@ -202,31 +202,14 @@ __device__ __forceinline__ uint32_t pack_h2_relu(float a, float b) {
   return d;
 }
 
-// Store 8 consecutive-k values of one row as fp16 (and, with TA == 2, their rounding residuals).
-template <int TA>
-__device__ __forceinline__ void store_group(unsigned char* a_hi, unsigned char* a_lo, int kg, int row, const float (&x)[8]) {
-  uint4 hi;
-  hi.x = pack_h2(x[0], x[1]);
-  hi.y = pack_h2(x[2], x[3]);
-  hi.z = pack_h2(x[4], x[5]);
-  hi.w = pack_h2(x[6], x[7]);
-  *reinterpret_cast<uint4*>(a_hi + kg * KG_BYTES + row * 16) = hi;
-  if (TA == 2) {
-    float r[8];
-    const __half2* hp = reinterpret_cast<const __half2*>(&hi);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float2 f = __half22float2(hp[e]);
-      r[2 * e] = x[2 * e] - f.x;
-      r[2 * e + 1] = x[2 * e + 1] - f.y;
-    }
-    uint4 lo;
-    lo.x = pack_h2(r[0], r[1]);
-    lo.y = pack_h2(r[2], r[3]);
-    lo.z = pack_h2(r[4], r[5]);
-    lo.w = pack_h2(r[6], r[7]);
-    *reinterpret_cast<uint4*>(a_lo + kg * KG_BYTES + row * 16) = lo;
-  }
+// Store 8 consecutive-k values of one row as fp16.
+__device__ __forceinline__ void store_group(unsigned char* a, int kg, int row, const float (&x)[8]) {
+  uint4 v;
+  v.x = pack_h2(x[0], x[1]);
+  v.y = pack_h2(x[2], x[3]);
+  v.z = pack_h2(x[4], x[5]);
+  v.w = pack_h2(x[6], x[7]);
+  *reinterpret_cast<uint4*>(a + kg * KG_BYTES + row * 16) = v;
 }
 
 }  // namespace
