@@ -6,28 +6,38 @@
 // mlp_mode 0: the fp32 network, operands as exact sums of three bf16 terms; mlp_mode 1: activations as fp16 hi + lo (see
 // gnr_split.cuh).  Biases, ReLU, the encodings and layer 3 are fp32 on the CUDA cores.
 //
-// Work split: one persistent CTA per SM, tiles of 128 samples (row = lane of tensor memory).  Two groups of 256 threads
-// (two per row) take alternate tiles and do the CUDA-core work; one warp issues every MMA.  Layer inputs travel in
-// CHUNKS of 32 columns (two K steps; in tensor memory 16 columns per term) through a ring of slots in tensor memory:
-// five chunks of layer 1, then four of layer 2, per tile.  A chunk's MMAs run as soon as its 8 warps have stored it, and
-// its slot is free when they have completed (tcgen05.commit), so the encoding of the next tile and the conversion of
-// layer 1's result into layer 2's input run beside the MMAs of earlier chunks.  The K order of layer 1 is
-// permuted so that each K step holds three values u with their sin u, sin 2u, cos u, cos 2u (and one zero): a thread
-// encodes three values, splits 16 numbers, and stores 8 columns per term.
-// Tensor memory: D1 (layer 1 result) [0, 128), D2 [128, 256), the ring [256, 512).  Shared memory: the weight images
-// (216 KB with three terms), biases, layer-3 weights.
+// Work split: one persistent CTA per SM, tiles of 128 samples (row = lane of tensor memory), three roles.
+//   * eight warps ENCODE (two threads per row): layer 1's input travels in chunks of 32 columns (two K steps) through a
+//     ring of slots in tensor memory.  The K order of layer 1 is permuted so that each K step holds three values u with
+//     their sin u, sin 2u, cos u, cos 2u (and one zero): a thread encodes three values, splits 16 numbers, and stores 8
+//     columns per term.  A slot is free when the MMAs of its chunk have completed (tcgen05.commit).
+//   * eight warps FINISH: relu(D1 + b1) becomes layer 2's input IN PLACE, terms h and m over the columns of D1 just read
+//     (term l beside it), so that the ring belongs to layer 1 alone and the next tile is encoded while this one goes
+//     through layer 2; then layer 3 from D2.
+//   * one warp issues every MMA.
+// Leading products are issued last, after the small ones of the layer: the sums in tensor memory do not round to nearest,
+// and this way few steps happen at full size (with three terms the ring holds four of the five chunks, so the fifth's
+// small products come after the leading ones of the first).  Error against fp64 on 119,185 samples: rms 2.3e-8; 2.6e-8
+// with all products chunk by chunk; 2.35e-8 with fp32 arithmetic on the CUDA cores.
+// What bounds it: the tensor pipe (70 % active: 108 MMAs of 78 cycles per tile with three terms, 8400 of 11,300 cycles),
+// then the chain D1 -> first chunk of layer 2.  752,149 samples: 237 us; 1,900 in fp32 on the CUDA cores; 327 with all
+// sixteen warps encoding and converting the same tile, 312 with two groups of warps on alternate tiles (in both, layer
+// 2's input took ring slots, so a tile could not be encoded while the one before was in the tensor pipe).
+// Tensor memory: D1 (layer 1 result, then terms h and m of layer 2's input) [0, 128), D2 [128, 256), term l [256, 320),
+// the ring [320, 512).  Shared memory: the weight images (216 KB with three terms), biases, layer-3 weights.
 //
 // Every wait is bounded; when one runs out the CTA raises status[GNR_ST_WAIT_EXPIRED] and all its roles stop.
 #include "gnr_split.cuh"
 
 namespace {
 
-constexpr int GROUP = 256;                 // threads of a group (two per row)
-constexpr int THREADS = 2 * GROUP + 32;    // + the warp that issues MMAs
-constexpr int L1_CHUNKS = 5, L2_CHUNKS = 4, CHUNKS = L1_CHUNKS + L2_CHUNKS;
+constexpr int ROLE_WARPS = 8;              // warps that encode, and warps that finish (two threads per row)
+constexpr int MMA_WARP = 2 * ROLE_WARPS;
+constexpr int THREADS = (2 * ROLE_WARPS + 1) * 32;
+constexpr int L1_CHUNKS = 5, L2_CHUNKS = 4;
 constexpr int CHUNK_COLS = 16;             // tensor-memory columns of one term of a chunk (32 values)
-constexpr int RING_COL = 256;
-constexpr int SLOTS = 5;
+constexpr int L_COL = 256, RING_COL = 320;
+constexpr int MAX_BARS = 24;
 constexpr int W1S_BYTES = 160 * HID * 2, W2S_BYTES = HID * HID * 2;  // one term of a weight image
 
 struct SplitArgs {
@@ -48,6 +58,8 @@ struct SplitArgs {
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_constant__ SplitArgs a) {
   using T = Split<MODE>;
+  constexpr int SLOT_COLS = T::TA * CHUNK_COLS, SLOTS = (512 - RING_COL) / SLOT_COLS;  // 4 with three terms, 6 with two
+  constexpr int AHEAD = SLOTS < L1_CHUNKS ? SLOTS : L1_CHUNKS;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* s_w1 = smem;                                  // [TW][W1S_BYTES]
   unsigned char* s_w2 = s_w1 + T::TW * W1S_BYTES;              // [TW][W2S_BYTES]
@@ -55,9 +67,10 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   float* s_b1 = s_w3 + 3 * HID;
   float* s_b2 = s_b1 + HID;
   float* s_b3 = s_b2 + HID;                                    // [4]
-  float* s_part = s_b3 + 4;                                    // [2 groups][128][3] layer-3 sums of the second half of a row
-  uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_part + 2 * ROWS * 3);
-  enum { FULL = 0, EMPTY = SLOTS, D1_READY = 2 * SLOTS, D2_READY, D2_FREE, WEIGHTS, DRAIN, PART, N_BARS = PART + 2 };
+  float* s_part = s_b3 + 4;                                    // [128][3] layer-3 sums of the second half of a row
+  uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_part + ROWS * 3);
+  enum { FULL = 0, EMPTY = SLOTS, A2_FULL = 2 * SLOTS, D1_READY = A2_FULL + L2_CHUNKS, D2_READY, D2_FREE, WEIGHTS, DRAIN, PART, N_BARS };
+  static_assert(N_BARS <= MAX_BARS, "barriers");
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + N_BARS);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
 
@@ -70,21 +83,23 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   const int my_tiles = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
   const uint32_t bars = smem_u32(s_bar);
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  auto wait = [&](int i, uint32_t parity) { return warp_wait(bar(i), parity & 1u, s_abort, a.status, a.wait_limit); };
 
   // ---- set-up: barriers, tensor memory; the weight images come in by bulk copies while the first tile is encoded ----
   constexpr uint32_t kImage = T::TW * (W1S_BYTES + W2S_BYTES);
-  if (warp == 2 * GROUP / 32) {
+  if (warp == MMA_WARP) {
     if (lane == 0) {
       for (int s = 0; s < SLOTS; ++s) {
-        mbar_init(bar(FULL + s), GROUP / 32);
+        mbar_init(bar(FULL + s), ROLE_WARPS);
         mbar_init(bar(EMPTY + s), 1);
       }
+      for (int c = 0; c < L2_CHUNKS; ++c) mbar_init(bar(A2_FULL + c), ROLE_WARPS);
       mbar_init(bar(D1_READY), 1);
       mbar_init(bar(D2_READY), 1);
-      mbar_init(bar(D2_FREE), GROUP / 32);
+      mbar_init(bar(D2_FREE), ROLE_WARPS);
       mbar_init(bar(WEIGHTS), 1);
       mbar_init(bar(DRAIN), 1);
-      for (int g = 0; g < 2; ++g) mbar_init(bar(PART + g), GROUP / 64);
+      mbar_init(bar(PART), ROLE_WARPS / 2);
       *s_abort = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -97,7 +112,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
         bulk_load(smem_u32(smem) + at, a.w_image + at, min(16384u, kImage - at), bar(WEIGHTS));
     }
   } else {
-    for (int i = tid; i < 3 * HID; i += 2 * GROUP) s_w3[i] = a.w3[i];
+    for (int i = tid; i < 3 * HID; i += MMA_WARP * 32) s_w3[i] = a.w3[i];
     if (tid < HID) {
       s_b1[tid] = a.b1[tid];
       s_b2[tid] = a.b2[tid];
@@ -108,50 +123,74 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
-  const uint32_t d1 = tmem, d2 = tmem + HID, ring = tmem + RING_COL;
+  const uint32_t d1 = tmem, d2 = tmem + HID, l2_low = tmem + L_COL, ring = tmem + RING_COL;
 
-  if (warp == 2 * GROUP / 32) {
-    // ---- the warp that issues MMAs: chunks strictly in order ---------------------------------------------------------
+  if (warp == MMA_WARP) {
+    // ---- MMAs ------------------------------------------------------------------------------------------------------------
+    // (WAR: layer 1 of the next tile overwrites D1, whose columns hold layer 2's operand; MMAs of one thread run in order)
     constexpr uint32_t kIdesc = kIdescHid | T::kFormat;
-    bool ok = warp_wait(bar(WEIGHTS), 0, s_abort, a.status, a.wait_limit);
+    bool ok = wait(WEIGHTS, 0);
     const uint32_t w1 = smem_u32(s_w1), w2 = smem_u32(s_w2);
-    int q = 0;  // chunks taken so far
+    int q = 0;  // chunks of layer 1 taken so far
     for (int n = 0; n < my_tiles && ok; ++n) {
-#pragma unroll 1
-      for (int layer = 0; layer < 2 && ok; ++layer) {
-        const int chunks = layer == 0 ? L1_CHUNKS : L2_CHUNKS;
-        const uint32_t d = layer == 0 ? d1 : d2, wb = layer == 0 ? w1 : w2, w_term = layer == 0 ? W1S_BYTES : W2S_BYTES;
-        auto products = [&](int i, int c, uint32_t leader) {
-          const uint32_t at = ring + (uint32_t)(((q + c) % SLOTS) * T::TA * CHUNK_COLS);
+      // layer 1
+      auto products1 = [&](int i, int c, uint32_t leader) {
+        const uint32_t at = ring + (uint32_t)((q + c) % SLOTS) * SLOT_COLS + T::a(i) * CHUNK_COLS;
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
-            mma_f16_ts(d, at + T::a(i) * CHUNK_COLS + ks * 8,
-                       make_desc(wb + T::w(i) * w_term + (uint32_t)(4 * c + 2 * ks) * KG_BYTES, KG_BYTES), kIdesc,
-                       (c > 0 || i > 0 || ks > 0) ? 1u : 0u, leader);
-        };
+        for (int ks = 0; ks < 2; ++ks)
+          mma_f16_ts(d1, at + ks * 8, make_desc(w1 + T::w(i) * W1S_BYTES + (uint32_t)(4 * c + 2 * ks) * KG_BYTES, KG_BYTES), kIdesc,
+                     (c > 0 || i > 0 || ks > 0) ? 1u : 0u, leader);
+      };
+      int led = 0;  // chunks whose leading products have been issued
 #pragma unroll 1
-        for (int c = 0; c < chunks && ok; ++c) {  // everything but the leading products, chunk by chunk as they arrive
-          ok = warp_wait(bar(FULL + (q + c) % SLOTS), (uint32_t)((q + c) / SLOTS) & 1u, s_abort, a.status, a.wait_limit);
-          if (ok && c == 0 && layer == 1 && n > 0)  // layer 2 of the tile before must have been read out
-            ok = warp_wait(bar(D2_FREE), (uint32_t)(n - 1) & 1u, s_abort, a.status, a.wait_limit);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t leader = elect_one();
-#pragma unroll
-          for (int i = 0; i + 1 < T::PRODUCTS; ++i) products(i, c, leader);
-        }
+      for (int c = 0; c < L1_CHUNKS && ok; ++c) {
+        ok = wait(FULL + (q + c) % SLOTS, (uint32_t)((q + c) / SLOTS));
         if (!ok) break;
+        tc_fence_after();
         const uint32_t leader = elect_one();
+#pragma unroll
+        for (int i = 0; i + 1 < T::PRODUCTS; ++i) products1(i, c, leader);
+        if (c + 1 >= AHEAD) {
+          // all chunks are in: the leading products of the rest; a slot short: those of the first chunk, whose slot the
+          // last one waits for
+          const int upto = c + 1 == L1_CHUNKS ? L1_CHUNKS : L1_CHUNKS - AHEAD;
 #pragma unroll 1
-        for (int c = 0; c < chunks; ++c) {  // the leading products
-          products(T::PRODUCTS - 1, c, leader);
-          mma_commit(bar(EMPTY + (q + c) % SLOTS), leader);
+          for (; led < upto; ++led) {
+            products1(T::PRODUCTS - 1, led, leader);
+            mma_commit(bar(EMPTY + (q + led) % SLOTS), leader);
+          }
         }
-        const bool skip = a.debug_skip_commit != 0 && blockIdx.x == 0 && n == 0 && layer == 0;
-        mma_commit(bar(layer == 0 ? D1_READY : D2_READY), skip ? 0u : leader);
-        __syncwarp();
-        q += chunks;
       }
+      if (!ok) break;
+      const bool skip = a.debug_skip_commit != 0 && blockIdx.x == 0 && n == 0;
+      mma_commit(bar(D1_READY), skip ? 0u : elect_one());
+      __syncwarp();
+      q += L1_CHUNKS;
+      // layer 2: chunk c = hidden units 16 c .. 16 c + 15 of either half (K steps c and 4 + c)
+      auto products2 = [&](int i, int c, uint32_t leader) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t at = T::a(i) == 2 ? l2_low + 32 * h + 8 * c : d1 + 64 * h + 32 * T::a(i) + 8 * c;
+          mma_f16_ts(d2, at, make_desc(w2 + T::w(i) * W2S_BYTES + (uint32_t)(8 * h + 2 * c) * KG_BYTES, KG_BYTES), kIdesc,
+                     (c > 0 || i > 0 || h > 0) ? 1u : 0u, leader);
+        }
+      };
+      if (n > 0) ok = wait(D2_FREE, (uint32_t)(n - 1));  // layer 2 of the tile before has been read out
+#pragma unroll 1
+      for (int c = 0; c < L2_CHUNKS && ok; ++c) {
+        ok = wait(A2_FULL + c, (uint32_t)n);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t leader = elect_one();
+#pragma unroll
+        for (int i = 0; i + 1 < T::PRODUCTS; ++i) products2(i, c, leader);
+      }
+      if (!ok) break;
+      const uint32_t leader = elect_one();
+#pragma unroll
+      for (int c = 0; c < L2_CHUNKS; ++c) products2(T::PRODUCTS - 1, c, leader);
+      mma_commit(bar(D2_READY), leader);
+      __syncwarp();
     }
     if (!ok) {
       // stop: wait (bounded) until nothing of this CTA runs in the tensor pipe
@@ -160,17 +199,12 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
       for (uint32_t it = 0; it < kWaitLimit && !mbar_try_wait(bar(DRAIN), 0); ++it) __nanosleep(64);
     }
   } else {
-    // ---- a group: tiles g, g + 2, ... of this CTA ----------------------------------------------------------------------
-    const int g = warp / (GROUP / 32), wg = warp % (GROUP / 32);
+    const int wg = warp & (ROLE_WARPS - 1);
     const int half = wg >> 2, row = ((wg & 3) << 5) | lane;
     const uint32_t lane_off = (uint32_t)((wg & 3) * 32) << 16;
-    const uint32_t ring_half = ring + lane_off + (uint32_t)(half * 8);  // this thread's 8 of a chunk's 16 columns
-    float* part = s_part + (size_t)(g * ROWS + row) * 3;
-    bool ok = true;
-    // one chunk (16 numbers of this thread) -> its slot of the ring; q = number of the chunk in this CTA
-    auto put_chunk = [&](int q, const float (&x)[16]) -> bool {
-      const int slot = q % SLOTS, use = q / SLOTS;
-      uint32_t t[T::TA][8];
+    auto tile_row = [&](int n) { return ((long long)blockIdx.x + (long long)n * gridDim.x) * ROWS + row; };
+    // 16 numbers -> T::TA terms of eight packed columns
+    auto split16 = [&](const float (&x)[16], uint32_t (&t)[T::TA][8]) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         uint32_t terms[T::TA];
@@ -178,125 +212,152 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
 #pragma unroll
         for (int i = 0; i < T::TA; ++i) t[i][e] = terms[i];
       }
-      if (use > 0 && !warp_wait(bar(EMPTY + slot), (uint32_t)(use - 1) & 1u, s_abort, a.status, a.wait_limit)) return false;
-      tc_fence_after();
-      const uint32_t at = ring_half + (uint32_t)(slot * T::TA * CHUNK_COLS);
-#pragma unroll
-      for (int i = 0; i < T::TA; ++i) tmem_st8(at + i * CHUNK_COLS, t[i]);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(FULL + slot));
-      return true;
     };
-    for (int n = g; n < my_tiles && ok; n += 2) {
-      const long long j = ((long long)blockIdx.x + (long long)n * gridDim.x) * ROWS + row;
-      const bool live = j < total;
-      const long long js = live ? j : total - 1;
-      // this thread's 15 values: 6 c + 3 half + i for chunk c; the last three of half 1 are the view direction
-      float u[15];
-      const float* fr = a.feat + (size_t)js * FEAT_STRIDE + 3 * half;
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-          if (c < 4 || half == 0) u[3 * c + i] = __ldg(fr + 6 * c + i);
-      }
-      if (half == 1) {
-        const float* vsrc;
-        if (a.crd.view_direct) {
-          vsrc = a.crd.view_direct + (size_t)js * a.crd.point_stride;
-        } else {
-          const uint32_t ray = __ldg(a.crd.ids + (a.crd.index ? (long long)__ldg(a.crd.index + js) : js)) >> a.kbits;
-          vsrc = a.crd.rays + (size_t)ray * 6 + 3;
+    bool ok = true;
+    if (warp < ROLE_WARPS) {
+      // ---- encode --------------------------------------------------------------------------------------------------------
+      // this thread's three values of chunk c: 6 c + 3 half .. of the features; the last three of half 1 are the view direction
+      const uint32_t ring_half = ring + lane_off + (uint32_t)(half * 8);  // this thread's 8 of a term's 16 columns
+      const float *fr, *last;
+      auto row_sources = [&](int n) {
+        const long long j = tile_row(n), js = j < total ? j : total - 1;
+        fr = a.feat + (size_t)js * FEAT_STRIDE + 3 * half;
+        last = fr + 6 * (L1_CHUNKS - 1);
+        if (half == 1) {
+          if (a.crd.view_direct) {
+            last = a.crd.view_direct + (size_t)js * a.crd.point_stride;
+          } else {
+            const uint32_t ray = __ldg(a.crd.ids + (a.crd.index ? (long long)__ldg(a.crd.index + js) : js)) >> a.kbits;
+            last = a.crd.rays + (size_t)ray * 6 + 3;
+          }
         }
+      };
+      auto load = [&](int c, float (&u)[3]) {
+        const float* src = c + 1 < L1_CHUNKS ? fr + 6 * c : last;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) u[12 + i] = __ldg(vsrc + i);
-      }
-      // ---- layer 1 input ------------------------------------------------------------------------------------------------
-#pragma unroll
-      for (int c = 0; c < L1_CHUNKS; ++c) {
+        for (int i = 0; i < 3; ++i) u[i] = __ldg(src + i);
+      };
+      float u[3], ahead[3];
+      row_sources(0);
+      load(0, u);
+      const int chunks = my_tiles * L1_CHUNKS;
+      int c = 0;  // chunk in its tile
+      // (not unrolled: the encoding is long, and unrolled it does not fit the instruction cache)
+#pragma unroll 1
+      for (int q = 0; q < chunks && ok; ++q) {
+        if (++c == L1_CHUNKS) {
+          c = 0;
+          if (q + 1 < chunks) row_sources(q / L1_CHUNKS + 1);
+        }
+        load(c, ahead);  // the values of the next chunk (behind the last one: the same row again)
         float x[16];
+        T::encode(u, x);
+        uint32_t t[T::TA][8];
+        split16(x, t);
+        const int slot = q % SLOTS;
+        if (q >= SLOTS) ok = wait(EMPTY + slot, (uint32_t)(q / SLOTS - 1));
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const float v = u[3 * c + i];
-          x[5 * i] = v;
-          T::encode(v, x[5 * i + 1], x[5 * i + 2], x[5 * i + 3], x[5 * i + 4]);
-        }
-        x[15] = 0.0f;
-        if (ok) ok = put_chunk(CHUNKS * n + c, x);
+        for (int i = 0; i < T::TA; ++i) tmem_st8(ring_half + (uint32_t)(slot * SLOT_COLS + i * CHUNK_COLS), t[i]);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(FULL + slot));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) u[i] = ahead[i];
       }
-      // ---- layer 2 input: relu(D1 + b1) ------------------------------------------------------------------------------------
-      if (ok) ok = warp_wait(bar(D1_READY), (uint32_t)n & 1u, s_abort, a.status, a.wait_limit);
-      if (!ok) break;
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < L2_CHUNKS; ++c) {
-        uint32_t v[16];
-        const int col = 32 * c + 16 * half;
-        tmem_ld16(d1 + lane_off + col, v);
+    } else {
+      // ---- finish ----------------------------------------------------------------------------------------------------------
+      const uint32_t d1_half = d1 + lane_off + 64u * (uint32_t)half, low_half = l2_low + lane_off + 32u * (uint32_t)half;
+#pragma unroll 1
+      for (int n = 0; n < my_tiles; ++n) {
+        // layer 2's input: relu(D1 + b1), 16 of this half's 64 units at a time; the upper 32 columns are read before term m
+        // overwrites them
+        if (!(ok = wait(D1_READY, (uint32_t)n))) break;
+        tc_fence_after();
+        uint32_t upper[32], v[16];
+        tmem_ld16(d1_half, v);
+        tmem_ld32(d1_half + 32, upper);
         tmem_ld_wait();
-        float x[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 b = *reinterpret_cast<const float4*>(s_b1 + col + 4 * q);
-          x[4 * q + 0] = fmaxf(__uint_as_float(v[4 * q + 0]) + b.x, 0.0f);
-          x[4 * q + 1] = fmaxf(__uint_as_float(v[4 * q + 1]) + b.y, 0.0f);
-          x[4 * q + 2] = fmaxf(__uint_as_float(v[4 * q + 2]) + b.z, 0.0f);
-          x[4 * q + 3] = fmaxf(__uint_as_float(v[4 * q + 3]) + b.w, 0.0f);
-        }
-        if (ok) ok = put_chunk(CHUNKS * n + L1_CHUNKS + c, x);
-      }
-      // ---- layer 3: rgb = sigmoid(W3 relu(D2 + b2) + b3), fp32; half h sums columns 64 h .. ------------------------------------
-      if (ok) ok = warp_wait(bar(D2_READY), (uint32_t)n & 1u, s_abort, a.status, a.wait_limit);
-      if (!ok) break;
-      tc_fence_after();
-      float2 p0 = make_float2(0.0f, 0.0f), p1 = p0, p2 = p0;
+        for (int c = 0; c < L2_CHUNKS; ++c) {
+          float x[16];
 #pragma unroll
-      for (int cb = 0; cb < 2; ++cb) {
-        uint32_t v[32];
-        const int col = 64 * half + 32 * cb;
-        tmem_ld32(d2 + lane_off + col, v);
-        tmem_ld_wait();
-        if (cb == 1) {  // the accumulator can be overwritten
+          for (int e = 0; e < 4; ++e) {
+            const float4 b = *reinterpret_cast<const float4*>(s_b1 + 64 * half + 16 * c + 4 * e);
+            const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t raw = c < 2 ? v[4 * e + i] : upper[16 * (c - 2) + 4 * e + i];
+              x[4 * e + i] = fmaxf(__uint_as_float(raw) + bb[i], 0.0f);
+            }
+          }
+          uint32_t t[T::TA][8];
+          split16(x, t);
+          if (c == 0) {  // the next 16 columns, before the first 8 are overwritten
+            tmem_ld16(d1_half + 16, v);
+            tmem_ld_wait();
+          }
+          tmem_st8(d1_half + 8 * c, t[0]);
+          tmem_st8(d1_half + 32 + 8 * c, t[1]);
+          if constexpr (T::TA == 3) tmem_st8(low_half + 8 * c, t[2]);
+          tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar(D2_FREE));
+          if (lane == 0) mbar_arrive(bar(A2_FULL + c));
         }
+        // layer 3: rgb = sigmoid(W3 relu(D2 + b2) + b3), fp32; half h sums columns 64 h ..
+        if (!(ok = wait(D2_READY, (uint32_t)n))) break;
+        tc_fence_after();
+        float2 p0 = make_float2(0.0f, 0.0f), p1 = p0, p2 = p0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 b = *reinterpret_cast<const float4*>(s_b2 + col + 4 * q);
-          const float2 xa = make_float2(fmaxf(__uint_as_float(v[4 * q + 0]) + b.x, 0.0f), fmaxf(__uint_as_float(v[4 * q + 1]) + b.y, 0.0f));
-          const float2 xb = make_float2(fmaxf(__uint_as_float(v[4 * q + 2]) + b.z, 0.0f), fmaxf(__uint_as_float(v[4 * q + 3]) + b.w, 0.0f));
-          const float4 wr = *reinterpret_cast<const float4*>(s_w3 + col + 4 * q);
-          const float4 wg4 = *reinterpret_cast<const float4*>(s_w3 + HID + col + 4 * q);
-          const float4 wb4 = *reinterpret_cast<const float4*>(s_w3 + 2 * HID + col + 4 * q);
-          p0 = __ffma2_rn(xb, make_float2(wr.z, wr.w), __ffma2_rn(xa, make_float2(wr.x, wr.y), p0));
-          p1 = __ffma2_rn(xb, make_float2(wg4.z, wg4.w), __ffma2_rn(xa, make_float2(wg4.x, wg4.y), p1));
-          p2 = __ffma2_rn(xb, make_float2(wb4.z, wb4.w), __ffma2_rn(xa, make_float2(wb4.x, wb4.y), p2));
+        for (int cb = 0; cb < 2; ++cb) {
+          const int col = 64 * half + 32 * cb;
+          tmem_ld32(d2 + lane_off + col, upper);
+          tmem_ld_wait();
+          if (cb == 1) {  // the accumulator can be overwritten
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(D2_FREE));
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float4 b = *reinterpret_cast<const float4*>(s_b2 + col + 4 * e);
+            const float2 xa = make_float2(fmaxf(__uint_as_float(upper[4 * e + 0]) + b.x, 0.0f), fmaxf(__uint_as_float(upper[4 * e + 1]) + b.y, 0.0f));
+            const float2 xb = make_float2(fmaxf(__uint_as_float(upper[4 * e + 2]) + b.z, 0.0f), fmaxf(__uint_as_float(upper[4 * e + 3]) + b.w, 0.0f));
+            const float4 wr = *reinterpret_cast<const float4*>(s_w3 + col + 4 * e);
+            const float4 wg4 = *reinterpret_cast<const float4*>(s_w3 + HID + col + 4 * e);
+            const float4 wb4 = *reinterpret_cast<const float4*>(s_w3 + 2 * HID + col + 4 * e);
+            p0 = __ffma2_rn(xb, make_float2(wr.z, wr.w), __ffma2_rn(xa, make_float2(wr.x, wr.y), p0));
+            p1 = __ffma2_rn(xb, make_float2(wg4.z, wg4.w), __ffma2_rn(xa, make_float2(wg4.x, wg4.y), p1));
+            p2 = __ffma2_rn(xb, make_float2(wb4.z, wb4.w), __ffma2_rn(xa, make_float2(wb4.x, wb4.y), p2));
+          }
         }
-      }
-      // (half 1 cannot overtake: its next sums follow MMAs that need half 0's next chunks, stored after the reads here)
-      if (half == 1) {
-        part[0] = p0.x + p0.y;
-        part[1] = p1.x + p1.y;
-        part[2] = p2.x + p2.y;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(PART + g));
-        continue;
-      }
-      ok = warp_wait(bar(PART + g), (uint32_t)(n >> 1) & 1u, s_abort, a.status, a.wait_limit);
-      if (ok && live) {
-        float* out = a.rgb_out + (size_t)j * 3;
-        out[0] = 1.0f / (1.0f + expf(-((p0.x + p0.y) + part[0] + s_b3[0])));
-        out[1] = 1.0f / (1.0f + expf(-((p1.x + p1.y) + part[1] + s_b3[1])));
-        out[2] = 1.0f / (1.0f + expf(-((p2.x + p2.y) + part[2] + s_b3[2])));
+        float* part = s_part + row * 3;
+        // (half 1 cannot overtake: its next sums follow MMAs that need half 0's next chunks, stored after the reads here)
+        if (half == 1) {
+          part[0] = p0.x + p0.y;
+          part[1] = p1.x + p1.y;
+          part[2] = p2.x + p2.y;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(PART));
+          continue;
+        }
+        if (!(ok = wait(PART, (uint32_t)n))) break;
+        const long long j = tile_row(n);
+        if (j < total) {
+          float* out = a.rgb_out + (size_t)j * 3;
+          out[0] = 1.0f / (1.0f + expf(-((p0.x + p0.y) + part[0] + s_b3[0])));
+          out[1] = 1.0f / (1.0f + expf(-((p1.x + p1.y) + part[1] + s_b3[1])));
+          out[2] = 1.0f / (1.0f + expf(-((p2.x + p2.y) + part[2] + s_b3[2])));
+        }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 2 * GROUP / 32) {
+  if (warp == MMA_WARP) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   }
@@ -352,8 +413,8 @@ int prepare_images(GnrModel* m, const float* basis_w, const float* w1, const flo
 
 template <int MODE>
 int launch_mode(const GnrModel* m, const SplitArgs& a, cudaStream_t st) {
-  constexpr size_t smem = (size_t)Split<MODE>::TW * (W1S_BYTES + W2S_BYTES) + (3 * HID + 2 * HID + 4 + 2 * ROWS * 3) * sizeof(float) +
-                          (2 * SLOTS + 7) * 8 + 16;
+  constexpr size_t smem = (size_t)Split<MODE>::TW * (W1S_BYTES + W2S_BYTES) + (3 * HID + 2 * HID + 4 + ROWS * 3) * sizeof(float) +
+                          MAX_BARS * 8 + 16;
   static_assert(smem <= 227 * 1024, "the weights of the split network must fit shared memory");
   cudaError_t e = cudaFuncSetAttribute(mlp_split_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;

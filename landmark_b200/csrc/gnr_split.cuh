@@ -16,6 +16,31 @@ namespace {
 template <int MODE>
 struct Split;
 
+// sin and cos to within 7.1e-8 (rms 1.7e-8, i.e. little more than the rounding of the result) for |x| <= 1000: the
+// multiple of pi/2 nearest to x is taken off in two steps (pi/2 as the sum of two floats; the fused multiply-adds round
+// once), what is left, |r| <= pi/4, goes into the Taylor polynomials up to r^9 and r^10 (next terms: 2e-9 and 1e-10), and
+// the quadrant picks and signs them.
+__device__ __forceinline__ void sincos_short(float x, float& s, float& c) {
+  const float m = fmaf(x, 0.636619772f, 12582912.0f);  // 1.5 x 2^23: the low bits of m are the quadrant
+  const float k = m - 12582912.0f;
+  const int q = __float_as_int(m);
+  float r = fmaf(-k, 1.57079637f, x);
+  r = fmaf(-k, -4.37113883e-8f, r);
+  const float z = r * r;
+  float sp = fmaf(z, 2.75573192e-6f, -1.98412698e-4f);
+  sp = fmaf(sp, z, 8.33333333e-3f);
+  sp = fmaf(sp, z, -1.66666667e-1f);
+  const float sr = fmaf(sp, z * r, r);
+  float cp = fmaf(z, -2.75573192e-7f, 2.48015873e-5f);
+  cp = fmaf(cp, z, -1.38888889e-3f);
+  cp = fmaf(cp, z, 4.16666667e-2f);
+  cp = fmaf(cp, z, -0.5f);
+  const float cr = fmaf(cp, z, 1.0f);
+  const float a = (q & 1) ? cr : sr, b = (q & 1) ? sr : cr;
+  s = __int_as_float(__float_as_int(a) ^ ((q & 2) << 30));
+  c = __int_as_float(__float_as_int(b) ^ (((q + 1) & 2) << 30));
+}
+
 template <>
 struct Split<0> {
   static constexpr int TA = 3, TW = 3, PRODUCTS = 6;
@@ -43,10 +68,36 @@ struct Split<0> {
     x -= __bfloat162float(b);
     return __bfloat16_as_ushort(b);
   }
-  // sin v, sin 2v, cos v, cos 2v
-  __device__ static __forceinline__ void encode(float v, float& s1, float& s2, float& c1, float& c2) {
-    sincosf(v, &s1, &c1);
-    sincosf(2.0f * v, &s2, &c2);
+  // three values -> one K step of layer 1: v, sin v, sin 2v, cos v, cos 2v of each, and a zero
+  __device__ static __forceinline__ void encode(const float (&v)[3], float (&x)[16]) {
+    // one test for all six angles, so that the short form has no branches between them
+    const bool large = !(fabsf(v[0]) <= 500.0f && fabsf(v[1]) <= 500.0f && fabsf(v[2]) <= 500.0f);
+    if (__any_sync(0xffffffffu, large)) {
+#pragma unroll 1
+      for (int i = 0; i < 3; ++i) {
+        const float u = i == 0 ? v[0] : i == 1 ? v[1] : v[2];
+        float s1, c1, s2, c2;
+        sincosf(u, &s1, &c1);
+        sincosf(2.0f * u, &s2, &c2);
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+          if (e == i) {
+            x[5 * e] = u;
+            x[5 * e + 1] = s1;
+            x[5 * e + 2] = s2;
+            x[5 * e + 3] = c1;
+            x[5 * e + 4] = c2;
+          }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        x[5 * i] = v[i];
+        sincos_short(v[i], x[5 * i + 1], x[5 * i + 3]);
+        sincos_short(2.0f * v[i], x[5 * i + 2], x[5 * i + 4]);
+      }
+    }
+    x[15] = 0.0f;
   }
 };
 
@@ -66,11 +117,19 @@ struct Split<1> {
     x -= __half2float(h);
     return __half_as_ushort(h);
   }
-  // (as the other kernels of this mode: one hardware sine and cosine, then the double-angle identities)
-  __device__ static __forceinline__ void encode(float v, float& s1, float& s2, float& c1, float& c2) {
-    sincos_reduced(v, s1, c1);
-    s2 = 2.0f * s1 * c1;
-    c2 = 1.0f - 2.0f * s1 * s1;
+  // (one hardware sine and cosine, then the double-angle identities)
+  __device__ static __forceinline__ void encode(const float (&v)[3], float (&x)[16]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      float s, c;
+      sincos_reduced(v[i], s, c);
+      x[5 * i] = v[i];
+      x[5 * i + 1] = s;
+      x[5 * i + 2] = 2.0f * s * c;
+      x[5 * i + 3] = c;
+      x[5 * i + 4] = 1.0f - 2.0f * s * s;
+    }
+    x[15] = 0.0f;
   }
 };
 
