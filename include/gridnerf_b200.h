@@ -179,6 +179,10 @@ int gnr_rgba8(const float* rgb, int64_t n, uint8_t* rgba, void* stream);
  * passes it to the calls below; contents carry no state between chunks. */
 int gnr_workspace_bytes(const GnrModel* m, int64_t n_rays, int n_samples, int64_t max_valid,
                         int64_t max_app, size_t* bytes_h);
+/* The same for the gnr_render_* entries, which need less: they keep no id lists and, where one kernel does the
+ * appearance path, no per-sample features or product tiles. */
+int gnr_render_workspace_bytes(const GnrModel* m, int64_t n_rays, int n_samples, int64_t max_valid,
+                               int64_t max_app, size_t* bytes_h);
 
 /* The whole per-chunk forward: GridBaseSequential.forward, dense-sampling branch
  * (app/models/gridnerf_sequential.py:448-504) = sample_ray (:244-281) + alphaMask filter
@@ -189,6 +193,29 @@ int gnr_workspace_bytes(const GnrModel* m, int64_t n_rays, int n_samples, int64_
 int gnr_render_chunk(GnrModel* m, const float* rays, int64_t n_rays, int n_samples, int white_bg,
                      void* workspace, size_t workspace_bytes, int64_t max_valid, int64_t max_app,
                      float* rgb_map, float* depth_map, void* stream);
+
+/* gnr_render_chunk for one chunk, waited for: returns the chunk's status block (GNR_ST_* words) in ``status_h``. */
+int gnr_render_forward(GnrModel* m, const float* rays, int64_t n_rays, int n_samples, int white_bg,
+                       void* workspace, size_t workspace_bytes, int64_t max_valid, int64_t max_app,
+                       float* rgb_map, float* depth_map, int32_t* status_h, void* stream);
+
+/* The chunk loop over device-resident rays (dist_render/ddp_infer/inferer_impl.py:95-120): chunks of
+ * ``chunk_rays`` take the ``n_lanes`` workspaces in turn; with more than one lane and more than one chunk every lane is
+ * a stream of the library's, forked from ``stream`` (or behind ``after``, a cudaEvent_t, if it is not NULL) and joined
+ * to it.  Each chunk leaves its status block in ``status`` (8 words per chunk; device or pinned host memory). */
+int gnr_render_batch(GnrModel* m, const float* rays, int64_t n_rays, int n_samples, int white_bg,
+                     int64_t chunk_rays, int n_lanes, void* const* workspaces_h, size_t workspace_bytes,
+                     int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, int32_t* status,
+                     void* after, void* stream);
+
+/* One frame, pose in, RGBA8 image out (dist_render/ddp_infer/nerf_inferer.py:393-410, :267-341, :345-378), nothing
+ * waited for: rays of the listed pixels (every pixel of the image once, in any order) into ``rays[H * W][6]``, the chunk
+ * loop of gnr_render_batch, each pixel's ``(uint8)(rgb * 255)`` and alpha 255 at its place in ``rgba[H][W][4]``
+ * (device), and the copy of that image to ``rgba_h`` (pinned). */
+int gnr_render_frame(GnrModel* m, const float* pose_h, const float* dir_x, const float* dir_y, int H, int W,
+                     const int32_t* pixel_ids, int n_samples, int white_bg, int64_t chunk_rays, int n_lanes,
+                     void* const* workspaces_h, size_t workspace_bytes, int64_t max_valid, int64_t max_app,
+                     float* rays, uint8_t* rgba, uint8_t* rgba_h, int32_t* status, void* stream);
 
 /* Same forward with HOST buffers: copies ``rays_h`` to the device in chunks of
  * ``chunk_rays``, renders, copies rgb/depth back, synchronises, and returns the status block.

@@ -4,6 +4,7 @@
 #include <stdarg.h>
 #include <string.h>
 
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -224,10 +225,13 @@ extern "C" int gnr_create(const GnrConfig* cfg, int device, GnrModel** out) {
     gnr_set_error("gnr_create: device %d not present (%d devices)", device, n_dev);
     return -1;
   }
-  cudaDeviceProp prop;
-  GNR_CUDA_OK(cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10) {
-    gnr_set_error("gnr_create: device %d is sm_%d%d; this library contains sm_100a code only", device, prop.major, prop.minor);
+  // (three attributes: cudaGetDeviceProperties asks the driver for all of them, which took 3 to 15 ms per model)
+  int major = 0, minor = 0, sms = 0;
+  GNR_CUDA_OK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  GNR_CUDA_OK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+  GNR_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  if (major != 10) {
+    gnr_set_error("gnr_create: device %d is sm_%d%d; this library contains sm_100a code only", device, major, minor);
     return -1;
   }
   GnrModel* m = new (std::nothrow) GnrModel();
@@ -238,7 +242,7 @@ extern "C" int gnr_create(const GnrConfig* cfg, int device, GnrModel** out) {
   memset(m, 0, sizeof(*m));
   m->cfg = *cfg;
   m->device = device;
-  m->sm_count = prop.multiProcessorCount > 0 ? prop.multiProcessorCount : GNR_SM_COUNT_FALLBACK;
+  m->sm_count = sms > 0 ? sms : GNR_SM_COUNT_FALLBACK;
   const int A = cfg->app_dim, V = cfg->view_pe > 0 ? cfg->view_pe : 0;
   m->mlp.in_dim = A + 3 + 2 * cfg->fea_pe * A + 2 * V * 3;
   m->mlp.k1_pad = (m->mlp.in_dim + 7) / 8 * 8;
@@ -282,6 +286,11 @@ extern "C" int gnr_destroy(GnrModel* m) {
   free_dev(m->host_rgb);
   free_dev(m->host_depth);
   if (m->host_status) cudaFreeHost(m->host_status);
+  if (m->forward_status) cudaFreeHost(m->forward_status);
+  for (int i = 0; i < GNR_MAX_LANES; ++i)
+    if (m->lane_streams[i]) cudaStreamDestroy(m->lane_streams[i]);
+  for (int i = 0; i <= GNR_MAX_LANES; ++i)
+    if (m->lane_events[i]) cudaEventDestroy(m->lane_events[i]);
   delete m->prof;
   for (int i = 0; i < 2; ++i) {
     if (m->host_streams[i]) cudaStreamDestroy(m->host_streams[i]);
@@ -658,11 +667,16 @@ extern "C" int gnr_sample_bits(int n_samples) {
   return b;
 }
 
-GnrWs gnr_ws_layout(const GnrModel* m, int64_t n, int S, int64_t max_valid, int64_t max_app) {
+// `render_only`: the layout of the gnr_render_* entries, which leaves out what they never touch: the id lists of the
+// stage-wise entries and, where one kernel does the appearance path, per-sample features and product tiles (all but 24
+// of 440 bytes per appearance entry).
+GnrWs gnr_ws_layout(const GnrModel* m, int64_t n, int S, int64_t max_valid, int64_t max_app, int render_only) {
   GnrWs L;
   memset(&L, 0, sizeof(L));
   const size_t words = (size_t)(S + 31) / 32;
   const size_t n_blocks = (size_t)(n + 1023) / 1024 + 1;
+  const bool lists = !render_only || gnr_march_lanes(m, n, S, max_valid) == 0;
+  const bool samples = !render_only || !gnr_app_fusable(m);
   L.feat_stride = (m->cfg.app_dim + 3) / 4 * 4;
   L.max_valid = max_valid;
   L.max_app = max_app;
@@ -679,20 +693,22 @@ GnrWs gnr_ws_layout(const GnrModel* m, int64_t n, int S, int64_t max_valid, int6
   L.counts = take((size_t)n * 4);
   L.offsets = take((size_t)(n + 1) * 4);
   L.block_sums = take(n_blocks * 4);
-  L.ids = take((size_t)max_valid * 4);
-  L.sigma_feat = take((size_t)max_valid * 4);
+  if (lists) {
+    L.ids = take((size_t)max_valid * 4);
+    L.sigma_feat = take((size_t)max_valid * 4);
+  }
   L.sigma = take((size_t)max_valid * 4);
   L.weight = take((size_t)max_valid * 4);
   L.acc = take((size_t)n * 4);
   L.depth = take((size_t)n * 4);
   L.app_counts = take((size_t)n * 4);
   L.app_offsets = take((size_t)(n + 1) * 4);
-  L.app_index = take((size_t)max_app * 4);
+  if (lists) L.app_index = take((size_t)max_app * 4);
   L.app_ids = take((size_t)max_app * 4);     // ray << kbits | sample of every appearance entry
   L.app_weight = take((size_t)max_app * 4);  // its compositing weight
-  L.app_feat = take((size_t)max_app * L.feat_stride * 4);
+  if (samples) L.app_feat = take((size_t)max_app * L.feat_stride * 4);
   L.app_rgb = take((size_t)max_app * 3 * 4);
-  if (gnr_tc_basis_fused(m)) {
+  if (samples && gnr_tc_basis_fused(m)) {
     const size_t tiles = (size_t)(max_app + 127) / 128;
     L.app_prod_tile = gnr_tc_tile_bytes(m);
     L.app_prod = take(tiles * (size_t)L.app_prod_tile);
@@ -769,7 +785,7 @@ int gnr_check_sampler(const GnrModel* m, int S) {
 }
 
 int gnr_check_chunk(const GnrModel* m, int64_t n, int S, int64_t max_valid, int64_t max_app, const void* ws,
-                    size_t ws_bytes) {
+                    size_t ws_bytes, int render_only) {
   if (!m) {
     gnr_set_error("null model");
     return -1;
@@ -801,7 +817,7 @@ int gnr_check_chunk(const GnrModel* m, int64_t n, int S, int64_t max_valid, int6
   }
   if (gnr_check_sampler(m, S)) return -1;
   if (gnr_check_lattice(m)) return -1;
-  GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app);
+  GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app, render_only);
   if (!ws || ws_bytes < L.total) {
     gnr_set_error("workspace too small: have %zu bytes, need %zu", ws_bytes, L.total);
     return -1;
@@ -820,6 +836,16 @@ extern "C" int gnr_workspace_bytes(const GnrModel* m, int64_t n_rays, int n_samp
     return -1;
   }
   *bytes_h = gnr_ws_layout(m, n_rays, n_samples, max_valid, max_app).total;
+  return 0;
+}
+
+extern "C" int gnr_render_workspace_bytes(const GnrModel* m, int64_t n_rays, int n_samples, int64_t max_valid, int64_t max_app,
+                                          size_t* bytes_h) {
+  if (!m || !bytes_h || n_rays < 0 || n_samples < 1 || max_valid < 0 || max_app < 0) {
+    gnr_set_error("gnr_render_workspace_bytes: bad argument");
+    return -1;
+  }
+  *bytes_h = gnr_ws_layout(m, n_rays, n_samples, max_valid, max_app, 1).total;
   return 0;
 }
 
@@ -1036,8 +1062,9 @@ extern "C" int gnr_composite(GnrModel* m, int64_t n, int white_bg, void* workspa
 }
 
 static int render_chunk_impl(GnrModel* m, const float* rays, int64_t n, int S, int white_bg, char* ws,
-                             int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, cudaStream_t st) {
-  GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app);
+                             int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, cudaStream_t st,
+                             const GnrPixelSink* sink = nullptr) {
+  GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app, 1);
   GnrSampleParams p = gnr_sample_params(m, S);
   const int lanes = gnr_march_lanes(m, n, S, max_valid);
   {
@@ -1092,7 +1119,7 @@ static int render_chunk_impl(GnrModel* m, const float* rays, int64_t n, int S, i
   }
   {
     StageScope sc(m, GNR_STAGE_COMPOSITE, 1, st);
-    GNR_LAUNCH_OK(launch_composite(m, n, white_bg, ws, L, rgb_map, depth_map, st, lanes));
+    GNR_LAUNCH_OK(launch_composite(m, n, white_bg, ws, L, rgb_map, depth_map, st, lanes, sink));
   }
   return 0;
 }
@@ -1138,9 +1165,8 @@ extern "C" int gnr_profile_collect(GnrModel* m, float* stage_ms_h, int64_t* laun
 extern "C" int gnr_render_chunk(GnrModel* m, const float* rays, int64_t n, int S, int white_bg, void* workspace,
                                 size_t ws_bytes, int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map,
                                 void* stream) {
-  int rc = gnr_check_chunk(m, n, S, max_valid, max_app, workspace, ws_bytes);
+  int rc = gnr_check_chunk(m, n, S, max_valid, max_app, workspace, ws_bytes, 1);
   if (rc) return rc;
-  if (n == 0) return 0;
   if (!rays) {
     gnr_set_error("gnr_render_chunk: null rays");
     return -1;
@@ -1148,6 +1174,112 @@ extern "C" int gnr_render_chunk(GnrModel* m, const float* rays, int64_t n, int S
   DeviceGuard g(m->device);
   return render_chunk_impl(m, rays, n, S, white_bg, (char*)workspace, max_valid, max_app, rgb_map, depth_map,
                            (cudaStream_t)stream);
+}
+
+extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int S, int white_bg, void* workspace, size_t ws_bytes,
+                                  int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, int32_t* status_h,
+                                  void* stream) {
+  int rc = gnr_check_chunk(m, n, S, max_valid, max_app, workspace, ws_bytes, 1);
+  if (rc) return rc;
+  if (!rays || !status_h) {
+    gnr_set_error("gnr_render_forward: null rays or status");
+    return -1;
+  }
+  DeviceGuard g(m->device);
+  // the compositing writes the status block into pinned memory: no copy is queued behind it
+  if (!m->forward_status) GNR_CUDA_OK(cudaMallocHost(&m->forward_status, GNR_ST_WORDS * sizeof(int32_t)));
+  const GnrPixelSink sink{nullptr, nullptr, m->forward_status};
+  rc = render_chunk_impl(m, rays, n, S, white_bg, (char*)workspace, max_valid, max_app, rgb_map, depth_map, (cudaStream_t)stream,
+                         &sink);
+  if (rc) return rc;
+  GNR_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
+  memcpy(status_h, m->forward_status, GNR_ST_WORDS * sizeof(int32_t));
+  return 0;
+}
+
+// Chunks of one call, dealt to the lanes in turn.  With several lanes each is a stream of the model's: forked from
+// `stream` (or behind `after`), joined to it at the end.  One call at a time forks (the events are the model's).
+static int render_batch_impl(GnrModel* m, const float* rays, int64_t n_rays, int S, int white_bg, int64_t chunk, int n_lanes,
+                             void* const* ws, int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, uint8_t* rgba,
+                             const int32_t* pixel_ids, int32_t* status, cudaEvent_t after, cudaStream_t stream) {
+  static std::mutex mutex;
+  const bool fork = n_lanes > 1 && n_rays > chunk;
+  std::unique_lock<std::mutex> lock(mutex, std::defer_lock);
+  if (fork) {
+    lock.lock();
+    for (int i = 0; i < n_lanes; ++i) {
+      if (!m->lane_streams[i]) GNR_CUDA_OK(cudaStreamCreateWithFlags(&m->lane_streams[i], cudaStreamNonBlocking));
+      if (!m->lane_events[i]) GNR_CUDA_OK(cudaEventCreateWithFlags(&m->lane_events[i], cudaEventDisableTiming));
+    }
+    if (!after) {
+      cudaEvent_t& e = m->lane_events[GNR_MAX_LANES];
+      if (!e) GNR_CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      GNR_CUDA_OK(cudaEventRecord(e, stream));
+      after = e;
+    }
+    for (int i = 0; i < n_lanes; ++i) GNR_CUDA_OK(cudaStreamWaitEvent(m->lane_streams[i], after, 0));
+  }
+  int rc = 0;
+  int64_t c = 0;
+  for (int64_t first = 0; first < n_rays && !rc; first += chunk, ++c) {
+    const int lane = fork ? (int)(c % n_lanes) : 0;
+    const int64_t n = first + chunk <= n_rays ? chunk : n_rays - first;
+    const GnrPixelSink sink{rgba, pixel_ids ? pixel_ids + first : nullptr, status ? status + c * GNR_ST_WORDS : nullptr};
+    rc = render_chunk_impl(m, rays + first * 6, n, S, white_bg, (char*)ws[lane], max_valid, max_app, rgb_map ? rgb_map + first * 3 : nullptr,
+                           depth_map ? depth_map + first : nullptr, fork ? m->lane_streams[lane] : stream, &sink);
+  }
+  if (fork) {  // (after an error too: nothing is left running beside the caller's stream)
+    for (int i = 0; i < n_lanes; ++i) {
+      GNR_CUDA_OK(cudaEventRecord(m->lane_events[i], m->lane_streams[i]));
+      GNR_CUDA_OK(cudaStreamWaitEvent(stream, m->lane_events[i], 0));
+    }
+  }
+  return rc;
+}
+
+static int check_batch(const char* who, const GnrModel* m, const void* rays, int64_t n_rays, int S, int64_t chunk, int n_lanes,
+                       void* const* ws, size_t ws_bytes, int64_t max_valid, int64_t max_app) {
+  if (!m || !rays || !ws || n_rays < 1 || chunk < 1 || n_lanes < 1 || n_lanes > GNR_MAX_LANES) {
+    gnr_set_error("%s: null model, rays or workspaces, or bad sizes (%lld rays, chunk %lld, %d lanes of at most %d)", who,
+                  (long long)n_rays, (long long)chunk, n_lanes, GNR_MAX_LANES);
+    return -1;
+  }
+  for (int i = 0; i < n_lanes; ++i) {
+    const int rc = gnr_check_chunk(m, chunk < n_rays ? chunk : n_rays, S, max_valid, max_app, ws[i], ws_bytes, 1);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+extern "C" int gnr_render_batch(GnrModel* m, const float* rays, int64_t n_rays, int S, int white_bg, int64_t chunk, int n_lanes,
+                                void* const* workspaces, size_t ws_bytes, int64_t max_valid, int64_t max_app, float* rgb_map,
+                                float* depth_map, int32_t* status, void* after, void* stream) {
+  const int rc = check_batch("gnr_render_batch", m, rays, n_rays, S, chunk, n_lanes, workspaces, ws_bytes, max_valid, max_app);
+  if (rc) return rc;
+  DeviceGuard g(m->device);
+  return render_batch_impl(m, rays, n_rays, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, rgb_map, depth_map, nullptr,
+                           nullptr, status, (cudaEvent_t)after, (cudaStream_t)stream);
+}
+
+extern "C" int gnr_render_frame(GnrModel* m, const float* pose_h, const float* dir_x, const float* dir_y, int H, int W,
+                                const int32_t* pixel_ids, int S, int white_bg, int64_t chunk, int n_lanes, void* const* workspaces,
+                                size_t ws_bytes, int64_t max_valid, int64_t max_app, float* rays, uint8_t* rgba, uint8_t* rgba_h,
+                                int32_t* status, void* stream) {
+  const int64_t n = (int64_t)H * W;
+  int rc = check_batch("gnr_render_frame", m, rays, n, S, chunk, n_lanes, workspaces, ws_bytes, max_valid, max_app);
+  if (rc) return rc;
+  if (!pixel_ids || !rgba || !rgba_h) {
+    gnr_set_error("gnr_render_frame: null pixel_ids, rgba or rgba_h");
+    return -1;
+  }
+  DeviceGuard g(m->device);
+  rc = gnr_generate_rays(pose_h, dir_x, dir_y, H, W, pixel_ids, 0, n, rays, stream);
+  if (rc) return rc;
+  rc = render_batch_impl(m, rays, n, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, nullptr, nullptr, rgba, pixel_ids,
+                         status, nullptr, (cudaStream_t)stream);
+  if (rc) return rc;
+  GNR_CUDA_OK(cudaMemcpyAsync(rgba_h, rgba, (size_t)n * 4, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  return 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1649,8 +1781,7 @@ extern "C" int gnr_render_host(GnrModel* m, const float* rays_h, int64_t n_rays,
   }
   DeviceGuard g(m->device);
   if (chunk > n_rays && n_rays > 0) chunk = n_rays;
-  GnrWs L = gnr_ws_layout(m, chunk, S, max_valid, max_app);
-  const size_t ws_one = align_up(L.total, 256);
+  const size_t ws_one = align_up(gnr_ws_layout(m, chunk, S, max_valid, max_app, 1).total, 256);
   if (m->host_chunk != chunk || m->host_ws_bytes < 2 * ws_one) {
     cudaDeviceSynchronize();
     free_dev(m->host_ws);
@@ -1671,7 +1802,7 @@ extern "C" int gnr_render_host(GnrModel* m, const float* rays_h, int64_t n_rays,
   for (int i = 0; i < 2; ++i) {
     if (!m->host_streams[i]) GNR_CUDA_OK(cudaStreamCreateWithFlags(&m->host_streams[i], cudaStreamNonBlocking));
   }
-  int rc = gnr_check_chunk(m, chunk, S, max_valid, max_app, m->host_ws, ws_one);
+  int rc = gnr_check_chunk(m, chunk, S, max_valid, max_app, m->host_ws, ws_one, 1);
   if (rc) return rc;
   const int64_t n_chunks = (n_rays + chunk - 1) / chunk;
   if (n_chunks > m->host_status_slots) {
@@ -1691,11 +1822,11 @@ extern "C" int gnr_render_host(GnrModel* m, const float* rays_h, int64_t n_rays,
     float* d_rgb = m->host_rgb + (size_t)b * chunk * 3;
     float* d_depth = m->host_depth + (size_t)b * chunk;
     GNR_CUDA_OK(cudaMemcpyAsync(d_rays, rays_h + first * 6, (size_t)n * 24, cudaMemcpyHostToDevice, st));
-    rc = render_chunk_impl(m, d_rays, n, S, white_bg, ws, max_valid, max_app, d_rgb, d_depth, st);
+    const GnrPixelSink sink{nullptr, nullptr, &st_all[(size_t)c * GNR_ST_WORDS]};
+    rc = render_chunk_impl(m, d_rays, n, S, white_bg, ws, max_valid, max_app, d_rgb, d_depth, st, &sink);
     if (rc) return rc;
     if (rgb_h) GNR_CUDA_OK(cudaMemcpyAsync(rgb_h + first * 3, d_rgb, (size_t)n * 12, cudaMemcpyDeviceToHost, st));
     if (depth_h) GNR_CUDA_OK(cudaMemcpyAsync(depth_h + first, d_depth, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
-    GNR_CUDA_OK(cudaMemcpyAsync(&st_all[(size_t)c * GNR_ST_WORDS], ws, GNR_ST_WORDS * 4, cudaMemcpyDeviceToHost, st));
   }
   GNR_CUDA_OK(cudaStreamSynchronize(m->host_streams[0]));
   GNR_CUDA_OK(cudaStreamSynchronize(m->host_streams[1]));

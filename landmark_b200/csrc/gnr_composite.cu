@@ -157,15 +157,31 @@ expand_app_packed_kernel(const float2* __restrict__ packed, int kbits,
 
 // rgb_map = sum_j w_j rgb_j (+ 1 - acc), clamp to [0,1]; depth_map = sum w t
 // (app/models/gridnerf_sequential.py:493-501).
+__device__ __forceinline__ uchar4 to_rgba8(float r, float g, float b) {  // x 255, truncated; alpha 255
+  return make_uchar4((unsigned char)__float2uint_rz(fminf(fmaxf(r * 255.0f, 0.0f), 255.0f)),
+                     (unsigned char)__float2uint_rz(fminf(fmaxf(g * 255.0f, 0.0f), 255.0f)),
+                     (unsigned char)__float2uint_rz(fminf(fmaxf(b * 255.0f, 0.0f), 255.0f)), 255);
+}
+
 __device__ __forceinline__ void write_pixel(float r, float g, float b, const float* __restrict__ acc, const float* __restrict__ depth,
-                                            int64_t ray, int white_bg, float* __restrict__ rgb_map, float* __restrict__ depth_map) {
+                                            int64_t ray, int white_bg, float* __restrict__ rgb_map, float* __restrict__ depth_map,
+                                            const GnrPixelSink& sink) {
+  const float bg = white_bg ? (1.0f - acc[ray]) : 0.0f;
+  r = fminf(fmaxf(r + bg, 0.0f), 1.0f);
+  g = fminf(fmaxf(g + bg, 0.0f), 1.0f);
+  b = fminf(fmaxf(b + bg, 0.0f), 1.0f);
   if (rgb_map) {
-    const float bg = white_bg ? (1.0f - acc[ray]) : 0.0f;
-    rgb_map[ray * 3 + 0] = fminf(fmaxf(r + bg, 0.0f), 1.0f);
-    rgb_map[ray * 3 + 1] = fminf(fmaxf(g + bg, 0.0f), 1.0f);
-    rgb_map[ray * 3 + 2] = fminf(fmaxf(b + bg, 0.0f), 1.0f);
+    rgb_map[ray * 3 + 0] = r;
+    rgb_map[ray * 3 + 1] = g;
+    rgb_map[ray * 3 + 2] = b;
   }
   if (depth_map) depth_map[ray] = depth[ray];
+  if (sink.rgba) reinterpret_cast<uchar4*>(sink.rgba)[sink.pixel_ids[ray]] = to_rgba8(r, g, b);
+}
+
+// The chunk's status block is complete when the compositing starts: its first block hands it on.
+__device__ __forceinline__ void write_status(const int32_t* __restrict__ status, const GnrPixelSink& sink) {
+  if (sink.status && blockIdx.x == 0 && threadIdx.x < GNR_ST_WORDS) sink.status[threadIdx.x] = status[threadIdx.x];
 }
 
 // One thread per ray, ranks in order, the loads of eight ranks in flight (one rank at a time, each step waited for its
@@ -174,7 +190,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 composite_kernel(const float* __restrict__ app_weight, const int32_t* __restrict__ app_counts,
                  const int32_t* __restrict__ app_offsets, const float* __restrict__ app_rgb, const float* __restrict__ acc, const float* __restrict__ depth,
                  int64_t n_rays, long long app_capacity, int white_bg, float* __restrict__ rgb_map,
-                 float* __restrict__ depth_map) {
+                 float* __restrict__ depth_map, const int32_t* __restrict__ status, GnrPixelSink sink) {
+  write_status(status, sink);
   const int lane = threadIdx.x & 31;
   const int64_t group = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (group * 32 >= n_rays) return;
@@ -206,7 +223,7 @@ composite_kernel(const float* __restrict__ app_weight, const int32_t* __restrict
       b = fmaf(w[i], cb[i], b);
     }
   }
-  if (has_ray) write_pixel(r, g, b, acc, depth, ray, white_bg, rgb_map, depth_map);
+  if (has_ray) write_pixel(r, g, b, acc, depth, ray, white_bg, rgb_map, depth_map, sink);
 }
 
 // Ray-by-ray lists (small chunks): one warp per ray, 32 entries loaded at a time, summed in order with shuffles.
@@ -214,7 +231,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 composite_rays_kernel(const float* __restrict__ app_weight, const int32_t* __restrict__ app_counts,
                       const int32_t* __restrict__ app_base, const float* __restrict__ app_rgb, const float* __restrict__ acc,
                       const float* __restrict__ depth, int64_t n_rays, long long app_capacity, int white_bg,
-                      float* __restrict__ rgb_map, float* __restrict__ depth_map) {
+                      float* __restrict__ rgb_map, float* __restrict__ depth_map, const int32_t* __restrict__ status,
+                      GnrPixelSink sink) {
+  write_status(status, sink);
   const int lane = threadIdx.x & 31;
   const int64_t ray = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (ray >= n_rays) return;
@@ -238,7 +257,7 @@ composite_rays_kernel(const float* __restrict__ app_weight, const int32_t* __res
       b = fmaf(wi, __shfl_sync(0xffffffffu, cb, i), b);
     }
   }
-  if (lane == 0) write_pixel(r, g, b, acc, depth, ray, white_bg, rgb_map, depth_map);
+  if (lane == 0) write_pixel(r, g, b, acc, depth, ray, white_bg, rgb_map, depth_map, sink);
 }
 
 }  // namespace
@@ -281,13 +300,15 @@ int launch_app_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, c
 }
 
 int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const GnrWs& L, float* rgb_map,
-                     float* depth_map, cudaStream_t st, int march_lanes) {
+                     float* depth_map, cudaStream_t st, int march_lanes, const GnrPixelSink* sink_in) {
   (void)m;
+  const GnrPixelSink sink = sink_in ? *sink_in : GnrPixelSink{nullptr, nullptr, nullptr};
+  const int32_t* status = (const int32_t*)(ws + L.status);
   if (march_lanes == 32) {  // ray-by-ray lists
     composite_rays_kernel<<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
         (const float*)(ws + L.app_weight), (const int32_t*)(ws + L.app_counts), (const int32_t*)(ws + L.app_offsets),
         (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc), (const float*)(ws + L.depth), n, L.max_app, white_bg, rgb_map,
-        depth_map);
+        depth_map, status, sink);
     return (int)cudaGetLastError();
   }
   const int64_t groups = (n + 31) / 32;
@@ -296,7 +317,7 @@ int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const
   composite_kernel<<<blocks, kWarpsPerBlock * 32, 0, st>>>(
       (const float*)(ws + L.app_weight), (const int32_t*)(ws + L.app_counts), (const int32_t*)(ws + L.app_offsets),
       (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc), (const float*)(ws + L.depth), n, app_capacity,
-      white_bg, rgb_map, depth_map);
+      white_bg, rgb_map, depth_map, status, sink);
   return (int)cudaGetLastError();
 }
 
@@ -304,10 +325,7 @@ namespace {
 __global__ void rgba8_kernel(const float* __restrict__ rgb, long long n, uchar4* __restrict__ out) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float r = rgb[i * 3 + 0] * 255.0f, g = rgb[i * 3 + 1] * 255.0f, b = rgb[i * 3 + 2] * 255.0f;
-  out[i] = make_uchar4((unsigned char)__float2uint_rz(fminf(fmaxf(r, 0.0f), 255.0f)),
-                       (unsigned char)__float2uint_rz(fminf(fmaxf(g, 0.0f), 255.0f)),
-                       (unsigned char)__float2uint_rz(fminf(fmaxf(b, 0.0f), 255.0f)), 255);
+  out[i] = to_rgba8(rgb[i * 3 + 0], rgb[i * 3 + 1], rgb[i * 3 + 2]);
 }
 }  // namespace
 

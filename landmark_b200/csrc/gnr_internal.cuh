@@ -8,6 +8,7 @@
 #include "gridnerf_b200.h"
 
 #define GNR_MAX_PLANES 9
+#define GNR_MAX_LANES 8
 #define GNR_SM_COUNT_FALLBACK 148
 
 // One plane/line pair in device layout: plane [H][W][C] channel-last, line [L][C];
@@ -93,6 +94,17 @@ struct GnrModel {
   int64_t host_status_slots;
   cudaStream_t host_streams[2];
   cudaEvent_t host_events[2];
+  // lanes of gnr_render_batch / gnr_render_frame
+  cudaStream_t lane_streams[GNR_MAX_LANES];
+  cudaEvent_t lane_events[GNR_MAX_LANES + 1];
+  int32_t* forward_status;  // pinned
+};
+
+// Where the compositing leaves a chunk's pixels and its status block, beside rgb_map / depth_map.
+struct GnrPixelSink {
+  uint8_t* rgba;             // null, or the RGBA8 image ...
+  const int32_t* pixel_ids;  // ... and the pixel of every ray of the chunk
+  int32_t* status;           // null, or 8 words of device or pinned host memory
 };
 
 // Scalar parameters every sampling-dependent kernel needs (passed by value).
@@ -146,14 +158,14 @@ struct GnrCoords {
 };
 
 void gnr_set_error(const char* fmt, ...);
-GnrWs gnr_ws_layout(const GnrModel* m, int64_t n_rays, int S, int64_t max_valid, int64_t max_app);
+GnrWs gnr_ws_layout(const GnrModel* m, int64_t n_rays, int S, int64_t max_valid, int64_t max_app, int render_only = 0);
 GnrSampleParams gnr_sample_params(const GnrModel* m, int S);
 // What every launch of the sampler needs from the model, checked on the host before anything is
 // enqueued: with sampling_mode 1 the hull tables must have been uploaded for exactly S samples.
 int gnr_check_sampler(const GnrModel* m, int S);
 int gnr_check_lattice(const GnrModel* m);  // refuses a lattice that is older than the density planes
 int gnr_check_chunk(const GnrModel* m, int64_t n_rays, int S, int64_t max_valid, int64_t max_app,
-                    const void* ws, size_t ws_bytes);
+                    const void* ws, size_t ws_bytes, int render_only = 0);
 
 // launchers (each enqueues on `st`, returns cudaGetLastError as int)
 // (`status`: also zero this status block)
@@ -230,7 +242,7 @@ int launch_mlp_tc(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& 
                   float* feat_out, const unsigned char* prod, int tile_bytes, float* rgb,
                   int32_t* status, int force_unfused, cudaStream_t st, int basis_only = 0);
 int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const GnrWs& L, float* rgb_map,
-                     float* depth_map, cudaStream_t st, int march_lanes = 0);
+                     float* depth_map, cudaStream_t st, int march_lanes = 0, const GnrPixelSink* sink = nullptr);
 int launch_exclusive_scan(const int32_t* counts, int32_t* offsets, int32_t* block_sums, int64_t n,
                           int32_t* status, int total_slot, int overflow_slot, int64_t capacity,
                           cudaStream_t st);

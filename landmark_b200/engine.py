@@ -47,6 +47,31 @@ class FrameRenderer:
         self.model.render_rays(rays, self.n_samples, self.white_bg, chunk=self.chunk, rgb_out=rgb_out,
                                overlap=self.streams if self.streams > 1 else False)
 
+    STATUS_RING = 8  # frames whose status blocks are kept apart
+
+    def render_frame(self, pose: np.ndarray, H: int, W: int, focal: float, pixel_ids: torch.Tensor, rgba: torch.Tensor,
+                     host_image: torch.Tensor):
+        """A whole frame on one GPU in one library call: rays of ``pixel_ids`` (every pixel once), chunk loop, RGBA8 pixels at
+        their places in ``rgba`` and their copy to ``host_image`` (pinned).  Returns the event behind it."""
+        from .rays import device_tables
+
+        n = H * W
+        bufs = self.__dict__.get("_frame_buffers")
+        if bufs is None or bufs[0].shape[0] != n:
+            n_chunks = (n + self.chunk - 1) // self.chunk
+            bufs = self._frame_buffers = (torch.empty((n, 6), dtype=torch.float32, device=self.device),
+                                          torch.zeros((self.STATUS_RING, n_chunks, 8), dtype=torch.int32).pin_memory())
+            self._frame_turn = 0
+        rays, ring = bufs
+        status = ring[self._frame_turn]
+        self._frame_turn = (self._frame_turn + 1) % self.STATUS_RING
+        self.model.render_frame(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg,
+                                self.chunk, self.streams, rays, rgba, host_image, status)
+        ev = torch.cuda.Event()
+        ev.record(torch.cuda.current_stream(self.device))
+        self.model._pending_status, self.model._pending_event = status, ev
+        return ev
+
     def finish(self):
         self.model.check_pending_status()
 
@@ -233,6 +258,8 @@ class NerfDDPRunner:
             raise RuntimeError("enqueue / run_batch is the main rank's call; other ranks run serve()")
         pose = np.asarray(single_pose.cpu() if isinstance(single_pose, torch.Tensor) else single_pose, dtype=np.float32)
         focal = self._focal_of(pose)
+        if self.world == 1 and host_image.is_pinned() and getattr(self.renderer, "render_frame", None) is not None:
+            return self.renderer.render_frame(pose[:3, :4], self.H, self.W, focal, self.shard.pixel_ids, self.rgba, host_image)
         pose, focal, _ = self._broadcast(pose[:3, :4], focal, False)
         self.renderer.render_pixels(pose, self.H, self.W, focal, self.shard.pixel_ids, self.rgb[: self.shard.n_local])
         self.shard.assemble(self.rgb, self.image)

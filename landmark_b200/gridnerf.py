@@ -325,6 +325,7 @@ class B200GridNeRF(torch.nn.Module):
         lines to channel-last, bit-packs the occupancy volume, re-tiles the MLP weights."""
         self._release()
         self._hull_tables_for = -1
+        self._ws_bytes.clear()
         dev_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         cfg = self._config()
         h = C.c_void_p(0)
@@ -500,8 +501,10 @@ class B200GridNeRF(torch.nn.Module):
         per_app = min(n_samples, self.app_capacity_per_ray)
         return max(1, n_rays * per_valid), max(1, n_rays * per_app)
 
-    def workspace(self, n_rays: int, n_samples: int, slot: int = 0):
-        """Scratch buffer of chunk slot ``slot`` (one per stream that renders chunks concurrently).
+    def workspace(self, n_rays: int, n_samples: int, slot: int = 0, stages: bool = False):
+        """Scratch buffer of chunk slot ``slot`` (one per stream that renders chunks concurrently), large enough for the
+        rendering entries; ``stages``: for the stage-wise entries, whose id lists, per-sample features and product tiles a
+        render does not need (90 % of the whole where one kernel does the appearance path).
 
         A slot keeps ONE buffer and only ever replaces it by a larger one: the library derives the
         layout from the call's arguments, so a larger buffer serves every smaller shape.  Before a
@@ -511,12 +514,12 @@ class B200GridNeRF(torch.nn.Module):
         (``GraphedFrameRenderer`` does), which keeps that memory out of the allocator for as long
         as the graph lives."""
         max_valid, max_app = self.capacities(n_rays, n_samples)
-        key = (n_rays, n_samples, max_valid, max_app)
+        key = (n_rays, n_samples, max_valid, max_app, stages)
         need = self._ws_bytes.get(key)
         if need is None:
             nbytes = C.c_size_t(0)
-            check(lib.gnr_workspace_bytes(self._handle, n_rays, n_samples, max_valid, max_app, C.byref(nbytes)),
-                  "gnr_workspace_bytes")
+            query = lib.gnr_workspace_bytes if stages else lib.gnr_render_workspace_bytes
+            check(query(self._handle, n_rays, n_samples, max_valid, max_app, C.byref(nbytes)), "gnr_workspace_bytes")
             if len(self._ws_bytes) > 256:
                 self._ws_bytes.clear()
             need = self._ws_bytes[key] = int(nbytes.value)
@@ -557,6 +560,8 @@ class B200GridNeRF(torch.nn.Module):
             raise RuntimeError("model parameters were never committed: call load(ckpt) or commit()")
         if rays_chunk.device != self.device and rays_chunk.device.type != "cuda":
             raise RuntimeError("rays must live on the model's CUDA device")
+        if rays_chunk.dtype == torch.float32 and rays_chunk.is_contiguous():
+            return rays_chunk
         return rays_chunk.detach().to(torch.float32).contiguous()
 
     def read_status(self, ws_ptr) -> np.ndarray:
@@ -587,12 +592,17 @@ class B200GridNeRF(torch.nn.Module):
         depth = torch.empty((n,), dtype=torch.float32, device=self.device)
         if n == 0:
             return {"rgb_map": rgb, "depth_map": depth}, {}
-        with torch.cuda.device(self.device):
-            keep, ws_ptr, ws_bytes, max_valid, max_app = self.workspace(n, s)
-            check(lib.gnr_render_chunk(self._handle, _ptr(rays), n, s, int(bool(white_bg)), ws_ptr, ws_bytes,
-                                       max_valid, max_app, _ptr(rgb), _ptr(depth), _stream()), "gnr_render_chunk")
-            if self.check_status_every_call:
-                self.raise_on_status(self.read_status(ws_ptr))
+        keep, ws_ptr, ws_bytes, max_valid, max_app = self.workspace(n, s)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        if self.check_status_every_call:  # one call: the chunk, the wait for it, its status block
+            st = (C.c_int32 * _lib.ST_WORDS)()
+            check(lib.gnr_render_forward(self._handle, rays.data_ptr(), n, s, int(bool(white_bg)), ws_ptr, ws_bytes, max_valid,
+                                         max_app, rgb.data_ptr(), depth.data_ptr(), st, stream), "gnr_render_forward")
+            self.last_status = np.frombuffer(st, dtype=np.int32).astype(np.int64)
+            self.raise_on_status(self.last_status)
+        else:
+            check(lib.gnr_render_chunk(self._handle, rays.data_ptr(), n, s, int(bool(white_bg)), ws_ptr, ws_bytes, max_valid,
+                                       max_app, rgb.data_ptr(), depth.data_ptr(), stream), "gnr_render_chunk")
         return {"rgb_map": rgb, "depth_map": depth}, {}
 
     # -- stage-wise access for parity tests and profiling --------------------------------------------
@@ -607,7 +617,7 @@ class B200GridNeRF(torch.nn.Module):
         dev = self.device
         out = {}
         with torch.cuda.device(dev):
-            keep, ws_ptr, ws_bytes, max_valid, max_app = self.workspace(n, s)
+            keep, ws_ptr, ws_bytes, max_valid, max_app = self.workspace(n, s, stages=True)
             words = (s + 31) // 32
             t_min = torch.empty(n, dtype=torch.float32, device=dev)
             counts = torch.empty(n, dtype=torch.int32, device=dev)
@@ -694,47 +704,56 @@ class B200GridNeRF(torch.nn.Module):
             rgb_out = torch.empty((n, 3), dtype=torch.float32, device=self.device)
         if depth_out is None:
             depth_out = torch.empty((n,), dtype=torch.float32, device=self.device)
+        if n == 0:
+            return rgb_out, depth_out
         chunk = max(1, min(chunk, n))
-        n_chunks = max(1, (n + chunk - 1) // chunk)
-        status = torch.zeros((n_chunks, _lib.ST_WORDS), dtype=torch.int32, device=self.device)
-        n_side = 2 if overlap is True else int(overlap or 0)
-        use_side = n_side > 1 and n_chunks > 1
-        with torch.cuda.device(self.device):
-            main = torch.cuda.current_stream()
-            if use_side:
-                if len(getattr(self, "_side_streams", None) or ()) < n_side:
-                    self._side_streams = [torch.cuda.Stream(device=self.device) for _ in range(n_side)]
-                for st_ in self._side_streams[:n_side]:
-                    if after is not None:
-                        st_.wait_event(after)
-                    else:
-                        st_.wait_stream(main)
-            used = {}
-            for ci, first in enumerate(range(0, n, chunk)):
-                m = min(chunk, n - first)
-                slot = ci % n_side if use_side else 0
-                keep, ws_ptr, ws_bytes, max_valid, max_app = self.workspace(chunk, s, slot)
-                used[slot] = keep
-                stream = self._side_streams[slot] if use_side else main
-                with torch.cuda.stream(stream):
-                    check(lib.gnr_render_chunk(self._handle, C.c_void_p(rays.data_ptr() + first * 24), m, s,
-                                               int(bool(white_bg)), ws_ptr, ws_bytes, max_valid, max_app,
-                                               C.c_void_p(rgb_out.data_ptr() + first * 12),
-                                               C.c_void_p(depth_out.data_ptr() + first * 4),
-                                               C.c_void_p(stream.cuda_stream)), "gnr_render_chunk")
-                    status[ci].copy_(keep[(-keep.data_ptr()) % 256:][: 4 * _lib.ST_WORDS].view(torch.int32))
-            if use_side:
-                for st_ in self._side_streams[:n_side]:
-                    main.wait_stream(st_)
-        self._pending_status = status
-        self._last_workspaces = list(used.values())
+        n_chunks = (n + chunk - 1) // chunk
+        status = torch.empty((n_chunks, _lib.ST_WORDS), dtype=torch.int32, device=self.device)
+        lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, n_chunks, overlap)
+        check(lib.gnr_render_batch(self._handle, rays.data_ptr(), n, s, int(bool(white_bg)), chunk, lanes, ws, ws_bytes, max_valid,
+                                   max_app, rgb_out.data_ptr(), depth_out.data_ptr(), status.data_ptr(),
+                                   after.cuda_event if after is not None and lanes > 1 else None,
+                                   torch.cuda.current_stream(self.device).cuda_stream), "gnr_render_batch")
+        self._pending_status, self._pending_event = status, None
         return rgb_out, depth_out
+
+    def _lanes(self, chunk: int, n_samples: int, n_chunks: int, overlap):
+        """Workspaces of a chunk loop: (lanes, their addresses, bytes of each, list capacities)."""
+        want = 2 if overlap is True else int(overlap or 1)
+        lanes = want if want > 1 and n_chunks > 1 else 1
+        ws = (C.c_void_p * lanes)()
+        self._last_workspaces = []
+        ws_bytes = None
+        for slot in range(lanes):
+            keep, ptr, nbytes, max_valid, max_app = self.workspace(chunk, n_samples, slot)
+            ws[slot] = ptr.value
+            ws_bytes = nbytes if ws_bytes is None else min(ws_bytes, nbytes)
+            self._last_workspaces.append(keep)
+        return lanes, ws, ws_bytes, max_valid, max_app
+
+    def render_frame(self, pose: np.ndarray, tables, H: int, W: int, pixel_ids: torch.Tensor, N_samples: int, white_bg: bool,
+                     chunk: int, overlap, rays: torch.Tensor, rgba: torch.Tensor, host_image: torch.Tensor, status: torch.Tensor):
+        """One frame without waiting (gnr_render_frame): ``pose`` ``[3, 4]`` float32, ``tables`` the two direction tables on
+        the device, ``pixel_ids`` every pixel once, ``rays [H * W, 6]`` and ``rgba`` device buffers, ``host_image`` pinned
+        ``uint8 [H, W, 4]``, ``status`` pinned ``int32 [n_chunks, 8]``, complete when the stream's work is."""
+        s = self._samples(N_samples)
+        n = H * W
+        chunk = max(1, min(chunk, n))
+        lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, (n + chunk - 1) // chunk, overlap)
+        pose_c = (C.c_float * 12).from_buffer_copy(pose.astype(np.float32, copy=False).tobytes())
+        check(lib.gnr_render_frame(self._handle, pose_c, tables[0].data_ptr(), tables[1].data_ptr(), H, W, pixel_ids.data_ptr(), s,
+                                   int(bool(white_bg)), chunk, lanes, ws, ws_bytes, max_valid, max_app, rays.data_ptr(),
+                                   rgba.data_ptr(), host_image.data_ptr(), status.data_ptr(),
+                                   torch.cuda.current_stream(self.device).cuda_stream), "gnr_render_frame")
 
     def check_pending_status(self):
         """Synchronise and raise if any chunk of the last ``render_rays`` overflowed a list."""
         st = getattr(self, "_pending_status", None)
         if st is None:
             return None
+        if getattr(self, "_pending_event", None) is not None:  # the status blocks lie in pinned memory
+            self._pending_event.synchronize()
+            self._pending_event = None
         h = st.cpu().numpy().astype(np.int64)
         agg = np.zeros(_lib.ST_WORDS, dtype=np.int64)
         agg[[0, 1, 4]] = h[:, [0, 1, 4]].max(0)

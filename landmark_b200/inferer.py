@@ -51,6 +51,8 @@ class B200NerfDDPInfererImpl:
     """Drop-in for ``TorchNerfDDPInfererImpl``: same constructor argument (a context with
     ``args_nerf`` and ``model_path``), same methods and properties."""
 
+    RENDER_CHUNK = 65536  # rays of a device chunk, unless render_batch_size is larger
+
     def __init__(self, context, profile_stages: bool = False, mlp_mode: Optional[int] = None, preset: str = "exact",
                  **model_options) -> None:
         """``preset`` picks a row of ``PRESETS`` ("exact" is the default so that a drop-in run first
@@ -125,4 +127,13 @@ class B200NerfDDPInfererImpl:
             # the reference's single-block inferer drops app_code (inferer_impl.py:144-145), which fails
             # for an encode_app checkpoint; here it reaches the model
             kw["app_code"] = app_code
+        if self._forward is self._model and not is_train and rays.shape[0] > 0:
+            # The same chunks as one library call: pixels do not depend on how rays are cut into chunks, so chunks of at
+            # least RENDER_CHUNK rays rotate over two lanes and the status blocks are read once at the end, instead of a
+            # wait per chunk of render_batch_size rays (960x540 in chunks of 8192: 64 waits).
+            with torch.inference_mode():
+                self._model.set_app_code(kw.get("app_code"))
+                rgb, _ = self._model.render_rays(rays, N_samples, white_bg, chunk=max(self._chunk_size, self.RENDER_CHUNK), overlap=2)
+                self._model.check_pending_status()
+            return rgb
         return renderer_fn(self._forward, rays, self._chunk_size, **kw)

@@ -205,7 +205,7 @@ class _Chunk:
         self.rays = model._prepare(rays)
         self.n = self.rays.shape[0]
         self.s = model._samples(n_samples)
-        self.keep, self.ws, self.ws_bytes, self.max_valid, self.max_app = model.workspace(self.n, self.s, slot)
+        self.keep, self.ws, self.ws_bytes, self.max_valid, self.max_app = model.workspace(self.n, self.s, slot, stages=True)
         self.kbits = lib.gnr_sample_bits(self.s)
         self.num_valid = self.num_app = 0
         self.ids = self.app_index = None

@@ -31,6 +31,18 @@ def direction_tables(H: int, W: int, focal: float):
 _table_cache = {}
 
 
+def device_tables(H: int, W: int, focal: float, device):
+    """``direction_tables`` on the device, kept per (size, focal length, device)."""
+    dev = torch.device(device)
+    key = (H, W, float(focal), str(dev))
+    if key not in _table_cache:
+        if len(_table_cache) > 8:
+            _table_cache.clear()
+        dx, dy = direction_tables(H, W, float(focal))
+        _table_cache[key] = (dx.to(dev), dy.to(dev))
+    return _table_cache[key]
+
+
 def generate_rays(single_pose, H, W, focal=None, device="cuda", pixel_ids: Optional[torch.Tensor] = None,
                   first_pixel: int = 0, n: Optional[int] = None) -> torch.Tensor:
     """Rays ``[n, 6]`` (origin, un-normalised direction) on ``device``.
@@ -46,13 +58,7 @@ def generate_rays(single_pose, H, W, focal=None, device="cuda", pixel_ids: Optio
         focal = focal.item()
     H, W = int(H), int(W)
     dev = torch.device(device)
-    key = (H, W, float(focal), str(dev))
-    if key not in _table_cache:
-        if len(_table_cache) > 8:
-            _table_cache.clear()
-        dx, dy = direction_tables(H, W, float(focal))
-        _table_cache[key] = (dx.to(dev), dy.to(dev))
-    dx, dy = _table_cache[key]
+    dx, dy = device_tables(H, W, float(focal), dev)
     if pixel_ids is not None:
         pixel_ids = pixel_ids.to(device=dev, dtype=torch.int32).contiguous()
         n = pixel_ids.numel()
