@@ -37,7 +37,7 @@ def renderer_fn(forward: Callable, rays: torch.Tensor, chunk_size: int, **kwargs
 
 
 # Precision presets of the drop-in inferer.  "exact": fp32 everywhere, no termination (what the
-# reference's torch path computes; about 11x slower than "fast" on a city frame).  "fast": the
+# reference's torch path computes; about 4x slower than "fast" on a city frame).  "fast": the
 # configuration the benchmark measures: tcgen05 MLP with fp16 operands, fp16 appearance planes,
 # rays stop at transmittance 2e-5, density from the pre-summed lattice; rgb stays within 1e-4 of
 # "exact" on the tested scenes.
@@ -51,7 +51,8 @@ class B200NerfDDPInfererImpl:
     """Drop-in for ``TorchNerfDDPInfererImpl``: same constructor argument (a context with
     ``args_nerf`` and ``model_path``), same methods and properties."""
 
-    RENDER_CHUNK = 65536  # rays of a device chunk, unless render_batch_size is larger
+    RENDER_CHUNK = 65536      # rays of a device chunk, unless render_batch_size is larger
+    RENDER_SAMPLES = 1 << 25  # and at most that many samples of them: the ids and lists of a chunk grow with both
 
     def __init__(self, context, profile_stages: bool = False, mlp_mode: Optional[int] = None, preset: str = "exact",
                  **model_options) -> None:
@@ -133,7 +134,8 @@ class B200NerfDDPInfererImpl:
             # wait per chunk of render_batch_size rays (960x540 in chunks of 8192: 64 waits).
             with torch.inference_mode():
                 self._model.set_app_code(kw.get("app_code"))
-                rgb, _ = self._model.render_rays(rays, N_samples, white_bg, chunk=max(self._chunk_size, self.RENDER_CHUNK), overlap=2)
+                fit = min(self.RENDER_CHUNK, self.RENDER_SAMPLES // self._model._samples(N_samples))
+                rgb, _ = self._model.render_rays(rays, N_samples, white_bg, chunk=max(self._chunk_size, fit), overlap=2)
                 self._model.check_pending_status()
             return rgb
         return renderer_fn(self._forward, rays, self._chunk_size, **kw)

@@ -122,3 +122,20 @@ def test_fp32_network_wait_expires_and_the_context_survives():
     model.debug_wait()
     again, _ = model(rays, N_samples=spec.n_samples)
     assert torch.equal(good["rgb_map"], again["rgb_map"])
+
+
+def test_inferer_chunks_fit_the_sample_ids():
+    """65536 rays of 40000 samples do not fit the 32-bit ids of a chunk, 8192 do: the drop-in loop takes what fits."""
+    from types import SimpleNamespace
+
+    from landmark_b200.inferer import B200NerfDDPInfererImpl
+
+    spec = scenes.tiny_spec(grid=32).lit()
+    args = scenes.model_args(spec, "cuda:0")
+    args.render_batch_size = 64
+    impl = B200NerfDDPInfererImpl(SimpleNamespace(args_nerf=args, checkpoint=scenes.make_checkpoint(spec), model_path=None))
+    impl.load_model(spec.height, spec.width)
+    impl.model.app_capacity_per_ray = impl.model.valid_capacity_per_ray = 64
+    rays = torch.zeros((65536, 6), device="cuda:0")
+    rays[:, 2], rays[:, 5] = 50.0, 1.0  # above the scene, looking away: no valid sample
+    assert torch.equal(impl.renderer_fn(rays, N_samples=40000), torch.ones_like(rays[:, :3]))
