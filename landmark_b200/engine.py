@@ -56,9 +56,11 @@ class FrameRenderer:
         from .rays import device_tables
 
         n = H * W
+        n_chunks = (n + self.chunk - 1) // self.chunk
         bufs = self.__dict__.get("_frame_buffers")
-        if bufs is None or bufs[0].shape[0] != n:
-            n_chunks = (n + self.chunk - 1) // self.chunk
+        if bufs is None or bufs[0].shape[0] != n or bufs[1].shape[1] != n_chunks:
+            if bufs is not None:  # frames in flight still write status blocks into the pinned ring
+                torch.cuda.synchronize(self.device)
             bufs = self._frame_buffers = (torch.empty((n, 6), dtype=torch.float32, device=self.device),
                                           torch.zeros((self.STATUS_RING, n_chunks, 8), dtype=torch.int32).pin_memory())
             self._frame_turn = 0
@@ -249,6 +251,15 @@ class NerfDDPRunner:
         self.shard.assemble(self.rgb, self.image)
         self.renderer.finish()
 
+    def _whole_frame(self, host_image: torch.Tensor) -> bool:
+        """One library call does the frame: a single rank, FrameRenderer's own stages over a model that has the call, and
+        an image the call can write as plain bytes.  Everything else goes stage by stage."""
+        r = self.renderer
+        return (self.world == 1 and isinstance(r, FrameRenderer) and type(r).render_pixels is FrameRenderer.render_pixels
+                and type(r).to_rgba8 is FrameRenderer.to_rgba8 and hasattr(r.model, "render_frame") and host_image.is_pinned()
+                and host_image.is_contiguous() and host_image.dtype == torch.uint8
+                and tuple(host_image.shape) == (self.H, self.W, 4))
+
     def enqueue(self, single_pose, host_image: torch.Tensor):
         """Everything ``run_batch`` does for one frame except waiting for it: broadcast, render, gather,
         RGBA8, and the copy of the image into ``host_image`` (``uint8 [H, W, 4]``, pinned for an
@@ -258,7 +269,7 @@ class NerfDDPRunner:
             raise RuntimeError("enqueue / run_batch is the main rank's call; other ranks run serve()")
         pose = np.asarray(single_pose.cpu() if isinstance(single_pose, torch.Tensor) else single_pose, dtype=np.float32)
         focal = self._focal_of(pose)
-        if self.world == 1 and host_image.is_pinned() and getattr(self.renderer, "render_frame", None) is not None:
+        if self._whole_frame(host_image):
             return self.renderer.render_frame(pose[:3, :4], self.H, self.W, focal, self.shard.pixel_ids, self.rgba, host_image)
         pose, focal, _ = self._broadcast(pose[:3, :4], focal, False)
         self.renderer.render_pixels(pose, self.H, self.W, focal, self.shard.pixel_ids, self.rgb[: self.shard.n_local])

@@ -139,3 +139,30 @@ def test_inferer_chunks_fit_the_sample_ids():
     rays = torch.zeros((65536, 6), device="cuda:0")
     rays[:, 2], rays[:, 5] = 50.0, 1.0  # above the scene, looking away: no valid sample
     assert torch.equal(impl.renderer_fn(rays, N_samples=40000), torch.ones_like(rays[:, :3]))
+
+
+def test_frames_of_one_renderer_in_changing_chunks_and_images():
+    """The frame call keeps its buffers per image and chunk count; images it cannot write as plain bytes, and renderers
+    with stages of their own, take the stage-wise path.  All give the same bytes."""
+    from landmark_b200.engine import FrameRenderer, NerfDDPRunner
+
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    renderer = FrameRenderer(model, spec.n_samples, chunk=4096)
+    runner = NerfDDPRunner(renderer, spec.height, spec.width, focal=spec.focal)
+    pose = scenes.make_pose(spec)
+    first = runner.run_batch(pose).copy()
+    renderer.chunk = 500  # more status blocks than the ring had
+    assert np.array_equal(first, runner.run_batch(pose))
+    wide = torch.zeros((spec.height, spec.width, 8), dtype=torch.uint8).pin_memory()
+    runner.enqueue(pose, wide[..., :4]).synchronize()
+    assert np.array_equal(first, wide[..., :4].numpy()) and not wide[..., 4:].any()
+    with pytest.raises(RuntimeError):
+        runner.enqueue(pose, torch.zeros((spec.height, spec.width - 1, 4), dtype=torch.uint8).pin_memory())
+
+    class Dark(FrameRenderer):
+        def to_rgba8(self, image, out):
+            super().to_rgba8(image * 0.0, out)
+
+    dark = NerfDDPRunner(Dark(model, spec.n_samples), spec.height, spec.width, focal=spec.focal).run_batch(pose)
+    assert not dark[..., :3].any() and (dark[..., 3] == 255).all()
