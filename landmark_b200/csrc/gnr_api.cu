@@ -397,51 +397,32 @@ extern "C" int gnr_upload_line(GnrModel* m, int kind, int idx, const float* src,
   return 0;
 }
 
-// Coarse occupancy: block (bx, by, bz) covers mask cells [4 b, 4 b + 4] on each axis (its own 4 and
-// the first cell of the next block: a trilinear test whose lower corner lies in the block reads
-// those).  A clear bit therefore proves that the fine test of any such sample sums to zero.
-__global__ void coarse_bits_kernel(const uint32_t* __restrict__ bits, int D, int H, int W, int cD, int cH, int cW,
-                                   uint32_t* __restrict__ coarse) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool in_range = c < (long long)cD * cH * cW;
-  bool any = false;
-  if (in_range) {
+// Coarse occupancy in blocks of 2x2x2 cells, by the lower corner of a trilinear test.  `coarse`: a test whose lower
+// corner lies in block (bx, by, bz) reads cells [2 b, 2 b + 2] on each axis; a clear bit proves that all of them are clear
+// and the test sums to zero.  `full`: every cell of the block itself is set (a cell outside the volume, which is nobody's
+// lower corner, does not count), so that the lower corner of the test is.
+__global__ void block_bits_kernel(const uint32_t* __restrict__ bits, int D, int H, int W, int cD, int cH, int cW,
+                                  uint32_t* __restrict__ coarse, uint32_t* __restrict__ full) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = (long long)cD * cH * cW;
+  bool any = false, all = c < n;
+  if (c < n) {
     const int bx = (int)(c % cW), by = (int)((c / cW) % cH), bz = (int)(c / ((long long)cW * cH));
-    for (int z = 4 * bz; z <= 4 * bz + 4 && z < D && !any; ++z)
-      for (int y = 4 * by; y <= 4 * by + 4 && y < H && !any; ++y)
-        for (int x = 4 * bx; x <= 4 * bx + 4 && x < W; ++x) {
-          const uint32_t bit = (uint32_t)(((long long)z * H + y) * W + x);
-          if ((bits[bit >> 5] >> (bit & 31)) & 1u) {
-            any = true;
-            break;
-          }
-        }
+    for (int e = 0; e < 27; ++e) {
+      const int dx = e % 3, dy = e / 3 % 3, dz = e / 9;
+      const int x = 2 * bx + dx, y = 2 * by + dy, z = 2 * bz + dz;
+      if (x < W && y < H && z < D) {
+        const long long bit = ((long long)z * H + y) * W + x;
+        const bool set = (bits[bit >> 5] >> (bit & 31)) & 1u;
+        any = any || set;
+        if (dx < 2 && dy < 2 && dz < 2) all = all && set;
+      }
+    }
   }
-  const uint32_t word = __ballot_sync(0xffffffffu, any);  // 32 consecutive blocks = one word
-  if ((threadIdx.x & 31) == 0 && c < (((long long)cD * cH * cW + 31) / 32) * 32) coarse[c >> 5] = word;
-}
-
-// The opposite bound: block (bx, by, bz) is "full" if every mask cell of [4 b, 4 b + 4]^3 exists and
-// is set.  A sample whose lower corner lies in a full block then has that corner occupied.
-__global__ void full_bits_kernel(const uint32_t* __restrict__ bits, int D, int H, int W, int cD, int cH, int cW,
-                                 uint32_t* __restrict__ full) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  bool all = c < (long long)cD * cH * cW;
-  if (all) {
-    const int bx = (int)(c % cW), by = (int)((c / cW) % cH), bz = (int)(c / ((long long)cW * cH));
-    all = 4 * bx + 4 < W && 4 * by + 4 < H && 4 * bz + 4 < D;
-    for (int z = 4 * bz; all && z <= 4 * bz + 4; ++z)
-      for (int y = 4 * by; all && y <= 4 * by + 4; ++y)
-        for (int x = 4 * bx; x <= 4 * bx + 4; ++x) {
-          const uint32_t bit = (uint32_t)(((long long)z * H + y) * W + x);
-          if (!((bits[bit >> 5] >> (bit & 31)) & 1u)) {
-            all = false;
-            break;
-          }
-        }
+  const uint32_t any_word = __ballot_sync(0xffffffffu, any), all_word = __ballot_sync(0xffffffffu, all);
+  if ((threadIdx.x & 31) == 0 && c < ((n + 31) / 32) * 32) {  // 32 consecutive blocks = one word
+    coarse[c >> 5] = any_word;
+    full[c >> 5] = all_word;
   }
-  const uint32_t word = __ballot_sync(0xffffffffu, all);
-  if ((threadIdx.x & 31) == 0 && c < (((long long)cD * cH * cW + 31) / 32) * 32) full[c >> 5] = word;
 }
 
 // Per cell: is any of the eight cells a trilinear test with this lower corner reads set (cells outside the volume are not)?
@@ -485,15 +466,12 @@ extern "C" int gnr_upload_alpha_mask(GnrModel* m, const uint8_t* vol, int D, int
   pack_bits_kernel<<<(unsigned)((n_words + 255) / 256), 256, 0, (cudaStream_t)stream>>>(vol, m->alpha_bits, n_vox, n_words);
   GNR_CUDA_OK(cudaGetLastError());
   {
-    const int cD = (D + 3) / 4, cH = (H + 3) / 4, cW = (W + 3) / 4;
+    const int cD = (D + 1) / 2, cH = (H + 1) / 2, cW = (W + 1) / 2;
     const long long n_blocks = (long long)cD * cH * cW, n_cwords = (n_blocks + 31) / 32;
     GNR_CUDA_OK(cudaMalloc(&m->alpha_coarse, (size_t)n_cwords * sizeof(uint32_t)));
-    coarse_bits_kernel<<<(unsigned)((n_cwords * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->alpha_bits, D, H, W, cD, cH,
-                                                                                            cW, m->alpha_coarse);
-    GNR_CUDA_OK(cudaGetLastError());
     GNR_CUDA_OK(cudaMalloc(&m->alpha_full, (size_t)n_cwords * sizeof(uint32_t)));
-    full_bits_kernel<<<(unsigned)((n_cwords * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->alpha_bits, D, H, W, cD, cH, cW,
-                                                                                          m->alpha_full);
+    block_bits_kernel<<<(unsigned)((n_cwords * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        m->alpha_bits, D, H, W, cD, cH, cW, m->alpha_coarse, m->alpha_full);
     GNR_CUDA_OK(cudaGetLastError());
     GNR_CUDA_OK(cudaMalloc(&m->alpha_any8, (size_t)n_words * sizeof(uint32_t)));
     any8_bits_kernel<<<(unsigned)((n_words * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->alpha_bits, D, H, W, m->alpha_any8);
@@ -742,9 +720,9 @@ GnrSampleParams gnr_sample_params(const GnrModel* m, int S) {
   p.a_half[0] = 0.5f * (float)(m->aW - 1);
   p.a_half[1] = 0.5f * (float)(m->aH - 1);
   p.a_half[2] = 0.5f * (float)(m->aD - 1);
-  p.cD = (m->aD + 3) / 4;
-  p.cH = (m->aH + 3) / 4;
-  p.cW = (m->aW + 3) / 4;
+  p.cD = (m->aD + 1) / 2;
+  p.cH = (m->aH + 1) / 2;
+  p.cW = (m->aW + 1) / 2;
   p.S = S;
   p.words = (S + 31) / 32;
   p.kbits = gnr_sample_bits(S);

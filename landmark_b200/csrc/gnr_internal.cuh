@@ -68,8 +68,8 @@ struct GnrModel {
   int lat_valid;  // 0 after a density plane or line was uploaded: the lattice must be rebuilt before the next launch
   // occupancy bits
   uint32_t* alpha_bits;
-  uint32_t* alpha_coarse;  // one bit per 4x4x4 block of mask cells (see coarse_bits_kernel)
-  uint32_t* alpha_full;    // one bit per block: every cell of the block and of its +1 border is set
+  uint32_t* alpha_coarse;  // one bit per 2x2x2 block of mask cells (see block_bits_kernel)
+  uint32_t* alpha_full;    // one bit per block: every cell of it is set
   uint32_t* alpha_any8;    // one bit per mask cell: set if any of the eight corners of the cell (itself and its +1 neighbours) is
   int aD, aH, aW;
   float a_lo[3], a_inv[3];
@@ -116,8 +116,8 @@ struct GnrSampleParams {
   int aD, aH, aW;
   int has_mask;
   const uint32_t* a_bits;
-  const uint32_t* a_coarse;  // null, or 1 bit per 4x4x4 block: set if any cell of the block or of its +1 border is set
-  const uint32_t* a_full;    // null, or 1 bit per 4x4x4 block: every cell of the block and its +1 border is set
+  const uint32_t* a_coarse;  // null, or 1 bit per 2x2x2 block: set if any cell of the block or of its +1 border is set
+  const uint32_t* a_full;    // null, or 1 bit per 2x2x2 block: every cell of the block is set
   const uint32_t* a_any8;    // null, or 1 bit per cell: any of its eight corners is set
   float a_half[3];           // (W - 1) / 2, (H - 1) / 2, (D - 1) / 2
   int cD, cH, cW;

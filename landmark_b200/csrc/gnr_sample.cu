@@ -144,7 +144,9 @@ struct RaySetup {  // what the sample tests need of a ray, in shared memory
 // argument (every operation is a correctly rounded monotone function), so along each axis every sample between the two
 // lies between them, without any tolerance: if both are inside the box all are, if both are outside on the same side
 // none is, and the mask cells of all samples lie in the range spanned by the cells of the two.
-// BLOCKS: the occupancy of that range is looked up in blocks of 4x4x4 cells, else cell by cell.
+// BLOCKS: the occupancy of that range is looked up in blocks of 2x2x2 cells, else cell by cell; a run that spans more
+// than four of either along an axis stays open.  (Blocks of 4x4x4 cells, two at most, left 55 % of a city frame's words
+// open; 22 % is what mixes valid and other samples.)
 template <bool BLOCKS>
 __device__ __forceinline__ int run_by_ends(const GnrSampleParams& p, const RaySetup& r, int k0, int k1) {
   const float t0 = gnr_sample_t(p, r.t_min, k0), t1 = gnr_sample_t(p, r.t_min, k1);
@@ -172,27 +174,33 @@ __device__ __forceinline__ int run_by_ends(const GnrSampleParams& p, const RaySe
     b0[a] = (int)lo;
     b1[a] = (int)hi;
     if (BLOCKS) {
-      b0[a] >>= 2;
-      b1[a] >>= 2;
+      b0[a] >>= 1;
+      b1[a] >>= 1;
     } else {
       inside_cell = inside_cell && b0[a] == b1[a] && (float)b0[a] != lo;
     }
-    if (b1[a] - b0[a] > 1) return 2;
+    if (b1[a] - b0[a] > 3) return 2;
   }
   const uint32_t nx = (uint32_t)(BLOCKS ? p.cW : p.aW), ny = (uint32_t)(BLOCKS ? p.cH : p.aH);
   const uint32_t* any_bits = BLOCKS ? p.a_coarse : p.a_any8;
   const uint32_t* all_bits = BLOCKS ? p.a_full : p.a_bits;
-  bool any = false, all = p.a_thres == 0.0f;
+  const uint32_t row_bits = (2u << (b1[0] - b0[0])) - 1u;  // the range along x: at most four neighbouring bits
+  uint32_t any = 0u, miss = 0u;
   for (int z = b0[2]; z <= b1[2]; ++z)
-    for (int y = b0[1]; y <= b1[1]; ++y)
-      for (int x = b0[0]; x <= b1[0]; ++x) {
-        const uint32_t at = ((uint32_t)z * ny + (uint32_t)y) * nx + (uint32_t)x;
-        any = any || ((__ldg(any_bits + (at >> 5)) >> (at & 31)) & 1u);
-        all = all && ((__ldg(all_bits + (at >> 5)) >> (at & 31)) & 1u);
+    for (int y = b0[1]; y <= b1[1]; ++y) {
+      const uint32_t at = ((uint32_t)z * ny + (uint32_t)y) * nx + (uint32_t)b0[0], word = at >> 5, s = at & 31u;
+      uint32_t a = __ldg(any_bits + word) >> s, f = __ldg(all_bits + word) >> s;
+      if (row_bits >> (31u - s) > 1u) {  // (the row goes on in the next word)
+        a |= __ldg(any_bits + word + 1) << (32u - s);
+        f |= __ldg(all_bits + word + 1) << (32u - s);
       }
+      any |= a & row_bits;
+      miss |= ~f & row_bits;
+    }
+  const bool all = miss == 0u && p.a_thres == 0.0f;
   // no occupied corner in reach: the sum is zero.  Threshold zero: with its lower corner occupied a sample has a positive
   // weight, (x0 + 1 - ix)(y0 + 1 - iy)(z0 + 1 - iz), wherever in the cell it lies; strictly inside a cell any corner will do
-  if (!any) return 0;
+  if (any == 0u) return 0;
   if (!BLOCKS && inside_cell && p.a_thres == 0.0f) return 1;
   return all ? 1 : 2;
 }
@@ -212,10 +220,10 @@ constexpr int kSampleWarps = 4;
 // samples; the words that stay open are cut into runs of eight samples, 32 runs at a time, and decided the same way cell
 // by cell; the runs that stay open are tested sample by sample, four runs at a time.  Each step queues what it leaves
 // open in shared memory, so that the lanes of the next one are full.
-// Bound by instruction issue (77 % of the slots).  A ray's latency is a few passes instead of one dependent step per
-// sample, and most samples are never looked at: of a city frame's words 40 % stay open after the first step and 0.5 runs
-// of each after the second.  98,304 rays x 256 samples: 65 us, 51 warp instructions per word (104 us and 87 when every
-// open word was tested sample by sample); 333 rays x 128 samples: 14 us, 121 us with a thread walking each ray.
+// Bound by instruction issue.  A ray's latency is a few passes instead of one dependent step per sample, and most samples
+// are never looked at: of a city frame's words 22 % stay open after the first step and 0.9 runs of each after the second.
+// 131,072 rays x 384 samples (12 words a ray): 89 us, 38 warp instructions per word (119 us with first-step blocks of
+// 4x4x4 cells, which left 55 % of the words open); 333 rays x 128 samples: 14 us, 121 us with a thread walking each ray.
 __global__ void __launch_bounds__(kSampleWarps * 32, 8)
 sample_words_kernel(const __grid_constant__ GnrSampleParams p, const float* __restrict__ rays, int64_t n_rays, int per_warp,
                     float* __restrict__ t_min_out, uint32_t* __restrict__ words_out, int32_t* __restrict__ counts_out,
