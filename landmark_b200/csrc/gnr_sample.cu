@@ -139,17 +139,28 @@ struct RaySetup {  // what the sample tests need of a ray, in shared memory
   float o[3], t_min, d[3], pad;
 };
 
-// What the two end samples of a run prove about all samples k0 .. k1 between them (dense sampler): 0 = none is valid,
-// 1 = all are, 2 = still open.  fl(t_min + fl(step k)), the point, and the mask index are each monotone in their
-// argument (every operation is a correctly rounded monotone function), so along each axis every sample between the two
-// lies between them, without any tolerance: if both are inside the box all are, if both are outside on the same side
-// none is, and the mask cells of all samples lie in the range spanned by the cells of the two.
+// What the two ends of a run prove about all its samples k0 .. k1: 0 = none is valid, 1 = all are, 2 = still open.
+// fl(t_min + fl(step k)), the point, and the mask index are each monotone in their argument (every operation is a
+// correctly rounded monotone function), so along each axis every sample between the two end samples lies between them,
+// without any tolerance: if both are inside the box all are, if both are outside on the same side none is, and the mask
+// cells of all samples lie in the range spanned by the cells of the two.  The hull sampler's distance is the sum of a
+// falling term, near (1 - u_k), and a monotone one, far u_k: its run lies between the sums of their smallest and of their
+// largest values, which for a near distance of 0.05 is hardly wider than the two end samples.
 // BLOCKS: the occupancy of that range is looked up in blocks of 2x2x2 cells, else cell by cell; a run that spans more
 // than four of either along an axis stays open.  (Blocks of 4x4x4 cells, two at most, left 55 % of a city frame's words
 // open; 22 % is what mixes valid and other samples.)
 template <bool BLOCKS>
 __device__ __forceinline__ int run_by_ends(const GnrSampleParams& p, const RaySetup& r, int k0, int k1) {
-  const float t0 = gnr_sample_t(p, r.t_min, k0), t1 = gnr_sample_t(p, r.t_min, k1);
+  float t0, t1;
+  if (p.mode == 0) {
+    t0 = gnr_sample_t(p, r.t_min, k0);
+    t1 = gnr_sample_t(p, r.t_min, k1);
+  } else {
+    if (!(fabsf(r.t_min) < 1e30f)) return 2;  // (far u_k is not monotone where 0 x inf comes up)
+    const float f0 = __fmul_rn(r.t_min, __ldg(p.hull_u + k0)), f1 = __fmul_rn(r.t_min, __ldg(p.hull_u + k1));
+    t0 = __fadd_rn(__ldg(p.hull_a + k1), fminf(f0, f1));
+    t1 = __fadd_rn(__ldg(p.hull_a + k0), fmaxf(f0, f1));
+  }
   float q0[3], q1[3];
   bool in = true;
 #pragma unroll
@@ -274,13 +285,10 @@ sample_words_kernel(const __grid_constant__ GnrSampleParams p, const float* __re
   const int W = p.words, items = mine * W;
   int ray = lane / W, word = lane - ray * W;  // this lane's item: word `word` of ray `ray` of the warp
   const int ray_step = 32 / W, word_step = 32 - ray_step * W;
-  // (the hull sampler's distances are a sum of a falling and a rising term and need not be monotone to the last bit:
-  // its samples are all tested one by one)
-  const bool dense = p.mode == 0;
   for (int i0 = 0; i0 < items; i0 += 32) {
     const bool has = i0 + lane < items;
     int verdict = 0;
-    if (has) verdict = dense ? run_by_ends<true>(p, s_ray[warp][ray], 32 * word, min(32 * word + 31, p.S - 1)) : 2;
+    if (has) verdict = run_by_ends<true>(p, s_ray[warp][ray], 32 * word, min(32 * word + 31, p.S - 1));
     const uint32_t open = __ballot_sync(0xffffffffu, verdict == 2);
     s_bits[warp][lane] = verdict != 1 ? 0u : (p.S - 32 * word >= 32 ? 0xffffffffu : (1u << (p.S - 32 * word)) - 1u);
     s_item[warp][lane] = ((uint32_t)ray << 16) | (uint32_t)word;
@@ -296,7 +304,7 @@ sample_words_kernel(const __grid_constant__ GnrSampleParams p, const float* __re
         const uint32_t it = s_item[warp][at];
         const int k = 32 * (int)(it & 0xffffu) + 8 * run;
         if (k < p.S) {
-          v = dense ? run_by_ends<false>(p, s_ray[warp][it >> 16], k, min(k + 7, p.S - 1)) : 2;
+          v = run_by_ends<false>(p, s_ray[warp][it >> 16], k, min(k + 7, p.S - 1));
           if (v == 1) atomicOr(&s_bits[warp][at], (k + 8 <= p.S ? 0xffu : (1u << (p.S - k)) - 1u) << (8 * run));
         }
       }

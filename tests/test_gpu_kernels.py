@@ -166,3 +166,54 @@ def test_frames_of_one_renderer_in_changing_chunks_and_images():
 
     dark = NerfDDPRunner(Dark(model, spec.n_samples), spec.height, spec.width, focal=spec.focal).run_batch(pose)
     assert not dark[..., :3].any() and (dark[..., 3] == 255).all()
+
+
+@pytest.mark.parametrize("n,samples,thres,mask", [
+    (1, 1, 0.0, True), (5, 33, 0.0, True), (130, 97, 0.5, True), (64, 128, 0.0, False), (6000, 64, 0.0, True), (3001, 1061, 0.0, True)])
+def test_hull_sampler_words_at_edges(n, samples, thres, mask):
+    """The hull sampler decides runs of samples from their ends too: words equal bit for bit to testing every sample, rays
+    that look up, (almost) along the ground plane (far up to infinity, or 0 / 0 on it) and from below it among them."""
+    from landmark_b200.gridnerf import B200GridNeRF
+
+    spec = scenes.tiny_spec().lit()
+    spec.alpha_filter_thres = thres
+    field, ckpt = oracle_field(spec)
+    if not mask:
+        ckpt = {k: v for k, v in ckpt.items() if not k.startswith("alphaMask")}
+    args = scenes.model_args(spec, "cuda:0")
+    args.sampling_opt, args.n_importance = 1, samples
+    kw = dict(ckpt["kwargs"])
+    kw.update({"device": "cuda:0", "args": args, "is_train": False})
+    model = B200GridNeRF(**kw)
+    model.load(ckpt)
+    g = torch.Generator().manual_seed(n + samples)
+    o = torch.rand((n, 3), generator=g) * 3.0 - 1.5
+    d = torch.randn((n, 3), generator=g)
+    o[::3] = (o[::3] * 16).round() / 16
+    d[1::5, 2] = -1e-38
+    d[2::7, 2] = -0.0
+    o[2::14, 2] = float(field.aabb[0, 2])
+    rays = torch.cat([o, d], 1).contiguous()
+    got = model.run_stages(rays.cuda(), samples, True, upto="sample")
+    a = field.aabb.numpy()
+    u = torch.linspace(0.0, 1.0, steps=samples)
+    near_term, u = (field.near * (1.0 - u)).numpy(), u.numpy()
+    with np.errstate(all="ignore"):
+        far = -((o[:, 2].numpy() - a[0, 2]) / d[:, 2].numpy())
+        far = np.where(d[:, 2].numpy() >= 0, np.float32(field.far), far)
+        z = near_term[None] + far[:, None] * u[None]
+        pts = o.numpy()[:, None] + d.numpy()[:, None] * z[:, :, None]
+        valid = snp.in_box(pts, a)
+        if mask:
+            m = field.alpha_aabb.numpy()
+            inv = (np.float32(1.0) / (m[1] - m[0])) * np.float32(2)
+            q = (pts[valid] - m[0]) * inv - np.float32(1)
+            finite = np.isfinite(q).all(1)
+            alpha = np.zeros(len(q), np.float32)
+            alpha[finite] = snp.trilinear_zero_pad(field.alpha_volume[0, 0].numpy(), q[finite])
+            at = np.nonzero(valid)
+            keep = alpha > np.float32(thres)
+            valid[at[0][~keep], at[1][~keep]] = False
+    assert z.dtype == pts.dtype == np.float32
+    assert np.array_equal(valid_bits_from_words(got["mask_words"], samples), valid)
+    assert np.array_equal(got["counts"].cpu().numpy(), valid.sum(1))
