@@ -1041,10 +1041,15 @@ extern "C" int gnr_composite(GnrModel* m, int64_t n, int white_bg, void* workspa
 
 static int render_chunk_impl(GnrModel* m, const float* rays, int64_t n, int S, int white_bg, char* ws,
                              int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, cudaStream_t st,
-                             const GnrPixelSink* sink = nullptr) {
+                             const GnrPixelSink* sink = nullptr, bool chained = false) {
   GnrWs L = gnr_ws_layout(m, n, S, max_valid, max_app, 1);
   GnrSampleParams p = gnr_sample_params(m, S);
   const int lanes = gnr_march_lanes(m, n, S, max_valid);
+  if (chained && lanes != 0) {  // (not where scans stand in between, nor in a capture: a graph has little latency to hide)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    GNR_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+    L.chained = capture == cudaStreamCaptureStatusNone;
+  }
   {
     StageScope sc(m, GNR_STAGE_SAMPLE, 1, st);
     GNR_LAUNCH_OK(launch_sample_mask(m, p, rays, n, ws, L, st, (int32_t*)(ws + L.status)));
@@ -1151,7 +1156,7 @@ extern "C" int gnr_render_chunk(GnrModel* m, const float* rays, int64_t n, int S
   }
   DeviceGuard g(m->device);
   return render_chunk_impl(m, rays, n, S, white_bg, (char*)workspace, max_valid, max_app, rgb_map, depth_map,
-                           (cudaStream_t)stream);
+                           (cudaStream_t)stream, nullptr, /*chained=*/true);
 }
 
 extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int S, int white_bg, void* workspace, size_t ws_bytes,
@@ -1168,7 +1173,7 @@ extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int
   if (!m->forward_status) GNR_CUDA_OK(cudaMallocHost(&m->forward_status, GNR_ST_WORDS * sizeof(int32_t)));
   const GnrPixelSink sink{nullptr, nullptr, m->forward_status};
   rc = render_chunk_impl(m, rays, n, S, white_bg, (char*)workspace, max_valid, max_app, rgb_map, depth_map, (cudaStream_t)stream,
-                         &sink);
+                         &sink, /*chained=*/true);
   if (rc) return rc;
   GNR_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
   memcpy(status_h, m->forward_status, GNR_ST_WORDS * sizeof(int32_t));
@@ -1204,7 +1209,7 @@ static int render_batch_impl(GnrModel* m, const float* rays, int64_t n_rays, int
     const int64_t n = first + chunk <= n_rays ? chunk : n_rays - first;
     const GnrPixelSink sink{rgba, pixel_ids ? pixel_ids + first : nullptr, status ? status + c * GNR_ST_WORDS : nullptr};
     rc = render_chunk_impl(m, rays + first * 6, n, S, white_bg, (char*)ws[lane], max_valid, max_app, rgb_map ? rgb_map + first * 3 : nullptr,
-                           depth_map ? depth_map + first : nullptr, fork ? m->lane_streams[lane] : stream, &sink);
+                           depth_map ? depth_map + first : nullptr, fork ? m->lane_streams[lane] : stream, &sink, /*chained=*/!fork);
   }
   if (fork) {  // (after an error too: nothing is left running beside the caller's stream)
     for (int i = 0; i < n_lanes; ++i) {

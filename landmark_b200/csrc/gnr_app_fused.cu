@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(FG * GT, 1) app_mlp_fused_kernel(GnrSamplePara
     constexpr int kAll = (WB_BYTES + W1_BYTES + W2_BYTES + W3_BYTES) / 16, kW1Beg = WB_BYTES / 16, kW1End = (WB_BYTES + W1_BYTES) / 16;
     for (int i = tid; i < kAll; i += FG * GT) dst[i] = (i >= kW1Beg && i < kW1End) ? src_w1p[i - kW1Beg] : src[i];
     if (tid < 4) s_b3[tid] = a.b3[tid];
+    griddep_wait();
     if (tid == 0) {
       for (int s = 0; s < FG; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_mbar[s])));
       s_rel[0] = 0u;
@@ -697,8 +698,7 @@ int launch_app_mlp_fused(const GnrModel* m, const GnrSampleParams& p, const GnrC
   auto launch = [&](auto kernel, int groups) -> int {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<m->sm_count, groups * GT, kFusedSmem, st>>>(p, set, a);
-    return 0;
+    return gnr_launch(kernel, m->sm_count, groups * GT, kFusedSmem, st, c.chained, p, set, a);
   };
   auto pick_variant = [&](auto groups_tag) -> int {
     constexpr int G = decltype(groups_tag)::value;

@@ -191,6 +191,7 @@ composite_kernel(const float* __restrict__ app_weight, const int32_t* __restrict
                  const int32_t* __restrict__ app_offsets, const float* __restrict__ app_rgb, const float* __restrict__ acc, const float* __restrict__ depth,
                  int64_t n_rays, long long app_capacity, int white_bg, float* __restrict__ rgb_map,
                  float* __restrict__ depth_map, const int32_t* __restrict__ status, GnrPixelSink sink) {
+  griddep_wait();
   write_status(status, sink);
   const int lane = threadIdx.x & 31;
   const int64_t group = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -233,6 +234,7 @@ composite_rays_kernel(const float* __restrict__ app_weight, const int32_t* __res
                       const float* __restrict__ depth, int64_t n_rays, long long app_capacity, int white_bg,
                       float* __restrict__ rgb_map, float* __restrict__ depth_map, const int32_t* __restrict__ status,
                       GnrPixelSink sink) {
+  griddep_wait();
   write_status(status, sink);
   const int lane = threadIdx.x & 31;
   const int64_t ray = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -305,19 +307,21 @@ int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const
   const GnrPixelSink sink = sink_in ? *sink_in : GnrPixelSink{nullptr, nullptr, nullptr};
   const int32_t* status = (const int32_t*)(ws + L.status);
   if (march_lanes == 32) {  // ray-by-ray lists
-    composite_rays_kernel<<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
-        (const float*)(ws + L.app_weight), (const int32_t*)(ws + L.app_counts), (const int32_t*)(ws + L.app_offsets),
-        (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc), (const float*)(ws + L.depth), n, L.max_app, white_bg, rgb_map,
-        depth_map, status, sink);
+    const int rc = gnr_launch(composite_rays_kernel, (unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st,
+                              L.chained, (const float*)(ws + L.app_weight), (const int32_t*)(ws + L.app_counts),
+                              (const int32_t*)(ws + L.app_offsets), (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc),
+                              (const float*)(ws + L.depth), n, L.max_app, white_bg, rgb_map, depth_map, status, sink);
+    if (rc) return rc;
     return (int)cudaGetLastError();
   }
   const int64_t groups = (n + 31) / 32;
   unsigned blocks = (unsigned)((groups + kWarpsPerBlock - 1) / kWarpsPerBlock);
   long long app_capacity = L.max_app;
-  composite_kernel<<<blocks, kWarpsPerBlock * 32, 0, st>>>(
-      (const float*)(ws + L.app_weight), (const int32_t*)(ws + L.app_counts), (const int32_t*)(ws + L.app_offsets),
-      (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc), (const float*)(ws + L.depth), n, app_capacity,
-      white_bg, rgb_map, depth_map, status, sink);
+  const int rc = gnr_launch(composite_kernel, blocks, kWarpsPerBlock * 32, 0, st, L.chained, (const float*)(ws + L.app_weight),
+                            (const int32_t*)(ws + L.app_counts), (const int32_t*)(ws + L.app_offsets),
+                            (const float*)(ws + L.app_rgb), (const float*)(ws + L.acc), (const float*)(ws + L.depth), n, app_capacity,
+                            white_bg, rgb_map, depth_map, status, sink);
+  if (rc) return rc;
   return (int)cudaGetLastError();
 }
 

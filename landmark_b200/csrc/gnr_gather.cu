@@ -453,6 +453,7 @@ __global__ void __launch_bounds__(kMarchBlock<G>, (LAT ? 40 : 16) / (kMarchBlock
 march_kernel(const __grid_constant__ GnrSampleParams p, const __grid_constant__ PlaneSet planes, LatticeRef lat,
              const __grid_constant__ MarchArgs a) {
   constexpr uint32_t kGroup = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+  griddep_wait();
   const int lane = threadIdx.x & 31, g = lane & (G - 1);
   const long long ray = (long long)blockIdx.x * (kMarchBlock<G> / G) + threadIdx.x / G;
   const bool has_ray = ray < a.n_rays;
@@ -841,6 +842,7 @@ GnrCoords gnr_coords_app(const float* rays, char* ws, const GnrWs& L, int lanes)
   c.ids = (const uint32_t*)(ws + L.app_ids);  // written in list order by the march or by expand_app_kernel
   c.total_ptr = lanes == 0 ? (const int32_t*)(ws + L.app_offsets) + L.n_rays : (const int32_t*)(ws + L.status) + GNR_ST_NUM_APP;
   c.capacity = L.max_app;
+  c.chained = L.chained;
   return c;
 }
 
@@ -1127,7 +1129,9 @@ int launch_march(const GnrModel* m, const GnrSampleParams& p, const float* rays,
   a.app_weight = (float*)(ws + L.app_weight);
   const unsigned rays_per_block = lanes == 32 ? 4 : 32;
   const unsigned grid = (unsigned)((n + rays_per_block - 1) / rays_per_block);
-#define GNR_MARCH_G(JJ, NPP, HH, LL, GG, LIST) march_kernel<JJ, NPP, HH, LL, GG, LIST><<<grid, kMarchBlock<GG>, 0, st>>>(p, set, lat, a)
+  int rc = 0;
+#define GNR_MARCH_G(JJ, NPP, HH, LL, GG, LIST) \
+  rc = gnr_launch(march_kernel<JJ, NPP, HH, LL, GG, LIST>, grid, kMarchBlock<GG>, 0, st, L.chained && LIST, p, set, lat, a)
 #define GNR_MARCH(JJ, NPP, HH, LL)                                   \
   do {                                                               \
     if (lanes == 0) GNR_MARCH_G(JJ, NPP, HH, LL, 4, false);          \
@@ -1150,5 +1154,6 @@ int launch_march(const GnrModel* m, const GnrSampleParams& p, const float* rays,
   }
 #undef GNR_MARCH
 #undef GNR_MARCH_G
+  if (rc) return rc;
   return (int)cudaGetLastError();
 }

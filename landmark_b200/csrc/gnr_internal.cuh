@@ -135,7 +135,35 @@ struct GnrWs {
   int feat_stride;  // floats per appearance feature row (app_dim rounded up to 4)
   long long max_valid, max_app;  // capacities of the two compacted lists
   long long n_rays;
+  int chained;                   // launch the chunk's kernels with gnr_launch's `chained`
 };
+
+// Chained launches: the kernels of a chunk run one after the other, each waiting for the one before.  A kernel launched
+// with `chained` starts its blocks when the last block of the kernel before it has ended, without waiting for that
+// kernel's writes to be flushed and for the launch to be set up, and then waits in griddep_wait until they are visible;
+// its set-up (weights into shared memory, barriers) runs meanwhile.  333 rays: 60.5 -> 54.0 us per call; 8192 rays, fp32:
+// 157 -> 147 us.  No kernel lets the next one start before its own last block has ended: early blocks settle on the SMs
+// that happen to have room, and the march of 10,000 rays, or the kernels behind it, then waits for the fullest SM (8192
+// rays: 163 us).  Chunks that share the GPU with another lane's are launched plainly.
+// A kernel that can be launched chained calls griddep_wait in every thread before it touches what earlier kernels write or
+// read (a kernel in the chain is complete only when the one before it is), and holds no tensor memory while it waits.  In
+// a kernel launched plainly the wait is over at once.
+__device__ __forceinline__ void griddep_wait() { cudaGridDependencySynchronize(); }
+
+template <typename... P, typename... A>
+int gnr_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool chained, A&&... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // Where a per-sample kernel finds item i: either through the chunk's compacted lists
 // (ids[index ? index[i] : i] -> ray, sample -> position recomputed from the ray) or, in point
@@ -155,6 +183,7 @@ struct GnrCoords {
   const int32_t* total_ptr;   // device count of items, or null ...
   long long total_direct;     // ... then this host count
   long long capacity;
+  int chained = 0;            // see GnrWs
 };
 
 void gnr_set_error(const char* fmt, ...);

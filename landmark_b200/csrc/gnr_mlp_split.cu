@@ -77,10 +77,6 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const long long total = min(a.crd.total_ptr ? (long long)*a.crd.total_ptr : a.crd.total_direct, a.crd.capacity);
-  const long long n_tiles = (total + ROWS - 1) / ROWS;
-  if ((long long)blockIdx.x >= n_tiles) return;  // (the whole CTA)
-  const int my_tiles = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
   const uint32_t bars = smem_u32(s_bar);
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   auto wait = [&](int i, uint32_t parity) { return warp_wait(bar(i), parity & 1u, s_abort, a.status, a.wait_limit); };
@@ -103,14 +99,12 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
       *s_abort = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(512u));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     if (lane == 0) {
       mbar_expect_tx(bar(WEIGHTS), kImage);
       for (uint32_t at = 0; at < kImage; at += 16384u)
         bulk_load(smem_u32(smem) + at, a.w_image + at, min(16384u, kImage - at), bar(WEIGHTS));
     }
+    __syncwarp();
   } else {
     for (int i = tid; i < 3 * HID; i += MMA_WARP * 32) s_w3[i] = a.w3[i];
     if (tid < HID) {
@@ -119,6 +113,14 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
     }
     if (tid < 4) s_b3[tid] = a.b3[tid];
   }
+  griddep_wait();
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  const long long total = min(a.crd.total_ptr ? (long long)*a.crd.total_ptr : a.crd.total_direct, a.crd.capacity);
+  const long long n_tiles = (total + ROWS - 1) / ROWS;
+  const int my_tiles = (int)max(0LL, (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -214,7 +216,9 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
       }
     };
     bool ok = true;
-    if (warp < ROLE_WARPS) {
+    if (my_tiles == 0) {
+      // (only the copies of the weights to see out, by the MMA warp)
+    } else if (warp < ROLE_WARPS) {
       // ---- encode --------------------------------------------------------------------------------------------------------
       // this thread's three values of chunk c: 6 c + 3 half .. of the features; the last three of half 1 are the view direction
       const uint32_t ring_half = ring + lane_off + (uint32_t)(half * 8);  // this thread's 8 of a term's 16 columns
@@ -418,7 +422,8 @@ int launch_mode(const GnrModel* m, const SplitArgs& a, cudaStream_t st) {
   static_assert(smem <= 227 * 1024, "the weights of the split network must fit shared memory");
   cudaError_t e = cudaFuncSetAttribute(mlp_split_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  mlp_split_kernel<MODE><<<m->sm_count, THREADS, smem, st>>>(a);
+  const int rc = gnr_launch(mlp_split_kernel<MODE>, m->sm_count, THREADS, smem, st, a.crd.chained, a);
+  if (rc) return rc;
   return (int)cudaGetLastError();
 }
 

@@ -60,6 +60,7 @@ project_split_kernel(const __grid_constant__ GnrSampleParams p, const __grid_con
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
+  griddep_wait();
   const long long total = coords_total(a.crd);
   const long long n_tiles = (total + ROWS - 1) / ROWS;
   // a contiguous share of the list per CTA: neighbouring tiles read the same texels
@@ -255,7 +256,8 @@ int launch_variant(const GnrModel* m, const GnrSampleParams& p, const PlaneSet& 
   const size_t smem = (size_t)Split<MODE>::TW * set.n * 2 * J * KGB_BYTES + (2 * SLOTS + 6) * 8 + 16;
   cudaError_t e = cudaFuncSetAttribute(project_split_kernel<MODE, J, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  project_split_kernel<MODE, J, NP><<<m->sm_count, THREADS, smem, st>>>(p, set, a);
+  const int rc = gnr_launch(project_split_kernel<MODE, J, NP>, m->sm_count, THREADS, smem, st, a.crd.chained, p, set, a);
+  if (rc) return rc;
   return (int)cudaGetLastError();
 }
 

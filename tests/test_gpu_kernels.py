@@ -217,3 +217,26 @@ def test_hull_sampler_words_at_edges(n, samples, thres, mask):
     assert z.dtype == pts.dtype == np.float32
     assert np.array_equal(valid_bits_from_words(got["mask_words"], samples), valid)
     assert np.array_equal(got["counts"].cpu().numpy(), valid.sum(1))
+
+
+@pytest.mark.parametrize("options", [{}, {"mlp_mode": 1}, {"mlp_mode": 2, "app_plane_fp16": True, "density_lattice": True, "ert_transmittance": 2e-5}])
+def test_chained_launches_keep_the_order_of_calls(options):
+    """Chunks of changing size queued back to back into one workspace, the kernels of each chained, between copies and
+    plain kernels of the caller: the pixels of every call equal those of the same call waited for by itself."""
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec, **options)
+    rays = tiny_rays(spec).cuda()
+    sizes = [1, 333, 9000, 40, 3100, 7000, 128, 2000] * 3
+    starts = [(977 * i) % (rays.shape[0] - n + 1) for i, n in enumerate(sizes)]
+    want = []
+    for a, n in zip(starts, sizes):
+        want.append(model(rays[a:a + n].contiguous(), N_samples=spec.n_samples)[0]["rgb_map"].clone())
+        torch.cuda.synchronize()
+    model.check_status_every_call = False
+    staged = torch.empty_like(rays)
+    got = []
+    for a, n in zip(starts, sizes):
+        staged[:n].copy_(rays[a:a + n])  # (into the buffer the call before still reads)
+        got.append(model(staged[:n], N_samples=spec.n_samples)[0]["rgb_map"] * 1.0)
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
