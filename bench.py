@@ -488,7 +488,7 @@ def main():
         del gr
         torch.cuda.empty_cache()
 
-    # ---- the same frame with every approximation off: fp32 CUDA-core MLP, fp32 planes, no early
+    # ---- the same frame with every approximation off: fp32 MLP, fp32 planes, no early
     # termination.  Its image is the full-frame check of the fast configuration. -----------------
     strict = None
     if world == 1 and not a.no_strict:
@@ -518,7 +518,7 @@ def main():
         ms2 = s0.elapsed_time(s1) / a.steps
         err2 = (rgb2[:n_local] - rgb[:n_local]).abs().max(dim=1).values
         strict = {"value": H * W / (ms2 * 1e-3) / 1e6, "unit": "Mrays/s", "ms_per_step": ms2,
-                  "config": "mlp_mode 0 (fp32 CUDA-core MLP), fp32 planes, ert_transmittance 0",
+                  "config": "mlp_mode 0 (fp32 MLP), fp32 planes, ert_transmittance 0",
                   "density_evaluated": float(st2[5]),
                   "fast_vs_strict_max_abs_rgb_diff": float(err2.max()), "fast_vs_strict_rays_above_1e-4": int((err2 > 1e-4).sum()),
                   "rays_compared": int(n_local)}
