@@ -9,9 +9,14 @@
 // One persistent CTA per SM, tiles of 128 samples (row = lane of tensor memory).  Sixteen warps gather: two groups of 256
 // threads, two per row, take alternate tiles; each thread interpolates half the channels of a pair, eight at a time (six
 // 256-bit loads), splits the products and stores them into a slot of a ring in tensor memory (one slot per pair, six
-// slots: two tiles of the usual three pairs).  One warp issues the MMAs, M 128 x N 32; four warps read the finished
-// features and store them.  The gatherers wait for nothing but a free slot, so the loads, which bound the kernel (192 bytes
-// per texel and pair through the L1 -> register port), never pause for a projection.
+// slots: two tiles of the usual three pairs).
+// A gatherer waits for its slot by the parity of the slot's use, which one bit tells apart only while the use before the
+// last is known to be consumed.  A group's last wait of a tile showed that all slots up to 7 + n_pairs before the first
+// of its next tile are; the parity needs 12 before.  From six pairs on the groups therefore take alternate pairs of every
+// tile instead: each then owns three slots and waits for every use of them.
+// One warp issues the MMAs, M 128 x N 32; four warps read the finished features and store them.  The gatherers wait for
+// nothing but a free slot, so the loads, which bound the kernel (192 bytes per texel and pair through the L1 -> register
+// port), never pause for a projection.
 // Tensor memory: the ring [0, 432), two feature accumulators [448, 512).
 //
 // Every wait is bounded; when one runs out the CTA raises status[GNR_ST_WAIT_EXPIRED] and all its roles stop.
@@ -176,8 +181,9 @@ project_split_kernel(const __grid_constant__ GnrSampleParams p, const __grid_con
     // ---- gather -------------------------------------------------------------------------------------------------------------
     const int g = warp >> 3, wg = warp & 7, half = wg >> 2, row = ((wg & 3) << 5) | lane;
     const uint32_t lane_off = (uint32_t)((wg & 3) * 32) << 16;
+    const bool by_pairs = n_pairs >= SLOTS;
     bool ok = true;
-    for (int n = g; n < my_tiles && ok; n += 2) {
+    for (int n = by_pairs ? 0 : g; n < my_tiles && ok; n += by_pairs ? 1 : 2) {
       const long long j = (t_beg + n) * ROWS + row;
       float x, y, z;
       sample_xyz(p, a.crd, j < total ? j : total - 1, x, y, z);  // (rows past the end repeat the last sample)
@@ -188,7 +194,7 @@ project_split_kernel(const __grid_constant__ GnrSampleParams p, const __grid_con
         tz = make_tap(z, planes.p[0].fl, planes.p[0].L);
       }
 #pragma unroll 1
-      for (int pi = 0; pi < n_pairs && ok; ++pi) {
+      for (int pi = by_pairs ? (g + n * n_pairs) & 1 : 0; pi < n_pairs && ok; pi += by_pairs ? 2 : 1) {
         const GnrPlane& pl = planes.p[pi];
         Tap tu, tv, tl;
         if (NP == 3) {

@@ -240,3 +240,75 @@ def test_chained_launches_keep_the_order_of_calls(options):
         got.append(model(staged[:n], N_samples=spec.n_samples)[0]["rgb_map"] * 1.0)
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+def _pairs_model(ndims, res_mode, channels, mode, **extra):
+    """A model with any layout of plane/line pairs, on a grid whose taps are exact for positions of 1/256."""
+    from landmark_b200.gridnerf import B200GridNeRF
+
+    spec = scenes.tiny_spec(grid=17).lit()
+    spec.app_n_comp = (channels,) * 3
+    g = torch.Generator().manual_seed(100 * ndims + len(res_mode))
+    sd = {k: v for k, v in scenes.make_state_dict(spec).items() if k.startswith("renderModule")}
+    for i in range(ndims):
+        m0, m1 = scenes.MAT_MODE[i]
+        for j, r in enumerate(res_mode):
+            size = [17 * r] * 3
+            for kind, c in (("density", 16), ("app", channels)):
+                sd[f"{kind}_plane.{i * len(res_mode) + j}"] = 0.1 * torch.randn((1, c, size[m1], size[m0]), generator=g)
+                sd[f"{kind}_line.{i * len(res_mode) + j}"] = 0.1 * torch.randn((1, c, size[scenes.VEC_MODE[i]], 1), generator=g)
+    k = ndims * len(res_mode) * channels
+    sd["basis_mat.weight"] = (torch.rand((27, k), generator=g) * 2 - 1) / k ** 0.5
+    ckpt = scenes.make_checkpoint(spec)
+    ckpt["state_dict"] = sd
+    args = scenes.model_args(spec, "cuda:0")
+    args.ndims, args.resMode = ndims, list(res_mode)
+    kw = dict(ckpt["kwargs"])
+    kw.update({"device": "cuda:0", "args": args, "is_train": False})
+    model = B200GridNeRF(**kw, mlp_mode=mode, **extra)
+    model.load(ckpt)
+    return model, sd
+
+
+def _features_fp64(sd, ndims, n_res, xyz, magnitudes=False):
+    """compute_appfeature in fp64; ``magnitudes``: the sums of the terms' magnitudes instead."""
+    parts = []
+    f = torch.abs if magnitudes else (lambda t: t)
+    for i in range(ndims * n_res):
+        d = i // n_res
+        uv = xyz[:, list(scenes.MAT_MODE[d])].double().view(1, -1, 1, 2)
+        line = xyz[:, scenes.VEC_MODE[d]].double()
+        line = torch.stack([torch.zeros_like(line), line], -1).view(1, -1, 1, 2)
+        p = torch.nn.functional.grid_sample(f(sd[f"app_plane.{i}"].cuda().double()), uv, align_corners=True)
+        l = torch.nn.functional.grid_sample(f(sd[f"app_line.{i}"].cuda().double()), line, align_corners=True)
+        parts.append((p * l)[0, :, :, 0].T)
+    w = f(sd["basis_mat.weight"].cuda().double())
+    return torch.cat(parts, 1) @ w.T, w
+
+
+@pytest.mark.parametrize("mode", [0])
+@pytest.mark.parametrize("ndims,res_mode,channels", [
+    (1, (1,), 48), (2, (1,), 48), (3, (1,), 48), (3, (1,), 16), (3, (1,), 24), (1, (1, 2, 4), 48), (2, (1, 2), 48), (2, (1, 2), 32),
+    (1, (1, 2, 1, 2, 1), 48), (1, (1, 2, 1, 2, 1), 16), (3, (1, 2), 48), (3, (1, 2), 16), (1, (1, 2, 1, 2, 1, 2, 1), 32),
+    (2, (1, 2, 1, 2), 48), (3, (1, 2, 4), 48), (3, (1, 2, 4), 10)])
+@pytest.mark.parametrize("n", [77, 7 * 148 * 128 + 77])
+def test_projected_features_of_every_layout(n, ndims, res_mode, channels, mode):
+    """Gather and projection of modes 0 and 1 against fp64, one to nine pairs of 16, 32 and 48 padded channels, a partial
+    tile alone and seven to eight tiles per CTA.  Bound per feature, against the sum of its terms' magnitudes: a product
+    has ten roundings (three tap weights, seven of the interpolation), a projection at most six times K / 16 accumulation steps
+    that need not round to nearest (2^-23).  Mode 1 with up to 152 products carries weights as one fp16 (2^-11) and
+    products as two (2^-25 where the second is subnormal); with more it is fp32, as mode 0."""
+    from landmark_b200.model_parallel import app_features_points
+
+    model, sd = _pairs_model(ndims, res_mode, channels, mode)
+    g = torch.Generator().manual_seed(n)
+    xyz = (torch.randint(-256, 257, (n, 3), generator=g) / 256.0).cuda()
+    got = app_features_points(model, xyz).double()
+    ref, _ = _features_fp64(sd, ndims, len(res_mode), xyz)
+    mag, w = _features_fp64(sd, ndims, len(res_mode), xyz, magnitudes=True)
+    k = ndims * len(res_mode) * (-(-channels // 16) * 16)
+    bound = (10 * 2.0 ** -24 + 6 * k / 16 * 2.0 ** -23) * mag + 1e-30
+    if mode == 1 and k <= 152:
+        bound = bound + 2.0 ** -11 * mag + 2.0 ** -25 * w.sum(1)
+    worst = ((got - ref).abs() / bound).max().item()
+    assert worst <= 1.0, f"error is {worst:.2f} of the bound"
