@@ -1,5 +1,5 @@
 // Appearance gather from fp32 planes and lines + basis projection, the projection on the tensor cores with operands as
-// sums of 16-bit terms (gnr_split.cuh): mlp_mode 0 and 1.
+// sums of 16-bit terms (gnr_split.cuh): mlp_mode 0, and mlp_mode 1 with up to 152 products per sample.
 //
 // compute_appfeature (app/models/gridnerf_sequential.py:829-871).  The plane x line products are computed in fp32 as
 // app_gather_kernel computes them (operations and order); app_dim x (pairs x channels) multiply-adds per sample follow,
@@ -276,8 +276,11 @@ int launch_mode(const GnrModel* m, const GnrSampleParams& p, const PlaneSet& set
 
 }  // namespace
 
+// Mode 1 projects in two fp16 terms (one for the weights) where its products fit one operand buffer, as it always has;
+// with more of them its features are fp32 ones from the CUDA cores.
 int gnr_project_split_usable(const GnrModel* m) {
-  return gnr_mlp_split_usable(m) && m->cfg.app_storage == 0 && m->app[0].C >= 16 && m->app[0].C <= 48;
+  return gnr_mlp_split_usable(m) && m->cfg.app_storage == 0 && m->app[0].C >= 16 && m->app[0].C <= 48 &&
+         (m->cfg.mlp_mode == 0 || m->mlp.n_prod + 8 <= MAX_K0);
 }
 
 int launch_project_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoords& c, int feat_stride, float* feat,

@@ -286,7 +286,7 @@ def _features_fp64(sd, ndims, n_res, xyz, magnitudes=False):
     return torch.cat(parts, 1) @ w.T, w
 
 
-@pytest.mark.parametrize("mode", [0])
+@pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("ndims,res_mode,channels", [
     (1, (1,), 48), (2, (1,), 48), (3, (1,), 48), (3, (1,), 16), (3, (1,), 24), (1, (1, 2, 4), 48), (2, (1, 2), 48), (2, (1, 2), 32),
     (1, (1, 2, 1, 2, 1), 48), (1, (1, 2, 1, 2, 1), 16), (3, (1, 2), 48), (3, (1, 2), 16), (1, (1, 2, 1, 2, 1, 2, 1), 32),
