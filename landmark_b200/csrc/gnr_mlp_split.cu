@@ -195,10 +195,12 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_split_kernel(const __grid_cons
       __syncwarp();
     }
     if (!ok) {
-      // stop: wait (bounded) until nothing of this CTA runs in the tensor pipe
+      // stop: wait (bounded, whatever limit the other waits have) until nothing of this CTA runs in the tensor pipe and
+      // no copy of the weights still writes its shared memory
       mma_commit(bar(DRAIN), elect_one());
       __syncwarp();
       for (uint32_t it = 0; it < kWaitLimit && !mbar_try_wait(bar(DRAIN), 0); ++it) __nanosleep(64);
+      for (uint32_t it = 0; it < kWaitLimit && !mbar_try_wait(bar(WEIGHTS), 0); ++it) __nanosleep(64);
     }
   } else {
     const int wg = warp & (ROLE_WARPS - 1);

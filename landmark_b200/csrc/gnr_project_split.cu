@@ -151,10 +151,12 @@ project_split_kernel(const __grid_constant__ GnrSampleParams p, const __grid_con
       q += n_pairs;
     }
     if (!ok) {
-      // stop: wait (bounded) until nothing of this CTA runs in the tensor pipe
+      // stop: wait (bounded, whatever limit the other waits have) until nothing of this CTA runs in the tensor pipe and
+      // no copy of the weights still writes its shared memory
       mma_commit(bar(DRAIN), elect_one());
       __syncwarp();
       for (uint32_t it = 0; it < kWaitLimit && !mbar_try_wait(bar(DRAIN), 0); ++it) __nanosleep(64);
+      for (uint32_t it = 0; it < kWaitLimit && !mbar_try_wait(bar(WEIGHTS), 0); ++it) __nanosleep(64);
     }
   } else if (warp >= GATHER_WARPS) {
     // ---- features: tensor memory -> global ------------------------------------------------------------------------------

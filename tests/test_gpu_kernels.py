@@ -124,6 +124,23 @@ def test_fp32_network_wait_expires_and_the_context_survives():
     assert torch.equal(good["rgb_map"], again["rgb_map"])
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+def test_waits_that_run_out_at_once_leave_no_copy_behind(mode):
+    """One poll per wait: roles of the split kernels give up while the copies of the weights are still on their way into
+    shared memory.  The kernels see them out before they leave, so that the launches behind them read what they loaded."""
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec, mlp_mode=mode)
+    rays = tiny_rays(spec).cuda()
+    good, _ = model(rays, N_samples=spec.n_samples)
+    model.check_status_every_call = False
+    for _ in range(5):
+        model.debug_wait(wait_limit=1)
+        model(rays, N_samples=spec.n_samples)
+        model.debug_wait()
+        again, _ = model(rays, N_samples=spec.n_samples)
+        assert torch.equal(good["rgb_map"], again["rgb_map"])
+
+
 def test_inferer_chunks_fit_the_sample_ids():
     """65536 rays of 40000 samples do not fit the 32-bit ids of a chunk, 8192 do: the drop-in loop takes what fits."""
     from types import SimpleNamespace
