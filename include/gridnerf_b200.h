@@ -447,7 +447,10 @@ int gnr_measure_l1_bandwidth(int device, int iters, float* gb_per_s_h);
  * tile in the MLP kernel, the commit of its first projection in the fused kernel), so that this wait
  * runs out: the group raises status[GNR_ST_WAIT_EXPIRED] and stops, the kernel frees its tensor memory
  * and returns, and the context stays usable.  ``expire`` = 0, ``wait_limit`` = 0 restores normal
- * operation.  Nothing in this hook faults, traps or spins without bound. */
+ * operation.  In mlp_mode 0 and 1, where the projection and the network are two kernels with such waits,
+ * GNR_EXPIRE_PROJECTION and GNR_EXPIRE_NETWORK pick one of them.  Nothing in this hook faults, traps or spins
+ * without bound. */
+enum { GNR_EXPIRE_ANY = 1, GNR_EXPIRE_PROJECTION = 2, GNR_EXPIRE_NETWORK = 3 };
 int gnr_debug_wait(GnrModel* m, int expire, int wait_limit);
 
 /* Measurement aid for the fused appearance kernel: with ``on`` != 0 the following launches let one thread

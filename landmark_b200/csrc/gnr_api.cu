@@ -832,7 +832,7 @@ extern "C" int gnr_debug_wait(GnrModel* m, int expire, int wait_limit) {
     gnr_set_error("gnr_debug_wait: bad argument");
     return -1;
   }
-  m->debug_expire_wait = expire ? 1 : 0;
+  m->debug_expire_wait = expire == GNR_EXPIRE_PROJECTION || expire == GNR_EXPIRE_NETWORK ? expire : (expire ? GNR_EXPIRE_ANY : 0);
   m->debug_wait_limit = wait_limit;
   return 0;
 }

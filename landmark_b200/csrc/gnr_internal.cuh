@@ -74,7 +74,7 @@ struct GnrModel {
   int aD, aH, aW;
   float a_lo[3], a_inv[3];
   GnrMlp mlp;
-  int debug_expire_wait;  // test hook (gnr_debug_wait): make one bounded wait of the tensor-core kernels run out
+  int debug_expire_wait;  // test hook (gnr_debug_wait): make one bounded wait of the tensor-core kernels run out (GNR_EXPIRE_*)
   int debug_wait_limit;   // polls a bounded wait may take; 0 = the default
   int32_t* route_scratch;  // per-CTA block counts and start rows of gnr_route_blocks
   size_t route_scratch_bytes;

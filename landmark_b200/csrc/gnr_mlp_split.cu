@@ -458,6 +458,6 @@ int launch_mlp_split(const GnrModel* m, const GnrSampleParams& p, const GnrCoord
   a.status = status;
   a.kbits = p.kbits;
   a.wait_limit = m->debug_wait_limit > 0 ? (uint32_t)m->debug_wait_limit : kWaitLimit;
-  a.debug_skip_commit = m->debug_expire_wait;
+  a.debug_skip_commit = m->debug_expire_wait == GNR_EXPIRE_ANY || m->debug_expire_wait == GNR_EXPIRE_NETWORK;
   return m->cfg.mlp_mode == 0 ? launch_mode<0>(m, a, st) : launch_mode<1>(m, a, st);
 }

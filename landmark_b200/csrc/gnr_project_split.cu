@@ -297,7 +297,7 @@ int launch_project_split(const GnrModel* m, const GnrSampleParams& p, const GnrC
   a.feat_out = feat;
   a.status = status;
   a.wait_limit = m->debug_wait_limit > 0 ? (uint32_t)m->debug_wait_limit : kWaitLimit;
-  a.debug_skip_commit = m->debug_expire_wait;
+  a.debug_skip_commit = m->debug_expire_wait == GNR_EXPIRE_ANY || m->debug_expire_wait == GNR_EXPIRE_PROJECTION;
   const PlaneSet set = make_set(m->app, m->cfg.n_pairs);
   return m->cfg.mlp_mode == 0 ? launch_mode<0>(m, p, set, a, st) : launch_mode<1>(m, p, set, a, st);
 }

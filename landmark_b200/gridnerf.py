@@ -671,8 +671,9 @@ class B200GridNeRF(torch.nn.Module):
 
     def debug_wait(self, expire: bool = False, wait_limit: int = 0):
         """Test hook (gnr_debug_wait): make one bounded device-side wait of the next tensor-core launches
-        run out, with ``wait_limit`` polls per wait; ``debug_wait()`` restores normal operation."""
-        check(lib.gnr_debug_wait(self._handle, int(bool(expire)), int(wait_limit)), "gnr_debug_wait")
+        run out, with ``wait_limit`` polls per wait; ``debug_wait()`` restores normal operation.  ``expire`` may also
+        be EXPIRE_PROJECTION or EXPIRE_NETWORK (``_lib``): that kernel alone, in mlp_mode 0 and 1."""
+        check(lib.gnr_debug_wait(self._handle, int(expire), int(wait_limit)), "gnr_debug_wait")
 
     def profile_enable(self, on: bool = True):
         check(lib.gnr_profile_enable(self._handle, int(on)), "gnr_profile_enable")

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from landmark_b200 import scenes
+from landmark_b200._lib import EXPIRE_ANY, EXPIRE_NETWORK, EXPIRE_PROJECTION
 from oracle import sampling_numpy as snp
 from tests._util import cuda_model, oracle_field, tiny_rays, valid_bits_from_words
 
@@ -111,12 +112,16 @@ def test_fp32_network_on_tensor_cores(n, scale):
     assert worst <= 1.0, f"error is {worst:.2f} of the bound"
 
 
-def test_fp32_network_wait_expires_and_the_context_survives():
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kernel", [EXPIRE_ANY, EXPIRE_PROJECTION, EXPIRE_NETWORK])
+def test_fp32_network_wait_expires_and_the_context_survives(kernel, mode):
+    """The projection and the network each report a wait that runs out (both write the chunk's one status block, so each is
+    made to run out alone)."""
     spec = scenes.tiny_spec().lit()
-    model = cuda_model(spec)
+    model = cuda_model(spec, mlp_mode=mode)
     rays = tiny_rays(spec).cuda()[4000:6000].contiguous()
     good, _ = model(rays, N_samples=spec.n_samples)
-    model.debug_wait(expire=True, wait_limit=2000)
+    model.debug_wait(expire=kernel, wait_limit=2000)
     with pytest.raises(RuntimeError, match="bounded device-side wait expired"):
         model(rays, N_samples=spec.n_samples)
     model.debug_wait()
