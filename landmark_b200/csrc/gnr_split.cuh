@@ -70,15 +70,21 @@ struct Split<0> {
   }
   // three values -> one K step of layer 1: v, sin v, sin 2v, cos v, cos 2v of each, and a zero
   __device__ static __forceinline__ void encode(const float (&v)[3], float (&x)[16]) {
-    // one test for all six angles, so that the short form has no branches between them
+    // one test for all six angles of the warp's rows, so that the short form has no branches between them; where it fails
+    // every value still takes the form that its own size asks for (a sample's bits do not depend on its neighbours)
     const bool large = !(fabsf(v[0]) <= 500.0f && fabsf(v[1]) <= 500.0f && fabsf(v[2]) <= 500.0f);
     if (__any_sync(0xffffffffu, large)) {
 #pragma unroll 1
       for (int i = 0; i < 3; ++i) {
         const float u = i == 0 ? v[0] : i == 1 ? v[1] : v[2];
         float s1, c1, s2, c2;
-        sincosf(u, &s1, &c1);
-        sincosf(2.0f * u, &s2, &c2);
+        if (fabsf(u) <= 500.0f) {
+          sincos_short(u, s1, c1);
+          sincos_short(2.0f * u, s2, c2);
+        } else {
+          sincosf(u, &s1, &c1);
+          sincosf(2.0f * u, &s2, &c2);
+        }
 #pragma unroll
         for (int e = 0; e < 3; ++e)
           if (e == i) {

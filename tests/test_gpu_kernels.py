@@ -112,6 +112,20 @@ def test_fp32_network_on_tensor_cores(n, scale):
     assert worst <= 1.0, f"error is {worst:.2f} of the bound"
 
 
+def test_fp32_network_bits_do_not_depend_on_the_order_of_samples():
+    """A few features beyond the range of the short sine among ordinary ones: every sample has the same bits in any order."""
+    from landmark_b200.model_parallel import mlp_features
+
+    spec = scenes.tiny_spec(grid=32).lit()
+    model = cuda_model(spec)
+    g = torch.Generator().manual_seed(1)
+    feats, view = torch.randn((4097, 27), generator=g), torch.randn((4097, 3), generator=g)
+    feats[::97, 3], feats[50::131, 26], view[7::500, 1] = 700.0, -1e6, 501.0
+    order = torch.randperm(feats.shape[0], generator=g)
+    rgb = mlp_features(model, feats.cuda(), view.cuda())
+    assert torch.equal(rgb[order.cuda()], mlp_features(model, feats[order].cuda(), view[order].cuda()))
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("kernel", [EXPIRE_ANY, EXPIRE_PROJECTION, EXPIRE_NETWORK])
 def test_fp32_network_wait_expires_and_the_context_survives(kernel, mode):
