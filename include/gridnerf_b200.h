@@ -152,7 +152,8 @@ int gnr_build_appearance_lattice(GnrModel* m, int enable, void* stream);
 /* Tables of the hull sampler for ``n_samples`` (= n_importance) samples per ray:
  * ``u[k] = torch.linspace(0, 1, n_samples)[k]`` and ``near_term[k] = near * (1.0 - u[k])``, both
  * evaluated by torch on the CPU so that ``z = near_term[k] + far * u[k]`` has the reference's bits
- * (app/models/gridnerf_sequential.py:303-304).  Device pointers; copied. */
+ * (app/models/gridnerf_sequential.py:303-304).  Device pointers; copied.  Any values in any order are sampled as given;
+ * ordered tables are the fast case. */
 int gnr_upload_hull_tables(GnrModel* m, int n_samples, const float* near_term, const float* u, void* stream);
 
 /* Ray generation from a pose.  Replaces generate_rays (dist_render/dataset/utils.py:92-113):

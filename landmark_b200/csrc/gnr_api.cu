@@ -272,6 +272,7 @@ extern "C" int gnr_destroy(GnrModel* m) {
   free_dev(m->alpha_any8);
   free_dev(m->hull_near_term);
   free_dev(m->hull_u);
+  free_dev(m->hull_ranges);
   free_dev(m->mlp.basis_blocked);
   free_dev(m->mlp.w1t);
   free_dev(m->mlp.w2t);
@@ -487,6 +488,26 @@ extern "C" int gnr_upload_alpha_mask(GnrModel* m, const uint8_t* vol, int D, int
   return 0;
 }
 
+// {smallest, largest near_term, smallest, largest u} of run r (8 samples; r < n_runs) or of word r - n_runs (32 samples).
+// NaN where a value is not of ordinary size: the sampler then leaves the run open.
+__global__ void hull_ranges_kernel(const float* __restrict__ near_term, const float* __restrict__ u, int n_samples, int n_runs,
+                                   int n_words, float4* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_runs + n_words) return;
+  const int beg = i < n_runs ? 8 * i : 32 * (i - n_runs), end = min(beg + (i < n_runs ? 8 : 32), n_samples);
+  float4 r = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+  bool ordinary = true;
+  for (int k = beg; k < end; ++k) {
+    ordinary = ordinary && fabsf(near_term[k]) <= 1e30f && fabsf(u[k]) <= 1e6f;
+    r.x = fminf(r.x, near_term[k]);
+    r.y = fmaxf(r.y, near_term[k]);
+    r.z = fminf(r.z, u[k]);
+    r.w = fmaxf(r.w, u[k]);
+  }
+  if (!ordinary) r.x = NAN;
+  out[i] = r;
+}
+
 extern "C" int gnr_upload_hull_tables(GnrModel* m, int n_samples, const float* near_term, const float* u, void* stream) {
   if (!m || n_samples < 1 || !near_term || !u) {
     gnr_set_error("gnr_upload_hull_tables: bad argument");
@@ -495,12 +516,19 @@ extern "C" int gnr_upload_hull_tables(GnrModel* m, int n_samples, const float* n
   DeviceGuard g(m->device);
   free_dev(m->hull_near_term);
   free_dev(m->hull_u);
+  free_dev(m->hull_ranges);
   m->hull_near_term = m->hull_u = nullptr;
+  m->hull_ranges = nullptr;
   m->hull_samples = 0;
   GNR_CUDA_OK(cudaMalloc(&m->hull_near_term, (size_t)n_samples * 4));
   GNR_CUDA_OK(cudaMalloc(&m->hull_u, (size_t)n_samples * 4));
   GNR_CUDA_OK(cudaMemcpyAsync(m->hull_near_term, near_term, (size_t)n_samples * 4, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
   GNR_CUDA_OK(cudaMemcpyAsync(m->hull_u, u, (size_t)n_samples * 4, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
+  const int n_runs = (n_samples - 1) / 8 + 1, n_words = (n_samples - 1) / 32 + 1;
+  GNR_CUDA_OK(cudaMalloc(&m->hull_ranges, (size_t)(n_runs + n_words) * sizeof(float4)));
+  hull_ranges_kernel<<<(n_runs + n_words + 127) / 128, 128, 0, (cudaStream_t)stream>>>(m->hull_near_term, m->hull_u, n_samples, n_runs,
+                                                                                   n_words, m->hull_ranges);
+  GNR_CUDA_OK(cudaGetLastError());
   m->hull_samples = n_samples;
   return 0;
 }
@@ -729,6 +757,7 @@ GnrSampleParams gnr_sample_params(const GnrModel* m, int S) {
   p.mode = m->cfg.sampling_mode;
   p.hull_a = m->hull_near_term;
   p.hull_u = m->hull_u;
+  p.hull_ranges = m->hull_ranges;
   return p;
 }
 
@@ -755,7 +784,7 @@ int gnr_check_sampler(const GnrModel* m, int S) {
     return -1;
   }
   // the hull sampler reads hull_near_term[k] and hull_u[k] for every k < S
-  if (m->cfg.sampling_mode == 1 && (m->hull_samples != S || !m->hull_u || !m->hull_near_term)) {
+  if (m->cfg.sampling_mode == 1 && (m->hull_samples != S || !m->hull_u || !m->hull_near_term || !m->hull_ranges)) {
     gnr_set_error("hull sampler: tables for %d samples per ray have not been uploaded (have %d)", S, m->hull_samples);
     return -1;
   }

@@ -82,6 +82,7 @@ struct GnrModel {
   // hull sampler tables (sampling_mode 1)
   float* hull_near_term;
   float* hull_u;
+  float4* hull_ranges;  // of both tables, per run of 8 samples, then per word of 32 (see hull_ranges_kernel)
   int hull_samples;
   // staging for gnr_render_host
   void* host_ws;
@@ -125,6 +126,7 @@ struct GnrSampleParams {
   int mode;                 // 0 dense sampler, 1 hull sampler
   const float* hull_a;      // near * (1 - u[k])
   const float* hull_u;      // u[k]
+  const float4* hull_ranges;  // smallest and largest of each over the runs of 8 samples, then over the words of 32
 };
 
 // Workspace layout (byte offsets), identical for every stage call with the same arguments.

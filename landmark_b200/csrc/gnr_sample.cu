@@ -143,9 +143,10 @@ struct RaySetup {  // what the sample tests need of a ray, in shared memory
 // fl(t_min + fl(step k)), the point, and the mask index are each monotone in their argument (every operation is a
 // correctly rounded monotone function), so along each axis every sample between the two end samples lies between them,
 // without any tolerance: if both are inside the box all are, if both are outside on the same side none is, and the mask
-// cells of all samples lie in the range spanned by the cells of the two.  The hull sampler's distance is the sum of a
-// falling term, near (1 - u_k), and a monotone one, far u_k: its run lies between the sums of their smallest and of their
-// largest values, which for a near distance of 0.05 is hardly wider than the two end samples.
+// cells of all samples lie in the range spanned by the cells of the two.  The hull sampler's distance is a_k + far u_k
+// with a_k and u_k from the caller's tables: the run lies between the sums of the terms' smallest and of their largest
+// values, whatever the order of the tables (their ranges over runs and words are kept beside them).  For
+// a_k = near (1 - u_k), rising u_k and a near distance of 0.05 that is hardly wider than the two end samples.
 // BLOCKS: the occupancy of that range is looked up in blocks of 2x2x2 cells, else cell by cell; a run that spans more
 // than four of either along an axis stays open.  (Blocks of 4x4x4 cells, two at most, left 55 % of a city frame's words
 // open; 22 % is what mixes valid and other samples.)
@@ -157,9 +158,11 @@ __device__ __forceinline__ int run_by_ends(const GnrSampleParams& p, const RaySe
     t1 = gnr_sample_t(p, r.t_min, k1);
   } else {
     if (!(fabsf(r.t_min) < 1e30f)) return 2;  // (far u_k is not monotone where 0 x inf comes up)
-    const float f0 = __fmul_rn(r.t_min, __ldg(p.hull_u + k0)), f1 = __fmul_rn(r.t_min, __ldg(p.hull_u + k1));
-    t0 = __fadd_rn(__ldg(p.hull_a + k1), fminf(f0, f1));
-    t1 = __fadd_rn(__ldg(p.hull_a + k0), fmaxf(f0, f1));
+    const float4 range = __ldg(p.hull_ranges + (BLOCKS ? (p.S + 7) / 8 + k0 / 32 : k0 / 8));
+    const float f0 = __fmul_rn(r.t_min, range.z), f1 = __fmul_rn(r.t_min, range.w);
+    t0 = __fadd_rn(range.x, fminf(f0, f1));
+    t1 = __fadd_rn(range.y, fmaxf(f0, f1));
+    if (!(t0 <= t1)) return 2;
   }
   float q0[3], q1[3];
   bool in = true;

@@ -348,3 +348,60 @@ def test_projected_features_of_every_layout(n, ndims, res_mode, channels, mode):
         bound = bound + 2.0 ** -11 * mag + 2.0 ** -25 * w.sum(1)
     worst = ((got - ref).abs() / bound).max().item()
     assert worst <= 1.0, f"error is {worst:.2f} of the bound"
+
+
+@pytest.mark.parametrize("mask", [True, False])
+@pytest.mark.parametrize("tables", ["negative near", "falling", "shuffled", "odd values"])
+def test_hull_sampler_words_for_any_tables(tables, mask):
+    """The sampler takes the tables as they are: a negative near distance (both terms rise), falling and shuffled tables,
+    and tables with values that no run can be decided from.  Words equal bit for bit to testing every sample."""
+    from landmark_b200._lib import check, lib
+    from landmark_b200.gridnerf import B200GridNeRF
+
+    samples, n = 133, 3001
+    spec = scenes.tiny_spec().lit()
+    field, ckpt = oracle_field(spec)
+    if not mask:
+        ckpt = {k: v for k, v in ckpt.items() if not k.startswith("alphaMask")}
+    args = scenes.model_args(spec, "cuda:0")
+    args.sampling_opt, args.n_importance = 1, samples
+    near = -0.7 if tables == "negative near" else 0.1
+    kw = dict(ckpt["kwargs"])
+    kw.update({"device": "cuda:0", "args": args, "is_train": False, "near_far": (near, 6.0)})
+    model = B200GridNeRF(**kw)
+    model.load(ckpt)
+    g = torch.Generator().manual_seed(samples)
+    u = torch.linspace(0.0, 1.0, steps=samples)
+    near_term = near * (1.0 - u)
+    if tables == "falling":
+        near_term, u = near_term.flip(0).contiguous(), u.flip(0).contiguous()
+    elif tables == "shuffled":
+        near_term, u = near_term[torch.randperm(samples, generator=g)], u[torch.randperm(samples, generator=g)]
+    elif tables == "odd values":
+        near_term[5], near_term[40], u[70], u[132] = float("nan"), float("inf"), float("nan"), -float("inf")
+    if tables != "negative near":  # (that one goes through the model's own tables)
+        assert model._samples(samples) == samples
+        a_dev, u_dev = near_term.cuda(), u.cuda()
+        check(lib.gnr_upload_hull_tables(model._handle, samples, a_dev.data_ptr(), u_dev.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+    o = torch.rand((n, 3), generator=g) * 3.0 - 1.5
+    d = torch.randn((n, 3), generator=g)
+    got = model.run_stages(torch.cat([o, d], 1).cuda(), samples, True, upto="sample")
+    a = field.aabb.numpy()
+    o, d, near_term, u = o.numpy(), d.numpy(), near_term.numpy(), u.numpy()
+    with np.errstate(all="ignore"):
+        far = np.where(d[:, 2] >= 0, np.float32(6.0), -((o[:, 2] - a[0, 2]) / d[:, 2]))
+        z = near_term[None] + far[:, None] * u[None]
+        pts = o[:, None] + d[:, None] * z[:, :, None]
+        valid = snp.in_box(pts, a)
+        if mask:
+            m = field.alpha_aabb.numpy()
+            inv = (np.float32(1.0) / (m[1] - m[0])) * np.float32(2)
+            q = (pts[valid] - m[0]) * inv - np.float32(1)
+            finite = np.isfinite(q).all(1)
+            alpha = np.zeros(len(q), np.float32)
+            alpha[finite] = snp.trilinear_zero_pad(field.alpha_volume[0, 0].numpy(), q[finite])
+            at = np.nonzero(valid)
+            valid[at[0][alpha <= 0], at[1][alpha <= 0]] = False
+    assert pts.dtype == np.float32
+    assert np.array_equal(valid_bits_from_words(got["mask_words"], samples), valid)
