@@ -182,6 +182,33 @@ int free_dev(void* p) {
 // ---------------------------------------------------------------------------------------------
 // lifetime
 // ---------------------------------------------------------------------------------------------
+// Pinned memory the compositing writes a chunk's status block into, one block per gnr_render_forward in work.
+struct GnrStatusBlock {
+  int32_t words[GNR_ST_WORDS];
+  GnrStatusBlock* next;
+};
+
+struct GnrHostSide {
+  std::mutex status_mutex;
+  GnrStatusBlock* free_status = nullptr;  // given back by finished calls; as many exist as calls ever ran at once
+};
+
+static int take_status_block(GnrModel* m, GnrStatusBlock** out) {
+  {
+    std::lock_guard<std::mutex> lock(m->host_side->status_mutex);
+    *out = m->host_side->free_status;
+    if (*out) m->host_side->free_status = (*out)->next;
+  }
+  if (!*out) GNR_CUDA_OK(cudaMallocHost(out, sizeof(GnrStatusBlock)));
+  return 0;
+}
+
+static void give_status_block(GnrModel* m, GnrStatusBlock* b) {
+  std::lock_guard<std::mutex> lock(m->host_side->status_mutex);
+  b->next = m->host_side->free_status;
+  m->host_side->free_status = b;
+}
+
 extern "C" int gnr_create(const GnrConfig* cfg, int device, GnrModel** out) {
   if (!cfg || !out) {
     gnr_set_error("gnr_create: null argument");
@@ -240,6 +267,12 @@ extern "C" int gnr_create(const GnrConfig* cfg, int device, GnrModel** out) {
     return -1;
   }
   memset(m, 0, sizeof(*m));
+  m->host_side = new (std::nothrow) GnrHostSide();
+  if (!m->host_side) {
+    delete m;
+    gnr_set_error("gnr_create: out of host memory");
+    return -1;
+  }
   m->cfg = *cfg;
   m->device = device;
   m->sm_count = sms > 0 ? sms : GNR_SM_COUNT_FALLBACK;
@@ -287,7 +320,11 @@ extern "C" int gnr_destroy(GnrModel* m) {
   free_dev(m->host_rgb);
   free_dev(m->host_depth);
   if (m->host_status) cudaFreeHost(m->host_status);
-  if (m->forward_status) cudaFreeHost(m->forward_status);
+  for (GnrStatusBlock *b = m->host_side->free_status, *next; b; b = next) {
+    next = b->next;
+    cudaFreeHost(b);
+  }
+  delete m->host_side;
   for (int i = 0; i < GNR_MAX_LANES; ++i)
     if (m->lane_streams[i]) cudaStreamDestroy(m->lane_streams[i]);
   for (int i = 0; i <= GNR_MAX_LANES; ++i)
@@ -1198,14 +1235,19 @@ extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int
     return -1;
   }
   DeviceGuard g(m->device);
-  // the compositing writes the status block into pinned memory: no copy is queued behind it
-  if (!m->forward_status) GNR_CUDA_OK(cudaMallocHost(&m->forward_status, GNR_ST_WORDS * sizeof(int32_t)));
-  const GnrPixelSink sink{nullptr, nullptr, m->forward_status};
+  // the compositing writes the status block into pinned memory: no copy is queued behind it.  The block is this call's own:
+  // other threads may be in here with workspaces and streams of theirs
+  GnrStatusBlock* block = nullptr;
+  rc = take_status_block(m, &block);
+  if (rc) return rc;
+  const GnrPixelSink sink{nullptr, nullptr, block->words};
   rc = render_chunk_impl(m, rays, n, S, white_bg, (char*)workspace, max_valid, max_app, rgb_map, depth_map, (cudaStream_t)stream,
                          &sink, /*chained=*/true);
+  const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);  // (after an error too: nothing writes the block any more)
+  memcpy(status_h, block->words, GNR_ST_WORDS * sizeof(int32_t));
+  give_status_block(m, block);
   if (rc) return rc;
-  GNR_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
-  memcpy(status_h, m->forward_status, GNR_ST_WORDS * sizeof(int32_t));
+  GNR_CUDA_OK(e);
   return 0;
 }
 

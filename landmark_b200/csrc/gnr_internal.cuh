@@ -42,6 +42,7 @@ struct GnrMlp {
 };
 
 struct GnrProfiler;
+struct GnrHostSide;
 
 struct GnrModel {
   GnrConfig cfg;
@@ -98,7 +99,7 @@ struct GnrModel {
   // lanes of gnr_render_batch / gnr_render_frame
   cudaStream_t lane_streams[GNR_MAX_LANES];
   cudaEvent_t lane_events[GNR_MAX_LANES + 1];
-  int32_t* forward_status;  // pinned
+  GnrHostSide* host_side;  // what calls of several host threads share
 };
 
 // Where the compositing leaves a chunk's pixels and its status block, beside rgb_map / depth_map.

@@ -1,5 +1,7 @@
 """GPU tests of single kernels at the sizes where their work split has its edges: partial tiles and words, the
 smallest and largest chunk a rule picks a form for.  References: the CPU oracle, or the same pixels computed another way."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -405,3 +407,50 @@ def test_hull_sampler_words_for_any_tables(tables, mask):
             valid[at[0][alpha <= 0], at[1][alpha <= 0]] = False
     assert pts.dtype == np.float32
     assert np.array_equal(valid_bits_from_words(got["mask_words"], samples), valid)
+
+
+def test_forward_from_two_threads_returns_each_calls_status():
+    """Two host threads call gnr_render_forward on one model, each with its own workspace and stream: every call returns its
+    own chunk's counts and flags (one thread's list overflows, the other's does not)."""
+    import threading
+
+    from landmark_b200._lib import ST_WORDS, check, lib
+
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    rays = tiny_rays(spec).cuda()
+    jobs = [(rays[4800:5100].contiguous(), 64), (rays[3000:7000].contiguous(), 1)]  # rays, list entries per ray
+    failures = []
+
+    def calls(chunk, per_ray, n_calls):
+        n, s = chunk.shape[0], spec.n_samples
+        need = C.c_size_t(0)
+        check(lib.gnr_render_workspace_bytes(model._handle, n, s, n * s, n * per_ray, C.byref(need)))
+        ws = torch.empty(need.value + 256, dtype=torch.uint8, device="cuda:0")
+        at = ws.data_ptr() + (-ws.data_ptr()) % 256
+        rgb = torch.empty((n, 3), device="cuda:0")
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        seen = []
+        for _ in range(n_calls):
+            st = (C.c_int32 * ST_WORDS)()
+            check(lib.gnr_render_forward(model._handle, chunk.data_ptr(), n, s, 1, at, need.value, n * s, n * per_ray, rgb.data_ptr(),
+                                         None, st, stream.cuda_stream))
+            seen.append(tuple(st))
+        return seen
+
+    want = [calls(*job, 1)[0] for job in jobs]
+    assert want[0][1] == 0 and want[1][1] == 1 and want[0][3] != want[1][3]
+
+    def worker(i):
+        try:
+            failures.extend(s for s in calls(*jobs[i], 400) if s != want[i])
+        except Exception as e:  # noqa: BLE001
+            failures.append(e)
+
+    threads = [threading.Thread(target=worker, args=(i % 2,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[:3]
