@@ -189,6 +189,7 @@ struct GnrStatusBlock {
 };
 
 struct GnrHostSide {
+  std::mutex lane_mutex;  // one call at a time deals chunks to the lanes
   std::mutex status_mutex;
   GnrStatusBlock* free_status = nullptr;  // given back by finished calls; as many exist as calls ever ran at once
 };
@@ -1256,9 +1257,8 @@ extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int
 static int render_batch_impl(GnrModel* m, const float* rays, int64_t n_rays, int S, int white_bg, int64_t chunk, int n_lanes,
                              void* const* ws, int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, uint8_t* rgba,
                              const int32_t* pixel_ids, int32_t* status, cudaEvent_t after, cudaStream_t stream) {
-  static std::mutex mutex;
   const bool fork = n_lanes > 1 && n_rays > chunk;
-  std::unique_lock<std::mutex> lock(mutex, std::defer_lock);
+  std::unique_lock<std::mutex> lock(m->host_side->lane_mutex, std::defer_lock);
   if (fork) {
     lock.lock();
     for (int i = 0; i < n_lanes; ++i) {

@@ -454,3 +454,33 @@ def test_forward_from_two_threads_returns_each_calls_status():
     for t in threads:
         t.join()
     assert not failures, failures[:3]
+
+
+def test_chunk_loops_of_two_models_and_threads():
+    """Chunk loops over lanes from several host threads, two models, two streams each: the lanes of a model are dealt to one
+    call at a time, and no model waits for another's.  Pixels as from one thread."""
+    import threading
+
+    spec = scenes.tiny_spec().lit()
+    models = [cuda_model(spec), cuda_model(spec, mlp_mode=2, app_plane_fp16=True)]
+    rays = tiny_rays(spec).cuda()
+    want = [m.render_rays(rays, spec.n_samples, chunk=1500, overlap=2)[0].clone() for m in models]
+    torch.cuda.synchronize()
+    failures = []
+
+    def worker(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(20):
+                    rgb, _ = models[i % 2].render_rays(rays, spec.n_samples, chunk=1500, overlap=2)
+                    if not torch.equal(rgb, want[i % 2]):
+                        failures.append(i)
+        except Exception as e:  # noqa: BLE001
+            failures.append(e)
+
+    threads = [threading.Thread(target=worker, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[:3]
