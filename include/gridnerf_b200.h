@@ -200,10 +200,12 @@ int gnr_render_forward(GnrModel* m, const float* rays, int64_t n_rays, int n_sam
                        void* workspace, size_t workspace_bytes, int64_t max_valid, int64_t max_app,
                        float* rgb_map, float* depth_map, int32_t* status_h, void* stream);
 
+#define GNR_MAX_LANES 8
 /* The chunk loop over device-resident rays (dist_render/ddp_infer/inferer_impl.py:95-120): chunks of
- * ``chunk_rays`` take the ``n_lanes`` workspaces in turn; with more than one lane and more than one chunk every lane is
- * a stream of the library's, forked from ``stream`` (or behind ``after``, a cudaEvent_t, if it is not NULL) and joined
- * to it.  Each chunk leaves its status block in ``status`` (8 words per chunk; device or pinned host memory). */
+ * ``chunk_rays`` take the ``n_lanes`` workspaces (1 .. GNR_MAX_LANES) in turn; with more than one lane and more than one
+ * chunk every lane is a stream of the library's, forked from ``stream`` (or behind ``after``, a cudaEvent_t, if it is not
+ * NULL) and joined to it.  Each chunk leaves its status block in ``status`` (8 words per chunk; device or pinned host
+ * memory). */
 int gnr_render_batch(GnrModel* m, const float* rays, int64_t n_rays, int n_samples, int white_bg,
                      int64_t chunk_rays, int n_lanes, void* const* workspaces_h, size_t workspace_bytes,
                      int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, int32_t* status,

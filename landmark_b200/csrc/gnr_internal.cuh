@@ -8,7 +8,6 @@
 #include "gridnerf_b200.h"
 
 #define GNR_MAX_PLANES 9
-#define GNR_MAX_LANES 8
 #define GNR_SM_COUNT_FALLBACK 148
 
 // One plane/line pair in device layout: plane [H][W][C] channel-last, line [L][C];

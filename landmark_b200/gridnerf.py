@@ -692,7 +692,7 @@ class B200GridNeRF(torch.nn.Module):
                     overlap=False, after: Optional["torch.cuda.Event"] = None):
         """Device-resident chunk loop: ``rays [N, 6]`` on the GPU -> ``rgb [N, 3]``, ``depth [N]``
         written in place, one status check at the end instead of one per chunk.
-        With ``overlap`` consecutive chunks rotate over that many side streams (``True`` = 2), each
+        With ``overlap`` consecutive chunks rotate over that many side streams (``True`` = 2; at most 8), each
         with its own workspace, so that one chunk's kernels run beside the other's: the stages are
         bound by different units (issue slots, L1, tensor pipe).
         ``after`` (with ``overlap``): the side streams wait for this event instead of for everything queued on the
@@ -721,7 +721,7 @@ class B200GridNeRF(torch.nn.Module):
     def _lanes(self, chunk: int, n_samples: int, n_chunks: int, overlap):
         """Workspaces of a chunk loop: (lanes, their addresses, bytes of each, list capacities)."""
         want = 2 if overlap is True else int(overlap or 1)
-        lanes = want if want > 1 and n_chunks > 1 else 1
+        lanes = max(1, min(want, n_chunks, _lib.MAX_LANES))  # (more chunks in flight than that share the lanes)
         ws = (C.c_void_p * lanes)()
         self._last_workspaces = []
         ws_bytes = None

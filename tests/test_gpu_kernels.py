@@ -484,3 +484,17 @@ def test_chunk_loops_of_two_models_and_threads():
     for t in threads:
         t.join()
     assert not failures, failures[:3]
+
+
+@pytest.mark.parametrize("chunk,overlap,lanes", [(500, 12, 8), (5000, 6, 2), (4000, 3, 3), (20000, 4, 1), (500, 1, 1), (500, True, 2)])
+def test_any_number_of_lanes_is_accepted(chunk, overlap, lanes):
+    """More side streams than the library has lanes, or than there are chunks: same pixels, a workspace per lane in use."""
+    from landmark_b200._lib import MAX_LANES
+
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    rays = tiny_rays(spec).cuda()
+    want, _ = model.render_rays(rays, spec.n_samples, chunk=10000)
+    model.release_workspaces()
+    got, _ = model.render_rays(rays, spec.n_samples, chunk=chunk, overlap=overlap)
+    assert torch.equal(got, want) and len(model._ws) == lanes <= MAX_LANES
