@@ -705,7 +705,8 @@ class B200GridNeRF(torch.nn.Module):
             rgb_out = torch.empty((n, 3), dtype=torch.float32, device=self.device)
         if depth_out is None:
             depth_out = torch.empty((n,), dtype=torch.float32, device=self.device)
-        if n == 0:
+        if n == 0:  # nothing to check (and not the status of the call before)
+            self._pending_status, self._pending_event = torch.zeros((1, _lib.ST_WORDS), dtype=torch.int32), None
             return rgb_out, depth_out
         chunk = max(1, min(chunk, n))
         n_chunks = (n + chunk - 1) // chunk

@@ -498,3 +498,13 @@ def test_any_number_of_lanes_is_accepted(chunk, overlap, lanes):
     model.release_workspaces()
     got, _ = model.render_rays(rays, spec.n_samples, chunk=chunk, overlap=overlap)
     assert torch.equal(got, want) and len(model._ws) == lanes <= MAX_LANES
+
+
+def test_status_of_an_empty_chunk_loop_is_its_own():
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    rays = tiny_rays(spec).cuda()
+    model.app_capacity_per_ray = 1
+    model.render_rays(rays, spec.n_samples)
+    assert model.render_rays(rays[:0], spec.n_samples)[0].shape == (0, 3)
+    assert not model.check_pending_status().any()
