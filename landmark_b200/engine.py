@@ -19,6 +19,7 @@ tiles and the colours come together with one all-gather (``landmark_b200.paralle
 from __future__ import annotations
 
 import ctypes as C
+import threading
 import time
 from typing import Callable, List, Optional
 
@@ -28,6 +29,42 @@ import torch
 from .parallel import TileSharding
 
 RENDER_1080P = (1080, 1920, 1483.6378)  # H, W, focal of the online renderer (nerf_inferer.py:385-404)
+
+
+class _StatusRing:
+    """Pinned status blocks of a renderer's whole-frame calls, ``SLOTS`` in turn, each large enough for the frame that asks.
+    A frame on another stream than the one that used its slot before waits (on the device) for that one's event; the host
+    waits for nothing."""
+
+    SLOTS = 8
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._slots = [None] * self.SLOTS  # (block [n, 8] int32, event behind its frame, that frame's stream)
+        self._outgrown = []                # smaller blocks: frames in flight may still write them
+        self._turn = 0
+
+    def take(self, n_chunks: int, stream):
+        """(slot, its first ``n_chunks`` rows); ``stream`` does not run ahead of the frame that used the slot before."""
+        with self._lock:
+            slot = self._turn
+            self._turn = (slot + 1) % self.SLOTS
+            block, event, other = self._slots[slot] or (None, None, None)
+            if block is None or block.shape[0] < n_chunks:
+                if block is not None:
+                    self._outgrown.append(block)
+                rows = max(64, 1 << (n_chunks - 1).bit_length())
+                block, event = torch.zeros((rows, 8), dtype=torch.int32).pin_memory(), None
+            self._slots[slot] = (block, event, other)
+            if event is not None and other != stream:
+                stream.wait_event(event)
+            return slot, block[:n_chunks]
+
+    def used(self, slot: int, status: torch.Tensor, event, stream):
+        with self._lock:
+            block = self._slots[slot][0]
+            if block.data_ptr() == status.data_ptr():
+                self._slots[slot] = (block, event, stream)
 
 
 class FrameRenderer:
@@ -47,30 +84,22 @@ class FrameRenderer:
         self.model.render_rays(rays, self.n_samples, self.white_bg, chunk=self.chunk, rgb_out=rgb_out,
                                overlap=self.streams if self.streams > 1 else False)
 
-    STATUS_RING = 8  # frames whose status blocks are kept apart
-
     def render_frame(self, pose: np.ndarray, H: int, W: int, focal: float, pixel_ids: torch.Tensor, rgba: torch.Tensor,
                      host_image: torch.Tensor):
         """A whole frame on one GPU in one library call: rays of ``pixel_ids`` (every pixel once), chunk loop, RGBA8 pixels at
-        their places in ``rgba`` and their copy to ``host_image`` (pinned).  Returns the event behind it."""
+        their places in ``rgba`` and their copy to ``host_image`` (pinned).  Returns the event behind it.  The frame's rays are
+        its own, so that frames on other streams may be in flight."""
         from .rays import device_tables
 
-        n = H * W
-        n_chunks = (n + self.chunk - 1) // self.chunk
-        bufs = self.__dict__.get("_frame_buffers")
-        if bufs is None or bufs[0].shape[0] != n or bufs[1].shape[1] != n_chunks:
-            if bufs is not None:  # frames in flight still write status blocks into the pinned ring
-                torch.cuda.synchronize(self.device)
-            bufs = self._frame_buffers = (torch.empty((n, 6), dtype=torch.float32, device=self.device),
-                                          torch.zeros((self.STATUS_RING, n_chunks, 8), dtype=torch.int32).pin_memory())
-            self._frame_turn = 0
-        rays, ring = bufs
-        status = ring[self._frame_turn]
-        self._frame_turn = (self._frame_turn + 1) % self.STATUS_RING
+        stream = torch.cuda.current_stream(self.device)
+        rays = torch.empty((H * W, 6), dtype=torch.float32, device=self.device)
+        ring = self.__dict__.get("_status_ring") or self.__dict__.setdefault("_status_ring", _StatusRing())
+        slot, status = ring.take((H * W + self.chunk - 1) // self.chunk, stream)
         self.model.render_frame(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg,
                                 self.chunk, self.streams, rays, rgba, host_image, status)
         ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(self.device))
+        ev.record(stream)
+        ring.used(slot, status, ev, stream)
         self.model._pending_status, self.model._pending_event = status, ev
         return ev
 

@@ -508,3 +508,51 @@ def test_status_of_an_empty_chunk_loop_is_its_own():
     model.render_rays(rays, spec.n_samples)
     assert model.render_rays(rays[:0], spec.n_samples)[0].shape == (0, 3)
     assert not model.check_pending_status().any()
+
+
+def _runners(model, spec, sizes, **kw):
+    """Runners of one renderer, an image size each."""
+    from landmark_b200.engine import FrameRenderer, NerfDDPRunner
+
+    renderer = FrameRenderer(model, spec.n_samples, **kw)
+    return [NerfDDPRunner(renderer, h, w, focal=spec.focal) for h, w in sizes]
+
+
+def test_frames_of_one_renderer_on_two_streams():
+    """Two runners share a renderer and enqueue frames of their own poses on a stream each, nothing waited for in between:
+    every image is that of its pose."""
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec, mlp_mode=2, app_plane_fp16=True)
+    runners = _runners(model, spec, [(100, 100), (100, 100)], chunk=3000)
+    poses = [scenes.look_at((1.2, 1.2, 1.0), (0.0, 0.0, 0.0)), scenes.look_at((-1.0, 1.4, 0.8), (0.0, 0.0, 0.0))]
+    want = [r.run_batch(p).copy() for r, p in zip(runners, poses)]
+    assert not np.array_equal(*want)
+    streams = [torch.cuda.Stream() for _ in runners]
+    images = [[torch.zeros((100, 100, 4), dtype=torch.uint8).pin_memory() for _ in range(30)] for _ in runners]
+    for k in range(30):
+        for r, p, s, im in zip(runners, poses, streams, images):
+            with torch.cuda.stream(s):
+                r.enqueue(p, im[k])
+    torch.cuda.synchronize()
+    for w, im in zip(want, images):
+        assert all(np.array_equal(w, i.numpy()) for i in im)
+    runners[0].renderer.finish()
+
+
+def test_frames_of_changing_size_wait_for_nothing(monkeypatch):
+    """A renderer that alternates between image sizes and chunk counts: no device-wide wait, and no new pinned memory once
+    every slot has been used."""
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    runners = _runners(model, spec, [(100, 100), (90, 70), (30, 30)])
+    pose = scenes.make_pose(spec)
+    want = [r.run_batch(pose).copy() for _ in range(8) for r in runners][-3:]
+
+    def fail(*a, **k):
+        raise AssertionError("waits or pins memory")
+
+    monkeypatch.setattr(torch.cuda, "synchronize", fail)
+    monkeypatch.setattr(torch.Tensor, "pin_memory", fail)
+    for _ in range(4):
+        for r, w in zip(runners, want):
+            assert np.array_equal(r.run_batch(pose), w)
