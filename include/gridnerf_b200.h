@@ -219,6 +219,13 @@ int gnr_render_frame(GnrModel* m, const float* pose_h, const float* dir_x, const
                      const int32_t* pixel_ids, int n_samples, int white_bg, int64_t chunk_rays, int n_lanes,
                      void* const* workspaces_h, size_t workspace_bytes, int64_t max_valid, int64_t max_app,
                      float* rays, uint8_t* rgba, uint8_t* rgba_h, int32_t* status, void* stream);
+/* gnr_render_frame that also leaves the colours in fp32 on the device: ``rgb[H * W][3]`` in the order of ``pixel_ids`` and
+ * ``image[H][W][3]`` (either may be NULL). */
+int gnr_render_frame_rgb(GnrModel* m, const float* pose_h, const float* dir_x, const float* dir_y, int H, int W,
+                         const int32_t* pixel_ids, int n_samples, int white_bg, int64_t chunk_rays, int n_lanes,
+                         void* const* workspaces_h, size_t workspace_bytes, int64_t max_valid, int64_t max_app,
+                         float* rays, float* rgb, float* image, uint8_t* rgba, uint8_t* rgba_h, int32_t* status,
+                         void* stream);
 
 /* Same forward with HOST buffers: copies ``rays_h`` to the device in chunks of
  * ``chunk_rays``, renders, copies rgb/depth back, synchronises, and returns the status block.

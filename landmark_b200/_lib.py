@@ -77,6 +77,8 @@ SIGNATURES = {
     "gnr_render_batch": (_INT, [_P, _P, _I64, _INT, _INT, _I64, _INT, C.POINTER(_P), _SZ, _I64, _I64, _P, _P, _P, _P, _P]),
     "gnr_render_frame": (_INT, [_P, C.POINTER(C.c_float), _P, _P, _INT, _INT, _P, _INT, _INT, _I64, _INT, C.POINTER(_P), _SZ,
                                 _I64, _I64, _P, _P, _P, _P, _P]),
+    "gnr_render_frame_rgb": (_INT, [_P, C.POINTER(C.c_float), _P, _P, _INT, _INT, _P, _INT, _INT, _I64, _INT, C.POINTER(_P), _SZ,
+                                    _I64, _I64, _P, _P, _P, _P, _P, _P, _P]),
     "gnr_render_chunk": (_INT, [_P, _P, _I64, _INT, _INT, _P, _SZ, _I64, _I64, _P, _P, _P]),
     "gnr_render_host": (_INT, [_P, _P, _I64, _INT, _INT, _I64, _I64, _I64, _P, _P, C.POINTER(C.c_int32)]),
     "gnr_sample": (_INT, [_P, _P, _I64, _INT, _P, _SZ, _I64, _P, _P, _P, _P, _P, _P]),

@@ -1241,7 +1241,8 @@ extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int
   GnrStatusBlock* block = nullptr;
   rc = take_status_block(m, &block);
   if (rc) return rc;
-  const GnrPixelSink sink{nullptr, nullptr, block->words};
+  GnrPixelSink sink{};
+  sink.status = block->words;
   rc = render_chunk_impl(m, rays, n, S, white_bg, (char*)workspace, max_valid, max_app, rgb_map, depth_map, (cudaStream_t)stream,
                          &sink, /*chained=*/true);
   const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);  // (after an error too: nothing writes the block any more)
@@ -1255,8 +1256,8 @@ extern "C" int gnr_render_forward(GnrModel* m, const float* rays, int64_t n, int
 // Chunks of one call, dealt to the lanes in turn.  With several lanes each is a stream of the model's: forked from
 // `stream` (or behind `after`), joined to it at the end.  One call at a time forks (the events are the model's).
 static int render_batch_impl(GnrModel* m, const float* rays, int64_t n_rays, int S, int white_bg, int64_t chunk, int n_lanes,
-                             void* const* ws, int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map, uint8_t* rgba,
-                             const int32_t* pixel_ids, int32_t* status, cudaEvent_t after, cudaStream_t stream) {
+                             void* const* ws, int64_t max_valid, int64_t max_app, float* rgb_map, float* depth_map,
+                             const GnrPixelSink& frame, cudaEvent_t after, cudaStream_t stream) {
   const bool fork = n_lanes > 1 && n_rays > chunk;
   std::unique_lock<std::mutex> lock(m->host_side->lane_mutex, std::defer_lock);
   if (fork) {
@@ -1278,7 +1279,9 @@ static int render_batch_impl(GnrModel* m, const float* rays, int64_t n_rays, int
   for (int64_t first = 0; first < n_rays && !rc; first += chunk, ++c) {
     const int lane = fork ? (int)(c % n_lanes) : 0;
     const int64_t n = first + chunk <= n_rays ? chunk : n_rays - first;
-    const GnrPixelSink sink{rgba, pixel_ids ? pixel_ids + first : nullptr, status ? status + c * GNR_ST_WORDS : nullptr};
+    GnrPixelSink sink = frame;
+    if (sink.pixel_ids) sink.pixel_ids += first;
+    if (sink.status) sink.status += c * GNR_ST_WORDS;
     rc = render_chunk_impl(m, rays + first * 6, n, S, white_bg, (char*)ws[lane], max_valid, max_app, rgb_map ? rgb_map + first * 3 : nullptr,
                            depth_map ? depth_map + first : nullptr, fork ? m->lane_streams[lane] : stream, &sink, /*chained=*/!fork);
   }
@@ -1311,14 +1314,16 @@ extern "C" int gnr_render_batch(GnrModel* m, const float* rays, int64_t n_rays, 
   const int rc = check_batch("gnr_render_batch", m, rays, n_rays, S, chunk, n_lanes, workspaces, ws_bytes, max_valid, max_app);
   if (rc) return rc;
   DeviceGuard g(m->device);
-  return render_batch_impl(m, rays, n_rays, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, rgb_map, depth_map, nullptr,
-                           nullptr, status, (cudaEvent_t)after, (cudaStream_t)stream);
+  GnrPixelSink sink{};
+  sink.status = status;
+  return render_batch_impl(m, rays, n_rays, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, rgb_map, depth_map, sink,
+                           (cudaEvent_t)after, (cudaStream_t)stream);
 }
 
-extern "C" int gnr_render_frame(GnrModel* m, const float* pose_h, const float* dir_x, const float* dir_y, int H, int W,
-                                const int32_t* pixel_ids, int S, int white_bg, int64_t chunk, int n_lanes, void* const* workspaces,
-                                size_t ws_bytes, int64_t max_valid, int64_t max_app, float* rays, uint8_t* rgba, uint8_t* rgba_h,
-                                int32_t* status, void* stream) {
+extern "C" int gnr_render_frame_rgb(GnrModel* m, const float* pose_h, const float* dir_x, const float* dir_y, int H, int W,
+                                    const int32_t* pixel_ids, int S, int white_bg, int64_t chunk, int n_lanes,
+                                    void* const* workspaces, size_t ws_bytes, int64_t max_valid, int64_t max_app, float* rays,
+                                    float* rgb, float* image, uint8_t* rgba, uint8_t* rgba_h, int32_t* status, void* stream) {
   const int64_t n = (int64_t)H * W;
   int rc = check_batch("gnr_render_frame", m, rays, n, S, chunk, n_lanes, workspaces, ws_bytes, max_valid, max_app);
   if (rc) return rc;
@@ -1329,11 +1334,24 @@ extern "C" int gnr_render_frame(GnrModel* m, const float* pose_h, const float* d
   DeviceGuard g(m->device);
   rc = gnr_generate_rays(pose_h, dir_x, dir_y, H, W, pixel_ids, 0, n, rays, stream);
   if (rc) return rc;
-  rc = render_batch_impl(m, rays, n, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, nullptr, nullptr, rgba, pixel_ids,
-                         status, nullptr, (cudaStream_t)stream);
+  GnrPixelSink sink{};
+  sink.rgba = rgba;
+  sink.image = image;
+  sink.pixel_ids = pixel_ids;
+  sink.status = status;
+  rc = render_batch_impl(m, rays, n, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, rgb, nullptr, sink, nullptr,
+                         (cudaStream_t)stream);
   if (rc) return rc;
   GNR_CUDA_OK(cudaMemcpyAsync(rgba_h, rgba, (size_t)n * 4, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   return 0;
+}
+
+extern "C" int gnr_render_frame(GnrModel* m, const float* pose_h, const float* dir_x, const float* dir_y, int H, int W,
+                                const int32_t* pixel_ids, int S, int white_bg, int64_t chunk, int n_lanes, void* const* workspaces,
+                                size_t ws_bytes, int64_t max_valid, int64_t max_app, float* rays, uint8_t* rgba, uint8_t* rgba_h,
+                                int32_t* status, void* stream) {
+  return gnr_render_frame_rgb(m, pose_h, dir_x, dir_y, H, W, pixel_ids, S, white_bg, chunk, n_lanes, workspaces, ws_bytes, max_valid,
+                              max_app, rays, nullptr, nullptr, rgba, rgba_h, status, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1876,7 +1894,8 @@ extern "C" int gnr_render_host(GnrModel* m, const float* rays_h, int64_t n_rays,
     float* d_rgb = m->host_rgb + (size_t)b * chunk * 3;
     float* d_depth = m->host_depth + (size_t)b * chunk;
     GNR_CUDA_OK(cudaMemcpyAsync(d_rays, rays_h + first * 6, (size_t)n * 24, cudaMemcpyHostToDevice, st));
-    const GnrPixelSink sink{nullptr, nullptr, &st_all[(size_t)c * GNR_ST_WORDS]};
+    GnrPixelSink sink{};
+    sink.status = &st_all[(size_t)c * GNR_ST_WORDS];
     rc = render_chunk_impl(m, d_rays, n, S, white_bg, ws, max_valid, max_app, d_rgb, d_depth, st, &sink);
     if (rc) return rc;
     if (rgb_h) GNR_CUDA_OK(cudaMemcpyAsync(rgb_h + first * 3, d_rgb, (size_t)n * 12, cudaMemcpyDeviceToHost, st));

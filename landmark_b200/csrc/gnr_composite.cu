@@ -176,7 +176,15 @@ __device__ __forceinline__ void write_pixel(float r, float g, float b, const flo
     rgb_map[ray * 3 + 2] = b;
   }
   if (depth_map) depth_map[ray] = depth[ray];
-  if (sink.rgba) reinterpret_cast<uchar4*>(sink.rgba)[sink.pixel_ids[ray]] = to_rgba8(r, g, b);
+  if (sink.rgba) {
+    const int64_t pixel = sink.pixel_ids[ray];
+    reinterpret_cast<uchar4*>(sink.rgba)[pixel] = to_rgba8(r, g, b);
+    if (sink.image) {
+      sink.image[pixel * 3 + 0] = r;
+      sink.image[pixel * 3 + 1] = g;
+      sink.image[pixel * 3 + 2] = b;
+    }
+  }
 }
 
 // The chunk's status block is complete when the compositing starts: its first block hands it on.
@@ -304,7 +312,7 @@ int launch_app_compact(const GnrModel* m, const GnrSampleParams& p, int64_t n, c
 int launch_composite(const GnrModel* m, int64_t n, int white_bg, char* ws, const GnrWs& L, float* rgb_map,
                      float* depth_map, cudaStream_t st, int march_lanes, const GnrPixelSink* sink_in) {
   (void)m;
-  const GnrPixelSink sink = sink_in ? *sink_in : GnrPixelSink{nullptr, nullptr, nullptr};
+  const GnrPixelSink sink = sink_in ? *sink_in : GnrPixelSink{};
   const int32_t* status = (const int32_t*)(ws + L.status);
   if (march_lanes == 32) {  // ray-by-ray lists
     const int rc = gnr_launch(composite_rays_kernel, (unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st,

@@ -104,6 +104,7 @@ struct GnrModel {
 // Where the compositing leaves a chunk's pixels and its status block, beside rgb_map / depth_map.
 struct GnrPixelSink {
   uint8_t* rgba;             // null, or the RGBA8 image ...
+  float* image;              // (null, or the same in fp32, three floats a pixel)
   const int32_t* pixel_ids;  // ... and the pixel of every ray of the chunk
   int32_t* status;           // null, or 8 words of device or pinned host memory
 };

@@ -85,10 +85,11 @@ class FrameRenderer:
                                overlap=self.streams if self.streams > 1 else False)
 
     def render_frame(self, pose: np.ndarray, H: int, W: int, focal: float, pixel_ids: torch.Tensor, rgba: torch.Tensor,
-                     host_image: torch.Tensor):
+                     host_image: torch.Tensor, rgb: Optional[torch.Tensor] = None, image: Optional[torch.Tensor] = None):
         """A whole frame on one GPU in one library call: rays of ``pixel_ids`` (every pixel once), chunk loop, RGBA8 pixels at
-        their places in ``rgba`` and their copy to ``host_image`` (pinned).  Returns the event behind it.  The frame's rays are
-        its own, so that frames on other streams may be in flight."""
+        their places in ``rgba`` and their copy to ``host_image`` (pinned); ``rgb`` and ``image``: the colours in fp32 too, in
+        the order of ``pixel_ids`` and of the image.  Returns the event behind it.  The frame's rays are its own, so that
+        frames on other streams may be in flight."""
         from .rays import device_tables
 
         stream = torch.cuda.current_stream(self.device)
@@ -96,7 +97,7 @@ class FrameRenderer:
         ring = self.__dict__.get("_status_ring") or self.__dict__.setdefault("_status_ring", _StatusRing())
         slot, status = ring.take((H * W + self.chunk - 1) // self.chunk, stream)
         self.model.render_frame(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg,
-                                self.chunk, self.streams, rays, rgba, host_image, status)
+                                self.chunk, self.streams, rays, rgba, host_image, status, rgb, image)
         ev = torch.cuda.Event()
         ev.record(stream)
         ring.used(slot, status, ev, stream)
@@ -299,7 +300,8 @@ class NerfDDPRunner:
         pose = np.asarray(single_pose.cpu() if isinstance(single_pose, torch.Tensor) else single_pose, dtype=np.float32)
         focal = self._focal_of(pose)
         if self._whole_frame(host_image):
-            return self.renderer.render_frame(pose[:3, :4], self.H, self.W, focal, self.shard.pixel_ids, self.rgba, host_image)
+            return self.renderer.render_frame(pose[:3, :4], self.H, self.W, focal, self.shard.pixel_ids, self.rgba, host_image,
+                                              self.rgb, self.image)
         pose, focal, _ = self._broadcast(pose[:3, :4], focal, False)
         self.renderer.render_pixels(pose, self.H, self.W, focal, self.shard.pixel_ids, self.rgb[: self.shard.n_local])
         self.shard.assemble(self.rgb, self.image)

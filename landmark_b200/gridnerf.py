@@ -734,19 +734,23 @@ class B200GridNeRF(torch.nn.Module):
         return lanes, ws, ws_bytes, max_valid, max_app
 
     def render_frame(self, pose: np.ndarray, tables, H: int, W: int, pixel_ids: torch.Tensor, N_samples: int, white_bg: bool,
-                     chunk: int, overlap, rays: torch.Tensor, rgba: torch.Tensor, host_image: torch.Tensor, status: torch.Tensor):
-        """One frame without waiting (gnr_render_frame): ``pose`` ``[3, 4]`` float32, ``tables`` the two direction tables on
+                     chunk: int, overlap, rays: torch.Tensor, rgba: torch.Tensor, host_image: torch.Tensor, status: torch.Tensor,
+                     rgb: Optional[torch.Tensor] = None, image: Optional[torch.Tensor] = None):
+        """One frame without waiting (gnr_render_frame_rgb): ``pose`` ``[3, 4]`` float32, ``tables`` the two direction tables on
         the device, ``pixel_ids`` every pixel once, ``rays [H * W, 6]`` and ``rgba`` device buffers, ``host_image`` pinned
-        ``uint8 [H, W, 4]``, ``status`` pinned ``int32 [n_chunks, 8]``, complete when the stream's work is."""
+        ``uint8 [H, W, 4]``, ``status`` pinned ``int32 [n_chunks, 8]``, complete when the stream's work is; ``rgb`` and
+        ``image``: the colours in fp32 too, ``[H * W, 3]`` in the order of ``pixel_ids`` and of the image."""
         s = self._samples(N_samples)
         n = H * W
         chunk = max(1, min(chunk, n))
         lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, (n + chunk - 1) // chunk, overlap)
         pose_c = (C.c_float * 12).from_buffer_copy(pose.astype(np.float32, copy=False).tobytes())
-        check(lib.gnr_render_frame(self._handle, pose_c, tables[0].data_ptr(), tables[1].data_ptr(), H, W, pixel_ids.data_ptr(), s,
-                                   int(bool(white_bg)), chunk, lanes, ws, ws_bytes, max_valid, max_app, rays.data_ptr(),
-                                   rgba.data_ptr(), host_image.data_ptr(), status.data_ptr(),
-                                   torch.cuda.current_stream(self.device).cuda_stream), "gnr_render_frame")
+        check(lib.gnr_render_frame_rgb(self._handle, pose_c, tables[0].data_ptr(), tables[1].data_ptr(), H, W,
+                                       pixel_ids.data_ptr(), s, int(bool(white_bg)), chunk, lanes, ws, ws_bytes, max_valid, max_app,
+                                       rays.data_ptr(), None if rgb is None else rgb.data_ptr(),
+                                       None if image is None else image.data_ptr(), rgba.data_ptr(), host_image.data_ptr(),
+                                       status.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream),
+              "gnr_render_frame_rgb")
 
     def check_pending_status(self):
         """Synchronise and raise if any chunk of the last ``render_rays`` overflowed a list."""

@@ -556,3 +556,20 @@ def test_frames_of_changing_size_wait_for_nothing(monkeypatch):
     for _ in range(4):
         for r, w in zip(runners, want):
             assert np.array_equal(r.run_batch(pose), w)
+
+
+def test_whole_frame_leaves_the_colours_in_the_runner():
+    """``rgb`` (tile order) and ``image`` (row order) of a runner hold the frame in fp32, as the stages leave them."""
+    from landmark_b200.engine import FrameRenderer, NerfDDPRunner
+
+    class Stages(FrameRenderer):
+        def to_rgba8(self, image, out):
+            super().to_rgba8(image, out)
+
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    for pose in (scenes.make_pose(spec), scenes.look_at((1.2, 1.2, 1.0), (0.0, 0.0, 0.0))):
+        for h, w in ((100, 100), (37, 61)):
+            whole, staged = (NerfDDPRunner(r(model, spec.n_samples, chunk=3000), h, w, focal=spec.focal) for r in (FrameRenderer, Stages))
+            assert np.array_equal(whole.run_batch(pose), staged.run_batch(pose))
+            assert torch.equal(whole.rgb, staged.rgb) and torch.equal(whole.image, staged.image) and whole.image.std() > 0
