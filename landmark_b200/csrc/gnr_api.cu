@@ -1338,6 +1338,7 @@ extern "C" int gnr_render_frame_rgb(GnrModel* m, const float* pose_h, const floa
   sink.rgba = rgba;
   sink.image = image;
   sink.pixel_ids = pixel_ids;
+  sink.n_pixels = n;
   sink.status = status;
   rc = render_batch_impl(m, rays, n, S, white_bg, chunk, n_lanes, workspaces, max_valid, max_app, rgb, nullptr, sink, nullptr,
                          (cudaStream_t)stream);

@@ -178,6 +178,7 @@ __device__ __forceinline__ void write_pixel(float r, float g, float b, const flo
   if (depth_map) depth_map[ray] = depth[ray];
   if (sink.rgba) {
     const int64_t pixel = sink.pixel_ids[ray];
+    if (pixel < 0 || pixel >= sink.n_pixels) return;
     reinterpret_cast<uchar4*>(sink.rgba)[pixel] = to_rgba8(r, g, b);
     if (sink.image) {
       sink.image[pixel * 3 + 0] = r;

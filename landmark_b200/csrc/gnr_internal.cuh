@@ -105,7 +105,8 @@ struct GnrModel {
 struct GnrPixelSink {
   uint8_t* rgba;             // null, or the RGBA8 image ...
   float* image;              // (null, or the same in fp32, three floats a pixel)
-  const int32_t* pixel_ids;  // ... and the pixel of every ray of the chunk
+  const int32_t* pixel_ids;  // ... and the pixel of every ray of the chunk (one outside the image is dropped)
+  int64_t n_pixels;
   int32_t* status;           // null, or 8 words of device or pinned host memory
 };
 

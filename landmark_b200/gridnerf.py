@@ -743,8 +743,23 @@ class B200GridNeRF(torch.nn.Module):
         s = self._samples(N_samples)
         n = H * W
         chunk = max(1, min(chunk, n))
-        lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, (n + chunk - 1) // chunk, overlap)
-        pose_c = (C.c_float * 12).from_buffer_copy(pose.astype(np.float32, copy=False).tobytes())
+        n_chunks = (n + chunk - 1) // chunk
+        pixel_ids = pixel_ids.to(device=self.device, dtype=torch.int32).contiguous()
+        pose = np.asarray(pose, dtype=np.float32)
+        if pose.shape != (3, 4) or pixel_ids.numel() != n:
+            raise ValueError(f"render_frame: a [3, 4] pose and {n} pixels, got {pose.shape} and {pixel_ids.numel()}")
+        for what, t, dtype, size in (("tables[0]", tables[0], torch.float32, W), ("tables[1]", tables[1], torch.float32, H),
+                                     ("rays", rays, torch.float32, 6 * n), ("rgba", rgba, torch.uint8, 4 * n),
+                                     ("rgb", rgb, torch.float32, 3 * n), ("image", image, torch.float32, 3 * n),
+                                     ("host_image", host_image, torch.uint8, 4 * n), ("status", status, torch.int32, 8 * n_chunks)):
+            if t is None and what in ("rgb", "image"):
+                continue
+            host = what in ("host_image", "status")
+            if t.dtype != dtype or t.numel() < size or not t.is_contiguous() or not (t.is_pinned() if host else t.is_cuda):
+                raise ValueError(f"render_frame: {what} must be contiguous {dtype} of at least {size} values "
+                                 f"{'in pinned memory' if host else 'on the device'}, got {t.dtype} {tuple(t.shape)} on {t.device}")
+        lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, n_chunks, overlap)
+        pose_c = (C.c_float * 12).from_buffer_copy(pose.tobytes())
         check(lib.gnr_render_frame_rgb(self._handle, pose_c, tables[0].data_ptr(), tables[1].data_ptr(), H, W,
                                        pixel_ids.data_ptr(), s, int(bool(white_bg)), chunk, lanes, ws, ws_bytes, max_valid, max_app,
                                        rays.data_ptr(), None if rgb is None else rgb.data_ptr(),

@@ -573,3 +573,41 @@ def test_whole_frame_leaves_the_colours_in_the_runner():
             whole, staged = (NerfDDPRunner(r(model, spec.n_samples, chunk=3000), h, w, focal=spec.focal) for r in (FrameRenderer, Stages))
             assert np.array_equal(whole.run_batch(pose), staged.run_batch(pose))
             assert torch.equal(whole.rgb, staged.rgb) and torch.equal(whole.image, staged.image) and whole.image.std() > 0
+
+
+def test_frame_call_checks_its_arguments():
+    """Pixel lists of any integer type are converted, as generate_rays does; buffers of another type, size or place, which
+    the library would write as raw memory, are refused."""
+    from landmark_b200.engine import FrameRenderer
+    from landmark_b200.rays import device_tables
+
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    runner = _runners(model, spec, [(60, 50)])[0]
+    pose = scenes.make_pose(spec)
+    want = runner.run_batch(pose).copy()
+    ids = runner.shard.pixel_ids
+    renderer = FrameRenderer(model, spec.n_samples)
+    for other in (ids.to(torch.int64), ids.cpu(), torch.stack([ids, ids], 1)[:, 0]):
+        image = torch.zeros((60, 50, 4), dtype=torch.uint8).pin_memory()
+        renderer.render_frame(pose, 60, 50, spec.focal, other, runner.rgba, image).synchronize()
+        assert np.array_equal(want, image.numpy())
+    dev = {"device": "cuda:0"}
+    good = {"rays": torch.empty((3000, 6), **dev), "rgba": torch.empty((3000, 4), dtype=torch.uint8, **dev),
+            "host_image": torch.empty((60, 50, 4), dtype=torch.uint8).pin_memory(), "status": torch.empty((1, 8), dtype=torch.int32).pin_memory(),
+            "rgb": torch.empty((3000, 3), **dev), "image": torch.empty((3000, 3), **dev), "pixel_ids": ids, "pose": pose}
+
+    def call(**changed):
+        a = dict(good, **changed)
+        model.render_frame(a["pose"], device_tables(60, 50, spec.focal, "cuda:0"), 60, 50, a["pixel_ids"], spec.n_samples, True, 131072, 2,
+                           a["rays"], a["rgba"], a["host_image"], a["status"], a["rgb"], a["image"])
+
+    call()
+    torch.cuda.synchronize()
+    assert np.array_equal(want, good["host_image"].numpy())
+    for changed in ({"rays": good["rays"].half()}, {"rays": good["rays"][:-1]}, {"rays": good["rays"].cpu()}, {"rgba": good["rgb"]},
+                    {"rgba": torch.empty((60, 100, 4), dtype=torch.uint8, **dev)[:, ::2]}, {"host_image": good["host_image"].clone()},
+                    {"host_image": good["rgba"]}, {"status": good["status"].clone()}, {"status": good["status"][:0]},
+                    {"rgb": good["rgb"].double()}, {"image": good["image"][1:]}, {"pixel_ids": ids[:-1]}, {"pose": pose[:2]}):
+        with pytest.raises(ValueError):
+            call(**changed)
