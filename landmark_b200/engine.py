@@ -282,13 +282,18 @@ class NerfDDPRunner:
         self.renderer.finish()
 
     def _whole_frame(self, host_image: torch.Tensor) -> bool:
-        """One library call does the frame: a single rank, FrameRenderer's own stages over a model that has the call, and
-        an image the call can write as plain bytes.  Everything else goes stage by stage."""
+        """One library call does the frame: a single rank, FrameRenderer's and the model's own stages, not replaced in a class
+        or on an object, and an image the call can write as plain bytes.  Everything else goes stage by stage."""
+        from .gridnerf import B200GridNeRF
+
         r = self.renderer
-        return (self.world == 1 and isinstance(r, FrameRenderer) and type(r).render_pixels is FrameRenderer.render_pixels
-                and type(r).to_rgba8 is FrameRenderer.to_rgba8 and hasattr(r.model, "render_frame") and host_image.is_pinned()
-                and host_image.is_contiguous() and host_image.dtype == torch.uint8
-                and tuple(host_image.shape) == (self.H, self.W, 4))
+        if self.world != 1 or not isinstance(r, FrameRenderer) or not isinstance(r.model, B200GridNeRF):
+            return False
+        for obj, base, stages in ((r, FrameRenderer, ("render_pixels", "to_rgba8")), (r.model, B200GridNeRF, ("render_rays",))):
+            if any(s in vars(obj) or getattr(type(obj), s) is not getattr(base, s) for s in stages):
+                return False
+        return (host_image.dtype == torch.uint8 and tuple(host_image.shape) == (self.H, self.W, 4) and host_image.is_contiguous()
+                and host_image.is_pinned())
 
     def enqueue(self, single_pose, host_image: torch.Tensor):
         """Everything ``run_batch`` does for one frame except waiting for it: broadcast, render, gather,

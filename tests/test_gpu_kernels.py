@@ -611,3 +611,35 @@ def test_frame_call_checks_its_arguments():
                     {"rgb": good["rgb"].double()}, {"image": good["image"][1:]}, {"pixel_ids": ids[:-1]}, {"pose": pose[:2]}):
         with pytest.raises(ValueError):
             call(**changed)
+
+
+def test_stages_replaced_on_objects_are_run():
+    """A renderer whose stages, or a model whose chunk loop, are replaced in a subclass or on the object: the frame goes
+    through them."""
+    from landmark_b200.gridnerf import B200GridNeRF
+
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    pose = scenes.make_pose(spec)
+    runner = _runners(model, spec, [(30, 30)])[0]
+    want = runner.run_batch(pose).copy()
+    ran = []
+
+    def noting(name, stage):
+        def f(*a, **k):
+            ran.append(name)
+            return stage(*a, **k)
+        return f
+
+    for obj, name in ((runner.renderer, "render_pixels"), (runner.renderer, "to_rgba8"), (model, "render_rays")):
+        setattr(obj, name, noting(name, getattr(obj, name)))
+        assert np.array_equal(runner.run_batch(pose), want) and ran[-1] == name
+        delattr(obj, name)
+
+    class Own(B200GridNeRF):
+        def render_rays(self, *a, **k):
+            ran.append("subclass")
+            return super().render_rays(*a, **k)
+
+    model.__class__ = Own
+    assert np.array_equal(runner.run_batch(pose), want) and ran[-1] == "subclass"
