@@ -95,9 +95,10 @@ class FrameRenderer:
         stream = torch.cuda.current_stream(self.device)
         rays = torch.empty((H * W, 6), dtype=torch.float32, device=self.device)
         ring = self.__dict__.get("_status_ring") or self.__dict__.setdefault("_status_ring", _StatusRing())
-        slot, status = ring.take((H * W + self.chunk - 1) // self.chunk, stream)
+        chunk = max(1, min(self.chunk, H * W))
+        slot, status = ring.take((H * W + chunk - 1) // chunk, stream)
         self.model.render_frame(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg,
-                                self.chunk, self.streams, rays, rgba, host_image, status, rgb, image)
+                                chunk, self.streams, rays, rgba, host_image, status, rgb, image)
         ev = torch.cuda.Event()
         ev.record(stream)
         ring.used(slot, status, ev, stream)

@@ -643,3 +643,13 @@ def test_stages_replaced_on_objects_are_run():
 
     model.__class__ = Own
     assert np.array_equal(runner.run_batch(pose), want) and ran[-1] == "subclass"
+
+
+def test_frame_with_a_chunk_size_below_one():
+    """Chunk sizes below one ray mean one ray, as in the chunk loop."""
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    pose = scenes.make_pose(spec)
+    want = _runners(model, spec, [(7, 9)])[0].run_batch(pose)
+    for chunk in (0, -3):
+        assert np.array_equal(_runners(model, spec, [(7, 9)], chunk=chunk)[0].run_batch(pose), want)
