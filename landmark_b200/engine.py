@@ -284,7 +284,7 @@ class NerfDDPRunner:
 
     def _whole_frame(self, host_image: torch.Tensor) -> bool:
         """One library call does the frame: a single rank, FrameRenderer's and the model's own stages, not replaced in a class
-        or on an object, and an image the call can write as plain bytes.  Everything else goes stage by stage."""
+        or on an object, an image the call can write as plain bytes, and no capture.  Everything else goes stage by stage."""
         from .gridnerf import B200GridNeRF
 
         r = self.renderer
@@ -294,7 +294,7 @@ class NerfDDPRunner:
             if any(s in vars(obj) or getattr(type(obj), s) is not getattr(base, s) for s in stages):
                 return False
         return (host_image.dtype == torch.uint8 and tuple(host_image.shape) == (self.H, self.W, 4) and host_image.is_contiguous()
-                and host_image.is_pinned())
+                and host_image.is_pinned() and not torch.cuda.is_current_stream_capturing())
 
     def enqueue(self, single_pose, host_image: torch.Tensor):
         """Everything ``run_batch`` does for one frame except waiting for it: broadcast, render, gather,

@@ -653,3 +653,21 @@ def test_frame_with_a_chunk_size_below_one():
     want = _runners(model, spec, [(7, 9)])[0].run_batch(pose)
     for chunk in (0, -3):
         assert np.array_equal(_runners(model, spec, [(7, 9)], chunk=chunk)[0].run_batch(pose), want)
+
+
+def test_a_frame_can_be_captured():
+    """enqueue under a CUDA graph capture goes stage by stage, which a graph can replay."""
+    spec = scenes.tiny_spec().lit()
+    model = cuda_model(spec)
+    pose = scenes.make_pose(spec)
+    runner = _runners(model, spec, [(50, 50)])[0]
+    want = runner.run_batch(pose).copy()
+    image = torch.zeros((50, 50, 4), dtype=torch.uint8).pin_memory()
+    model.render_rays(runner.rgb.new_zeros((2500, 6)), spec.n_samples)  # (workspace)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        runner.enqueue(pose, image)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(image.numpy(), want)
