@@ -671,3 +671,53 @@ def test_a_frame_can_be_captured():
     graph.replay()
     torch.cuda.synchronize()
     assert np.array_equal(image.numpy(), want)
+
+
+def _inferer(spec, chunk, **options):
+    from types import SimpleNamespace
+
+    from landmark_b200.inferer import B200NerfDDPInfererImpl
+
+    args = scenes.model_args(spec, "cuda:0")
+    args.render_batch_size = chunk
+    impl = B200NerfDDPInfererImpl(SimpleNamespace(args_nerf=args, checkpoint=scenes.make_checkpoint(spec), model_path=None), **options)
+    impl.load_model(spec.height, spec.width)
+    return impl
+
+
+def test_inferer_runs_what_is_hooked_to_the_forward():
+    """Forward hooks of the model, global ones, and a forward replaced on the object or in a subclass run once per chunk of
+    render_batch_size rays, as in the plain chunk loop."""
+    from landmark_b200.gridnerf import B200GridNeRF
+
+    spec = scenes.tiny_spec().lit()
+    impl = _inferer(spec, 2048)
+    model = impl.model
+    rays = tiny_rays(spec).cuda()
+    want = impl.renderer_fn(rays, N_samples=spec.n_samples)
+    ran = []
+
+    def count(*a, **k):
+        ran.append(1)
+
+    for register in (model.register_forward_hook, model.register_forward_pre_hook,
+                     torch.nn.modules.module.register_module_forward_hook, torch.nn.modules.module.register_module_forward_pre_hook):
+        ran.clear()
+        handle = register(count)
+        assert torch.equal(impl.renderer_fn(rays, N_samples=spec.n_samples), want)
+        handle.remove()
+        assert len(ran) == 5
+    ran.clear()
+    forward = model.forward
+    model.forward = lambda *a, **k: (count(), forward(*a, **k))[1]
+    assert torch.equal(impl.renderer_fn(rays, N_samples=spec.n_samples), want) and len(ran) == 5
+    del model.forward
+
+    class Own(B200GridNeRF):
+        def forward(self, *a, **k):
+            count()
+            return super().forward(*a, **k)
+
+    ran.clear()
+    model.__class__ = Own
+    assert torch.equal(impl.renderer_fn(rays, N_samples=spec.n_samples), want) and len(ran) == 5
