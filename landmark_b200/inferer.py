@@ -145,6 +145,7 @@ class B200NerfDDPInfererImpl:
                 self._model.set_app_code(kw.get("app_code"))
                 fit = min(self.RENDER_CHUNK, self.RENDER_SAMPLES // self._model._samples(N_samples))
                 rgb, _ = self._model.render_rays(rays, N_samples, white_bg, chunk=max(self._chunk_size, fit), overlap=2)
-                self._model.check_pending_status()
+                if self._model.check_status_every_call:
+                    self._model.check_pending_status()
             return rgb
         return renderer_fn(self._forward, rays, self._chunk_size, **kw)

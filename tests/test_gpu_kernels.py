@@ -721,3 +721,18 @@ def test_inferer_runs_what_is_hooked_to_the_forward():
     ran.clear()
     model.__class__ = Own
     assert torch.equal(impl.renderer_fn(rays, N_samples=spec.n_samples), want) and len(ran) == 5
+
+
+def test_inferer_without_status_checks():
+    """With ``check_status_every_call`` off renderer_fn neither waits for the status nor raises, as its chunks' forwards; the
+    status is there to be asked for."""
+    spec = scenes.tiny_spec().lit()
+    impl = _inferer(spec, 2048)
+    rays = tiny_rays(spec).cuda()
+    impl.model.app_capacity_per_ray = 1
+    with pytest.raises(RuntimeError, match="appearance-sample list overflow"):
+        impl.renderer_fn(rays, N_samples=spec.n_samples)
+    impl.model.check_status_every_call = False
+    assert impl.renderer_fn(rays, N_samples=spec.n_samples).shape == (10000, 3)
+    with pytest.raises(RuntimeError, match="appearance-sample list overflow"):
+        impl.model.check_pending_status()
