@@ -501,6 +501,20 @@ class B200GridNeRF(torch.nn.Module):
         per_app = min(n_samples, self.app_capacity_per_ray)
         return max(1, n_rays * per_valid), max(1, n_rays * per_app)
 
+    def workspace_bytes(self, n_rays: int, n_samples: int, stages: bool = False) -> int:
+        """Bytes of scratch a chunk of that shape needs (see ``workspace``)."""
+        max_valid, max_app = self.capacities(n_rays, n_samples)
+        key = (n_rays, n_samples, max_valid, max_app, stages)
+        need = self._ws_bytes.get(key)
+        if need is None:
+            nbytes = C.c_size_t(0)
+            query = lib.gnr_workspace_bytes if stages else lib.gnr_render_workspace_bytes
+            check(query(self._handle, n_rays, n_samples, max_valid, max_app, C.byref(nbytes)), "gnr_workspace_bytes")
+            if len(self._ws_bytes) > 256:
+                self._ws_bytes.clear()
+            need = self._ws_bytes[key] = int(nbytes.value)
+        return need
+
     def workspace(self, n_rays: int, n_samples: int, slot: int = 0, stages: bool = False):
         """Scratch buffer of chunk slot ``slot`` (one per stream that renders chunks concurrently), large enough for the
         rendering entries; ``stages``: for the stage-wise entries, whose id lists, per-sample features and product tiles a
@@ -514,15 +528,7 @@ class B200GridNeRF(torch.nn.Module):
         (``GraphedFrameRenderer`` does), which keeps that memory out of the allocator for as long
         as the graph lives."""
         max_valid, max_app = self.capacities(n_rays, n_samples)
-        key = (n_rays, n_samples, max_valid, max_app, stages)
-        need = self._ws_bytes.get(key)
-        if need is None:
-            nbytes = C.c_size_t(0)
-            query = lib.gnr_workspace_bytes if stages else lib.gnr_render_workspace_bytes
-            check(query(self._handle, n_rays, n_samples, max_valid, max_app, C.byref(nbytes)), "gnr_workspace_bytes")
-            if len(self._ws_bytes) > 256:
-                self._ws_bytes.clear()
-            need = self._ws_bytes[key] = int(nbytes.value)
+        need = self.workspace_bytes(n_rays, n_samples, stages)
         buf = self._ws.get(slot)
         if buf is None or buf.numel() < need + 256:
             if buf is not None:

@@ -51,8 +51,9 @@ class B200NerfDDPInfererImpl:
     """Drop-in for ``TorchNerfDDPInfererImpl``: same constructor argument (a context with
     ``args_nerf`` and ``model_path``), same methods and properties."""
 
-    RENDER_CHUNK = 65536      # rays of a device chunk, unless render_batch_size is larger
+    RENDER_CHUNK = 65536      # rays of a device chunk, unless render_batch_size is larger (0: always render_batch_size)
     RENDER_SAMPLES = 1 << 25  # and at most that many samples of them: the ids and lists of a chunk grow with both
+    RENDER_MEMORY = 0.125     # and as long as the workspaces take no more than that share of the free device memory
 
     def __init__(self, context, profile_stages: bool = False, mlp_mode: Optional[int] = None, preset: str = "exact",
                  **model_options) -> None:
@@ -74,6 +75,7 @@ class B200NerfDDPInfererImpl:
         self._model = None
         self._model_path = getattr(context, "model_path", None)
         self._ckpt = getattr(context, "checkpoint", None)  # an already loaded checkpoint dict
+        self._out_of_memory = False  # larger device chunks did not fit once: render_batch_size from then on
 
     @property
     def args(self):
@@ -129,6 +131,26 @@ class B200NerfDDPInfererImpl:
                 and type(m).__call__ is torch.nn.Module.__call__ and "forward" not in vars(m)
                 and not (m._forward_hooks or m._forward_pre_hooks or hooks._global_forward_hooks or hooks._global_forward_pre_hooks))
 
+    def _device_chunk(self, n_rays: int, n_samples: int):
+        """(rays of a device chunk, lanes) of a call: RENDER_CHUNK rays on two lanes, halved while their workspaces would take
+        too much of the memory; at the least what ``render_batch_size`` says, in one workspace."""
+        m, least = self._model, self._chunk_size
+        chunk = least if self._out_of_memory else max(least, min(self.RENDER_CHUNK, self.RENDER_SAMPLES // n_samples))
+        while not self._out_of_memory:
+            need = m.workspace_bytes(min(chunk, n_rays), n_samples) + 256
+            lanes = 2 if n_rays > chunk else 1
+            missing = sum(need for slot in range(lanes) if slot not in m._ws or m._ws[slot].numel() < need)
+            if not missing:
+                return chunk, lanes
+            free = (torch.cuda.mem_get_info(m.device)[0] + torch.cuda.memory_reserved(m.device)
+                    - torch.cuda.memory_allocated(m.device))
+            if missing <= self.RENDER_MEMORY * free:
+                return chunk, lanes
+            if chunk <= least:
+                break
+            chunk = max(least, chunk // 2)
+        return least, 1
+
     def renderer_fn(self, rays, N_samples=-1, white_bg=True, is_train=False, app_code=None):
         if self._forward is None:
             raise RuntimeError("load_model() has not been called")
@@ -138,14 +160,22 @@ class B200NerfDDPInfererImpl:
             # for an encode_app checkpoint; here it reaches the model
             kw["app_code"] = app_code
         if self._plain_forward() and not is_train and rays.shape[0] > 0:
-            # The same chunks as one library call: pixels do not depend on how rays are cut into chunks, so chunks of at
-            # least RENDER_CHUNK rays rotate over two lanes and the status blocks are read once at the end, instead of a
-            # wait per chunk of render_batch_size rays (960x540 in chunks of 8192: 64 waits).
+            # The same chunks as one library call: pixels do not depend on how rays are cut into chunks, so larger chunks
+            # rotate over two lanes and the status blocks are read once at the end, instead of a wait per chunk of
+            # render_batch_size rays (960x540 in chunks of 8192: 64 waits).
             with torch.inference_mode():
-                self._model.set_app_code(kw.get("app_code"))
-                fit = min(self.RENDER_CHUNK, self.RENDER_SAMPLES // self._model._samples(N_samples))
-                rgb, _ = self._model.render_rays(rays, N_samples, white_bg, chunk=max(self._chunk_size, fit), overlap=2)
-                if self._model.check_status_every_call:
-                    self._model.check_pending_status()
+                model = self._model
+                model.set_app_code(kw.get("app_code"))
+                chunk, lanes = self._device_chunk(rays.shape[0], model._samples(N_samples))
+                try:
+                    rgb, _ = model.render_rays(rays, N_samples, white_bg, chunk=chunk, overlap=lanes)
+                except torch.cuda.OutOfMemoryError:
+                    if (chunk, lanes) == (self._chunk_size, 1):
+                        raise
+                    self._out_of_memory = True
+                    model.release_workspaces()
+                    rgb, _ = model.render_rays(rays, N_samples, white_bg, chunk=self._chunk_size)
+                if model.check_status_every_call:
+                    model.check_pending_status()
             return rgb
         return renderer_fn(self._forward, rays, self._chunk_size, **kw)

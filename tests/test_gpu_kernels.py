@@ -736,3 +736,39 @@ def test_inferer_without_status_checks():
     assert impl.renderer_fn(rays, N_samples=spec.n_samples).shape == (10000, 3)
     with pytest.raises(RuntimeError, match="appearance-sample list overflow"):
         impl.model.check_pending_status()
+
+
+def test_inferer_stays_within_memory(monkeypatch):
+    """render_batch_size is what a caller sized its memory for: larger device chunks are taken only where their workspaces
+    are a small share of the free memory, and given up when an allocation fails.  Same pixels."""
+    spec = scenes.tiny_spec().lit()
+    rays = tiny_rays(spec).cuda()
+    impl = _inferer(spec, 1000)
+    model = impl.model
+    one = model.workspace_bytes(1000, spec.n_samples)
+    assert impl._device_chunk(10000, spec.n_samples) == (65536, 1) and impl._device_chunk(200000, spec.n_samples) == (65536, 2)
+    want = impl.renderer_fn(rays, N_samples=spec.n_samples)
+    for share, lanes in ((20.0, 1), (3.0, 2), (0.5, 1)):  # free memory in workspaces of 1000 rays
+        model.release_workspaces()
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (int(8 * share * one), 1 << 40))
+        monkeypatch.setattr(torch.cuda, "memory_reserved", lambda *a: 0)
+        monkeypatch.setattr(torch.cuda, "memory_allocated", lambda *a: 0)
+        assert torch.equal(impl.renderer_fn(rays, N_samples=spec.n_samples), want)
+        held = sum(w.numel() for w in model._ws.values())
+        assert len(model._ws) == lanes and held <= max(share, 1.0) * one + 1024, (share, held / one)
+    monkeypatch.undo()
+    model.release_workspaces()
+    made = model.workspace
+
+    def no_room(n, *a, **k):
+        if n > 1000:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return made(n, *a, **k)
+
+    monkeypatch.setattr(model, "workspace", no_room)
+    for _ in range(2):
+        assert torch.equal(impl.renderer_fn(rays, N_samples=spec.n_samples), want)
+        assert len(model._ws) == 1 and model._ws[0].numel() <= one + 512
+    monkeypatch.setattr(model, "workspace", lambda *a, **k: no_room(1001))
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        impl.renderer_fn(rays, N_samples=spec.n_samples)
