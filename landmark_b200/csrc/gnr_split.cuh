@@ -16,10 +16,11 @@ namespace {
 template <int MODE>
 struct Split;
 
-// sin and cos to within 7.1e-8 (rms 1.7e-8, i.e. little more than the rounding of the result) for |x| <= 1000: the
-// multiple of pi/2 nearest to x is taken off in two steps (pi/2 as the sum of two floats; the fused multiply-adds round
-// once), what is left, |r| <= pi/4, goes into the Taylor polynomials up to r^9 and r^10 (next terms: 2e-9 and 1e-10), and
-// the quadrant picks and signs them.
+// sin and cos to within 7.1e-8 (rms 1.7e-8, i.e. little more than the rounding of the result) for |x| <= 1000.  Cody and
+// Waite's argument reduction (Software Manual for the Elementary Functions, 1980): the multiple of pi/2 nearest to x is
+// taken off in two steps (pi/2 as the sum of two floats; the fused multiply-adds round once).  What is left,
+// |r| <= pi/4, goes into the Taylor polynomials up to r^9 and r^10 (next terms: 2e-9 and 1e-10), and the quadrant picks
+// and signs them.
 __device__ __forceinline__ void sincos_short(float x, float& s, float& c) {
   const float m = fmaf(x, 0.636619772f, 12582912.0f);  // 1.5 x 2^23: the low bits of m are the quadrant
   const float k = m - 12582912.0f;
