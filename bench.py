@@ -190,7 +190,7 @@ def main():
     ap.add_argument("--chunk", type=int, default=262144,
                     help="rays per library call (lowered so that every stream of a rank has a chunk)")
     ap.add_argument("--mlp-mode", type=int, default=2,
-                    help="0 fp32 CUDA cores, 1 tcgen05 fp16 hi+lo activations, 2 tcgen05 fp16 (default)")
+                    help="0 fp32 (three bf16 terms per operand), 1 tcgen05 fp16 hi+lo activations, 2 tcgen05 fp16 (default)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--frame", choices=sorted(FRAMES), default="1080p",
                     help="frame size (the focal length scales with the width); 4k is the tile-parallel configuration's frame")
@@ -687,13 +687,13 @@ def main():
                                      "hbm": hbm_part("app_gather_kernel", n_app, per_launch["app_gather"])}
     if per_launch["mlp"] > 0 and n_app > 0:
         fused_app = per_launch["app_gather"] == 0 and a.mlp_mode == 2  # gather + basis + MLP in one kernel
-        flop = MLP_FLOP_PER_SAMPLE + (BASIS_FLOP_PER_SAMPLE if a.mlp_mode else 0)
+        flop = MLP_FLOP_PER_SAMPLE + (BASIS_FLOP_PER_SAMPLE if a.mlp_mode == 2 else 0)  # (modes 0 and 1 project before)
         ach = n_app * flop / (per_launch["mlp"] * 1e-3) / 1e12
         key = "app_mlp_fused_kernel" if fused_app else "mlp_kernel"
         roof["mlp_kernel"] = {"bound": "tensor", "achieved": ach, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                               "frac": ach / pk["bf16_tflops"], "ms_per_frame": per_launch["mlp"], "flop_per_sample": flop,
                               "hbm": hbm_part(key, n_app, per_launch["mlp"]),
-                              "note": "fp32 CUDA-core kernel" if a.mlp_mode == 0 else
+                              "note": "tcgen05 kernel, operands as sums of 16-bit terms (mlp_split_kernel)" if a.mlp_mode != 2 else
                                       ("tcgen05 kernel with the appearance gather inside (app_mlp_fused_kernel)" if fused_app
                                        else "tcgen05 kernel (basis + MLP)")}
         if fused_app:

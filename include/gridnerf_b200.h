@@ -49,8 +49,10 @@ typedef struct GnrConfig {
   int32_t fea_pe, view_pe;  /* positional-encoding octaves (mlp_render_fea.py:20-27)      */
   int32_t hidden;           /* featureC (128)                                             */
   int32_t has_bias;         /* bias_enable                                                */
-  int32_t mlp_mode;         /* 0 = fp32 CUDA-core MLP, 1 = tcgen05 split-precision MLP (fp32-grade),
-                               2 = tcgen05 MLP with single fp16 operands, fp32 accumulate (fast) */
+  int32_t mlp_mode;         /* 0 = fp32 (tcgen05 with every operand as an exact sum of three bf16 terms, fp32
+                               accumulate; on the CUDA cores for other layer sizes than app_dim 27, fea_pe 2,
+                               view_pe 2, featureC 128), 1 = tcgen05 with activations as fp16 hi + lo, weights as one
+                               fp16, 2 = tcgen05 with single fp16 operands, fp32 accumulate (fast)            */
   int32_t sampling_mode;    /* 0 = sample_ray (:244-281), 1 = sample_ray_within_hull (:283-319,
                                args.sampling_opt); mode 1 needs gnr_upload_hull_tables             */
   float ert_transmittance;  /* early ray termination of the fused density + weights pass: a ray stops
@@ -373,8 +375,8 @@ int gnr_appearance_list(GnrModel* owner, const GnrModel* sampler, const float* r
  * gnr_composite_rgb; the per-sample weight array and the valid-list index of the entries are not produced. */
 int gnr_weights_from_rows(GnrModel* m, int64_t n_rays, int n_samples, void* workspace, size_t workspace_bytes,
                           int64_t max_valid, int64_t max_app, const float* sigma_rows, const int32_t* rows, void* stream);
-/* compute_appfeature only (gather + basis projection; on the tensor cores with mlp_mode 1/2, in fp32
- * on the CUDA cores with mode 0) for the appearance list of the workspace: with a channel slice of
+/* compute_appfeature only (gather + basis projection; on the tensor cores in every mlp_mode where the layout
+ * allows it: mode 0 with three bf16 terms per operand, i.e. in fp32) for the appearance list of the workspace: with a channel slice of
  * the planes and the matching columns of basis_mat these are the partial sums a tensor-parallel
  * rank contributes (gridnerf_tensor_parallel.py:284-300).  ``features[n_features][app_dim]``
  * receives the first n_features rows of the list (the caller read the list length from the status
