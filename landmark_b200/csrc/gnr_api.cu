@@ -786,6 +786,7 @@ GnrSampleParams gnr_sample_params(const GnrModel* m, int S) {
   p.a_half[0] = 0.5f * (float)(m->aW - 1);
   p.a_half[1] = 0.5f * (float)(m->aH - 1);
   p.a_half[2] = 0.5f * (float)(m->aD - 1);
+  for (int a = 0; a < 3; ++a) p.a_end[a] = fminf(2.0f * p.a_half[a], 4194304.0f);
   p.cD = (m->aD + 1) / 2;
   p.cH = (m->aH + 1) / 2;
   p.cW = (m->aW + 1) / 2;

@@ -123,6 +123,7 @@ struct GnrSampleParams {
   const uint32_t* a_full;    // null, or 1 bit per 2x2x2 block: every cell of the block is set
   const uint32_t* a_any8;    // null, or 1 bit per cell: any of its eight corners is set
   float a_half[3];           // (W - 1) / 2, (H - 1) / 2, (D - 1) / 2
+  float a_end[3];            // W - 1, H - 1, D - 1, at most 2^22: below it the sampler takes floors the short way
   int cD, cH, cW;
   int S, words, kbits;
   int mode;                 // 0 dense sampler, 1 hull sampler

@@ -122,7 +122,8 @@ __device__ __forceinline__ bool occupancy_test(const GnrSampleParams& p, float p
   const float ix = mask_index(px, p.a_lo[0], p.a_inv[0], p.a_half[0]);
   const float iy = mask_index(py, p.a_lo[1], p.a_inv[1], p.a_half[1]);
   const float iz = mask_index(pz, p.a_lo[2], p.a_inv[2], p.a_half[2]);
-  if (p.a_thres == 0.0f && fminf(fminf(ix, iy), iz) > 0.0f && ix < (float)(p.aW - 1) && iy < (float)(p.aH - 1) && iz < (float)(p.aD - 1)) {
+  if (p.a_thres == 0.0f && fminf(fminf(ix, iy), iz) > 0.0f && ix < p.a_end[0] && iy < p.a_end[1] &&
+      iz < p.a_end[2]) {
     int x0, y0, z0;
     const float fx = floor_small(ix, x0), fy = floor_small(iy, y0), fz = floor_small(iz, z0);
     // strictly inside a cell all eight corner weights are positive (differences of floats that are not equal; their

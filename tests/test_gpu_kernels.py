@@ -772,3 +772,29 @@ def test_inferer_stays_within_memory(monkeypatch):
     monkeypatch.setattr(model, "workspace", lambda *a, **k: no_room(1001))
     with pytest.raises(torch.cuda.OutOfMemoryError):
         impl.renderer_fn(rays, N_samples=spec.n_samples)
+
+
+def test_sampler_words_in_a_mask_longer_than_its_floats():
+    """A mask of 2 x 2 x (2^23 + 2^21) cells, where the index of a far sample has no fraction left: words as the test of
+    every sample gives them."""
+    from landmark_b200.gridnerf import AlphaGridMask, B200GridNeRF
+
+    spec = scenes.tiny_spec(grid=16).lit()
+    ckpt = scenes.make_checkpoint(spec)
+    kw = dict(ckpt["kwargs"])
+    kw.update({"device": "cuda:0", "args": scenes.model_args(spec, "cuda:0"), "is_train": False})
+    model = B200GridNeRF(**kw)
+    width = (1 << 23) + (1 << 21)
+    g = torch.Generator().manual_seed(5)
+    volume = (torch.rand((2, 2, width), generator=g) < 0.1)
+    model.alphaMask = AlphaGridMask(torch.device("cuda:0"), ckpt["alphaMask.aabb"].cuda(), volume.float().cuda())
+    model.load({k: v for k, v in ckpt.items() if not k.startswith("alphaMask")})
+    n, samples = 2000, 64
+    o = torch.rand((n, 3), generator=g) * 2.0 - 1.0
+    d = torch.randn((n, 3), generator=g) * torch.tensor([1.0, 0.1, 0.1])
+    got = model.run_stages(torch.cat([o, d], 1).cuda(), samples, True, upto="sample")
+    field, _ = oracle_field(spec)
+    valid, _ = snp.valid_mask(torch.cat([o, d], 1).numpy(), field.aabb.numpy(), field.near, field.far, field.step_size.item(), samples,
+                              volume.float().numpy(), field.alpha_aabb.numpy(), 0.0)
+    assert 0.05 < valid.mean() < 0.95
+    assert np.array_equal(valid_bits_from_words(got["mask_words"], samples), valid)
