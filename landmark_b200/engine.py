@@ -31,6 +31,10 @@ from .parallel import TileSharding
 RENDER_1080P = (1080, 1920, 1483.6378)  # H, W, focal of the online renderer (nerf_inferer.py:385-404)
 
 
+def _plain(t: torch.Tensor, dtype: torch.dtype, size: int) -> bool:
+    return t.dtype == dtype and t.numel() == size and t.is_contiguous()
+
+
 class _StatusRing:
     """Pinned status blocks of a renderer's whole-frame calls, ``SLOTS`` in turn, each large enough for the frame that asks.
     A frame on another stream than the one that used its slot before waits (on the device) for that one's event; the host
@@ -40,31 +44,29 @@ class _StatusRing:
 
     def __init__(self):
         self._lock = threading.Lock()
-        self._slots = [None] * self.SLOTS  # (block [n, 8] int32, event behind its frame, that frame's stream)
-        self._outgrown = []                # smaller blocks: frames in flight may still write them
+        self._slots = [(None, None, None, None)] * self.SLOTS  # block [n, 8], its rows in use, event behind their frame, its stream
+        self._outgrown = []  # smaller blocks: frames in flight may still write them
         self._turn = 0
 
     def take(self, n_chunks: int, stream):
-        """(slot, its first ``n_chunks`` rows); ``stream`` does not run ahead of the frame that used the slot before."""
+        """(``n_chunks`` status rows, the event to record behind their frame); ``stream`` does not run ahead of the frame that
+        used the rows before."""
         with self._lock:
             slot = self._turn
             self._turn = (slot + 1) % self.SLOTS
-            block, event, other = self._slots[slot] or (None, None, None)
+            block, rows, event, other = self._slots[slot]
             if block is None or block.shape[0] < n_chunks:
                 if block is not None:
                     self._outgrown.append(block)
-                rows = max(64, 1 << (n_chunks - 1).bit_length())
-                block, event = torch.zeros((rows, 8), dtype=torch.int32).pin_memory(), None
-            self._slots[slot] = (block, event, other)
+                block = torch.zeros((max(64, 1 << (n_chunks - 1).bit_length()), 8), dtype=torch.int32).pin_memory()
+                rows = event = None
+            if rows is None or rows.shape[0] != n_chunks:
+                rows = block[:n_chunks]
             if event is not None and other != stream:
                 stream.wait_event(event)
-            return slot, block[:n_chunks]
-
-    def used(self, slot: int, status: torch.Tensor, event, stream):
-        with self._lock:
-            block = self._slots[slot][0]
-            if block.data_ptr() == status.data_ptr():
-                self._slots[slot] = (block, event, stream)
+            event = torch.cuda.Event()
+            self._slots[slot] = (block, rows, event, stream)
+            return rows, event
 
 
 class FrameRenderer:
@@ -90,20 +92,30 @@ class FrameRenderer:
         their places in ``rgba`` and their copy to ``host_image`` (pinned); ``rgb`` and ``image``: the colours in fp32 too, in
         the order of ``pixel_ids`` and of the image.  Returns the event behind it.  The frame's rays are its own, so that
         frames on other streams may be in flight."""
+        return self._frame(lambda *a: self.model.render_frame(*a[:-1]), pose, H, W, focal, pixel_ids, rgba, host_image, rgb, image)
+
+    def _frame(self, call, pose, H, W, focal, pixel_ids, rgba, host_image, rgb, image):
+        """``call``: the model's ``render_frame``, or ``_frame`` where the buffers are known to be what it asks for."""
         from .rays import device_tables
 
         stream = torch.cuda.current_stream(self.device)
         rays = torch.empty((H * W, 6), dtype=torch.float32, device=self.device)
         ring = self.__dict__.get("_status_ring") or self.__dict__.setdefault("_status_ring", _StatusRing())
         chunk = max(1, min(self.chunk, H * W))
-        slot, status = ring.take((H * W + chunk - 1) // chunk, stream)
-        self.model.render_frame(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg,
-                                chunk, self.streams, rays, rgba, host_image, status, rgb, image)
-        ev = torch.cuda.Event()
+        status, ev = ring.take(-(-H * W // chunk), stream)
+        call(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg, chunk, self.streams,
+             rays, rgba, host_image, status, rgb, image, stream)
         ev.record(stream)
-        ring.used(slot, status, ev, stream)
         self.model._pending_status, self.model._pending_event = status, ev
         return ev
+
+    def has_own_stages(self) -> bool:
+        """No subclass and no object attribute stands in for a stage of a frame."""
+        cls = type(self)
+        return (cls is FrameRenderer or all(getattr(cls, s) is getattr(FrameRenderer, s) for s in self._STAGES)
+                ) and self.__dict__.keys().isdisjoint(self._STAGES)
+
+    _STAGES = ("render_pixels", "to_rgba8", "render_frame")
 
     def finish(self):
         self.model.check_pending_status()
@@ -285,16 +297,16 @@ class NerfDDPRunner:
     def _whole_frame(self, host_image: torch.Tensor) -> bool:
         """One library call does the frame: a single rank, FrameRenderer's and the model's own stages, not replaced in a class
         or on an object, an image the call can write as plain bytes, and no capture.  Everything else goes stage by stage."""
-        from .gridnerf import B200GridNeRF
-
         r = self.renderer
-        if self.world != 1 or not isinstance(r, FrameRenderer) or not isinstance(r.model, B200GridNeRF):
+        if self.world != 1 or not isinstance(r, FrameRenderer) or not r.has_own_stages():
             return False
-        for obj, base, stages in ((r, FrameRenderer, ("render_pixels", "to_rgba8")), (r.model, B200GridNeRF, ("render_rays",))):
-            if any(s in vars(obj) or getattr(type(obj), s) is not getattr(base, s) for s in stages):
-                return False
-        return (host_image.dtype == torch.uint8 and tuple(host_image.shape) == (self.H, self.W, 4) and host_image.is_contiguous()
-                and host_image.is_pinned() and not torch.cuda.is_current_stream_capturing())
+        own = getattr(r.model, "has_own_chunk_loop", None)
+        if own is None or not own() or torch.cuda.is_current_stream_capturing():
+            return False
+        n = self.H * self.W
+        return (host_image.shape == (self.H, self.W, 4) and _plain(host_image, torch.uint8, 4 * n) and host_image.is_pinned()
+                and _plain(self.rgba, torch.uint8, 4 * n) and self.rgba.is_cuda and _plain(self.rgb, torch.float32, 3 * n)
+                and self.rgb.is_cuda and _plain(self.image, torch.float32, 3 * n) and self.image.is_cuda)
 
     def enqueue(self, single_pose, host_image: torch.Tensor):
         """Everything ``run_batch`` does for one frame except waiting for it: broadcast, render, gather,
@@ -306,8 +318,9 @@ class NerfDDPRunner:
         pose = np.asarray(single_pose.cpu() if isinstance(single_pose, torch.Tensor) else single_pose, dtype=np.float32)
         focal = self._focal_of(pose)
         if self._whole_frame(host_image):
-            return self.renderer.render_frame(pose[:3, :4], self.H, self.W, focal, self.shard.pixel_ids, self.rgba, host_image,
-                                              self.rgb, self.image)
+            r = self.renderer
+            return r._frame(r.model._frame, pose[:3, :4], self.H, self.W, focal, self.shard.pixel_ids, self.rgba, host_image,
+                            self.rgb, self.image)
         pose, focal, _ = self._broadcast(pose[:3, :4], focal, False)
         self.renderer.render_pixels(pose, self.H, self.W, focal, self.shard.pixel_ids, self.rgb[: self.shard.n_local])
         self.shard.assemble(self.rgb, self.image)

@@ -746,10 +746,8 @@ class B200GridNeRF(torch.nn.Module):
         the device, ``pixel_ids`` every pixel once, ``rays [H * W, 6]`` and ``rgba`` device buffers, ``host_image`` pinned
         ``uint8 [H, W, 4]``, ``status`` pinned ``int32 [n_chunks, 8]``, complete when the stream's work is; ``rgb`` and
         ``image``: the colours in fp32 too, ``[H * W, 3]`` in the order of ``pixel_ids`` and of the image."""
-        s = self._samples(N_samples)
         n = H * W
-        chunk = max(1, min(chunk, n))
-        n_chunks = (n + chunk - 1) // chunk
+        n_chunks = -(-n // max(1, min(chunk, n)))
         pixel_ids = pixel_ids.to(device=self.device, dtype=torch.int32).contiguous()
         pose = np.asarray(pose, dtype=np.float32)
         if pose.shape != (3, 4) or pixel_ids.numel() != n:
@@ -764,14 +762,28 @@ class B200GridNeRF(torch.nn.Module):
             if t.dtype != dtype or t.numel() < size or not t.is_contiguous() or not (t.is_pinned() if host else t.is_cuda):
                 raise ValueError(f"render_frame: {what} must be contiguous {dtype} of at least {size} values "
                                  f"{'in pinned memory' if host else 'on the device'}, got {t.dtype} {tuple(t.shape)} on {t.device}")
-        lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, n_chunks, overlap)
+        self._frame(pose, tables, H, W, pixel_ids, N_samples, white_bg, chunk, overlap, rays, rgba, host_image, status, rgb, image,
+                    torch.cuda.current_stream(self.device))
+
+    def has_own_chunk_loop(self) -> bool:
+        """No subclass and no object attribute stands in for the chunk loop or the frame call."""
+        cls = type(self)
+        return (cls is B200GridNeRF or (cls.render_rays is B200GridNeRF.render_rays and cls.render_frame is B200GridNeRF.render_frame)
+                ) and self.__dict__.keys().isdisjoint(("render_rays", "render_frame"))
+
+    def _frame(self, pose, tables, H, W, pixel_ids, N_samples, white_bg, chunk, overlap, rays, rgba, host_image, status, rgb, image,
+               stream):
+        """``render_frame`` with buffers that are known to be what it asks for."""
+        s = self._samples(N_samples)
+        n = H * W
+        chunk = max(1, min(chunk, n))
+        lanes, ws, ws_bytes, max_valid, max_app = self._lanes(chunk, s, -(-n // chunk), overlap)
         pose_c = (C.c_float * 12).from_buffer_copy(pose.tobytes())
         check(lib.gnr_render_frame_rgb(self._handle, pose_c, tables[0].data_ptr(), tables[1].data_ptr(), H, W,
                                        pixel_ids.data_ptr(), s, int(bool(white_bg)), chunk, lanes, ws, ws_bytes, max_valid, max_app,
                                        rays.data_ptr(), None if rgb is None else rgb.data_ptr(),
                                        None if image is None else image.data_ptr(), rgba.data_ptr(), host_image.data_ptr(),
-                                       status.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream),
-              "gnr_render_frame_rgb")
+                                       status.data_ptr(), stream.cuda_stream), "gnr_render_frame_rgb")
 
     def check_pending_status(self):
         """Synchronise and raise if any chunk of the last ``render_rays`` overflowed a list."""
