@@ -503,13 +503,14 @@ class B200GridNeRF(torch.nn.Module):
 
     def workspace_bytes(self, n_rays: int, n_samples: int, stages: bool = False) -> int:
         """Bytes of scratch a chunk of that shape needs (see ``workspace``)."""
-        max_valid, max_app = self.capacities(n_rays, n_samples)
-        key = (n_rays, n_samples, max_valid, max_app, stages)
+        return self._workspace_need(n_rays, n_samples, *self.capacities(n_rays, n_samples), stages)
+
+    def _workspace_need(self, *key):
         need = self._ws_bytes.get(key)
         if need is None:
             nbytes = C.c_size_t(0)
-            query = lib.gnr_workspace_bytes if stages else lib.gnr_render_workspace_bytes
-            check(query(self._handle, n_rays, n_samples, max_valid, max_app, C.byref(nbytes)), "gnr_workspace_bytes")
+            query = lib.gnr_workspace_bytes if key[-1] else lib.gnr_render_workspace_bytes
+            check(query(self._handle, *key[:-1], C.byref(nbytes)), "gnr_workspace_bytes")
             if len(self._ws_bytes) > 256:
                 self._ws_bytes.clear()
             need = self._ws_bytes[key] = int(nbytes.value)
@@ -528,7 +529,7 @@ class B200GridNeRF(torch.nn.Module):
         (``GraphedFrameRenderer`` does), which keeps that memory out of the allocator for as long
         as the graph lives."""
         max_valid, max_app = self.capacities(n_rays, n_samples)
-        need = self.workspace_bytes(n_rays, n_samples, stages)
+        need = self._workspace_need(n_rays, n_samples, max_valid, max_app, stages)
         buf = self._ws.get(slot)
         if buf is None or buf.numel() < need + 256:
             if buf is not None:

@@ -53,7 +53,8 @@ class B200NerfDDPInfererImpl:
 
     RENDER_CHUNK = 65536      # rays of a device chunk, unless render_batch_size is larger (0: always render_batch_size)
     RENDER_SAMPLES = 1 << 25  # and at most that many samples of them: the ids and lists of a chunk grow with both
-    RENDER_MEMORY = 0.125     # and as long as the workspaces take no more than that share of the free device memory
+    RENDER_MEMORY = 0.125     # and as long as the workspaces take no more than that share of the free device memory ...
+    RENDER_UNASKED = 1 << 30  # ... which is asked for (0.3 ms) when they need more than this
 
     def __init__(self, context, profile_stages: bool = False, mlp_mode: Optional[int] = None, preset: str = "exact",
                  **model_options) -> None:
@@ -139,12 +140,12 @@ class B200NerfDDPInfererImpl:
         while not self._out_of_memory:
             need = m.workspace_bytes(min(chunk, n_rays), n_samples) + 256
             lanes = 2 if n_rays > chunk else 1
-            missing = sum(need for slot in range(lanes) if slot not in m._ws or m._ws[slot].numel() < need)
-            if not missing:
-                return chunk, lanes
-            free = (torch.cuda.mem_get_info(m.device)[0] + torch.cuda.memory_reserved(m.device)
-                    - torch.cuda.memory_allocated(m.device))
-            if missing <= self.RENDER_MEMORY * free:
+            missing = 0
+            for slot in range(lanes):
+                held = m._ws.get(slot)
+                if held is None or held.numel() < need:
+                    missing += need
+            if missing <= self.RENDER_UNASKED or missing <= self.RENDER_MEMORY * torch.cuda.mem_get_info(m.device)[0]:
                 return chunk, lanes
             if chunk <= least:
                 break
