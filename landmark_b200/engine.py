@@ -106,7 +106,7 @@ class FrameRenderer:
         call(pose, device_tables(H, W, focal, self.device), H, W, pixel_ids, self.n_samples, self.white_bg, chunk, self.streams,
              rays, rgba, host_image, status, rgb, image, stream)
         ev.record(stream)
-        self.model._pending_status, self.model._pending_event = status, ev
+        self.model._note(_pending_status=status, _pending_event=ev)
         return ev
 
     def has_own_stages(self) -> bool:

@@ -213,6 +213,8 @@ class B200GridNeRF(torch.nn.Module):
         self._ws: Dict[int, torch.Tensor] = {}        # chunk slot -> scratch buffer (grows, never shrinks)
         self._ws_bytes: Dict[tuple, int] = {}          # chunk shape -> bytes the library asks for
         self._last_workspaces: list = []               # buffers the last render_rays call used
+        self._pending_status: Optional[torch.Tensor] = None  # status blocks of the last chunk loop or frame ...
+        self._pending_event: Optional["torch.cuda.Event"] = None  # ... and, if they lie in pinned memory, the event behind them
         # capacities of the two compacted sample lists, per ray of a chunk
         self.valid_capacity_per_ray: Optional[int] = None  # None = n_samples (can never overflow)
         self.app_capacity_per_ray = 192
@@ -723,21 +725,25 @@ class B200GridNeRF(torch.nn.Module):
                                    max_app, rgb_out.data_ptr(), depth_out.data_ptr(), status.data_ptr(),
                                    after.cuda_event if after is not None and lanes > 1 else None,
                                    torch.cuda.current_stream(self.device).cuda_stream), "gnr_render_batch")
-        self._pending_status, self._pending_event = status, None
+        self._note(_pending_status=status, _pending_event=None)
         return rgb_out, depth_out
+
+    def _note(self, **state):
+        """Plain attributes set once per call, past torch.nn.Module.__setattr__ (1 to 2 us each)."""
+        self.__dict__.update(state)
 
     def _lanes(self, chunk: int, n_samples: int, n_chunks: int, overlap):
         """Workspaces of a chunk loop: (lanes, their addresses, bytes of each, list capacities)."""
         want = 2 if overlap is True else int(overlap or 1)
         lanes = max(1, min(want, n_chunks, _lib.MAX_LANES))  # (more chunks in flight than that share the lanes)
         ws = (C.c_void_p * lanes)()
-        self._last_workspaces = []
-        ws_bytes = None
+        used, ws_bytes = [], None
         for slot in range(lanes):
             keep, ptr, nbytes, max_valid, max_app = self.workspace(chunk, n_samples, slot)
             ws[slot] = ptr.value
             ws_bytes = nbytes if ws_bytes is None else min(ws_bytes, nbytes)
-            self._last_workspaces.append(keep)
+            used.append(keep)
+        self._note(_last_workspaces=used)
         return lanes, ws, ws_bytes, max_valid, max_app
 
     def render_frame(self, pose: np.ndarray, tables, H: int, W: int, pixel_ids: torch.Tensor, N_samples: int, white_bg: bool,
@@ -788,18 +794,16 @@ class B200GridNeRF(torch.nn.Module):
 
     def check_pending_status(self):
         """Synchronise and raise if any chunk of the last ``render_rays`` overflowed a list."""
-        st = getattr(self, "_pending_status", None)
+        st = self._pending_status
         if st is None:
             return None
-        if getattr(self, "_pending_event", None) is not None:  # the status blocks lie in pinned memory
+        if self._pending_event is not None:  # the status blocks lie in pinned memory
             self._pending_event.synchronize()
-            self._pending_event = None
         h = st.cpu().numpy().astype(np.int64)
         agg = np.zeros(_lib.ST_WORDS, dtype=np.int64)
         agg[[0, 1, 4]] = h[:, [0, 1, 4]].max(0)
         agg[[2, 3, 5]] = h[:, [2, 3, 5]].sum(0)
-        self.last_status = agg
-        self._pending_status = None
+        self._note(last_status=agg, _pending_status=None, _pending_event=None)
         self.raise_on_status(agg)
         return agg
 
