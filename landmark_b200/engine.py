@@ -36,15 +36,16 @@ def _plain(t: torch.Tensor, dtype: torch.dtype, size: int) -> bool:
 
 
 class _StatusRing:
-    """Pinned status blocks of a renderer's whole-frame calls, ``SLOTS`` in turn, each large enough for the frame that asks.
-    A frame on another stream than the one that used its slot before waits (on the device) for that one's event; the host
-    waits for nothing."""
+    """Pinned status blocks of a renderer's whole-frame calls: ``SLOTS`` of them in turn, each large enough for any frame so
+    far.  A frame on another stream than the one that used its slot before waits (on the device) for that one's event; the
+    host waits for nothing."""
 
     SLOTS = 8
 
     def __init__(self):
         self._lock = threading.Lock()
-        self._slots = [(None, None, None, None)] * self.SLOTS  # block [n, 8], its rows in use, event behind their frame, its stream
+        self._blocks = None  # [SLOTS, n, 8]
+        self._slots = [(None, None, None)] * self.SLOTS  # rows in use, event behind their frame, its stream
         self._outgrown = []  # smaller blocks: frames in flight may still write them
         self._turn = 0
 
@@ -52,20 +53,20 @@ class _StatusRing:
         """(``n_chunks`` status rows, the event to record behind their frame); ``stream`` does not run ahead of the frame that
         used the rows before."""
         with self._lock:
+            if self._blocks is None or self._blocks.shape[1] < n_chunks:
+                self._outgrown.append(self._blocks)
+                rows = max(64, 1 << (n_chunks - 1).bit_length())
+                self._blocks = torch.zeros((self.SLOTS, rows, 8), dtype=torch.int32).pin_memory()
+                self._slots = [(None, None, None)] * self.SLOTS
             slot = self._turn
             self._turn = (slot + 1) % self.SLOTS
-            block, rows, event, other = self._slots[slot]
-            if block is None or block.shape[0] < n_chunks:
-                if block is not None:
-                    self._outgrown.append(block)
-                block = torch.zeros((max(64, 1 << (n_chunks - 1).bit_length()), 8), dtype=torch.int32).pin_memory()
-                rows = event = None
+            rows, event, other = self._slots[slot]
             if rows is None or rows.shape[0] != n_chunks:
-                rows = block[:n_chunks]
+                rows = self._blocks[slot, :n_chunks]
             if event is not None and other != stream:
                 stream.wait_event(event)
             event = torch.cuda.Event()
-            self._slots[slot] = (block, rows, event, stream)
+            self._slots[slot] = (rows, event, stream)
             return rows, event
 
 
