@@ -54,7 +54,7 @@ class B200NerfDDPInfererImpl:
     RENDER_CHUNK = 65536      # rays of a device chunk, unless render_batch_size is larger (0: always render_batch_size)
     RENDER_SAMPLES = 1 << 25  # and at most that many samples of them: the ids and lists of a chunk grow with both
     RENDER_MEMORY = 0.125     # and as long as the workspaces take no more than that share of the free device memory ...
-    RENDER_UNASKED = 1 << 30  # ... which is asked for (0.3 ms) when they need more than this
+    RENDER_UNASKED = 1 << 28  # ... which is asked for (70 us) when they need more than this
 
     def __init__(self, context, profile_stages: bool = False, mlp_mode: Optional[int] = None, preset: str = "exact",
                  **model_options) -> None:
